@@ -1,16 +1,20 @@
-"""ctypes binding of libb200fp4.so, the C-ABI in ``include/b200fp4.h``.
+"""Bindings of libb200fp4.so, the C-ABI in ``include/b200fp4.h``: ctypes for every function, and the compiled host
+path of the hot operators (``native``, csrc/torch_binding.cpp).
 
-There is deliberately no fallback: if the library has not been built the import
+There is deliberately no fallback: if either has not been built the import
 fails, and every failing C call is turned into a Python exception carrying the
 library's own message.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "lib", "libb200fp4.so")
+BINDING_PATH = os.path.join(_PKG, "lib", "_b200fp4_torch.so")
 
 OK, INVALID_ARGUMENT, UNSUPPORTED, CUDA_ERROR, DEVICE_TIMEOUT, NOT_INITIALISED = range(6)
 
@@ -66,6 +70,21 @@ lib = _load()
 
 class B200Fp4Error(RuntimeError):
     pass
+
+
+def _load_native():
+    import torch  # noqa: F401  (its libraries must be in the process before the extension's are resolved)
+
+    if not os.path.exists(BINDING_PATH):
+        raise ImportError(f"{BINDING_PATH} is missing: build it with `python {os.path.join(_PKG, 'build.py')}`")
+    loader = importlib.machinery.ExtensionFileLoader("_b200fp4_torch", BINDING_PATH)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200fp4_torch", loader))
+    loader.exec_module(mod)
+    mod.set_error_class(B200Fp4Error)
+    return mod
+
+
+native = _load_native()
 
 
 def check(rc: int) -> None:

@@ -57,18 +57,6 @@ def _dtype_token(d) -> _DType:
     return _BY_NAME[name]
 
 
-def _as_lmk(t: torch.Tensor, what: str) -> torch.Tensor:
-    """Accept [R, C], [L, R, C] or the demo's (R, C, L) view with L slowest in memory;
-    return a contiguous-in-memory [L, R, C] view without copying."""
-    if t.dim() == 2:
-        t = t.unsqueeze(0)
-    elif t.dim() == 3 and not t.is_contiguous() and t.permute(2, 0, 1).is_contiguous():
-        t = t.permute(2, 0, 1)
-    if t.dim() != 3 or not t.is_contiguous():
-        raise ValueError(f"{what} must be contiguous [rows, cols], [L, rows, cols] or an (rows, cols, L) view of it")
-    return t
-
-
 def gemm_workspace_bytes(m: int, n: int, k: int) -> int:
     """Bytes of f32 scratch with which an [m, k] x [n, k] problem runs split-K (0: it does not split)."""
     return int(_lib.lib.b200fp4_nvfp4_gemm_workspace_bytes(m, n, k))
@@ -86,49 +74,7 @@ def nvfp4_gemm(a: torch.Tensor, b: torch.Tensor, sfa: torch.Tensor, sfb: torch.T
     ``workspace=`` (uint8, ``gemm_workspace_bytes(m, n, k)`` bytes) opts a problem with few output tiles and a long
     reduction into split-K.  It is off by default: at M = 128, N = K = 8192 the split kernel takes the same 15 us as
     the unsplit 64-wide tiles and the reduction adds 4."""
-    if not (a.is_cuda and b.is_cuda and sfa.is_cuda and sfb.is_cuda):
-        raise ValueError("operands must be CUDA tensors (there is no CPU implementation)")
-    a3, b3 = _as_lmk(a.view(torch.uint8), "a"), _as_lmk(b.view(torch.uint8), "b")
-    l, m, kh = a3.shape
-    lb, n, khb = b3.shape
-    if lb != l or khb != kh:
-        raise ValueError(f"a {tuple(a3.shape)} and b {tuple(b3.shape)} disagree on batch or K")
-    k = kh * 2
-    if k % 32 != 0 or n % 8 != 0:
-        raise ValueError("Invalid tensor alignment")
-    if sf_vec_size not in (16, 32):
-        raise NotImplementedError("sf_vec_size must be 16 (NVFP4) or 32 (MXFP4)")
-    need_a = l * swizzled_sf_numel(m, ceil_div(k, sf_vec_size))
-    need_b = l * swizzled_sf_numel(n, ceil_div(k, sf_vec_size))
-    if sfa.element_size() != 1 or sfb.element_size() != 1 or sfa.numel() < need_a or sfb.numel() < need_b:
-        raise ValueError(f"scale factors must be 1-byte tensors in the 128x4 tiled layout "
-                         f"({need_a} and {need_b} bytes)")
-    if out is None:
-        shape = (m, n) if a.dim() == 2 else (l, m, n)
-        out = torch.empty(shape, dtype=out_dtype, device=a.device)
-    out3 = _as_lmk(out, "c")
-    if tuple(out3.shape) != (l, m, n) or out.dtype not in _C_CODES:
-        raise ValueError(f"c must be [{m}, {n}] (x{l}) in float16, bfloat16 or float32")
-    if alpha is not None and (alpha.dtype != torch.float32 or not alpha.is_cuda):
-        raise ValueError("alpha must be a float32 CUDA tensor")
-    if sf_vec_size == 32:
-        with _lib.on_device(a.device):
-            _lib.check(_lib.lib.b200fp4_mxfp4_gemm(
-                a3.data_ptr(), b3.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), out3.data_ptr(), _lib.ptr(alpha),
-                m, n, k, l, _C_CODES[out.dtype], tile_n, _lib.current_stream_ptr(a.device)))
-        return out
-    ws_ptr, ws_bytes = None, 0
-    if workspace is not None and tile_n == 0:
-        ws_bytes = gemm_workspace_bytes(m, n, k)
-        if ws_bytes:
-            if not workspace.is_cuda or workspace.device != a.device or workspace.numel() * workspace.element_size() < ws_bytes:
-                raise ValueError(f"workspace must be a CUDA tensor on {a.device} of at least {ws_bytes} bytes")
-            ws_ptr = workspace.data_ptr()
-    with _lib.on_device(a.device):
-        _lib.check(_lib.lib.b200fp4_nvfp4_gemm_ws(
-            a3.data_ptr(), b3.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), out3.data_ptr(), _lib.ptr(alpha),
-            m, n, k, l, _C_CODES[out.dtype], tile_n, ws_ptr, ws_bytes, _lib.current_stream_ptr(a.device)))
-    return out
+    return _lib.native.nvfp4_gemm(a, b, sfa, sfb, alpha, out, out_dtype, tile_n, workspace, sf_vec_size)
 
 
 def mxfp8_gemm(a: torch.Tensor, b: torch.Tensor, sfa: torch.Tensor, sfb: torch.Tensor,
@@ -137,34 +83,7 @@ def mxfp8_gemm(a: torch.Tensor, b: torch.Tensor, sfa: torch.Tensor, sfb: torch.T
     """MXFP8 flavour: A ``[M, K]`` and B ``[N, K]`` are ``torch.float8_e4m3fn`` or ``torch.float8_e5m2`` (each
     operand its own format), scale factors ue8m0 bytes, one per 32 K-elements, in the 128x4 tiled layout
     (``swizzled_sf_numel(rows, ceil(K / 32))`` bytes).  Same kernel family as ``nvfp4_gemm``; single-CTA tiles."""
-    fmts = {torch.float8_e4m3fn: 0, torch.float8_e5m2: 1}
-    if a.dtype not in fmts or b.dtype not in fmts:
-        raise ValueError("a and b must be float8_e4m3fn or float8_e5m2 tensors")
-    if not (a.is_cuda and b.is_cuda and sfa.is_cuda and sfb.is_cuda):
-        raise ValueError("operands must be CUDA tensors (there is no CPU implementation)")
-    a3, b3 = _as_lmk(a.view(torch.uint8), "a"), _as_lmk(b.view(torch.uint8), "b")
-    l, m, k = a3.shape
-    lb, n, kb_ = b3.shape
-    if lb != l or kb_ != k:
-        raise ValueError(f"a {tuple(a3.shape)} and b {tuple(b3.shape)} disagree on batch or K")
-    if k % 16 != 0 or n % 8 != 0:
-        raise ValueError("Invalid tensor alignment")
-    need_a = l * swizzled_sf_numel(m, ceil_div(k, 32))
-    need_b = l * swizzled_sf_numel(n, ceil_div(k, 32))
-    if sfa.element_size() != 1 or sfb.element_size() != 1 or sfa.numel() < need_a or sfb.numel() < need_b:
-        raise ValueError(f"scale factors must be 1-byte tensors in the 128x4 tiled layout ({need_a} and {need_b} bytes)")
-    if out is None:
-        out = torch.empty((m, n) if a.dim() == 2 else (l, m, n), dtype=out_dtype, device=a.device)
-    out3 = _as_lmk(out, "c")
-    if tuple(out3.shape) != (l, m, n) or out.dtype not in _C_CODES:
-        raise ValueError(f"c must be [{m}, {n}] (x{l}) in float16, bfloat16 or float32")
-    if alpha is not None and (alpha.dtype != torch.float32 or not alpha.is_cuda):
-        raise ValueError("alpha must be a float32 CUDA tensor")
-    with _lib.on_device(a.device):
-        _lib.check(_lib.lib.b200fp4_mxfp8_gemm(
-            a3.data_ptr(), b3.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), out3.data_ptr(), _lib.ptr(alpha),
-            m, n, k, l, _C_CODES[out.dtype], tile_n, fmts[a.dtype], fmts[b.dtype], _lib.current_stream_ptr(a.device)))
-    return out
+    return _lib.native.mxfp8_gemm(a, b, sfa, sfb, alpha, out, out_dtype, tile_n)
 
 
 class Sm120BlockScaledGemmKernel:
@@ -362,13 +281,4 @@ def mm_fp4(a: torch.Tensor, b: torch.Tensor, a_descale: torch.Tensor, b_descale:
     ``b_descale`` likewise (tiled over [n, k/16]).  ``alpha`` = 1 / (global_scale_a * global_scale_b)."""
     if block_size != 16 or use_8x4_sf_layout:
         raise NotImplementedError("only NVFP4 (block_size=16) with the 128x4 scale layout is implemented")
-    if out_dtype not in (torch.bfloat16, torch.float16, torch.float32):
-        raise NotImplementedError(f"out_dtype {out_dtype}")
-    bu = b.view(torch.uint8)
-    if bu.dim() == 2 and not bu.is_contiguous() and bu.t().is_contiguous():
-        bu = bu.t()
-    sfb = b_descale
-    if sfb.dim() == 2 and not sfb.is_contiguous() and sfb.t().is_contiguous():
-        sfb = sfb.t()
-    return nvfp4_gemm(a.view(torch.uint8), bu, a_descale.contiguous().view(torch.uint8), sfb.contiguous().view(torch.uint8),
-                      alpha=alpha, out=out, out_dtype=out_dtype)
+    return _lib.native.mm_fp4(a, b, a_descale, b_descale, alpha, out, out_dtype)

@@ -6,8 +6,8 @@ tools/perf/bench_flashinfer_b12x.py:77-81).  One call = a fixed sequence of CUDA
 kernels on the current stream inside ``b200fp4_moe_fused``: (route +) count,
 quantise + place, grouped FC1 with SwiGLU and re-quantisation, grouped FC2,
 weighted combine.  Scratch memory comes from ``workspace=`` or from a
-``B12xMoEWrapper`` (allocated once); without either, a per-device buffer that
-only grows is used.
+``B12xMoEWrapper`` (allocated once); without either, it is taken from the
+current stream's allocator pool for the duration of the call.
 """
 from __future__ import annotations
 
@@ -18,20 +18,9 @@ import torch
 from . import _lib
 from .layout import pack_e2m1, six_mode_to_storage, swizzle_sf
 
-_WORKSPACES = {}
-
 
 def moe_workspace_bytes(tokens: int, hidden: int, intermediate: int, local_experts: int, top_k: int) -> int:
     return int(_lib.lib.b200fp4_moe_workspace_bytes(tokens, hidden, intermediate, local_experts, top_k))
-
-
-def _workspace(device, nbytes: int) -> torch.Tensor:
-    key = (device.type, device.index)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = ws
-    return ws
 
 
 def _on_device(device, **tensors) -> None:
@@ -59,16 +48,7 @@ def _sf_storage(sf: torch.Tensor, experts: int, rows: int, k: int, name: str) ->
 
 def topk_route(router_logits: torch.Tensor, top_k: int, renormalize: bool = True):
     """softmax -> top-k -> (renormalised) weights on the GPU; returns (ids int32, weights float32)."""
-    if not router_logits.is_cuda or router_logits.dtype != torch.float32 or router_logits.dim() != 2:
-        raise ValueError("router_logits must be a float32 CUDA tensor [tokens, experts]")
-    logits = router_logits.contiguous()
-    t, e = logits.shape
-    ids = torch.empty(t, top_k, dtype=torch.int32, device=logits.device)
-    w = torch.empty(t, top_k, dtype=torch.float32, device=logits.device)
-    with _lib.on_device(logits.device):
-        _lib.check(_lib.lib.b200fp4_topk_route(logits.data_ptr(), ids.data_ptr(), w.data_ptr(), t, e, top_k,
-                                               1 if renormalize else 0, _lib.current_stream_ptr(logits.device)))
-    return ids, w
+    return _lib.native.topk_route(router_logits, top_k, renormalize)
 
 
 def b12x_fused_moe(
@@ -117,79 +97,10 @@ def b12x_fused_moe(
         raise NotImplementedError("only NVFP4 weights with NVFP4 activations are implemented")
     if activation not in ("silu", "swiglu"):
         raise NotImplementedError(f"activation {activation!r}: only silu (SwiGLU) is implemented")
-    if output_dtype not in (torch.bfloat16, torch.float32) or x.dtype != torch.bfloat16:
-        raise NotImplementedError("tokens must be bfloat16 and the output bfloat16 (or float32 partial sums)")
-    if not x.is_cuda:
-        raise ValueError("x must be a CUDA tensor (there is no CPU implementation)")
-    if x.dim() != 2 or not x.is_contiguous():
-        raise ValueError("x must be contiguous [tokens, hidden]")
-    tokens, hidden = x.shape
-    dev = x.device
-    local = num_experts if num_local_experts is None else num_local_experts
-    ids, scales = token_selected_experts, token_final_scales
-    _on_device(dev, w1_weight=w1_weight, w1_weight_sf=w1_weight_sf, w2_weight=w2_weight, w2_weight_sf=w2_weight_sf,
-               token_selected_experts=ids, token_final_scales=scales, w1_alpha=w1_alpha, w2_alpha=w2_alpha,
-               fc2_input_scale=fc2_input_scale, output=output, workspace=workspace, router_logits=router_logits)
-    w1 = w1_weight.view(torch.uint8)
-    w2 = w2_weight.view(torch.uint8)
-    if w1.dim() != 3 or w1.shape[0] != local or w1.shape[2] * 2 != hidden or not w1.is_contiguous():
-        raise ValueError(f"w1_weight must be contiguous [{local}, 2*I, {hidden // 2}]")
-    inter = w1.shape[1] // 2
-    if tuple(w2.shape) != (local, hidden, inter // 2) or not w2.is_contiguous():
-        raise ValueError(f"w2_weight must be contiguous [{local}, {hidden}, {inter // 2}]")
-    if router_logits is not None:
-        if (router_logits.dtype != torch.float32 or tuple(router_logits.shape) != (tokens, num_experts)
-                or not router_logits.is_contiguous()):
-            raise ValueError(f"router_logits must be contiguous float32 [{tokens}, {num_experts}]")
-        if ids is None:
-            ids = torch.empty(tokens, top_k, dtype=torch.int32, device=dev)
-        if scales is None:
-            scales = torch.empty(tokens, top_k, dtype=torch.float32, device=dev)
-    elif ids is None or scales is None:
-        raise ValueError("token_selected_experts and token_final_scales are required without router_logits")
-    if ids.dtype != torch.int32 or tuple(ids.shape) != (tokens, top_k) or not ids.is_contiguous():
-        raise ValueError("token_selected_experts must be contiguous int32 [tokens, top_k]")
-    if scales.dtype != torch.float32 or tuple(scales.shape) != (tokens, top_k) or not scales.is_contiguous():
-        raise ValueError("token_final_scales must be contiguous float32 [tokens, top_k]")
-    s1 = _sf_storage(w1_weight_sf, local, 2 * inter, hidden, "w1_weight_sf")
-    s2 = _sf_storage(w2_weight_sf, local, hidden, inter, "w2_weight_sf")
-    for name, a in (("w1_alpha", w1_alpha), ("w2_alpha", w2_alpha)):
-        if a is not None and (a.dtype != torch.float32 or a.numel() != local or not a.is_contiguous()):
-            raise ValueError(f"{name} must be float32 [{local}]")
-    if fc2_input_scale is not None and (fc2_input_scale.dtype != torch.float32 or fc2_input_scale.numel() != 1):
-        raise ValueError("fc2_input_scale must be one float32")
-    if output is None:
-        output = torch.empty(tokens, hidden, dtype=output_dtype, device=dev)
-        if accumulate:
-            output.zero_()
-    elif (tuple(output.shape) != (tokens, hidden) or output.dtype not in (torch.bfloat16, torch.float32)
-          or not output.is_contiguous()):
-        raise ValueError("output must be contiguous bfloat16 or float32 [tokens, hidden]")
-    if slot_rows_dtype is None:
-        slot_rows_dtype = torch.float32 if output.dtype == torch.float32 else torch.bfloat16
-    if slot_rows_dtype not in (torch.bfloat16, torch.float32):
-        raise ValueError("slot_rows_dtype must be torch.bfloat16 or torch.float32")
-    if output.dtype == torch.float32 and slot_rows_dtype != torch.float32:
-        raise NotImplementedError("a float32 output keeps float32 per-slot rows")
-    if tokens == 0:
-        return output
-    need = moe_workspace_bytes(tokens, hidden, inter, local, top_k)
-    ws = _workspace(dev, need) if workspace is None else workspace
-    if ws.numel() * ws.element_size() < need:
-        raise ValueError(f"workspace too small: {need} bytes needed")
-    out_code = 2 if output.dtype == torch.float32 else (3 if slot_rows_dtype == torch.bfloat16 else 1)
-    tail = (_lib.ptr(w1_alpha), _lib.ptr(w2_alpha), _lib.ptr(fc2_input_scale), output.data_ptr(), tokens, hidden,
-            inter, local, top_k, int(local_expert_offset), 1 if accumulate else 0, out_code, ws.data_ptr(),
-            ws.numel() * ws.element_size(), _lib.current_stream_ptr(dev))
-    with _lib.on_device(dev):
-        if router_logits is None:
-            _lib.check(_lib.lib.b200fp4_moe_fused(x.data_ptr(), w1.data_ptr(), s1.data_ptr(), w2.data_ptr(),
-                                                  s2.data_ptr(), ids.data_ptr(), scales.data_ptr(), *tail))
-        else:
-            _lib.check(_lib.lib.b200fp4_moe_fused_routed(
-                x.data_ptr(), router_logits.data_ptr(), num_experts, 1 if renormalize else 0, w1.data_ptr(),
-                s1.data_ptr(), w2.data_ptr(), s2.data_ptr(), ids.data_ptr(), scales.data_ptr(), *tail))
-    return output
+    return _lib.native.moe(x, w1_weight, w1_weight_sf, w2_weight, w2_weight_sf, token_selected_experts, token_final_scales,
+                           num_experts, top_k, w1_alpha, w2_alpha, fc2_input_scale, num_local_experts,
+                           local_expert_offset, output, output_dtype, accumulate, workspace, slot_rows_dtype,
+                           router_logits, renormalize)
 
 
 class B12xMoEWrapper:
@@ -229,9 +140,9 @@ class B12xMoEWrapper:
         if tokens > self.max_num_tokens:
             raise ValueError(f"{tokens} tokens exceed max_num_tokens={self.max_num_tokens}")
         if router_logits is not None and token_selected_experts is None:
-            token_selected_experts, token_final_scales = self._ids[:tokens], self._scales[:tokens]
-        if output is None:
-            output = torch.empty(tokens, self.hidden_size, dtype=self.output_dtype, device=x.device)
+            whole = tokens == self.max_num_tokens
+            token_selected_experts = self._ids if whole else self._ids[:tokens]
+            token_final_scales = self._scales if whole else self._scales[:tokens]
         return b12x_fused_moe(
             x, w1_weight, w1_weight_sf, w2_weight, w2_weight_sf, token_selected_experts, token_final_scales,
             self.num_experts, self.top_k, w1_alpha=w1_alpha, w2_alpha=w2_alpha, fc2_input_scale=fc2_input_scale,
