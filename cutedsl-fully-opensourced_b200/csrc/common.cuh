@@ -52,6 +52,16 @@ __device__ __forceinline__ U32x8 ld_stream_32B(const void* p) {
   return r;
 }
 
+// read-only, read again by other blocks of the SM: through L1
+__device__ __forceinline__ U32x8 ld_cached_32B(const void* p) {
+  U32x8 r;
+  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+                 "=r"(r.v[6]), "=r"(r.v[7])
+               : "l"(p));
+  return r;
+}
+
 // data that the same kernel writes back later (no .nc)
 __device__ __forceinline__ U32x8 ld_32B(const void* p) {
   U32x8 r;
@@ -149,6 +159,65 @@ __device__ __forceinline__ uint32_t f32x2_to_pair16(uint64_t v) {
 }
 
 // ---------------------------------------------------------------------------
+// packed 16-bit arithmetic: a product of two 16-bit floats rounded once to the type (the same bits as the f32 product,
+// which is exact, rounded to the type), and the largest magnitudes of two pairs
+// ---------------------------------------------------------------------------
+template <typename T>
+struct Pack16;
+template <>
+struct Pack16<__nv_bfloat16> {
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("{\n.reg .b32 x, y;\nabs.bf16x2 x, %1;\nabs.bf16x2 y, %2;\nmax.bf16x2 %0, x, y;\n}" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+};
+template <>
+struct Pack16<__half> {
+  static __device__ __forceinline__ uint32_t mul(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+  static __device__ __forceinline__ uint32_t max_abs(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("{\n.reg .b32 x, y;\nabs.f16x2 x, %1;\nabs.f16x2 y, %2;\nmax.f16x2 %0, x, y;\n}" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+  }
+};
+
+// ---------------------------------------------------------------------------
+// programmatic dependent launch: a kernel launched with the attribute may start while the kernel before it in the
+// stream drains.  grid_dependency_wait() returns when that kernel is complete and its writes are visible: nothing that
+// an earlier kernel may write or read is touched before it.  let_dependents_launch() lets the next kernel's blocks be
+// scheduled as soon as every block of this one has called it (or has exited).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// launch with that attribute
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                             Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // e4m3 scale factors
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t e4m3_encode_rn(float x) {   // 0 <= x <= 448
@@ -203,7 +272,8 @@ __device__ __forceinline__ uint32_t e2m1x8_drop_negative_zero(uint32_t x) {
 }
 
 // a / 6 rounded to nearest, without the division routine: q = a*c, one exact
-// residual and one correction with c = RN(1/6).  Checked against a/6.0f for
+// residual and one correction with c = RN(1/6) (division by a constant known in
+// advance: Brisebarre, Muller, Raina, IEEE Trans. Computers 53(8), 2004).  Checked against a/6.0f for
 // every positive float whose quotient is a normal number; for denormal
 // quotients (far below the smallest scale factor) it may be one ulp off,
 // which the e4m3 rounding to zero hides.
@@ -234,50 +304,73 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // ---------------------------------------------------------------------------
 // The arithmetic runs on the packed f32x2 instructions of sm_100 (two IEEE round-to-nearest f32
 // operations per instruction): a block is eight register pairs.
-template <bool kImplicitOne>
-__device__ __forceinline__ void quantize_block16(const uint64_t (&v2)[8], float gs, uint32_t& codes_lo,
-                                                 uint32_t& codes_hi, uint32_t& sf_bits) {
-  float amax = 0.0f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) amax = fmaxf(fmaxf(amax, fabsf(f32x2_lo(v2[i]))), fabsf(f32x2_hi(v2[i])));
+//
+// pair(i): elements 2i and 2i + 1 of the block as an f32x2, in a form that `scale` turns into the values times gs up to
+// a few ulp; exact(i): the same two values exactly as the golden computes them (only evaluated when a bracket is
+// open: one warp in a hundred; a loop over the open values instead of sixteen copies of the exact rounding made the norm
+// kernel 20 to 40 % slower, it keeps the compiler from interleaving a thread's blocks); amax: the exact largest
+// magnitude.  kOneBranch: one branch for the block instead of one per eight values (2 to 3 % faster in the norm kernel,
+// 1 % slower in the epilogue of the MoE's first GEMM).
+template <bool kImplicitOne, bool kOneBranch, typename Pair, typename Exact>
+__device__ __forceinline__ void quantize_block16(Pair&& pair, Exact&& exact, float amax, float scale, float gs,
+                                                 uint32_t& codes_lo, uint32_t& codes_hi, uint32_t& sf_bits) {
   const float sf = fminf(div_by_6(__fmul_rn(amax, gs)), 448.0f);
   sf_bits = e4m3_encode_rn(sf);
   const float div = kImplicitOne ? e4m3_decode_implicit_one(sf_bits) : e4m3_decode(sf_bits);
-  // k only has to be within a few ulp of gs/div: the brackets are 2^-19 wide
-  const float k = div > 0.0f ? gs * rcp_approx(div) : 0.0f;
+  // k only has to be within a few ulp of scale / div: the brackets are 2^-19 wide
+  const float k = div > 0.0f ? scale * rcp_approx(div) : 0.0f;
   const float k_hi = k * 1.0000019073486328125f;   // 1 + 2^-19
   const float k_lo = k * 0.9999980926513671875f;   // 1 - 2^-19
   const uint64_t k_hi2 = f32x2_pack(k_hi, k_hi);
   const uint64_t k_lo2 = f32x2_pack(k_lo, k_lo);
-  uint32_t out[2];
+  uint32_t ch[2], cl[2];
+  auto redo = [&](int g) {
+    ch[g] = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t v = exact(4 * g + i);
+      ch[g] |= e2m1_code_exact(__fmul_rn(f32x2_lo(v), gs), div) << (8 * i);
+      ch[g] |= e2m1_code_exact(__fmul_rn(f32x2_hi(v), gs), div) << (8 * i + 4);
+    }
+  };
 #pragma unroll
   for (int g = 0; g < 2; ++g) {
     float uh[8], ul[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint64_t h = f32x2_mul(v2[4 * g + i], k_hi2);
-      const uint64_t l = f32x2_mul(v2[4 * g + i], k_lo2);
+      const uint64_t v = pair(4 * g + i);
+      const uint64_t h = f32x2_mul(v, k_hi2);
+      const uint64_t l = f32x2_mul(v, k_lo2);
       uh[2 * i] = f32x2_lo(h);
       uh[2 * i + 1] = f32x2_hi(h);
       ul[2 * i] = f32x2_lo(l);
       ul[2 * i + 1] = f32x2_hi(l);
     }
-    uint32_t ch = e2m1x8_hw(uh);
-    const uint32_t cl = e2m1x8_hw(ul);
-    if (ch != cl) {
-      ch = 0;
-      if (div > 0.0f) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          ch |= e2m1_code_exact(__fmul_rn(f32x2_lo(v2[4 * g + i]), gs), div) << (8 * i);
-          ch |= e2m1_code_exact(__fmul_rn(f32x2_hi(v2[4 * g + i]), gs), div) << (8 * i + 4);
-        }
-      }
+    ch[g] = e2m1x8_hw(uh);
+    cl[g] = e2m1x8_hw(ul);
+    if constexpr (!kOneBranch) {
+      if (ch[g] != cl[g]) redo(g);
     }
-    out[g] = e2m1x8_drop_negative_zero(ch);
   }
-  codes_lo = out[0];
-  codes_hi = out[1];
+  if constexpr (kOneBranch) {
+    if (((ch[0] ^ cl[0]) | (ch[1] ^ cl[1])) != 0) {
+      redo(0);
+      redo(1);
+    }
+  }
+  codes_lo = e2m1x8_drop_negative_zero(ch[0]);
+  codes_hi = e2m1x8_drop_negative_zero(ch[1]);
+}
+
+// the values themselves in registers
+template <bool kImplicitOne, bool kOneBranch = false>
+__device__ __forceinline__ void quantize_block16(const uint64_t (&v2)[8], float gs, uint32_t& codes_lo,
+                                                 uint32_t& codes_hi, uint32_t& sf_bits) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(fmaxf(amax, fabsf(f32x2_lo(v2[i]))), fabsf(f32x2_hi(v2[i])));
+  auto value = [&](int i) { return v2[i]; };
+  quantize_block16<kImplicitOne, kOneBranch>(value, value, amax, gs, gs, codes_lo, codes_hi, sf_bits);
 }
 
 // the same for sixteen scalars

@@ -4,17 +4,18 @@
 // (call sites tests/python/test_flashinfer_norm_verbatim.py:134,155-164); the
 // arithmetic contract is the reference's torch golden (same file, lines 58-99).
 //
-// One pass over HBM: a row is read once (x, and residual for the add variant),
-// kept in registers across the row reduction, and written once (residual, e2m1
-// codes, e4m3 scale factors).  Each thread owns kVec adjacent 16-element scale
-// blocks (one 256-bit load per block and tensor), so a block's amax, scale
-// factor and code bytes never leave the thread; neighbouring lanes merge their
-// scale bytes into one 32-bit store, which is contiguous both in the row-major
-// and in the 128x4 tiled scale-factor layout.  The grid is persistent (a
-// multiple of the SM count); every thread parks the f32 copy of its own slice
-// of the weight vector in shared memory once and re-reads it per row.
-#include <atomic>
-
+// One pass over HBM: a row is read once (x, and residual for the add variant), kept in registers across the row
+// reduction, and written once (residual, e2m1 codes, e4m3 scale factors).  Each thread owns kVec adjacent 16-element
+// scale blocks (one 256-bit load per block and tensor), so a block's amax, scale factor and code bytes never leave the
+// thread; neighbouring lanes merge their scale bytes into one 32-bit store, which is contiguous both in the row-major
+// and in the 128x4 tiled scale-factor layout.
+//
+// One block per row, in hardware order: several blocks share an SM, so one row's loads overlap another's reduction and
+// quantisation, and the last rows spread over all SMs.  (A persistent grid that looped over rows with the weights parked
+// in shared memory as f32 was 10 % slower on the largest shapes and 40 % on middle ones: a last wave that was nearly
+// empty, and a launch that had to load the weights first.)  What bounds it: DRAM for the add variant -- [8192, 7168]
+// bf16, 385 MB: 61 us = 6.3 TB/s, 66 us before -- and the issue slots for the plain one ([4096, 5120] fp16: 22.6 ->
+// 13.7 us; [8192, 7168] bf16: 45 -> 34 us).
 #include "common.cuh"
 
 namespace b200fp4 {
@@ -36,16 +37,8 @@ struct NormParams {
   int hidden;
   int64_t x_row_stride;     // elements
   int64_t res_row_stride;   // elements
+  bool y_vec16;             // rows of y are 16-byte aligned
 };
-
-template <typename T>
-__device__ __forceinline__ void unpack16(const U32x8& p, float (&f)[16]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    f[2 * i] = Pair16<T>::lo(p.v[i]);
-    f[2 * i + 1] = Pair16<T>::hi(p.v[i]);
-  }
-}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -53,284 +46,234 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// A "unit" is kVec adjacent 16-element chunks; thread t of a team handles units
-// t, t+team, ... (kUnits of them).  kWarpRow: the team is one warp and a CTA
-// works on one row per warp (hidden <= 512); otherwise the team is the CTA.
-// kCap: upper bound of the block size of this instantiation; small blocks ask the compiler for a
-// register budget that lets five of them share an SM.
-// kPipe: the loads of the team's next row are issued as soon as the current row's registers have been consumed
-// (before the row reduction), so DRAM requests stay in flight through the reduction, the quantisation and the
-// stores; costs the 32 load registers per thread for the whole loop, hence fewer resident CTAs.
-template <typename T, bool kAdd, int kVec, int kUnits, bool kWarpRow, int kCap, bool kPipe = false>
-__global__ void __launch_bounds__(kCap, kPipe ? 3 : (kCap <= 256 ? 5 : 2)) norm_quant_kernel(const NormParams p) {
-  extern __shared__ float4 wsm[];          // per-thread weight slices, f32
-  __shared__ float red[2][kMaxThreads / 32];
+// Rows that only pad the last 128-row tile of tiled scale factors: their bytes read as zero.  Blocks past the last row
+// of data write them, so that a call is one launch (a separate memset cost a decode-sized call a third of its time).
+__device__ __forceinline__ void zero_padding_row(const NormParams& p, int64_t row, int rk, int tid, int team) {
+  for (int i = tid; i < rk; i += team)
+    *reinterpret_cast<uint32_t*>(p.sf_swizzled + sf_swizzled_offset(row, 4 * i, rk)) = 0u;
+}
+
+// The sum over all 32 slots of red[] in the order of a butterfly over 32 lanes (distance 16, 8, 4, 2, 1), of which only
+// the first kN can be non-zero; every thread adds for itself from broadcast reads, without shuffles.
+template <int kN>
+__device__ __forceinline__ float butterfly_sum(const float* red) {
+  float v[kN];
+#pragma unroll
+  for (int i = 0; i < kN; i += 4) {
+    const float4 q = *reinterpret_cast<const float4*>(red + i);
+    v[i] = q.x, v[i + 1] = q.y, v[i + 2] = q.z, v[i + 3] = q.w;
+  }
+#pragma unroll
+  for (int o = kN / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < o; ++i) v[i] = __fadd_rn(v[i], v[i + o]);
+  }
+  return v[0];
+}
+
+// A "unit" is kVec adjacent 16-element chunks; thread t of a row's team handles units
+// t, t+team, ... (kUnits of them).  kWarpRow: the team is one warp and a block
+// works on one row per warp (hidden <= 1024); otherwise the team is the block.
+template <typename T, bool kAdd, int kVec, int kUnits, bool kWarpRow, int kCap, int kMinCtas>
+__global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormParams p) {
+  constexpr int kSlots = kCap <= 256 ? 8 : 16;             // warps of a team
+  __shared__ __align__(16) float red[kSlots];
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const int nwarps = blockDim.x >> 5;
   const int nchunks = p.hidden >> 4;
   const int team = kWarpRow ? 32 : blockDim.x;
   const int tid = kWarpRow ? lane : threadIdx.x;
   const int rk = (nchunks + 3) >> 2;
-  const float gs = __ldg(p.global_scale);
-  const float n_as_float = static_cast<float>(p.hidden);
-  const T* __restrict__ xg = static_cast<const T*>(p.x);
-  T* rg = static_cast<T*>(p.residual);
-  const bool sf_row_vec = (nchunks & 3) == 0;                  // row-major SF rows are 4-byte aligned
-  const bool y_vec16 = ((p.hidden >> 1) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0;
-  constexpr int kSlots = kUnits * kVec * 4;                    // float4 slots per thread
-  float4* wmine = wsm + (kWarpRow ? warp * kSlots * 32 : 0) + tid;   // slot s lives at wmine[s * team]
+  const int64_t row = kWarpRow ? static_cast<int64_t>(blockIdx.x) * (kCap / 32) + warp : blockIdx.x;
+  if constexpr (!kWarpRow) {
+    if (tid < kSlots && tid >= (team >> 5)) red[tid] = 0.0f;       // slots without a warp
+  }
+  let_dependents_launch();
+  grid_dependency_wait();
+  if (row >= p.rows) {                       // only tiled outputs have blocks past the data
+    if (p.sf_swizzled != nullptr && row < ((p.rows + 127) & ~int64_t{127})) zero_padding_row(p, row, rk, tid, team);
+    return;
+  }
+  const T* __restrict__ xrow = static_cast<const T*>(p.x) + row * p.x_row_stride;
+  T* rrow = static_cast<T*>(p.residual) + (kAdd ? row * p.res_row_stride : 0);
+  const T* __restrict__ wg = static_cast<const T*>(p.weight);
 
+  // ---- phase 1: load, (add, round, write residual), sum of squares; all f32 math on register pairs.  Everything the
+  // thread reads from DRAM is requested before anything is used.
+  U32x8 xin[kUnits * kVec], rin[kAdd ? kUnits * kVec : 1], win[kUnits * kVec];
 #pragma unroll
   for (int u = 0; u < kUnits; ++u) {
 #pragma unroll
     for (int v = 0; v < kVec; ++v) {
-      const int chunk = (tid + u * team) * kVec + v;
-      float wf[16];
+      const int c = u * kVec + v, chunk = (tid + u * team) * kVec + v;
       if (chunk < nchunks) {
-        unpack16<T>(ld_stream_32B(static_cast<const T*>(p.weight) + chunk * 16), wf);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) wf[i] = 0.0f;
+        xin[c] = ld_stream_32B(xrow + chunk * 16);
+        if constexpr (kAdd) rin[c] = ld_32B(rrow + chunk * 16);
+        else win[c] = ld_cached_32B(wg + chunk * 16);
       }
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        wmine[((u * kVec + v) * 4 + q) * team] = make_float4(wf[4 * q], wf[4 * q + 1], wf[4 * q + 2], wf[4 * q + 3]);
     }
   }
-  // each thread only ever reads back its own slots: no barrier needed
-
-  const int64_t row0 = kWarpRow ? static_cast<int64_t>(blockIdx.x) * nwarps + warp : blockIdx.x;
-  const int64_t row_step = kWarpRow ? static_cast<int64_t>(gridDim.x) * nwarps : gridDim.x;
-  int parity = 0;
-  const uint32_t row_bytes = static_cast<uint32_t>(p.hidden) * 2u;
-  // kPipe: raw rows travel in these registers from one iteration to the next
-  U32x8 xnext[kPipe ? kUnits * kVec : 1], rnext[kPipe && kAdd ? kUnits * kVec : 1];
-  auto load_row = [&](int64_t r) {
+  const float gs = __ldg(p.global_scale);
+  // what phase 2 normalises, kept as packed 16-bit pairs so that few registers live across the row reduction
+  uint32_t h[kUnits * kVec][8];
+  uint64_t ssq2 = 0;                         // {0.0f, 0.0f}
 #pragma unroll
-    for (int u = 0; u < kUnits; ++u) {
+  for (int u = 0; u < kUnits; ++u) {
 #pragma unroll
-      for (int v = 0; v < kVec; ++v) {
-        const int chunk = (tid + u * team) * kVec + v;
-        if (chunk < nchunks) {
-          xnext[u * kVec + v] = ld_stream_32B(xg + r * p.x_row_stride + chunk * 16);
-          if constexpr (kAdd) rnext[u * kVec + v] = ld_32B(rg + r * p.res_row_stride + chunk * 16);
-        }
-      }
-    }
-  };
-  if constexpr (kPipe) {
-    if (row0 < p.rows) load_row(row0);
-  }
-  for (int64_t row = row0; row < p.rows; row += row_step, parity ^= 1) {
-    // pull the row this team will work on next (kPipe: the one after it) into L2 while the current one is processed
-    const int64_t ahead = row + (kPipe ? 2 : 1) * row_step;
-    if (tid == 0 && ahead < p.rows) {
-      prefetch_l2_bulk(xg + ahead * p.x_row_stride, row_bytes);
-      if constexpr (kAdd) prefetch_l2_bulk(rg + ahead * p.res_row_stride, row_bytes);
-    }
-    // ---- phase 1: load, (add, round, write residual), sum of squares; all f32 math on register pairs
-    // what phase 2 normalises, kept as packed 16-bit pairs so that few registers live across the row reduction
-    uint32_t h[kUnits * kVec][8];
-    uint64_t ssq2 = 0;                       // {0.0f, 0.0f}
-#pragma unroll
-    for (int u = 0; u < kUnits; ++u) {
-#pragma unroll
-      for (int v = 0; v < kVec; ++v) {
-        const int c = u * kVec + v;
-        const int chunk = (tid + u * team) * kVec + v;
-        if (chunk < nchunks) {
-          const U32x8 xv = kPipe ? xnext[c] : ld_stream_32B(xg + row * p.x_row_stride + chunk * 16);
-          if constexpr (kAdd) {
-            T* rptr = rg + row * p.res_row_stride + chunk * 16;
-            const U32x8 rv = kPipe ? rnext[c] : ld_32B(rptr);
-            U32x8 outv;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint64_t s2 = f32x2_add(pair16_to_f32x2<T>(xv.v[i]), pair16_to_f32x2<T>(rv.v[i]));
-              ssq2 = f32x2_fma(s2, s2, ssq2);
-              outv.v[i] = f32x2_to_pair16<T>(s2);
-              h[c][i] = outv.v[i];                         // the normalised value is built from the ROUNDED residual
-            }
-            st_32B(rptr, outv);
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float4 w4 = wmine[(c * 4 + q) * team];
-              const uint64_t x0 = pair16_to_f32x2<T>(xv.v[2 * q]);
-              const uint64_t x1 = pair16_to_f32x2<T>(xv.v[2 * q + 1]);
-              ssq2 = f32x2_fma(x0, x0, ssq2);
-              ssq2 = f32x2_fma(x1, x1, ssq2);
-              // x*w is rounded to the input type before the f32 scaling
-              h[c][2 * q] = f32x2_to_pair16<T>(f32x2_mul(x0, f32x2_pack(w4.x, w4.y)));
-              h[c][2 * q + 1] = f32x2_to_pair16<T>(f32x2_mul(x1, f32x2_pack(w4.z, w4.w)));
-            }
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) h[c][i] = 0;
-        }
-      }
-    }
-    float ssq = __fadd_rn(f32x2_lo(ssq2), f32x2_hi(ssq2));
-    if constexpr (kPipe) {
-      if (row + row_step < p.rows) load_row(row + row_step);      // in flight until the next iteration's phase 1
-    }
-
-    // ---- row reduction: lanes, then (CTA teams) warps through shared memory
-    ssq = warp_sum(ssq);
-    if constexpr (!kWarpRow) {
-      if (lane == 0) red[parity][warp] = ssq;
-      __syncthreads();
-      ssq = warp_sum(lane < nwarps ? red[parity][lane] : 0.0f);
-    }
-    // 1/sqrt(mean + eps) with IEEE division and square root
-    const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssq, n_as_float), p.eps)));
-    const uint64_t rstd2 = f32x2_pack(rstd, rstd);
-
-    // ---- phase 2: scale, quantise, store
-#pragma unroll
-    for (int u = 0; u < kUnits; ++u) {
-      uint32_t codes[kVec][2];
-      uint32_t sfb[kVec];
-      const int chunk0 = (tid + u * team) * kVec;
-#pragma unroll
-      for (int v = 0; v < kVec; ++v) {
-        const int c = u * kVec + v;
-        uint64_t val[8];
+    for (int v = 0; v < kVec; ++v) {
+      const int c = u * kVec + v, chunk = (tid + u * team) * kVec + v;
+      if (chunk < nchunks) {
         if constexpr (kAdd) {
+          U32x8 outv;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 w4 = wmine[(c * 4 + q) * team];
-            val[2 * q] = f32x2_mul(f32x2_mul(pair16_to_f32x2<T>(h[c][2 * q]), rstd2), f32x2_pack(w4.x, w4.y));
-            val[2 * q + 1] =
-                f32x2_mul(f32x2_mul(pair16_to_f32x2<T>(h[c][2 * q + 1]), rstd2), f32x2_pack(w4.z, w4.w));
+          for (int i = 0; i < 8; ++i) {
+            const uint64_t s2 = f32x2_add(pair16_to_f32x2<T>(xin[c].v[i]), pair16_to_f32x2<T>(rin[c].v[i]));
+            ssq2 = f32x2_fma(s2, s2, ssq2);
+            outv.v[i] = f32x2_to_pair16<T>(s2);
+            h[c][i] = outv.v[i];             // the normalised value is built from the ROUNDED residual
           }
+          st_32B(rrow + chunk * 16, outv);
         } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) val[i] = f32x2_mul(pair16_to_f32x2<T>(h[c][i]), rstd2);
-        }
-        quantize_block16<false>(val, gs, codes[v][0], codes[v][1], sfb[v]);
-        if (chunk0 + v >= nchunks) sfb[v] = 0;
-      }
-      // codes: kVec * 8 contiguous bytes per thread
-      uint8_t* yrow = p.y + row * (p.hidden >> 1);
-      if constexpr (kVec == 2) {
-        if (chunk0 + 1 < nchunks) {
-          if (y_vec16) {
-            *reinterpret_cast<uint4*>(yrow + chunk0 * 8) =
-                make_uint4(codes[0][0], codes[0][1], codes[1][0], codes[1][1]);
-          } else {
-            *reinterpret_cast<uint2*>(yrow + chunk0 * 8) = make_uint2(codes[0][0], codes[0][1]);
-            *reinterpret_cast<uint2*>(yrow + chunk0 * 8 + 8) = make_uint2(codes[1][0], codes[1][1]);
+          for (int i = 0; i < 8; ++i) {
+            const uint64_t x2 = pair16_to_f32x2<T>(xin[c].v[i]);
+            ssq2 = f32x2_fma(x2, x2, ssq2);
+            h[c][i] = Pack16<T>::mul(xin[c].v[i], win[c].v[i]);   // x*w is rounded to the input type before the scaling
           }
-        } else if (chunk0 < nchunks) {
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) h[c][i] = 0;
+      }
+    }
+  }
+  if constexpr (kAdd) {
+#pragma unroll
+    for (int u = 0; u < kUnits; ++u) {
+#pragma unroll
+      for (int v = 0; v < kVec; ++v) {
+        const int c = u * kVec + v, chunk = (tid + u * team) * kVec + v;
+        if (chunk < nchunks) {
+          win[c] = ld_cached_32B(wg + chunk * 16);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) win[c].v[i] = 0;
+        }
+      }
+    }
+  }
+
+  // ---- row reduction: lanes, then (CTA teams) warps through shared memory
+  float ssq = warp_sum(__fadd_rn(f32x2_lo(ssq2), f32x2_hi(ssq2)));
+  if constexpr (!kWarpRow) {
+    if (lane == 0) red[warp] = ssq;
+    __syncthreads();
+    ssq = butterfly_sum<kSlots>(red);
+  }
+  // 1/sqrt(mean + eps) with IEEE division and square root
+  const float rstd = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ssq, static_cast<float>(p.hidden)), p.eps)));
+  const uint64_t rstd2 = f32x2_pack(rstd, rstd);
+
+  // ---- phase 2: scale, quantise, store
+#pragma unroll
+  for (int u = 0; u < kUnits; ++u) {
+    uint32_t codes[kVec][2];
+    uint32_t sfb[kVec];
+    const int chunk0 = (tid + u * team) * kVec;
+#pragma unroll
+    for (int v = 0; v < kVec; ++v) {
+      const int c = u * kVec + v;
+      if constexpr (kAdd) {
+        uint64_t val[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          val[i] = f32x2_mul(f32x2_mul(pair16_to_f32x2<T>(h[c][i]), rstd2), pair16_to_f32x2<T>(win[c].v[i]));
+        quantize_block16<false, true>(val, gs, codes[v][0], codes[v][1], sfb[v]);
+      } else {
+        // h * rstd rounds monotonically in |h|, so the block's largest value comes from its largest |h|, which packed
+        // 16-bit maxima find; the common factor rstd goes into the quantiser's scale
+        uint32_t m = Pack16<T>::max_abs(h[c][0], h[c][1]);
+#pragma unroll
+        for (int i = 2; i < 8; ++i) m = Pack16<T>::max_abs(m, h[c][i]);
+        const float amax = __fmul_rn(fmaxf(Pair16<T>::lo(m), Pair16<T>::hi(m)), rstd);
+        quantize_block16<false, true>([&](int i) { return pair16_to_f32x2<T>(h[c][i]); },
+                                [&](int i) { return f32x2_mul(pair16_to_f32x2<T>(h[c][i]), rstd2); }, amax, rstd * gs, gs,
+                                codes[v][0], codes[v][1], sfb[v]);
+      }
+      if (chunk0 + v >= nchunks) sfb[v] = 0;
+    }
+    // codes: kVec * 8 contiguous bytes per thread
+    uint8_t* yrow = p.y + row * (p.hidden >> 1);
+    if constexpr (kVec == 2) {
+      if (chunk0 + 1 < nchunks) {
+        if (p.y_vec16) {
+          *reinterpret_cast<uint4*>(yrow + chunk0 * 8) = make_uint4(codes[0][0], codes[0][1], codes[1][0], codes[1][1]);
+        } else {
           *reinterpret_cast<uint2*>(yrow + chunk0 * 8) = make_uint2(codes[0][0], codes[0][1]);
+          *reinterpret_cast<uint2*>(yrow + chunk0 * 8 + 8) = make_uint2(codes[1][0], codes[1][1]);
         }
-      } else {
-        if (chunk0 < nchunks) *reinterpret_cast<uint2*>(yrow + chunk0 * 8) = make_uint2(codes[0][0], codes[0][1]);
+      } else if (chunk0 < nchunks) {
+        *reinterpret_cast<uint2*>(yrow + chunk0 * 8) = make_uint2(codes[0][0], codes[0][1]);
       }
-      // scale bytes: the lane whose first chunk is a multiple of 4 collects four K-blocks
-      uint32_t quad;
-      bool leader;
-      if constexpr (kVec == 2) {
-        const uint32_t pair = sfb[0] | (sfb[1] << 8);
-        quad = pair | (__shfl_down_sync(0xffffffffu, pair, 1) << 16);
-        leader = (lane & 1) == 0;
-      } else {
-        quad = sfb[0];
-        quad |= __shfl_down_sync(0xffffffffu, sfb[0], 1) << 8;
-        quad |= __shfl_down_sync(0xffffffffu, sfb[0], 2) << 16;
-        quad |= __shfl_down_sync(0xffffffffu, sfb[0], 3) << 24;
-        leader = (lane & 3) == 0;
-      }
-      if (leader && chunk0 < nchunks) {
-        if (p.sf_swizzled != nullptr) {
-          *reinterpret_cast<uint32_t*>(p.sf_swizzled + sf_swizzled_offset(row, chunk0, rk)) = quad;
-        }
-        if (p.sf_rowmajor != nullptr) {
-          uint8_t* dst = p.sf_rowmajor + row * nchunks + chunk0;
-          if (sf_row_vec) {
-            *reinterpret_cast<uint32_t*>(dst) = quad;
-          } else {
-            for (int j = 0; j < 4 && chunk0 + j < nchunks; ++j) dst[j] = static_cast<uint8_t>(quad >> (8 * j));
-          }
+    } else {
+      if (chunk0 < nchunks) *reinterpret_cast<uint2*>(yrow + chunk0 * 8) = make_uint2(codes[0][0], codes[0][1]);
+    }
+    // scale bytes: the lane whose first chunk is a multiple of 4 collects four K-blocks
+    uint32_t quad;
+    bool leader;
+    if constexpr (kVec == 2) {
+      const uint32_t pair = sfb[0] | (sfb[1] << 8);
+      quad = pair | (__shfl_down_sync(0xffffffffu, pair, 1) << 16);
+      leader = (lane & 1) == 0;
+    } else {
+      quad = sfb[0];
+      quad |= __shfl_down_sync(0xffffffffu, sfb[0], 1) << 8;
+      quad |= __shfl_down_sync(0xffffffffu, sfb[0], 2) << 16;
+      quad |= __shfl_down_sync(0xffffffffu, sfb[0], 3) << 24;
+      leader = (lane & 3) == 0;
+    }
+    if (leader && chunk0 < nchunks) {
+      if (p.sf_swizzled != nullptr) *reinterpret_cast<uint32_t*>(p.sf_swizzled + sf_swizzled_offset(row, chunk0, rk)) = quad;
+      if (p.sf_rowmajor != nullptr) {
+        uint8_t* dst = p.sf_rowmajor + row * nchunks + chunk0;
+        if ((nchunks & 3) == 0) {            // row-major rows are 4-byte aligned
+          *reinterpret_cast<uint32_t*>(dst) = quad;
+        } else {
+          for (int j = 0; j < 4 && chunk0 + j < nchunks; ++j) dst[j] = static_cast<uint8_t>(quad >> (8 * j));
         }
       }
     }
   }
 }
 
-constexpr int kMaxDevices = 64;
-
-int current_device_ordinal() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return dev >= 0 && dev < kMaxDevices ? dev : 0;
-}
-
-// SM count, cached per device ordinal
-int sm_count(int dev) {
-  static std::atomic<int> cached[kMaxDevices];
-  int n = cached[dev].load(std::memory_order_relaxed);
-  if (n == 0) {
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-    cached[dev].store(n, std::memory_order_relaxed);
-  }
-  return n;
-}
-
-template <typename T, bool kAdd, int kVec, int kUnits, bool kWarpRow, int kCap, bool kPipe = false>
+template <typename T, bool kAdd, int kVec, int kUnits, bool kWarpRow, int kCap, int kMinCtas>
 int launch_one(const NormParams& p, int threads, cudaStream_t stream) {
-  auto kern = norm_quant_kernel<T, kAdd, kVec, kUnits, kWarpRow, kCap, kPipe>;
-  const size_t smem = static_cast<size_t>(kUnits) * kVec * 4 * sizeof(float4) * threads;
-  // Shared-memory opt-in and occupancy are per device and per block size: queried once for each (this
-  // instantiation, device, block size) and remembered -- the two driver calls cost more host time than the
-  // launch of a small problem.  per_sm_cache holds (threads << 8 | resident CTAs), 0 = not yet known.
-  static std::atomic<int> per_sm_cache[kMaxDevices];
-  const int dev = current_device_ordinal();
-  int per_sm = 0;
-  const int cached = per_sm_cache[dev].load(std::memory_order_acquire);
-  if (cached != 0 && (cached >> 8) == threads) {
-    per_sm = cached & 0xff;
-  } else {
-    if (smem > 48 * 1024) {
-      B200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    }
-    B200_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-    if (per_sm < 1) return fail(kUnsupported, "norm_quant_kernel does not fit on an SM (%zu bytes of shared memory)", smem);
-    if (per_sm > 255) per_sm = 255;
-    per_sm_cache[dev].store((threads << 8) | per_sm, std::memory_order_release);
-  }
-  // the residual-add variant is DRAM-bound with four resident CTAs per SM already; more of them only
-  // lengthen the last wave (measured on B200: 70 us with 4, 74 us with 6 at [8192, 7168])
-  if (kAdd && !kWarpRow && per_sm > 4) per_sm = 4;
-  const int64_t rows_per_cta = kWarpRow ? threads / 32 : 1;
-  const int64_t want = (p.rows + rows_per_cta - 1) / rows_per_cta;
-  int64_t grid = static_cast<int64_t>(sm_count(dev)) * per_sm;
-  if (grid > want) grid = want;
-  kern<<<static_cast<unsigned>(grid), threads, smem, stream>>>(p);
-  return check_cuda(cudaGetLastError(), "norm_quant_kernel launch");
+  const int64_t rows = p.sf_swizzled != nullptr ? (p.rows + 127) / 128 * 128 : p.rows;
+  const int64_t per_cta = kWarpRow ? kCap / 32 : 1;
+  return check_cuda(launch_dependent(norm_quant_kernel<T, kAdd, kVec, kUnits, kWarpRow, kCap, kMinCtas>,
+                                     dim3(static_cast<unsigned>((rows + per_cta - 1) / per_cta)),
+                                     dim3(kWarpRow ? kCap : threads), 0, stream, p),
+                    "norm_quant_kernel launch");
 }
 
 template <typename T, bool kAdd>
 int dispatch(const NormParams& p, cudaStream_t stream) {
   const int nchunks = p.hidden / 16;
-  if (nchunks <= 32) return launch_one<T, kAdd, 1, 1, true, 128>(p, 128, stream);
+  // up to 1024 columns a warp holds a row (one chunk per lane, or two) and a block of four warps four rows: blocks of a
+  // single warp would leave half of an SM's warp slots empty ([16384, 1024]: 18.3 -> 11.1 us plain, 21.8 -> 20.3 add)
+  if (nchunks <= 32) return launch_one<T, kAdd, 1, 1, true, 128, 1>(p, 32, stream);
   const int nunits = (nchunks + 1) / 2;                       // two adjacent chunks per unit
   const int units = (nunits + kMaxThreads - 1) / kMaxThreads;
   const int threads = (((nunits + units - 1) / units) + 31) / 32 * 32;
   switch (units) {
     case 1:
-      // the residual-add variant keeps its next row's loads in flight in registers (three resident CTAs instead
-      // of four: 71.2 -> 70.0 us at [8192, 7168]; with four pipelined CTAs 77 us); the plain variant, with half
-      // the bytes per row, does better with more resident CTAs and the L2 prefetch alone
-      if (kAdd && threads <= 256) return launch_one<T, kAdd, 2, 1, false, 256, kAdd>(p, threads, stream);
-      return threads <= 256 ? launch_one<T, kAdd, 2, 1, false, 256>(p, threads, stream)
-                            : launch_one<T, kAdd, 2, 1, false, kMaxThreads>(p, threads, stream);
-    case 2: return launch_one<T, kAdd, 2, 2, false, kMaxThreads>(p, threads, stream);
+      if (threads == 32) return launch_one<T, kAdd, 2, 1, true, 128, 8>(p, threads, stream);
+      // resident blocks: 64 registers for the add variant (five blocks of 48 are no faster, six spill), 48 for the plain
+      // one, which has half the loads ([8192, 7168]: 34 us against 38 with 64 registers)
+      return threads <= 256 ? launch_one<T, kAdd, 2, 1, false, 256, kAdd ? 4 : 5>(p, threads, stream)
+                            : launch_one<T, kAdd, 2, 1, false, kMaxThreads, 2>(p, threads, stream);
+    case 2: return launch_one<T, kAdd, 2, 2, false, kMaxThreads, 1>(p, threads, stream);
     default: return fail(kUnsupported, "hidden=%d exceeds the supported maximum of %d", p.hidden,
                          32 * kMaxThreads * kMaxUnitsPerThread);
   }
@@ -376,12 +319,8 @@ int norm_fp4quant_launch(const void* x, void* residual, const void* weight, void
   p.x_row_stride = x_row_stride;
   p.res_row_stride = res_row_stride;
 
-  const int nchunks = hidden / 16;
-  if (p.sf_swizzled != nullptr && ((rows & 127) != 0 || (nchunks & 3) != 0)) {
-    // rows / K-blocks that only pad a 128x4 tile must read as zero
-    const size_t bytes = static_cast<size_t>((rows + 127) / 128) * ((nchunks + 3) / 4) * 512;
-    B200_CUDA(cudaMemsetAsync(p.sf_swizzled, 0, bytes, stream));
-  }
+  p.y_vec16 = hidden % 32 == 0 && (reinterpret_cast<uintptr_t>(y_fp4) & 15) == 0;
+  if (rows > (1LL << 30)) return fail(kUnsupported, "too many rows");
   const bool add = residual != nullptr;
   if (dtype == 1) return add ? dispatch<__nv_bfloat16, true>(p, stream) : dispatch<__nv_bfloat16, false>(p, stream);
   return add ? dispatch<__half, true>(p, stream) : dispatch<__half, false>(p, stream);

@@ -130,6 +130,13 @@ def test_ragged_shapes_and_layouts(b200, rows, hidden):
     assert np.array_equal(s3u.cpu().numpy(), s1n)
 
 
+@pytest.mark.parametrize("rows,hidden", [(1, 1024), (5, 528), (127, 1008), (129, 1024), (3, 512), (130, 1056), (256, 4096)])
+def test_rows_of_one_warp_and_padding_blocks(b200, rows, hidden):
+    """One warp per row up to 1024 columns (one or two chunks per lane), one block per row beyond, and the blocks that
+    clear the padding rows of tiled scale factors."""
+    test_ragged_shapes_and_layouts(b200, rows, hidden)
+
+
 def test_three_dim_input_and_strided_rows(b200):
     torch.manual_seed(11)
     base = torch.randn(4, 6, 2 * 512).to(torch.bfloat16).cuda()
