@@ -241,8 +241,14 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   int grid = sm_count_of_current_device();
   if (grid > max_tiles) grid = max_tiles;
   if (grid < 1) return kOk;
-  kern<<<grid, gemm_threads(kBlockN, kSwigluB, kEpi), L.total, stream>>>(ta, tb, tc, p, epi);
-  return check_cuda(cudaGetLastError(), "nvfp4_gemm_kernel launch");
+  // the expert-parallel launches keep full stream order: other ranks' kernels follow their own signals
+  if (p.peer.world > 1) {
+    kern<<<grid, gemm_threads(kBlockN, kSwigluB, kEpi), L.total, stream>>>(ta, tb, tc, p, epi);
+    return check_cuda(cudaGetLastError(), "nvfp4_gemm_kernel launch");
+  }
+  return check_cuda(launch_dependent(kern, dim3(grid), dim3(gemm_threads(kBlockN, kSwigluB, kEpi)), L.total, stream, ta, tb,
+                                     tc, p, epi),
+                    "nvfp4_gemm_kernel launch");
 }
 
 // CTA-pair variant: 256 x 256 tiles on 2-CTA clusters
@@ -283,13 +289,15 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   cfg.blockDim = dim3(kPairThreads, 1, 1);
   cfg.dynamicSmemBytes = kPairSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, p, epi), "nvfp4_gemm_pair_kernel launch");
 }
 
@@ -302,6 +310,8 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
 template <typename OutT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits, int64_t stride,
                                      const float* __restrict__ alpha, OutT* __restrict__ c, int64_t n4) {
+  grid_dependency_wait();
+  let_dependents_launch();
   const float scale = alpha == nullptr ? 1.0f : __ldg(alpha);
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -367,9 +377,9 @@ int gemm_dense_splitk(const void* a, const void* b, const void* sfa, const void*
   if (rc) return rc;
   const int64_t n4 = static_cast<int64_t>(m) * n / 4;
   const int grid = static_cast<int>(std::min<int64_t>((n4 + 255) / 256, 4 * sm_count_of_current_device()));
-  splitk_reduce_kernel<OutT><<<grid, 256, 0, stream>>>(workspace, splits, static_cast<int64_t>(m) * n, alpha,
-                                                        static_cast<OutT*>(c), n4);
-  return check_cuda(cudaGetLastError(), "splitk_reduce_kernel launch");
+  return check_cuda(launch_dependent(splitk_reduce_kernel<OutT>, dim3(grid), dim3(256), 0, stream, workspace, splits,
+                                     static_cast<int64_t>(m) * n, alpha, static_cast<OutT*>(c), n4),
+                    "splitk_reduce_kernel launch");
 }
 
 // ---------------------------------------------------------------------------
@@ -499,7 +509,8 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
                  const float* w1_alpha, const float* fc2_input_scale, const int* num_m_blocks_dev,
                  const int* m_block_expert, const int* m_block_rows, int max_m_blocks, int hidden, int inter,
                  int experts, int few_rows, int* status, cudaStream_t stream, const PeerSync* peer,
-                 int sfa_row_pitch) {
+                 int sfa_row_pitch, int early_b) {
+  // early_b: the block tables are older than the kernel before this one
   // sfa_row_pitch: 0 = xq_sf holds 128x4 tiles; else plain rows of scale bytes with that pitch
   // few_rows: no row block holds more than 32 rows (the caller knows: at most 32 tokens) -> stages of 32 rows of A
   // Tile width: [up 128 | gate 128] tiles by default.  They have one accumulator, but the epilogue hands it back
@@ -537,6 +548,8 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
   p.status = status;
   p.row_block_major = 1;
   if (peer != nullptr) p.peer = *peer;
+  p.early_b = early_b;
+  p.early_trigger = few_rows;
   CUtensorMap tsfa{};
   if (sfa_row_pitch != 0) {
     rc = make_sfa_rows_map(&tsfa, xq_sf, static_cast<int64_t>(max_m_blocks) * 128, hidden, sfa_row_pitch);
@@ -588,7 +601,7 @@ template <typename RowT>
 int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2, const void* w2_sf, RowT* partial,
                        const float* w2_alpha, const int* num_m_blocks_dev, const int* m_block_expert,
                        const int* m_block_rows, int max_m_blocks, int hidden, int inter, int experts, int few_rows,
-                       int* status, cudaStream_t stream) {
+                       int* status, cudaStream_t stream, int early_b) {
   CUtensorMap ta, tb;
   // Short reductions with 16-bit rows: 256-wide tiles whose rows leave through TMA stores (EpilogueStoreWide, three
   // stages).  FC2 of the prefill shape: 128-wide tiles with TMA stores 67 us, 256-wide with register stores 64,
@@ -622,6 +635,7 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   p.m_block_rows = m_block_rows;
   p.status = status;
   p.row_block_major = 1;
+  p.early_b = early_b;
   EpilogueStore<RowT> epi{partial, hidden, w2_alpha, 1};
   CUtensorMap tc{};
   rc = make_output_map(&tc, partial, static_cast<int64_t>(max_m_blocks) * 128, static_cast<int64_t>(hidden) * sizeof(RowT),
@@ -691,14 +705,14 @@ int gemm_moe_fc2_push(const void* act_codes, const void* act_sf, const void* w2,
 int gemm_moe_fc2(const void* act_codes, const void* act_sf, const void* w2, const void* w2_sf, void* partial,
                  int rows_bf16, const float* w2_alpha, const int* num_m_blocks_dev, const int* m_block_expert,
                  const int* m_block_rows, int max_m_blocks, int hidden, int inter, int experts, int few_rows,
-                 int* status, cudaStream_t stream) {
+                 int* status, cudaStream_t stream, int early_b) {
   if (rows_bf16)
     return gemm_moe_fc2_typed(act_codes, act_sf, w2, w2_sf, static_cast<__nv_bfloat16*>(partial), w2_alpha,
                               num_m_blocks_dev, m_block_expert, m_block_rows, max_m_blocks, hidden, inter, experts,
-                              few_rows, status, stream);
+                              few_rows, status, stream, early_b);
   return gemm_moe_fc2_typed(act_codes, act_sf, w2, w2_sf, static_cast<float*>(partial), w2_alpha, num_m_blocks_dev,
                             m_block_expert, m_block_rows, max_m_blocks, hidden, inter, experts, few_rows, status,
-                            stream);
+                            stream, early_b);
 }
 
 }  // namespace b200fp4

@@ -95,6 +95,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   ptx::cluster_sync();                                   // both CTAs' barriers exist before anyone signals them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  grid_dependency_wait();
 
   const int num_tiles = p.num_m_blocks * p.num_n_blocks; // num_m_blocks counts 256-row blocks here
 

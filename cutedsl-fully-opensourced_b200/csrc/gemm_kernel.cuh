@@ -30,6 +30,8 @@
 #ifdef B200FP4_ACCT
 #include <cstdio>
 #endif
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 
@@ -116,6 +118,13 @@ struct GemmParams {
   // peer.signal_phase >= 0: the last CTA to finish raises that signal at every peer (its epilogue stored rows
   // into their memory).
   PeerSync peer;
+  // Launched as a dependent of the kernel before it (programmatic dependent launch): the block tables and B are older
+  // than that kernel, so the producer asks for the first stages of B before it waits for the rows of A.
+  int early_b;
+  // Let the next kernel's blocks take over the SMs of blocks that have finished.  Measured: FC1 of a one-token step gains
+  // (57.7 against 59.9 us for the step), launches with more than a few tiles per SM lose (a 16 x 8192 x 8192 GEMM 18.3
+  // against 16.9 us, a prefill step 3 to 5 us), so only the few-row FC1 sets it.
+  int early_trigger;
 };
 
 struct SmemLayout {
@@ -691,6 +700,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
+  if (!p.early_b) grid_dependency_wait();
 
   // grouped launches read the number of row blocks from device memory; never trust it beyond the table size
   const int num_m_blocks =
@@ -730,19 +740,60 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         // peers wrote the rows with ordinary stores; the loads below go through the async proxy
         asm volatile("fence.proxy.async;" ::: "memory");
       }
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int m_blk = tile_m(tile);
+      const int tps = 4 >> p.sf_block32;                            // 512-byte scale tiles per stage: 4, 2 or 1
+      // what the loads of a tile have in common
+      int m_blk = 0, group = 0, b_row[kBPieces];
+      const uint8_t *sfa_row = nullptr, *sfb_row[kBPieces];
+      auto begin_tile = [&](int tile) {
+        m_blk = tile_m(tile);
         const int n_blk = tile_n(tile);
-        const int group =
-            p.m_block_group != nullptr ? max(0, min(__ldg(p.m_block_group + m_blk), p.num_groups - 1)) : 0;
-        int b_row[kBPieces];
-        if constexpr (kSwigluB) {
-          b_row[0] = n_blk * kBPieceRows;
-          b_row[1] = p.gate_row_offset + n_blk * kBPieceRows;
-        } else {
+        group = p.m_block_group != nullptr ? max(0, min(__ldg(p.m_block_group + m_blk), p.num_groups - 1)) : 0;
+        sfa_row = p.sfa + static_cast<int64_t>(m_blk) * p.rk * 512;
 #pragma unroll
-          for (int i = 0; i < kBPieces; ++i) b_row[i] = n_blk * kBlockN + kBPieceRows * i;
+        for (int i = 0; i < kBPieces; ++i) {
+          b_row[i] = kSwigluB ? (i == 0 ? 0 : p.gate_row_offset) + n_blk * kBPieceRows : n_blk * kBlockN + kBPieceRows * i;
+          sfb_row[i] = p.sfb + (static_cast<int64_t>(group) * p.b_row_tiles + (b_row[i] >> 7)) * p.rk * 512;
         }
+      };
+      // One K step.  The scale slabs go first and report to their own barrier: the movers carry them into tensor memory
+      // while the operand tiles are still on their way.
+      // kA / kB: whether the A and the B part of the stage are requested.
+      auto issue = [&](int kt, int stage, auto a_part, auto b_part) {
+        constexpr bool kA = decltype(a_part)::value, kB = decltype(b_part)::value;
+        const uint32_t sa = smem_base + stage * L.stage_bytes, sb = sa + L.a_bytes;
+        const uint32_t ssfa = sb + L.b_bytes, ssfb = ssfa + L.sfa_bytes;
+        const uint32_t sf_bytes = static_cast<uint32_t>(min(tps, p.rk - tps * kt)) * 512u;
+        const uint32_t sbar = sf_loaded_bar(stage), bar = full_bar(stage);
+        // B announces the bytes of the whole stage; a box always delivers its full size
+        if constexpr (kB) ptx::mbar_expect_tx(sbar, (p.sfa_row_major ? 2048u : sf_bytes) + sf_bytes * kBPieces);
+        if constexpr (kA) {
+          if (p.sfa_row_major) ptx::tma_load_2d(ssfa, &tmap_aux, kt * 16, m_blk * kBlockM, sbar);
+          else ptx::bulk_load(ssfa, sfa_row + tps * kt * 512, sf_bytes, sbar);
+        }
+        if constexpr (kB) {
+#pragma unroll
+          for (int i = 0; i < kBPieces; ++i) ptx::bulk_load(ssfb + i * 2048, sfb_row[i] + tps * kt * 512, sf_bytes, sbar);
+          ptx::mbar_expect_tx(bar, L.a_bytes + L.b_bytes);
+        }
+        if constexpr (kA) ptx::tma_load_2d(sa, &tmap_a, kt * 128, m_blk * kBlockM, bar);
+        if constexpr (kB) {
+#pragma unroll
+          for (int i = 0; i < kBPieces; ++i)
+            ptx::tma_load_3d(sb + i * kBPieceRows * 128, &tmap_b, kt * 128, b_row[i], group, bar);
+        }
+      };
+      int primed = 0;                    // stages whose B is under way
+      if (p.early_b) {
+        for (int tile = blockIdx.x; tile < num_tiles && primed < kStages; tile += gridDim.x) {
+          begin_tile(tile);
+          for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end && primed < kStages; ++kt)
+            issue(kt, primed++, std::false_type{}, std::true_type{});
+        }
+        grid_dependency_wait();
+      }
+      if (p.early_trigger) let_dependents_launch();
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        begin_tile(tile);
         if (kARows < kBlockM && p.m_block_rows != nullptr && __ldg(p.m_block_rows + m_blk) > kARows)
           atomicOr(p.status, kStatusRowsExceedTile);      // results of this block are wrong: tell the host
         for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end; ++kt) {
@@ -751,33 +802,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             ok = false;
             break;
           }
-          const uint32_t sa = smem_base + st.stage * L.stage_bytes;
-          const uint32_t sb = sa + L.a_bytes;
-          const uint32_t ssfa = sb + L.b_bytes;
-          const uint32_t ssfb = ssfa + L.sfa_bytes;
-          const int tps = 4 >> p.sf_block32;                            // 512-byte scale tiles per stage: 4, 2 or 1
-          const int k_sf_tiles = min(tps, p.rk - tps * kt);
-          const uint32_t sf_bytes = static_cast<uint32_t>(k_sf_tiles) * 512u;
-          // the scale slabs go first and report to their own barrier: the movers carry them into tensor
-          // memory while the operand tiles are still on their way
-          const uint32_t sbar = sf_loaded_bar(st.stage);
-          if (p.sfa_row_major) {
-            ptx::mbar_expect_tx(sbar, 2048u + sf_bytes * kBPieces);     // a box always delivers its full size
-            ptx::tma_load_2d(ssfa, &tmap_aux, kt * 16, m_blk * kBlockM, sbar);
+          if (primed > 0) {
+            --primed;
+            issue(kt, st.stage, std::true_type{}, std::false_type{});
           } else {
-            ptx::mbar_expect_tx(sbar, sf_bytes * (1 + kBPieces));
-            ptx::bulk_load(ssfa, p.sfa + (static_cast<int64_t>(m_blk) * p.rk + tps * kt) * 512, sf_bytes, sbar);
+            issue(kt, st.stage, std::true_type{}, std::true_type{});
           }
-#pragma unroll
-          for (int i = 0; i < kBPieces; ++i) {
-            const int64_t tile_idx = static_cast<int64_t>(group) * p.b_row_tiles + (b_row[i] >> 7);
-            ptx::bulk_load(ssfb + i * 2048, p.sfb + (tile_idx * p.rk + tps * kt) * 512, sf_bytes, sbar);
-          }
-          const uint32_t bar = full_bar(st.stage);
-          ptx::mbar_expect_tx(bar, L.a_bytes + L.b_bytes);
-          ptx::tma_load_2d(sa, &tmap_a, kt * 128, m_blk * kBlockM, bar);
-#pragma unroll
-          for (int i = 0; i < kBPieces; ++i) ptx::tma_load_3d(sb + i * kBPieceRows * 128, &tmap_b, kt * 128, b_row[i], group, bar);
           st.advance(kStages);
         }
       }
@@ -965,6 +995,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int quarter = warp & 3;                      // TMEM lanes this warp may touch
     const int part = (warp - 2) >> 2;                  // which share of the columns (two warps per quarter)
     const int row = quarter * 32 + lane;
+    if (p.early_b) grid_dependency_wait();
     PipeState acc;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const int m_blk = tile_m(tile);

@@ -17,6 +17,7 @@
 //
 // All intermediate buffers live in a caller-provided workspace.
 #include <algorithm>
+#include <utility>
 
 #include "gemm_kernel.cuh"
 
@@ -26,11 +27,11 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
                  const float* w1_alpha, const float* fc2_input_scale, const int* num_m_blocks_dev,
                  const int* m_block_expert, const int* m_block_rows, int max_m_blocks, int hidden, int inter,
                  int experts, int few_rows, int* status, cudaStream_t stream, const PeerSync* peer = nullptr,
-                 int sfa_row_pitch = 0);
+                 int sfa_row_pitch = 0, int early_b = 0);
 int gemm_moe_fc2(const void* act_codes, const void* act_sf, const void* w2, const void* w2_sf, void* partial,
                  int rows_bf16, const float* w2_alpha, const int* num_m_blocks_dev, const int* m_block_expert,
                  const int* m_block_rows, int max_m_blocks, int hidden, int inter, int experts, int few_rows,
-                 int* status, cudaStream_t stream);
+                 int* status, cudaStream_t stream, int early_b = 0);
 
 int sm_count_of_current_device();
 
@@ -108,6 +109,8 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int* __restr
                                   int tokens, int experts, int top_k, int renormalize) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
+  grid_dependency_wait();
+  let_dependents_launch();
   if (warp >= tokens) return;
   int my_id;
   float my_w;
@@ -229,6 +232,8 @@ moe_count_kernel(const float* __restrict__ logits, int route_experts, int renorm
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int token0 = blockIdx.x * tokens_per_cta;
   const int n_tokens = min(tokens_per_cta, tokens - token0);
+  grid_dependency_wait();
+  let_dependents_launch();
   for (int e = threadIdx.x; e < experts_total; e += kCountThreads) s_hist[e] = 0;
   __syncthreads();
   for (int lt = warp; lt < n_tokens; lt += kCountThreads >> 5) {
@@ -311,6 +316,8 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
   __shared__ int s_flag;
   __shared__ int s_rows[kWarps][64];
   __shared__ int s_dst[kWarps][64];
+  grid_dependency_wait();
+  let_dependents_launch();
   if (!wait_all_ranks(ex, 0, ctrl, status, &s_flag)) return;
 
   const int rpb = rows_per_block;
@@ -450,6 +457,8 @@ moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, in
   __shared__ int s_expert[1024];
   const int t = threadIdx.x;
   s_count[t] = 0;
+  grid_dependency_wait();
+  let_dependents_launch();
   if constexpr (kRoutePerLane > 0) {
     const int lane = t & 31;
     for (int token = t >> 5; token * top_k < n_slots; token += 32) {
@@ -524,6 +533,8 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __
                               uint8_t* xq_sf, int hidden, int top_k) {
   __shared__ int s_rows[64];
   const int token = blockIdx.x;
+  grid_dependency_wait();
+  let_dependents_launch();
   if (threadIdx.x < top_k) s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
   __syncthreads();
   const int nchunks = hidden >> 4;
@@ -567,6 +578,8 @@ __global__ void moe_combine_kernel(const RowT* __restrict__ partial, const int* 
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
   const int token = blockIdx.x;
+  grid_dependency_wait();
+  let_dependents_launch();
   if (threadIdx.x < top_k) {
     s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
     s_w[threadIdx.x] = weights[static_cast<int64_t>(token) * top_k + threadIdx.x];
@@ -619,6 +632,8 @@ __global__ void moe_combine_few_kernel(const RowT* __restrict__ partial, const i
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
   const int token = blockIdx.x;
+  grid_dependency_wait();
+  let_dependents_launch();
   if (threadIdx.x < top_k) {
     s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
     s_w[threadIdx.x] = weights[static_cast<int64_t>(token) * top_k + threadIdx.x];
@@ -678,6 +693,8 @@ __global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ part
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
   const int token = blockIdx.x;
+  grid_dependency_wait();
+  let_dependents_launch();
   if (threadIdx.x < top_k) {
     s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
     s_w[threadIdx.x] = weights[static_cast<int64_t>(token) * top_k + threadIdx.x];
@@ -800,6 +817,16 @@ MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int expert
   return w;
 }
 
+// a launch that may overlap the tail of its predecessor on a single GPU; the expert-parallel steps, whose kernels wait for
+// and signal other ranks, keep full stream order
+template <typename... Params, typename... Args>
+cudaError_t launch_in_order(int world, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                            Args&&... args) {
+  if (world == 1) return launch_dependent(kern, grid, block, smem, stream, std::forward<Args>(args)...);
+  kern<<<grid, block, smem, stream>>>(static_cast<Params>(args)...);
+  return cudaGetLastError();
+}
+
 // launch of the count kernel: routing from logits when `logits` is given (ids_out / weights_out receive the
 // result), else the caller's ids
 int launch_count(const float* logits, int route_experts, int renormalize, const int* ids_in, int* ids_out,
@@ -809,16 +836,17 @@ int launch_count(const float* logits, int route_experts, int renormalize, const 
   const dim3 grid((tokens + tpc - 1) / tpc);
   const size_t smem = sizeof(int) * 2 * experts_total;
 #define B200_COUNT(PL)                                                                                             \
-  moe_count_kernel<PL><<<grid, std::min(count_threads(PL), 32 * tpc), smem, stream>>>(                             \
-      logits, route_experts, renormalize, ids_in, ids_out, weights_out, tokens, top_k, expert_lo, experts_total,    \
-      my_counts, slot_pos, ctrl, ex, tpc)
-  if (logits == nullptr) B200_COUNT(0);
-  else if (route_experts <= 64) B200_COUNT(2);
-  else if (route_experts <= 128) B200_COUNT(4);
-  else if (route_experts <= 256) B200_COUNT(8);
-  else B200_COUNT(kRouteMaxPerLane);
+  launch_in_order(ex.world, moe_count_kernel<PL>, grid, dim3(std::min(count_threads(PL), 32 * tpc)), smem, stream,   \
+                  logits, route_experts, renormalize, ids_in, ids_out, weights_out, tokens, top_k, expert_lo,        \
+                  experts_total, my_counts, slot_pos, ctrl, ex, tpc)
+  cudaError_t err;
+  if (logits == nullptr) err = B200_COUNT(0);
+  else if (route_experts <= 64) err = B200_COUNT(2);
+  else if (route_experts <= 128) err = B200_COUNT(4);
+  else if (route_experts <= 256) err = B200_COUNT(8);
+  else err = B200_COUNT(kRouteMaxPerLane);
 #undef B200_COUNT
-  return check_cuda(cudaGetLastError(), "moe_count_kernel launch");
+  return check_cuda(err, "moe_count_kernel launch");
 }
 
 int launch_place(const void* x, const int* ids, const int* slot_pos, const Exchange& ex, int tokens, int hidden,
@@ -828,10 +856,11 @@ int launch_place(const void* x, const int* ids, const int* slot_pos, const Excha
   // eight warps per CTA, one token per warp at a time; enough CTAs that every SM holds several
   const int grid = std::max(1, std::min((tokens + 7) / 8, 6 * sm_count_of_current_device()));
   const size_t smem = sizeof(int) * 3 * experts_total;
-  moe_quant_place_kernel<256><<<grid, 256, smem, stream>>>(
+  const cudaError_t err = launch_in_order(
+      ex.world, moe_quant_place_kernel<256>, dim3(grid), dim3(256), smem, stream,
       static_cast<const __nv_bfloat16*>(x), ids, slot_pos, ex, tokens, hidden, top_k, expert_lo, experts_total,
       max_m_blocks, rows_per_block, slot_row, num_m_blocks, m_block_expert, m_block_rows, ctrl, status, weights);
-  return check_cuda(cudaGetLastError(), "moe_quant_place_kernel launch");
+  return check_cuda(err, "moe_quant_place_kernel launch");
 }
 
 int route_check(int tokens, int experts, int top_k) {
@@ -851,16 +880,19 @@ int route_topk(const float* logits, int* ids, float* weights, int tokens, int ex
   if (tokens == 0) return kOk;
   const int warps_per_cta = 4;
   const dim3 grid((tokens + warps_per_cta - 1) / warps_per_cta), block(32 * warps_per_cta);
+  auto route = [&](auto kern) {
+    return check_cuda(launch_dependent(kern, grid, block, 0, stream, logits, ids, weights, tokens, experts, top_k, renormalize),
+                      "route_topk_kernel launch");
+  };
   if (experts <= 64)
-    route_topk_kernel<2><<<grid, block, 0, stream>>>(logits, ids, weights, tokens, experts, top_k, renormalize);
+    rc = route(route_topk_kernel<2>);
   else if (experts <= 128)
-    route_topk_kernel<4><<<grid, block, 0, stream>>>(logits, ids, weights, tokens, experts, top_k, renormalize);
+    rc = route(route_topk_kernel<4>);
   else if (experts <= 256)
-    route_topk_kernel<8><<<grid, block, 0, stream>>>(logits, ids, weights, tokens, experts, top_k, renormalize);
+    rc = route(route_topk_kernel<8>);
   else
-    route_topk_kernel<kRouteMaxPerLane><<<grid, block, 0, stream>>>(logits, ids, weights, tokens, experts, top_k,
-                                                                     renormalize);
-  return check_cuda(cudaGetLastError(), "route_topk_kernel launch");
+    rc = route(route_topk_kernel<kRouteMaxPerLane>);
+  return rc;
 }
 
 size_t moe_workspace_bytes(int64_t tokens, int hidden, int inter, int experts, int top_k) {
@@ -905,13 +937,14 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
   const int few_rows = moe_few_rows(tokens, top_k);
 
   if (slots <= 1024) {
-    B200_CUDA(cudaMemsetAsync(ws.xq_sf, 0, ws.xq_sf_bytes, stream));    // rows that only pad a block read as zero
+    // rows that only pad a block keep whatever their scale bytes held: a row of the accumulator depends on its own row of A
+    // only, and rows without data are never read back
     // few slots: one CTA counts, scans and assigns rows in slot order; quantisation splits a token's columns
     // over several CTAs (a decode step is mostly the latency of these small kernels)
 #define B200_PREPARE(PL)                                                                                          \
-  moe_prepare_small_kernel<PL><<<1, 1024, 0, stream>>>(logits, route_experts, renormalize, top_k, ids, route_w, slots, \
-                                                       expert_lo, ws.h, experts, ws.max_m_blocks, max_rows,          \
-                                                       few_rows ? 32 : 128)
+  B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL>, dim3(1), dim3(1024), 0, stream, logits, route_experts,   \
+                             renormalize, top_k, ids, route_w, slots, expert_lo, ws.h, experts, ws.max_m_blocks,    \
+                             max_rows, few_rows ? 32 : 128))
     if (logits == nullptr) {
       B200_PREPARE(0);
     } else if (route_experts <= 64) {
@@ -928,8 +961,8 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     }
 #undef B200_PREPARE
     const int parts = std::max(1, std::min(8, (hidden / 16) / 128));
-    moe_scatter_quant_rows_kernel<128><<<dim3(static_cast<unsigned>(tokens), parts), 128, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, hidden, top_k);
+    B200_CUDA(launch_dependent(moe_scatter_quant_rows_kernel<128>, dim3(static_cast<unsigned>(tokens), parts), dim3(128), 0,
+                               stream, static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, hidden, top_k));
   } else {
     // two launches for any number of tokens: (route +) count, then scan + quantise + place
     B200_CUDA(cudaMemsetAsync(ws.ctrl, 0, ws.clear_bytes, stream));
@@ -952,35 +985,39 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
                       ws.ctrl, status, stream);
     if (rc) return rc;
   }
-  B200_CUDA(cudaGetLastError());
+  // the small front end's block tables are two launches old when FC1 starts, the other one's are its predecessor's work
   int rc = gemm_moe_fc1(ws.xq, ws.xq_sf, w1, w1_sf, ws.act, ws.act_sf, w1_alpha, fc2_input_scale, ws.h.num_m_blocks,
                         ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, few_rows,
-                        status, stream, nullptr, slots <= 1024 ? 0 : sf_row_pitch(hidden));
+                        status, stream, nullptr, slots <= 1024 ? 0 : sf_row_pitch(hidden), slots <= 1024);
   if (rc) return rc;
   rc = gemm_moe_fc2(ws.act, ws.act_sf, w2, w2_sf, ws.partial, rows_bf16, w2_alpha, ws.h.num_m_blocks, ws.h.m_block_expert,
-                    ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, few_rows, status, stream);
+                    ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, few_rows, status, stream, 1);
   if (rc) return rc;
   const int threads = hidden / 4 >= 256 ? 256 : 128;
+  auto combine = [&](auto kern, dim3 grid, int block, auto... args) {
+    return check_cuda(launch_dependent(kern, grid, dim3(block), 0, stream, args...), "moe_combine_kernel launch");
+  };
   if (tokens <= 256 && out_dtype == 3) {
     const dim3 cgrid(static_cast<unsigned>(tokens), (hidden / 4 + threads - 1) / threads);
-    moe_combine_few_kernel<__nv_bfloat16, __nv_bfloat16><<<cgrid, threads, 0, stream>>>(
+    return combine(
+        moe_combine_few_kernel<__nv_bfloat16, __nv_bfloat16>, cgrid, threads,
         reinterpret_cast<const __nv_bfloat16*>(ws.partial), ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out),
         hidden, top_k, accumulate);
   } else if (out_dtype == 2) {
-    moe_combine_kernel<float, float><<<static_cast<unsigned>(tokens), threads, 0, stream>>>(
-        ws.partial, ws.h.slot_row, route_w, static_cast<float*>(out), hidden, top_k, accumulate);
+    return combine(
+        moe_combine_kernel<float, float>, dim3(static_cast<unsigned>(tokens)), threads, ws.partial, ws.h.slot_row, route_w, static_cast<float*>(out), hidden, top_k, accumulate);
   } else if (rows_bf16) {
     // hidden is a multiple of 64 (checked above): whole 16-byte pieces (32.8 -> 27.9 us at the prefill shape against
     // 8-byte accesses with one row in flight)
     const int t8 = hidden / 8 >= 256 ? 256 : 128;
-    moe_combine_bf16x8_kernel<<<static_cast<unsigned>(tokens), t8, 0, stream>>>(
+    return combine(
+        moe_combine_bf16x8_kernel, dim3(static_cast<unsigned>(tokens)), t8,
         reinterpret_cast<const __nv_bfloat16*>(ws.partial), ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out),
         hidden, top_k, accumulate);
   } else {
-    moe_combine_kernel<__nv_bfloat16, float><<<static_cast<unsigned>(tokens), threads, 0, stream>>>(
-        ws.partial, ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out), hidden, top_k, accumulate);
+    return combine(
+        moe_combine_kernel<__nv_bfloat16, float>, dim3(static_cast<unsigned>(tokens)), threads, ws.partial, ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out), hidden, top_k, accumulate);
   }
-  return check_cuda(cudaGetLastError(), "moe_combine_kernel launch");
 }
 
 }  // namespace b200fp4
