@@ -121,6 +121,13 @@ struct Pair16<__half> {
 template <typename T>
 __device__ __forceinline__ uint64_t pair16_to_f32x2(uint32_t u);
 
+template <typename T>
+__device__ __forceinline__ T to_out(float v);
+template <>
+__device__ __forceinline__ __nv_bfloat16 to_out<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <>
+__device__ __forceinline__ __half to_out<__half>(float v) { return __float2half_rn(v); }
+
 // ---------------------------------------------------------------------------
 // packed f32x2 arithmetic (sm_100): two IEEE round-to-nearest f32 operations per instruction,
 // operands are register pairs viewed as one 64-bit value {lo, hi}

@@ -10,6 +10,7 @@
 
 #include "gemm2cta_kernel.cuh"
 #include "gemm_kernel.cuh"
+#include "gemm_stream_kernel.cuh"
 
 namespace b200fp4 {
 
@@ -251,16 +252,42 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
                     "nvfp4_gemm_kernel launch");
 }
 
+template <typename OutT, int kFlavour>
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsa, const CUtensorMap& tsb,
+                const GemmParams& p, const EpilogueStore<OutT>& epi, cudaStream_t stream) {
+  auto kern = nvfp4_gemm_pair_kernel<EpilogueStore<OutT>, kFlavour>;
+  static std::atomic<bool> configured[kMaxDevices];
+  int rc = configure_smem_once(configured, kern, static_cast<int>(kPairSmemBytes));
+  if (rc) return rc;
+  const int pairs = std::min(sm_count_of_current_device() / 2, p.num_m_blocks * p.num_n_blocks);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.blockDim = dim3(kPairThreads, 1, 1);
+  cfg.dynamicSmemBytes = kPairSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, p, epi), "nvfp4_gemm_pair_kernel launch");
+}
+
 // CTA-pair variant: 256 x 256 tiles on 2-CTA clusters
 template <typename OutT>
 int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha, int m,
-                    int n, int k, cudaStream_t stream) {
+                    int n, int k, int sf_vec, int fmt8, cudaStream_t stream) {
   CUtensorMap ta, tb, tsa, tsb;
-  int rc = make_operand_map(&ta, a, m, k, 0);
+  const int k_nibbles = fmt8 >= 0 ? 2 * k : k;
+  int rc = make_operand_map(&ta, a, m, k_nibbles, 0);
   if (rc) return rc;
-  rc = make_operand_map(&tb, b, n, k, 1);
+  rc = make_operand_map(&tb, b, n, k_nibbles, 1);
   if (rc) return rc;
-  const int64_t rk = (k + 63) / 64;
+  const int64_t rk = sf_vec == 32 ? (k + 127) / 128 : (k + 63) / 64;
   rc = make_sf_map(&tsa, sfa, static_cast<int64_t>((m + 127) / 128) * rk * 512);
   if (rc) return rc;
   rc = make_sf_map(&tsb, sfb, static_cast<int64_t>((n + 127) / 128) * rk * 512);
@@ -269,36 +296,20 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   p.m_rows = m;
   p.n_cols = n;
   p.k = k;
-  p.k_bytes = k / 2;
+  p.k_bytes = fmt8 >= 0 ? k : k / 2;
+  p.sf_block32 = fmt8 >= 0 ? 2 : (sf_vec == 32 ? 1 : 0);
+  p.a_fmt8 = fmt8 >= 0 ? (fmt8 & 1) : 0;
+  p.b_fmt8 = fmt8 >= 0 ? (fmt8 >> 1) : 0;
   p.rk = static_cast<int>(rk);
-  p.num_k_tiles = (k + kBlockK - 1) / kBlockK;
+  p.num_k_tiles = (p.k_bytes + 127) / 128;
   p.num_m_blocks = (m + 255) / 256;
   p.num_n_blocks = (n + 255) / 256;
   rc = device_status_word(&p.status);
   if (rc) return rc;
   EpilogueStore<OutT> epi{static_cast<OutT*>(c), n, alpha, 0};
-  auto kern = nvfp4_gemm_pair_kernel<EpilogueStore<OutT>>;
-  static std::atomic<bool> configured[kMaxDevices];
-  rc = configure_smem_once(configured, kern, static_cast<int>(kPairSmemBytes));
-  if (rc) return rc;
-  int pairs = sm_count_of_current_device() / 2;
-  const int tiles = p.num_m_blocks * p.num_n_blocks;
-  if (pairs > tiles) pairs = tiles;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
-  cfg.blockDim = dim3(kPairThreads, 1, 1);
-  cfg.dynamicSmemBytes = kPairSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, p, epi), "nvfp4_gemm_pair_kernel launch");
+  if (p.sf_block32 == 2) return launch_pair<OutT, 2>(ta, tb, tsa, tsb, p, epi, stream);
+  if (p.sf_block32 == 1) return launch_pair<OutT, 1>(ta, tb, tsa, tsb, p, epi, stream);
+  return launch_pair<OutT, 0>(ta, tb, tsa, tsb, p, epi, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -382,6 +393,65 @@ int gemm_dense_splitk(const void* a, const void* b, const void* sfa, const void*
                     "splitk_reduce_kernel launch");
 }
 
+// Few output tiles: the streaming kernel (gemm_stream_kernel.cuh) with `tok` rows of A per tile and `splits` CTAs per tile
+template <int kTok, typename OutT>
+int launch_stream(const CUtensorMap& tw, const CUtensorMap& tx, const GemmParams& p, OutT* c, const float* alpha,
+                  cudaStream_t stream) {
+  auto kern = nvfp4_gemm_stream_kernel<kTok, OutT>;
+  constexpr StreamLayout L = stream_layout(kTok);
+  static std::atomic<bool> configured[kMaxDevices];
+  int rc = configure_smem_once(configured, kern, static_cast<int>(L.total));
+  if (rc) return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.num_n_blocks) * p.k_splits, static_cast<unsigned>(p.num_m_blocks), 1);
+  cfg.blockDim = dim3(kStreamThreads, 1, 1);
+  cfg.dynamicSmemBytes = L.total;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.k_splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, tw, tx, p, c, alpha), "nvfp4_gemm_stream_kernel launch");
+}
+
+template <typename OutT>
+int gemm_dense_stream(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha, int m,
+                      int n, int k, int tok, int splits, int sf_vec, int fmt8, cudaStream_t stream) {
+  CUtensorMap tw, tx;
+  const int k_nibbles = fmt8 >= 0 ? 2 * k : k;
+  int rc = make_operand_map(&tw, b, n, k_nibbles, 1);
+  if (rc) return rc;
+  rc = make_operand_map(&tx, a, m, k_nibbles, 0, tok);
+  if (rc) return rc;
+  GemmParams p{};
+  p.sfa = static_cast<const uint8_t*>(sfa);
+  p.sfb = static_cast<const uint8_t*>(sfb);
+  p.m_rows = m;
+  p.n_cols = n;
+  p.k = k;
+  p.k_bytes = fmt8 >= 0 ? k : k / 2;
+  p.sf_block32 = fmt8 >= 0 ? 2 : (sf_vec == 32 ? 1 : 0);
+  p.a_fmt8 = fmt8 >= 0 ? (fmt8 & 1) : 0;
+  p.b_fmt8 = fmt8 >= 0 ? (fmt8 >> 1) : 0;
+  p.rk = sf_vec == 32 ? (k + 127) / 128 : (k + 63) / 64;
+  p.num_k_tiles = (p.k_bytes + 127) / 128;
+  p.num_n_blocks = (n + 127) / 128;
+  p.num_m_blocks = (m + tok - 1) / tok;
+  p.k_splits = splits;
+  rc = device_status_word(&p.status);
+  if (rc) return rc;
+  OutT* out = static_cast<OutT*>(c);
+  if (tok == 16) return launch_stream<16>(tw, tx, p, out, alpha, stream);
+  if (tok == 32) return launch_stream<32>(tw, tx, p, out, alpha, stream);
+  if (tok == 64) return launch_stream<64>(tw, tx, p, out, alpha, stream);
+  return launch_stream<128>(tw, tx, p, out, alpha, stream);
+}
+
 // ---------------------------------------------------------------------------
 // dense GEMM: C[l][m][n] = alpha * A[l][m][k] . B[l][n][k]^T
 // ---------------------------------------------------------------------------
@@ -389,7 +459,9 @@ template <typename OutT>
 int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha, int m,
                      int n, int k, int tile_n, int sf_vec, int fmt8, cudaStream_t stream) {
   // fmt8 < 0: e2m1 operands; else MXFP8 with operand formats a = fmt8 & 1, b = fmt8 >> 1 (0 e4m3, 1 e5m2)
-  if (tile_n == 512) return gemm_dense_pair<OutT>(a, b, sfa, sfb, c, alpha, m, n, k, stream);
+  if (tile_n >= 1000)
+    return gemm_dense_stream<OutT>(a, b, sfa, sfb, c, alpha, m, n, k, tile_n % 1000, tile_n / 1000, sf_vec, fmt8, stream);
+  if (tile_n == 512) return gemm_dense_pair<OutT>(a, b, sfa, sfb, c, alpha, m, n, k, sf_vec, fmt8, stream);
   CUtensorMap ta, tb;
   const int k_nibbles = fmt8 >= 0 ? 2 * k : k;           // operand maps count 4-bit units
   int rc = make_operand_map(&ta, a, m, k_nibbles, 0);
@@ -432,6 +504,50 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
   return launch_gemm<128, false>(ta, tb, tc, p, epi, p.num_m_blocks * p.num_n_blocks, stream);
 }
 
+// ---------------------------------------------------------------------------
+// Which kernel: the least estimated time.  Times of the variants over 1 <= m <= 8192 and n, k from 1024 to 8192 (launches
+// back to back, operands larger than L2) follow, within 10 to 15 %,
+//
+//   one CTA or pair per tile:  base + waves * k_steps * step      waves = ceil(tiles / SMs or pairs)
+//   streaming kernel:          base + k_steps / splits * step + bytes of B / 6.5 TB/s      (one wave, two CTAs per SM)
+//
+// base: launch, pipeline fill and the last tile's epilogue; step: one 256-wide (128 bytes) K step of a stage, which grows
+// with the bytes a stage brings in.  Where the lines cross:
+//   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 64, n = 2048, k = 7168: 12.5 against 7.4
+//   m = 512, n = k = 4096: 128-wide tiles 10.2 us, 64-wide 15.2; m = 1024: 256-wide pairs 12.9, 128-wide 16.3
+//   m = 2048, n = 2048, k = 7168: pairs 16.8 us, 128-wide 24.5
+// Returns a tile_n code.
+// ---------------------------------------------------------------------------
+int choose_tile(int m, int n, int k_bytes, int sms) {
+  const int64_t mb = (m + 127) / 128;
+  const int kt = (k_bytes + 127) / 128;
+  auto blocks = [](int v, int b) { return static_cast<int64_t>((v + b - 1) / b); };
+  auto waves = [](int64_t tiles, int slots) { return static_cast<double>((tiles + slots - 1) / slots); };
+  int best = 64;
+  double best_us = 3.4 + waves(mb * blocks(n, 64), sms) * kt * 0.345;
+  auto consider = [&](int code, double us) {
+    if (us < best_us) best = code, best_us = us;
+  };
+  consider(128, 4.3 + waves(mb * blocks(n, 128), sms) * kt * 0.375);
+  consider(256, 5.0 + waves(mb * blocks(n, 256), sms) * kt * 0.50);
+  consider(512, 5.6 + waves(blocks(m, 256) * blocks(n, 256), sms / 2) * kt * 0.43);
+  const int tok = m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128));
+  for (int t = tok; t >= 32 || t == tok; t /= 2) {          // narrower tiles read B again, but spread over more SMs
+    const double base = t <= 16 ? 3.9 : (t <= 32 ? 4.3 : (t <= 64 ? 5.2 : 6.6));
+    const double step = t <= 32 ? 0.32 : (t <= 64 ? 0.38 : 0.48);
+    const int64_t tiles = blocks(m, t) * blocks(n, 128);
+    for (int s = 1; s <= 8; s *= 2) {
+      const int steps = (kt + s - 1) / s;
+      // clusters of eight only while every CTA has an SM of its own (two to an SM leave the last ones waiting: m = 281,
+      // n = 1536, k = 5888 took 19.0 instead of 11.5 us)
+      if (4 * s > t || tiles * s > (s == 8 ? sms : 2 * sms) || s > kt) continue;
+      consider(1000 * s + t, base + steps * step + (tiles * s > sms ? 0.8 : 0.0) +
+                                 static_cast<double>(n) * k_bytes * blocks(m, t) / 6.5e6);
+    }
+  }
+  return best;
+}
+
 // workspace: optional f32 scratch of gemm_workspace_bytes(m, n, k) bytes; with it, problems with few output tiles
 // and a long reduction run split-K (tile_n 0 only).  Without it they run unsplit.
 // sf_vec: 16 = NVFP4 (e4m3 scale per 16 elements), 32 = MXFP4 (ue8m0 scale per 32 elements; single-CTA tiles only)
@@ -440,7 +556,6 @@ int gemm_dense(const void* a, const void* b, const void* sfa, const void* sfb, v
                cudaStream_t stream) {
   if (sf_vec != 16 && sf_vec != 32) return fail(kUnsupported, "sf_vec=%d (16 = NVFP4, 32 = MXFP4 / MXFP8)", sf_vec);
   if (fmt8 >= 0 && (sf_vec != 32 || fmt8 > 3)) return fail(kUnsupported, "8-bit operands take ue8m0 scales per 32 elements");
-  if (sf_vec == 32 && tile_n == 512) return fail(kUnsupported, "the MX flavours run on single-CTA tiles (tile_n 0, 64, 128, 256)");
   if (sf_vec == 32) workspace = nullptr;
   if (a == nullptr || b == nullptr || sfa == nullptr || sfb == nullptr || c == nullptr)
     return fail(kInvalidArgument, "null pointer argument");
@@ -454,8 +569,14 @@ int gemm_dense(const void* a, const void* b, const void* sfa, const void* sfb, v
        reinterpret_cast<uintptr_t>(sfb) | reinterpret_cast<uintptr_t>(c)) & 15)
     return fail(kInvalidArgument, "Invalid tensor alignment: pointers must be 16-byte aligned");
   if (c_dtype < 0 || c_dtype > 2) return fail(kUnsupported, "c_dtype code %d (0 fp16, 1 bf16, 2 f32)", c_dtype);
-  if (tile_n != 0 && tile_n != 64 && tile_n != 128 && tile_n != 256 && tile_n != 512)
-    return fail(kInvalidArgument, "tile_n must be 0, 64, 128, 256 or 512 (512 = 256 x 256 tiles on CTA pairs)");
+  if (tile_n >= 1000) {
+    const int tok = tile_n % 1000, s = tile_n / 1000, k_tiles = ((fmt8 >= 0 ? k : k / 2) + 127) / 128;
+    if ((tok != 16 && tok != 32 && tok != 64 && tok != 128) || (s != 1 && s != 2 && s != 4 && s != 8) || (tok == 16 && m > 16) || 4 * s > tok ||
+        s > k_tiles)
+      return fail(kInvalidArgument, "tile_n=%d: 1000 * splits + rows, splits 1, 2, 4 or 8 (at most one per K step), rows 16 (m <= 16), 32, 64 or 128", tile_n);
+  } else if (tile_n != 0 && tile_n != 64 && tile_n != 128 && tile_n != 256 && tile_n != 512) {
+    return fail(kInvalidArgument, "tile_n must be 0, 64, 128, 256, 512 (256 x 256 tiles on CTA pairs) or 1000 * splits + rows");
+  }
   int splits = 1;
   if (tile_n == 0 && workspace != nullptr) {
     splits = splitk_slices(m, n, k);
@@ -464,17 +585,7 @@ int gemm_dense(const void* a, const void* b, const void* sfa, const void* sfb, v
       return fail(kInvalidArgument, "split-K workspace must hold %zu bytes, 16-byte aligned",
                   static_cast<size_t>(splits) * m * n * sizeof(float));
   }
-  if (tile_n == 0) {
-    // wide tiles halve the operand traffic per flop; keep narrow ones while they are needed to fill the SMs
-    const int sms = sm_count_of_current_device();
-    const int64_t m_blocks = (m + 127) / 128;
-    static const bool no_pairs = getenv("B200FP4_NO_PAIRS") != nullptr;
-    // a full wave of 256 x 256 tiles on CTA pairs: each CTA fills 38 KB per K step instead of 54 KB
-    if (!no_pairs && sf_vec == 16 && fmt8 < 0 && ((m + 255) / 256) * static_cast<int64_t>((n + 255) / 256) >= sms / 2 && k >= 1024) tile_n = 512;
-    else if (m_blocks * ((n + 255) / 256) >= sms) tile_n = 256;
-    else if (m_blocks * ((n + 127) / 128) >= sms) tile_n = 128;
-    else tile_n = 64;            // few rows (weight streaming): narrow tiles put more SMs on the stream of B
-  }
+  if (tile_n == 0) tile_n = choose_tile(m, n, fmt8 >= 0 ? k : k / 2, sm_count_of_current_device());
   const int64_t m_tiles = (m + 127) / 128, n_tiles = (n + 127) / 128, rk = sf_vec == 32 ? (k + 127) / 128 : (k + 63) / 64;
   const size_t c_elem = c_dtype == 2 ? 4 : 2;
   for (int i = 0; i < l; ++i) {

@@ -36,7 +36,8 @@ constexpr uint32_t kPairStageBytes = 16384 + 16384 + 2048 + 4096;    // A, B hal
 constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + 1024 + 256;
 constexpr int kPairThreads = 64 + 8 * 32 + 128;     // TMA, MMA, 8 epilogue warps, 4 scale-slab movers
 
-template <typename Epilogue>
+// kFlavour: GemmParams::sf_block32 (0 NVFP4, 1 MXFP4, 2 MXFP8)
+template <typename Epilogue, int kFlavour>
 __global__ void __launch_bounds__(kPairThreads, 1)
 nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
@@ -104,6 +105,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     if (lane == 0) {
       PipeState st;
       bool ok = true;
+      const int tps = 4 >> p.sf_block32;                 // 512-byte scale tiles per stage: 4, 2 or 1
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const int m2 = tile % p.num_m_blocks;
         const int n_blk = tile / p.num_m_blocks;
@@ -123,10 +125,11 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           // while the operand tiles are still on their way
           const uint32_t sbar = sf_loaded_bar(st.stage);
           ptx::mbar_expect_tx(sbar, kSfaBytes + 4096);
-          ptx::tma_load_2d(ssfa, &tmap_sfa, 0, (m_tile * p.rk + 4 * kt) * 2, sbar);
+          // a box is four 512-byte scale tiles, whatever the flavour uses of them; rows past the end read as zero
+          ptx::tma_load_2d(ssfa, &tmap_sfa, 0, (m_tile * p.rk + tps * kt) * 2, sbar);
 #pragma unroll
           for (int i = 0; i < 2; ++i)
-            ptx::tma_load_2d(ssfb + i * 2048, &tmap_sfb, 0, ((n_blk * 2 + i) * p.rk + 4 * kt) * 2, sbar);
+            ptx::tma_load_2d(ssfb + i * 2048, &tmap_sfb, 0, ((n_blk * 2 + i) * p.rk + tps * kt) * 2, sbar);
           if (rank == 0) ptx::mbar_expect_tx(full_bar(st.stage), 2 * (kABytes + kBBytes));
           ptx::tma2_load_2d(sa, &tmap_a, kt * 128, m_tile * 128, bar);
           ptx::tma2_load_3d(sb, &tmap_b, kt * 128, n_blk * 256 + static_cast<int>(rank) * 128, 0, bar);
@@ -175,11 +178,29 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           const uint32_t sfb_t = sfa_t + 16;
           const int kblocks = kt + 1 == p.num_k_tiles ? last_kblocks : 4;
           if (ptx::elect_one()) {
-            ptx::mma2_mxf4nvf4(tmem_base, da, db, kIdesc, sfa_t, sfb_t, kt != 0 ? 1u : 0u);
+            if constexpr (kFlavour == 2) {               // one scale tile per stage, instruction kb reads byte kb
 #pragma unroll
-            for (int kb = 1; kb < 4; ++kb) {
-              if (kb < kblocks)
-                ptx::mma2_mxf4nvf4(tmem_base, da + 2 * kb, db + 2 * kb, kIdesc, sfa_t + 4 * kb, sfb_t + 8 * kb, 1u);
+              for (int kb = 0; kb < 4; ++kb) {
+                if (kb < kblocks)
+                  ptx::mma2_mxf8_block32(tmem_base, da + 2 * kb, db + 2 * kb,
+                                         ptx::idesc_m256(ptx::idesc_mxf8_block32(kBlockN, p.a_fmt8, p.b_fmt8, kb)), sfa_t, sfb_t,
+                                         (kt != 0 || kb != 0) ? 1u : 0u);
+              }
+            } else if constexpr (kFlavour == 1) {        // a scale tile serves two instructions
+#pragma unroll
+              for (int kb = 0; kb < 4; ++kb) {
+                if (kb < kblocks)
+                  ptx::mma2_mxf4_block32(tmem_base, da + 2 * kb, db + 2 * kb,
+                                         ptx::idesc_m256(ptx::idesc_mxf4_block32(kBlockN, (kb & 1) * 2)), sfa_t + 4 * (kb >> 1),
+                                         sfb_t + 8 * (kb >> 1), (kt != 0 || kb != 0) ? 1u : 0u);
+              }
+            } else {
+              ptx::mma2_mxf4nvf4(tmem_base, da, db, kIdesc, sfa_t, sfb_t, kt != 0 ? 1u : 0u);
+#pragma unroll
+              for (int kb = 1; kb < 4; ++kb) {
+                if (kb < kblocks)
+                  ptx::mma2_mxf4nvf4(tmem_base, da + 2 * kb, db + 2 * kb, kIdesc, sfa_t + 4 * kb, sfb_t + 8 * kb, 1u);
+              }
             }
             ptx::tc2_commit_mcast(empty_bar(st.stage), 3);      // frees the stage in both CTAs
           }

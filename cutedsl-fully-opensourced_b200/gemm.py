@@ -69,11 +69,11 @@ def nvfp4_gemm(a: torch.Tensor, b: torch.Tensor, sfa: torch.Tensor, sfb: torch.T
     """C = alpha * (A*SFA) @ (B*SFB)^T with f32 accumulation on the tensor cores.
 
     ``sf_vec_size`` 16: NVFP4 (one e4m3 scale byte per 16 K-elements); 32: MXFP4 (one ue8m0 scale byte per 32
-    K-elements, same 128x4 tiles; single-CTA tile variants only).
+    K-elements, same 128x4 tiles).
 
     ``workspace=`` (uint8, ``gemm_workspace_bytes(m, n, k)`` bytes) opts a problem with few output tiles and a long
-    reduction into split-K.  It is off by default: at M = 128, N = K = 8192 the split kernel takes the same 15 us as
-    the unsplit 64-wide tiles and the reduction adds 4."""
+    reduction into split-K through global memory.  It is off by default: such problems already take a kernel that deals
+    the K steps to a cluster of CTAs."""
     return _lib.native.nvfp4_gemm(a, b, sfa, sfb, alpha, out, out_dtype, tile_n, workspace, sf_vec_size)
 
 
@@ -82,7 +82,7 @@ def mxfp8_gemm(a: torch.Tensor, b: torch.Tensor, sfa: torch.Tensor, sfb: torch.T
                out_dtype: torch.dtype = torch.bfloat16, tile_n: int = 0) -> torch.Tensor:
     """MXFP8 flavour: A ``[M, K]`` and B ``[N, K]`` are ``torch.float8_e4m3fn`` or ``torch.float8_e5m2`` (each
     operand its own format), scale factors ue8m0 bytes, one per 32 K-elements, in the 128x4 tiled layout
-    (``swizzled_sf_numel(rows, ceil(K / 32))`` bytes).  Same kernel family as ``nvfp4_gemm``; single-CTA tiles."""
+    (``swizzled_sf_numel(rows, ceil(K / 32))`` bytes).  Same kernel family as ``nvfp4_gemm``."""
     return _lib.native.mxfp8_gemm(a, b, sfa, sfb, alpha, out, out_dtype, tile_n)
 
 

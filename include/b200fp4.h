@@ -63,7 +63,9 @@ int b200fp4_add_rmsnorm_fp4quant(const void* x, void* residual, const void* weig
  * SFA / SFB: e4m3 bytes, one per 16 K-elements, in 128x4 tiles [l][ceil(rows/128)][ceil(k/64)][32][4][4]
  * (padding bytes zero).  C row-major, c_dtype 0 = fp16, 1 = bf16, 2 = f32; f32 accumulation.
  * alpha: one f32 in device memory, or NULL for 1.  tile_n: 0 = choose (by problem size), or force one of
- * 64 / 128 / 256 (output columns per single-CTA tile) or 512 (256 x 256 tiles on CTA pairs).
+ * 64 / 128 / 256 (output columns per single-CTA tile), 512 (256 x 256 tiles on CTA pairs) or
+ * 1000 * splits + rows (the streaming kernel for few tiles: 16, 32, 64 or 128 rows of A against 128 of B per tile, the
+ * reduction dealt to a cluster of 1, 2, 4 or 8 CTAs; at least four rows per CTA, 16 rows only for m <= 16).
  * Stands in for Sm120BlockScaledGemmKernel.__call__ and its kernel:
  *   third_party/cutlass/examples/python/CuTeDSL/cute/blackwell_geforce/kernel/blockscaled_gemm/
  *   dense_blockscaled_gemm_persistent_cooperative.py:281-439 (host), :443-1185 (device),

@@ -341,3 +341,40 @@ def test_mxfp8_through_the_demo_entry(b200):
                    c_major="n", tile_shape_mnk=(128, 128, 128), epi_tile=(128, 128), tolerance=0.1,
                    warmup_iterations=0, iterations=1, skip_ref_check=False)
         assert us > 0
+
+
+@pytest.mark.parametrize("m,n,k,tile_n", [(1, 128, 256, 1016), (16, 264, 1056, 4016), (7, 520, 2304, 4016), (32, 256, 512, 1032),
+                                          (33, 136, 1184, 2032), (31, 1024, 4096, 8032), (60, 264, 1184, 1064), (70, 384, 2080, 4064),
+                                          (64, 136, 4096, 8064), (128, 128, 256, 1128), (300, 520, 2080, 2128), (100, 136, 8192, 8128)])
+def test_streaming_kernel(b200, m, n, k, tile_n):
+    """Weights on the 128-row side, K steps dealt to a cluster: ragged rows, columns and last K step, row tiles that start
+    inside a 128-row scale tile, every split; NVFP4 with integer-valued operands exact, MXFP4 and MXFP8 against the oracle."""
+    ac, sfa, bc, sfb = O.integer_gemm_operands(m, n, k, seed=m + n + k)
+    a, b, sa, sb = _dev_operands(ac, sfa, bc, sfb)
+    for out_dtype in (torch.float32, torch.bfloat16, torch.float16):
+        c = b200.nvfp4_gemm(a, b, sa, sb, alpha=torch.tensor([0.5], device="cuda"), out_dtype=out_dtype, tile_n=tile_n)
+        assert torch.equal(c.cpu().float(), O.gemm_nvfp4_ref(ac, sfa, bc, sfb, alpha=0.5).to(out_dtype).float())
+    _mx_flavours(b200, m, n, k, tile_n)
+    _check_status(b200)
+
+
+@pytest.mark.parametrize("m,n,k", [(256, 256, 256), (200, 264, 1056), (300, 520, 2080)])
+def test_mx_flavours_on_cta_pairs(b200, m, n, k):
+    _mx_flavours(b200, m, n, k, 512)
+    _check_status(b200)
+
+
+def _mx_flavours(b200, m, n, k, tile_n):
+    rng = np.random.default_rng(m + n + k)
+    kb = -(-k // 32)
+    sfa, sfb = (rng.integers(122, 131, size=(r, kb), dtype=np.uint8) for r in (m, n))
+    ac, bc = (rng.integers(0, 16, size=(r, k), dtype=np.uint8) for r in (m, n))
+    a, b, sa, sb = _dev_operands(ac, sfa, bc, sfb)
+    ab, bb = (rng.integers(0, 2, size=(r, k), dtype=np.uint8) << 7 | rng.integers(24, 80, size=(r, k), dtype=np.uint8) for r in (m, n))
+    got4 = b200.nvfp4_gemm(a, b, sa, sb, out_dtype=torch.float32, tile_n=tile_n, sf_vec_size=32)
+    got8 = b200.mxfp8_gemm(torch.from_numpy(ab).cuda().view(torch.float8_e4m3fn), torch.from_numpy(bb).cuda().view(torch.float8_e5m2),
+                           sa, sb, out_dtype=torch.float32, tile_n=tile_n)
+    for got, ref in ((got4, O.gemm_nvfp4_ref(ac, sfa, bc, sfb, alpha=1.0, sf_vec=32)),
+                     (got8, O.gemm_mxfp8_ref(ab, sfa, bb, sfb, alpha=1.0, a_e5m2=False, b_e5m2=True))):
+        err = torch.linalg.vector_norm(got.cpu() - ref) / torch.linalg.vector_norm(ref)
+        assert err <= 1e-5, float(err)
