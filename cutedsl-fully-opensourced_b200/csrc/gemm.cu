@@ -11,6 +11,7 @@
 #include "gemm2cta_kernel.cuh"
 #include "gemm_kernel.cuh"
 #include "gemm_stream_kernel.cuh"
+#include "moe_stream_kernel.cuh"
 
 namespace b200fp4 {
 
@@ -127,17 +128,17 @@ int make_sf_map(CUtensorMap* map, const void* base, int64_t total_bytes) {
   return kOk;
 }
 
-// Row-major scale factors of A: [rows][k / 16] bytes, `pitch` bytes between rows; boxes of 128 rows x 16 bytes (the
+// Row-major scale factors of A: [rows][k / 16] bytes, `pitch` bytes between rows; boxes of box_rows rows x 16 bytes (the
 // scale bytes of one 256-wide K step).  Columns beyond k / 16 read as zero.
-int make_sfa_rows_map(CUtensorMap* map, const void* base, int64_t rows, int k, int64_t pitch) {
+int make_sfa_rows_map(CUtensorMap* map, const void* base, int64_t rows, int k, int64_t pitch, int box_rows = 128) {
   const MapKey key{4, reinterpret_cast<uint64_t>(base), static_cast<uint64_t>(rows), static_cast<uint64_t>(k),
-                   static_cast<uint64_t>(pitch), 0};
+                   static_cast<uint64_t>(pitch), static_cast<uint64_t>(box_rows)};
   if (cached_map(key, map)) return kOk;
   EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr) return fail(kCudaError, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(k / 16), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch)};
-  cuuint32_t box[2] = {16, 128};
+  cuuint32_t box[2] = {16, static_cast<cuuint32_t>(box_rows)};
   cuuint32_t elem[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -824,6 +825,86 @@ int gemm_moe_fc2(const void* act_codes, const void* act_sf, const void* w2, cons
   return gemm_moe_fc2_typed(act_codes, act_sf, w2, w2_sf, static_cast<float*>(partial), w2_alpha, num_m_blocks_dev,
                             m_block_expert, m_block_rows, max_m_blocks, hidden, inter, experts, few_rows, status,
                             stream, early_b);
+}
+
+// ---------------------------------------------------------------------------
+// the grouped GEMMs with few rows per expert (moe_stream_kernel.cuh): blocks of at most `tok` rows, `tok` apart.  small:
+// the block tables are older than the kernel before FC1.
+// ---------------------------------------------------------------------------
+template <int kTok, typename Epi>
+int launch_moe_stream(const void* x, const void* x_sf, int x_sf_pitch, const void* w, const void* w_sf, int w_rows, int k,
+                      int gate_row_offset, int num_n_blocks, const int* num_blocks_dev, const int* block_expert,
+                      const int* block_rows, int max_blocks, int experts, int early_b, int trigger, int* status, const Epi& epi,
+                      cudaStream_t stream) {
+  CUtensorMap tw, tx, tsf;
+  const int64_t rows = static_cast<int64_t>(max_blocks) * kTok;
+  int rc = make_operand_map(&tw, w, w_rows, k, experts);
+  if (rc) return rc;
+  rc = make_operand_map(&tx, x, rows, k, 0, kTok);
+  if (rc) return rc;
+  rc = make_sfa_rows_map(&tsf, x_sf, rows, k, x_sf_pitch, kTok);
+  if (rc) return rc;
+  GemmParams p{};
+  p.sfb = static_cast<const uint8_t*>(w_sf);
+  p.k = k;
+  p.k_bytes = k / 2;
+  p.rk = (k + 63) / 64;
+  p.num_k_tiles = (k + kBlockK - 1) / kBlockK;
+  p.num_n_blocks = num_n_blocks;
+  p.b_row_tiles = (w_rows + 127) / 128;
+  p.gate_row_offset = gate_row_offset;
+  p.num_m_blocks_dev = num_blocks_dev;
+  p.num_m_blocks = max_blocks;
+  p.m_block_group = block_expert;
+  p.num_groups = experts;
+  p.m_block_rows = block_rows;
+  p.status = status;
+  p.early_b = early_b;
+  p.early_trigger = trigger;
+  auto kern = moe_stream_gemm_kernel<kTok, Epi>;
+  constexpr MoeStreamLayout L = moe_stream_layout(kTok, Epi::kParkElem);
+  static std::atomic<bool> configured[kMaxDevices];
+  rc = configure_smem_once(configured, kern, static_cast<int>(L.total));
+  if (rc) return rc;
+  const int grid = std::min(sm_count_of_current_device(), max_blocks * num_n_blocks);
+  return check_cuda(launch_dependent(kern, dim3(grid), dim3(kMoeStreamThreads), L.total, stream, tw, tx, tsf, p, epi),
+                    "moe_stream_gemm_kernel launch");
+}
+
+template <int kTok>
+int moe_stream_gemms_tok(const void* xq, const void* xq_sf, int xq_sf_pitch, const void* w1, const void* w1_sf, void* act,
+                         void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
+                         const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
+                         const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
+                         int small, int* status, cudaStream_t stream) {
+  const MoeStreamFc1 e1{static_cast<uint8_t*>(act), static_cast<uint8_t*>(act_sf), w1_alpha, fc2_input_scale, inter, act_sf_pitch};
+  int rc = launch_moe_stream<kTok>(xq, xq_sf, xq_sf_pitch, w1, w1_sf, 2 * inter, hidden, inter, inter / 128, num_blocks_dev,
+                                   block_expert, block_rows, max_blocks, experts, small, small, status, e1, stream);
+  if (rc) return rc;
+  const int n_blocks = (hidden + 255) / 256;
+  if (rows_bf16) {
+    const MoeStreamFc2<__nv_bfloat16> e2{static_cast<__nv_bfloat16*>(partial), w2_alpha, hidden};
+    return launch_moe_stream<kTok>(act, act_sf, act_sf_pitch, w2, w2_sf, hidden, inter, 0, n_blocks, num_blocks_dev,
+                                   block_expert, block_rows, max_blocks, experts, 1, 0, status, e2, stream);
+  }
+  const MoeStreamFc2<float> e2{static_cast<float*>(partial), w2_alpha, hidden};
+  return launch_moe_stream<kTok>(act, act_sf, act_sf_pitch, w2, w2_sf, hidden, inter, 0, n_blocks, num_blocks_dev, block_expert,
+                                 block_rows, max_blocks, experts, 1, 0, status, e2, stream);
+}
+
+int moe_stream_gemms(int tok, const void* xq, const void* xq_sf, int xq_sf_pitch, const void* w1, const void* w1_sf, void* act,
+                     void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
+                     const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
+                     const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
+                     int small, int* status, cudaStream_t stream) {
+  auto run = [&](auto fn) {
+    return fn(xq, xq_sf, xq_sf_pitch, w1, w1_sf, act, act_sf, act_sf_pitch, w2, w2_sf, partial, rows_bf16, w1_alpha, w2_alpha,
+              fc2_input_scale, num_blocks_dev, block_expert, block_rows, max_blocks, hidden, inter, experts, small, status,
+              stream);
+  };
+  if (tok == 16) return run(moe_stream_gemms_tok<16>);
+  if (tok == 32) return run(moe_stream_gemms_tok<32>);
+  return run(moe_stream_gemms_tok<64>);
 }
 
 }  // namespace b200fp4

@@ -17,6 +17,7 @@
 //
 // All intermediate buffers live in a caller-provided workspace.
 #include <algorithm>
+#include <cmath>
 #include <utility>
 
 #include "gemm_kernel.cuh"
@@ -32,6 +33,12 @@ int gemm_moe_fc2(const void* act_codes, const void* act_sf, const void* w2, cons
                  int rows_bf16, const float* w2_alpha, const int* num_m_blocks_dev, const int* m_block_expert,
                  const int* m_block_rows, int max_m_blocks, int hidden, int inter, int experts, int few_rows,
                  int* status, cudaStream_t stream, int early_b = 0);
+
+int moe_stream_gemms(int tok, const void* xq, const void* xq_sf, int xq_sf_pitch, const void* w1, const void* w1_sf, void* act,
+                     void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
+                     const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
+                     const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
+                     int trigger, int* status, cudaStream_t stream);
 
 int sm_count_of_current_device();
 
@@ -125,9 +132,6 @@ __global__ void route_topk_kernel(const float* __restrict__ logits, int* __restr
 // bookkeeping header at the start of the workspace
 // ---------------------------------------------------------------------------
 struct MoeHeader {           // all int32, contiguous
-  int* counts;               // [experts]     rows routed to each local expert
-  int* cursor;               // [experts]     next free row inside the expert's segment
-  int* offsets;              // [experts + 1] first row of each expert's padded segment
   int* num_m_blocks;         // [1]
   int* m_block_expert;       // [max_m_blocks]
   int* m_block_rows;         // [max_m_blocks] rows of the block that hold data (the rest pads it to 128)
@@ -296,16 +300,16 @@ moe_count_kernel(const float* __restrict__ logits, int route_experts, int renorm
   if (threadIdx.x == 0) ctrl[kCtrlTicketCount] = 0;
 }
 
-// place: see the section comment.  rows_per_block: valid rows that a 128-row block may hold (128, or 32 for the
-// few-row GEMM variants).  One warp per token at a time; a lane quantises groups of four adjacent 16-element
+// place: see the section comment.  rows_per_block: valid rows that a block may hold; block_stride: rows from one block's
+// first to the next one's (128 and 128; 32 and 128 for the few-row GEMM variants; both kTok for the streaming GEMMs).  One warp per token at a time; a lane quantises groups of four adjacent 16-element
 // blocks (128 bytes of the token in flight per lane) and writes, per slot, their 32 bytes of codes and their four
 // scale bytes (adjacent in the 128x4 tiles) with one store each.  Dynamic shared memory: 3 * experts_total ints.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
 moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ ids,
                        const int* __restrict__ slot_pos, Exchange ex, int tokens, int hidden, int top_k,
-                       int expert_lo, int experts_total, int max_m_blocks, int rows_per_block, int* slot_row,
-                       int* num_m_blocks, int* m_block_expert, int* m_block_rows, int* ctrl, int* status,
+                       int expert_lo, int experts_total, int max_m_blocks, int rows_per_block, int block_stride,
+                       int* slot_row, int* num_m_blocks, int* m_block_expert, int* m_block_rows, int* ctrl, int* status,
                        const float* __restrict__ weights) {
   extern __shared__ int s_dyn[];
   int* s_base = s_dyn;                       // blocks before expert e (over all experts, in expert order)
@@ -393,8 +397,8 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
       if (e >= 0 && e < experts_total && pos >= 0) {
         d = e / el;
         const int r = s_myoff[e] + pos;
-        row = (s_base[e] - s_base[d * el] + r / rpb) * 128 + r % rpb;
-        if (row >= max_m_blocks * 128) row = -1;
+        row = (s_base[e] - s_base[d * el] + r / rpb) * block_stride + r % rpb;
+        if (row >= max_m_blocks * block_stride) row = -1;
         else reinterpret_cast<int*>(ex.peers.p[d] + ex.row_tag)[row] = (ex.rank << 24) | static_cast<int>(slot);
       }
       s_rows[warp][j] = row;
@@ -441,8 +445,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
 
 // Few slots (<= 1024): count, scan and row assignment in one CTA -- one launch instead of a memset and three
 // kernels, which is most of a decode step's bookkeeping time.  Rows of an expert go to its slots in slot order.
-// rows_per_block: valid rows that a 128-row block may hold.  128 normally; 32 for the few-row GEMM variants, which
-// load only the first 32 rows of every block (an expert with more rows than that simply gets more blocks).
+// rows_per_block, block_stride: as in the place kernel.
 // kRoutePerLane > 0: the router runs here first (one warp per token, the CTA's 32 warps take the tokens in turn;
 // experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
 // step.  0: the ids are inputs.
@@ -450,18 +453,21 @@ template <int kRoutePerLane>
 __global__ void __launch_bounds__(1024)
 moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, int renormalize, int top_k, int* ids,
                          float* weights, int n_slots, int expert_lo, MoeHeader h, int experts, int max_m_blocks,
-                         int max_rows, int rows_per_block) {
-  __shared__ int s_count[1024];
-  __shared__ int s_blocks[1024];
-  __shared__ int s_offset[1024];
-  __shared__ int s_expert[1024];
-  const int t = threadIdx.x;
-  s_count[t] = 0;
+                         int rows_per_block, int block_stride) {
+  __shared__ __align__(16) uint8_t s_cnt[32][1024];      // slots of warp w's 32 that named expert e
+  __shared__ int s_first[1024];                            // expert -> its first block
+  __shared__ int s_ids[1024];
+  __shared__ int s_warp[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int used = (n_slots + 31) >> 5;                    // warps that hold slots
+  {
+    uint4* clear = reinterpret_cast<uint4*>(s_cnt[warp]);
+    if (warp < used) clear[lane] = clear[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+  }
   grid_dependency_wait();
   let_dependents_launch();
   if constexpr (kRoutePerLane > 0) {
-    const int lane = t & 31;
-    for (int token = t >> 5; token * top_k < n_slots; token += 32) {
+    for (int token = warp; token * top_k < n_slots; token += 32) {
       int my_id;
       float my_w;
       route_one_token<kRoutePerLane>(logits + static_cast<int64_t>(token) * route_experts, lane, route_experts, top_k,
@@ -469,41 +475,46 @@ moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, in
       if (lane < top_k) {
         ids[token * top_k + lane] = my_id;
         weights[token * top_k + lane] = my_w;
-        s_blocks[token * top_k + lane] = my_id;          // handed to the slot's thread below
+        s_ids[token * top_k + lane] = my_id;               // handed to the slot's thread below
       }
     }
     __syncthreads();
   }
-  int e = -1, rank_in_expert = 0;
+  int e = -1, rank = 0;
   if (t < n_slots) {
-    e = (kRoutePerLane > 0 ? s_blocks[t] : ids[t]) - expert_lo;
+    e = (kRoutePerLane > 0 ? s_ids[t] : ids[t]) - expert_lo;
     if (e < 0 || e >= experts) e = -1;
   }
-  s_expert[t] = e;
+  __syncwarp();
+  // position of the slot among the slots of its expert, in slot order: earlier lanes of the warp, then earlier warps
+  const uint32_t same = __match_any_sync(0xffffffffu, e);
+  rank = __popc(same & ((1u << lane) - 1u));
+  if (e >= 0 && rank == 0) s_cnt[warp][e] = static_cast<uint8_t>(__popc(same));
   __syncthreads();
-  // position of the slot among the slots of its expert, in slot order: count earlier slots with the same expert
-  if (e >= 0) {
-    atomicAdd(s_count + e, 1);
-    for (int i = 0; i < t; ++i) rank_in_expert += s_expert[i] == e;
-  }
-  __syncthreads();
-  const int count = t < experts ? s_count[t] : 0;
+  if (e >= 0)
+    for (int w = 0; w < warp; ++w) rank += s_cnt[w][e];
+  int count = 0;
+  if (t < experts)
+    for (int w = 0; w < used; ++w) count += s_cnt[w][t];
   const int blocks = (count + rows_per_block - 1) / rows_per_block;
-  s_blocks[t] = blocks;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int add = t >= o ? s_blocks[t - o] : 0;
-    __syncthreads();
-    s_blocks[t] += add;
-    __syncthreads();
+  int incl = blocks;                                       // scan over the experts: lanes, then warps
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
   }
-  const int incl = s_blocks[t];
+  if (lane == 31) s_warp[warp] = incl;
+  __syncthreads();
+  int before = s_warp[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += v;
+  }
+  incl += warp == 0 ? 0 : __shfl_sync(0xffffffffu, before, warp - 1);
   const int excl = incl - blocks;
-  s_offset[t] = excl * 128;
+  s_first[t] = excl;
   if (t < experts) {
-    h.counts[t] = count;
-    h.offsets[t] = excl * 128;
-    h.cursor[t] = count;
     for (int b = 0; b < blocks; ++b) {
       if (excl + b < max_m_blocks) {
         h.m_block_expert[excl + b] = t;
@@ -511,16 +522,13 @@ moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, in
       }
     }
   }
-  if (t == experts - 1) {
-    h.offsets[experts] = incl * 128;
-    *h.num_m_blocks = min(incl, max_m_blocks);
-  }
+  if (t == experts - 1) *h.num_m_blocks = min(incl, max_m_blocks);
   __syncthreads();
   if (t < n_slots) {
     int row = -1;
     if (e >= 0) {
-      row = s_offset[e] + (rank_in_expert / rows_per_block) * 128 + rank_in_expert % rows_per_block;
-      if (row >= max_rows) row = -1;
+      row = (s_first[e] + rank / rows_per_block) * block_stride + rank % rows_per_block;
+      if (row >= max_m_blocks * block_stride) row = -1;
     }
     h.slot_row[t] = row;
   }
@@ -530,7 +538,7 @@ moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, in
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
 moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_row, uint8_t* xq,
-                              uint8_t* xq_sf, int hidden, int top_k) {
+                              uint8_t* xq_sf, int sf_pitch, int hidden, int top_k) {
   __shared__ int s_rows[64];
   const int token = blockIdx.x;
   grid_dependency_wait();
@@ -538,7 +546,6 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __
   if (threadIdx.x < top_k) s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
   __syncthreads();
   const int nchunks = hidden >> 4;
-  const int rk = (nchunks + 3) >> 2;
   for (int chunk = blockIdx.y * kThreads + threadIdx.x; chunk < nchunks; chunk += gridDim.y * kThreads) {
     const U32x8 raw = ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16);
     float v[16];
@@ -553,7 +560,7 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __
       const int row = s_rows[j];
       if (row < 0) continue;
       *reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * (hidden >> 1) + chunk * 8) = make_uint2(lo, hi);
-      xq_sf[sf_swizzled_offset(row, chunk, rk)] = static_cast<uint8_t>(sfb);
+      xq_sf[static_cast<int64_t>(row) * sf_pitch + chunk] = static_cast<uint8_t>(sfb);
     }
   }
 }
@@ -744,23 +751,30 @@ __global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ part
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// With at most 32 tokens (and few enough slots for the single-CTA bookkeeping kernel) the wide GEMM variants keep
-// only 32 rows of A per stage, which buys another stage of weights in flight.  The bookkeeping then fills every
-// 128-row block with at most 32 rows, so an expert that is named more than 32 times (ids may repeat inside a
-// token: the reference's own bench draws them with replacement, tools/perf/bench_flashinfer_b12x.py:70-71)
-// gets several blocks instead of wrong results.
+// With at most 32 tokens in the whole group the expert-parallel GEMMs keep only 32 rows of A per stage, which buys
+// another stage of weights in flight.  Every 128-row block then holds at most 32 rows, so an expert that is named more
+// than 32 times (ids may repeat inside a token: the reference's own bench draws them with replacement,
+// tools/perf/bench_flashinfer_b12x.py:70-71) gets several blocks instead of wrong results.
 inline bool moe_few_rows(int64_t tokens, int top_k) { return tokens <= 32 && tokens * top_k <= 1024; }
 
-// Scale bytes of the FC1 operand.  The general front end writes them as plain rows, sf_row_pitch(hidden) bytes
-// apart (a multiple of 16, as the tensor map wants); the few-slot front end writes 128x4 tiles.  The buffer fits
-// either.  Rows that only pad a 128-row block are never written and never cleared: a row of the accumulator
-// depends on its own row of A and of its scale bytes only, and rows without data are never read back.
-inline int sf_row_pitch(int hidden) { return ((hidden / 16) + 15) / 16 * 16; }
-inline size_t xq_sf_buffer_bytes(int64_t blocks, int hidden) {
-  const size_t tiled = static_cast<size_t>(blocks) * ((hidden + 63) / 64) * 512;
-  const size_t rows = static_cast<size_t>(blocks) * 128 * sf_row_pitch(hidden);
-  return std::max(tiled, rows);
+// Rows per block of the streaming GEMMs (moe_stream_kernel.cuh), 0 = the 128-row kernels.  The narrowest block that an
+// expert with the average number of rows and two standard deviations more still fits (an expert that does not gets a
+// second block, whose weights then come from L2); blocks of 64 up to an average of 60.  Whole steps, us, 128-row kernels /
+// blocks of 16 / 32 / 64, at averages of 4, 16, 32, 56 and 80 rows:
+//   hidden 2048, inter 768, 128 experts    96/78/79/80   103/91/90/91   105/106/95/94   111/152/109/105   117/197/137/126
+//   hidden 4096, inter 3584, 8 experts     56/47/47/48   61/56/52/53    67/67/63/60     76/96/73/69       81/118/89/82
+inline int stream_rows(int64_t tokens, int top_k, int experts) {
+  const int64_t slots = tokens * top_k;
+  const double mean = static_cast<double>(slots) / static_cast<double>(std::min<int64_t>(experts, slots));
+  for (int tok = 16; tok <= 32; tok *= 2)
+    if (mean + 2.0 * std::sqrt(mean) <= tok) return tok;
+  return mean <= 60.0 ? 64 : 0;
 }
+
+// Scale bytes of the FC1 operand (and of FC2's, for the streaming GEMMs): plain rows, sf_row_pitch(columns) bytes apart
+// (a multiple of 16, as the tensor map wants).  Rows that only pad a block are never written and never cleared: a row of
+// the accumulator depends on its own row of A and of its scale bytes only, and rows without data are never read back.
+inline int sf_row_pitch(int columns) { return ((columns / 16) + 15) / 16 * 16; }
 
 struct MoeWorkspace {
   MoeHeader h;
@@ -775,18 +789,18 @@ struct MoeWorkspace {
   uint8_t* act_sf;
   float* partial;
   size_t clear_bytes;      // ctrl + my_counts
-  size_t xq_sf_bytes;
   size_t total;
   int max_m_blocks;
 };
 
-MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int experts, int top_k) {
+// tok: rows per block and from block to block (stream_rows), 0 = 128
+MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int experts, int top_k, int tok) {
   MoeWorkspace w{};
   const int64_t slots = tokens * top_k;
-  // few-row launches (see moe_fused) fill a block with at most 32 rows
-  const int64_t blocks = std::min<int64_t>(experts, slots) + slots / (moe_few_rows(tokens, top_k) ? 32 : 128);
+  const int64_t per_block = tok != 0 ? tok : 128;
+  const int64_t blocks = std::min<int64_t>(experts, slots) + slots / per_block;
   w.max_m_blocks = static_cast<int>(blocks);
-  const int64_t rows = blocks * 128;
+  const int64_t rows = blocks * per_block;
   uint8_t* p = static_cast<uint8_t*>(base);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -794,9 +808,6 @@ MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int expert
     off = align_up(off + bytes, 256);
     return r;
   };
-  w.h.counts = reinterpret_cast<int*>(take(sizeof(int) * experts));
-  w.h.cursor = reinterpret_cast<int*>(take(sizeof(int) * experts));
-  w.h.offsets = reinterpret_cast<int*>(take(sizeof(int) * (experts + 1)));
   w.h.num_m_blocks = reinterpret_cast<int*>(take(sizeof(int)));
   w.h.m_block_expert = reinterpret_cast<int*>(take(sizeof(int) * blocks));
   w.h.m_block_rows = reinterpret_cast<int*>(take(sizeof(int) * blocks));
@@ -807,10 +818,10 @@ MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int expert
   w.counts_all = reinterpret_cast<int*>(take(sizeof(int) * experts));
   w.slot_pos = reinterpret_cast<int*>(take(sizeof(int) * slots));
   w.row_tag = reinterpret_cast<int*>(take(sizeof(int) * rows));
-  w.xq_sf_bytes = xq_sf_buffer_bytes(blocks, hidden);
-  w.xq_sf = take(w.xq_sf_bytes);
+  w.xq_sf = take(static_cast<size_t>(rows) * sf_row_pitch(hidden));
   w.xq = take(static_cast<size_t>(rows) * (hidden / 2));
-  w.act_sf = take(static_cast<size_t>(blocks) * ((inter + 63) / 64) * 512);
+  w.act_sf = take(tok != 0 ? static_cast<size_t>(rows) * sf_row_pitch(inter)
+                           : static_cast<size_t>(blocks) * ((inter + 63) / 64) * 512);
   w.act = take(static_cast<size_t>(rows) * (inter / 2));
   w.partial = reinterpret_cast<float*>(take(static_cast<size_t>(rows) * hidden * sizeof(float)));
   w.total = off;
@@ -850,7 +861,7 @@ int launch_count(const float* logits, int route_experts, int renormalize, const 
 }
 
 int launch_place(const void* x, const int* ids, const int* slot_pos, const Exchange& ex, int tokens, int hidden,
-                 int top_k, int expert_lo, int experts_total, int max_m_blocks, int rows_per_block, int* slot_row,
+                 int top_k, int expert_lo, int experts_total, int max_m_blocks, int rows_per_block, int block_stride, int* slot_row,
                  int* num_m_blocks, int* m_block_expert, int* m_block_rows, int* ctrl, int* status,
                  cudaStream_t stream, const float* weights = nullptr) {
   // eight warps per CTA, one token per warp at a time; enough CTAs that every SM holds several
@@ -859,7 +870,7 @@ int launch_place(const void* x, const int* ids, const int* slot_pos, const Excha
   const cudaError_t err = launch_in_order(
       ex.world, moe_quant_place_kernel<256>, dim3(grid), dim3(256), smem, stream,
       static_cast<const __nv_bfloat16*>(x), ids, slot_pos, ex, tokens, hidden, top_k, expert_lo, experts_total,
-      max_m_blocks, rows_per_block, slot_row, num_m_blocks, m_block_expert, m_block_rows, ctrl, status, weights);
+      max_m_blocks, rows_per_block, block_stride, slot_row, num_m_blocks, m_block_expert, m_block_rows, ctrl, status, weights);
   return check_cuda(err, "moe_quant_place_kernel launch");
 }
 
@@ -896,7 +907,9 @@ int route_topk(const float* logits, int* ids, float* weights, int tokens, int ex
 }
 
 size_t moe_workspace_bytes(int64_t tokens, int hidden, int inter, int experts, int top_k) {
-  return carve(nullptr, tokens, hidden, inter, experts, top_k).total;
+  // enough for 128-row blocks whatever the number of rows: one workspace then serves every smaller batch as well
+  return std::max(carve(nullptr, tokens, hidden, inter, experts, top_k, 0).total,
+                  carve(nullptr, tokens, hidden, inter, experts, top_k, stream_rows(tokens, top_k, experts)).total);
 }
 
 // status: device word that the GEMM kernels OR failure bits into.
@@ -929,12 +942,12 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     if (rc) return rc;
   }
   if (tokens == 0) return kOk;
-  MoeWorkspace ws = carve(workspace, tokens, hidden, inter, experts, top_k);
+  const int tok = stream_rows(tokens, top_k, experts);
+  const int per_block = tok != 0 ? tok : 128;
+  MoeWorkspace ws = carve(workspace, tokens, hidden, inter, experts, top_k, tok);
   if (workspace_bytes < ws.total)
     return fail(kInvalidArgument, "workspace holds %zu bytes, %zu needed", workspace_bytes, ws.total);
   const int slots = static_cast<int>(tokens * top_k);
-  const int max_rows = ws.max_m_blocks * 128;
-  const int few_rows = moe_few_rows(tokens, top_k);
 
   if (slots <= 1024) {
     // rows that only pad a block keep whatever their scale bytes held: a row of the accumulator depends on its own row of A
@@ -944,7 +957,7 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
 #define B200_PREPARE(PL)                                                                                          \
   B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL>, dim3(1), dim3(1024), 0, stream, logits, route_experts,   \
                              renormalize, top_k, ids, route_w, slots, expert_lo, ws.h, experts, ws.max_m_blocks,    \
-                             max_rows, few_rows ? 32 : 128))
+                             per_block, per_block))
     if (logits == nullptr) {
       B200_PREPARE(0);
     } else if (route_experts <= 64) {
@@ -962,7 +975,8 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
 #undef B200_PREPARE
     const int parts = std::max(1, std::min(8, (hidden / 16) / 128));
     B200_CUDA(launch_dependent(moe_scatter_quant_rows_kernel<128>, dim3(static_cast<unsigned>(tokens), parts), dim3(128), 0,
-                               stream, static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, hidden, top_k));
+                               stream, static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, sf_row_pitch(hidden), hidden,
+                               top_k));
   } else {
     // two launches for any number of tokens: (route +) count, then scan + quantise + place
     B200_CUDA(cudaMemsetAsync(ws.ctrl, 0, ws.clear_bytes, stream));
@@ -981,18 +995,26 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
                           expert_lo, experts, ws.my_counts, ws.slot_pos, ws.ctrl, ex, stream);
     if (rc) return rc;
     rc = launch_place(x, ids, ws.slot_pos, ex, static_cast<int>(tokens), hidden, top_k, expert_lo, experts,
-                      ws.max_m_blocks, 128, ws.h.slot_row, ws.h.num_m_blocks, ws.h.m_block_expert, ws.h.m_block_rows,
+                      ws.max_m_blocks, per_block, per_block, ws.h.slot_row, ws.h.num_m_blocks, ws.h.m_block_expert, ws.h.m_block_rows,
                       ws.ctrl, status, stream);
     if (rc) return rc;
   }
-  // the small front end's block tables are two launches old when FC1 starts, the other one's are its predecessor's work
-  int rc = gemm_moe_fc1(ws.xq, ws.xq_sf, w1, w1_sf, ws.act, ws.act_sf, w1_alpha, fc2_input_scale, ws.h.num_m_blocks,
-                        ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, few_rows,
-                        status, stream, nullptr, slots <= 1024 ? 0 : sf_row_pitch(hidden), slots <= 1024);
-  if (rc) return rc;
-  rc = gemm_moe_fc2(ws.act, ws.act_sf, w2, w2_sf, ws.partial, rows_bf16, w2_alpha, ws.h.num_m_blocks, ws.h.m_block_expert,
-                    ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, few_rows, status, stream, 1);
-  if (rc) return rc;
+  int rc;
+  if (tok != 0) {
+    rc = moe_stream_gemms(tok, ws.xq, ws.xq_sf, sf_row_pitch(hidden), w1, w1_sf, ws.act, ws.act_sf, sf_row_pitch(inter), w2,
+                          w2_sf, ws.partial, rows_bf16, w1_alpha, w2_alpha, fc2_input_scale, ws.h.num_m_blocks,
+                          ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, slots <= 1024,
+                          status, stream);
+    if (rc) return rc;
+  } else {
+    rc = gemm_moe_fc1(ws.xq, ws.xq_sf, w1, w1_sf, ws.act, ws.act_sf, w1_alpha, fc2_input_scale, ws.h.num_m_blocks,
+                      ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, 0, status, stream,
+                      nullptr, sf_row_pitch(hidden), slots <= 1024);
+    if (rc) return rc;
+    rc = gemm_moe_fc2(ws.act, ws.act_sf, w2, w2_sf, ws.partial, rows_bf16, w2_alpha, ws.h.num_m_blocks, ws.h.m_block_expert,
+                      ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, 0, status, stream, 1);
+    if (rc) return rc;
+  }
   const int threads = hidden / 4 >= 256 ? 256 : 128;
   auto combine = [&](auto kern, dim3 grid, int block, auto... args) {
     return check_cuda(launch_dependent(kern, grid, dim3(block), 0, stream, args...), "moe_combine_kernel launch");
@@ -1088,8 +1110,7 @@ EpLayout ep_layout(int64_t tokens_local, int hidden, int inter, int experts_loca
   L.flags = take(sizeof(int) * kSignalPhases * kMaxPeers);
   L.counts_all = take(sizeof(int) * world * experts_total);
   L.xq_sf_pitch = sf_row_pitch(hidden);
-  L.xq_sf_bytes = xq_sf_buffer_bytes(blocks, hidden);
-  L.xq_sf = take(L.xq_sf_bytes);
+  L.xq_sf = take(static_cast<size_t>(blocks) * 128 * sf_row_pitch(hidden));
   L.xq = take(static_cast<size_t>(rows) * (hidden / 2));
   L.row_tag = take(sizeof(int) * rows);
   // output rows cross NVLink as bf16 rows (f32 accumulation in the combine): one per slot, or one per (token,
@@ -1425,7 +1446,7 @@ int moe_ep_dispatch(const void* x, const int* ids, const float* weights, const f
   if (phases & 2) {
     rc = launch_place(x, logits != nullptr ? ids_buf : ids, reinterpret_cast<int*>(b + L.slot_pos), ex,
                       static_cast<int>(tokens_local), hidden, top_k, 0, experts_total, L.max_m_blocks,
-                      L.rows_per_block, nullptr, reinterpret_cast<int*>(b + L.num_m_blocks),
+                      L.rows_per_block, 128, nullptr, reinterpret_cast<int*>(b + L.num_m_blocks),
                       reinterpret_cast<int*>(b + L.m_block_expert), reinterpret_cast<int*>(b + L.m_block_rows), ctrl,
                       status, stream, logits != nullptr ? w_buf : weights);
     if (rc) return rc;

@@ -54,6 +54,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// named barrier over `threads` threads that tells whether all of them came with `ok`
+__device__ __forceinline__ bool bar_all(int id, int threads, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "bar.red.and.pred q, %2, %3, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u), "r"(id), "r"(threads)
+      : "memory");
+  return r != 0;
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05)
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -102,6 +102,15 @@ def test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k,
     assert rel_l2(out, ref) <= 1e-2
 
 
+@pytest.mark.parametrize("tokens,experts,hidden,inter,top_k", [
+    (20, 4, 320, 128, 1), (24, 2, 192, 128, 1), (60, 4, 320, 384, 2), (40, 1, 256, 128, 1), (700, 24, 576, 256, 2), (900, 24, 576, 256, 2)])
+@pytest.mark.parametrize("slot_rows", [None, torch.float32], ids=["rows_bf16", "rows_f32"])
+def test_few_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_rows):
+    """The streaming GEMMs with blocks of 16, 32 and 64 rows, experts that overflow a block, hidden sizes that do not fill the
+    last 256-wide column block, and both front ends (few and many slots); the last case is past their range."""
+    test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
+
+
 def test_hot_expert_and_expert_parallel_split(b200):
     """All tokens share one hot expert (several 128-row blocks of one expert), and the same problem computed as two
     expert-parallel halves accumulated into one output."""
