@@ -225,7 +225,8 @@ __global__ void __launch_bounds__(count_threads(kPerLane))
 moe_count_kernel(const float* __restrict__ logits, int route_experts, int renormalize, const int* __restrict__ ids_in,
                  int* __restrict__ ids_out, float* __restrict__ weights_out, int tokens, int top_k, int expert_lo,
                  int experts_total, int* my_counts, int* __restrict__ slot_pos, int* ctrl, Exchange ex,
-                 int tokens_per_cta) {
+                 int tokens_per_cta,
+                 int rows_per_block, int max_m_blocks, int* num_m_blocks, int* m_block_expert, int* m_block_rows) {
   const int kCountThreads = blockDim.x;
   extern __shared__ int s_dyn[];
   int* s_hist = s_dyn;
@@ -287,11 +288,37 @@ moe_count_kernel(const float* __restrict__ logits, int route_experts, int renorm
   const bool live = *reinterpret_cast<volatile int*>(ctrl + kCtrlAbort) == 0;
   for (int e = threadIdx.x; e < experts_total; e += blockDim.x) {
     const int c = atomicExch(my_counts + e, 0);
+    s_hist[e] = c;
     for (int d = 0; d < ex.world; ++d)
       if (d == ex.rank || live)
         reinterpret_cast<int*>(ex.peers.p[d] + ex.counts_all)[ex.rank * experts_total + e] = c;
   }
   __syncthreads();
+  if (num_m_blocks != nullptr) {         // single GPU: the block tables of the grouped GEMMs, one launch ahead of them
+    __shared__ int s_sum[32];
+    const int per_thread = (experts_total + kCountThreads - 1) / kCountThreads, e0 = threadIdx.x * per_thread;
+    int blocks = 0;
+    for (int e = e0; e < min(e0 + per_thread, experts_total); ++e) blocks += (s_hist[e] + rows_per_block - 1) / rows_per_block;
+    int incl = blocks;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    int at = incl - blocks;
+    for (int w = 0; w < warp; ++w) at += s_sum[w];
+    for (int e = e0; e < min(e0 + per_thread, experts_total); ++e) {
+      for (int left = s_hist[e]; left > 0; left -= rows_per_block, ++at) {
+        if (at < max_m_blocks) {
+          m_block_expert[at] = e;
+          m_block_rows[at] = min(rows_per_block, left);
+        }
+      }
+    }
+    if (threadIdx.x == kCountThreads - 1) *num_m_blocks = min(at, max_m_blocks);
+  }
   if (threadIdx.x < ex.world && threadIdx.x != ex.rank && live) {
     __threadfence_system();
     const int epoch = *reinterpret_cast<volatile int*>(ctrl + kCtrlEpoch) + 1;
@@ -320,6 +347,32 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
   __shared__ int s_flag;
   __shared__ int s_rows[kWarps][64];
   __shared__ int s_dst[kWarps][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int groups = hidden >> 6;            // groups of four 16-element blocks
+  auto quantise = [&](int token, int g, U32x8& codes, uint32_t& quad) {
+    const __nv_bfloat16* xrow = x + static_cast<int64_t>(token) * hidden;
+    U32x8 raw[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) raw[c] = ld_stream_32B(xrow + g * 64 + c * 16);
+    quad = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint64_t v2[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(raw[c].v[i]);
+      uint32_t sfb;
+      quantize_block16<true>(v2, 1.0f, codes.v[2 * c], codes.v[2 * c + 1], sfb);
+      quad |= (sfb & 0xffu) << (8 * c);
+    }
+  };
+  // The tokens are older than the count kernel, so the warp reads and quantises (the start of) its first token while that
+  // kernel still runs; most launches have one token per warp.
+  U32x8 pre[2];
+  uint32_t pre_quad[2];
+  const int first_token = blockIdx.x * kWarps + warp;
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+    if (first_token < tokens && lane + 32 * u < groups) quantise(first_token, lane + 32 * u, pre[u], pre_quad[u]);
   grid_dependency_wait();
   let_dependents_launch();
   if (!wait_all_ranks(ex, 0, ctrl, status, &s_flag)) return;
@@ -345,7 +398,6 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
     }
   }
   // exclusive scan of my_blocks over the CTA's threads
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int incl = my_blocks;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -366,7 +418,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
   }
   __syncthreads();
 
-  if (blockIdx.x == 0) {               // block tables of this rank's experts for the grouped GEMMs
+  if (blockIdx.x == 0 && num_m_blocks != nullptr) {      // block tables of this rank's experts for the grouped GEMMs
     const int first = ex.rank * el;
     const int seg0 = s_base[first];
     for (int le = threadIdx.x; le < el; le += kThreads) {
@@ -386,8 +438,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
     }
   }
 
-  const int groups = hidden >> 6;            // groups of four 16-element blocks
-  for (int token = blockIdx.x * kWarps + warp; token < tokens; token += gridDim.x * kWarps) {
+  for (int token = first_token; token < tokens; token += gridDim.x * kWarps) {
     __syncwarp();
     for (int j = lane; j < top_k; j += 32) {
       const int64_t slot = static_cast<int64_t>(token) * top_k + j;
@@ -413,22 +464,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
       }
     }
     __syncwarp();
-    const __nv_bfloat16* xrow = x + static_cast<int64_t>(token) * hidden;
-    for (int g = lane; g < groups; g += 32) {
-      U32x8 raw[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) raw[c] = ld_stream_32B(xrow + g * 64 + c * 16);
-      U32x8 codes;
-      uint32_t quad = 0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint64_t v2[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(raw[c].v[i]);
-        uint32_t sfb;
-        quantize_block16<true>(v2, 1.0f, codes.v[2 * c], codes.v[2 * c + 1], sfb);
-        quad |= (sfb & 0xffu) << (8 * c);
-      }
+    auto write = [&](int g, const U32x8& codes, uint32_t quad) {
       for (int j = 0; j < top_k; ++j) {
         const int row = s_rows[warp][j];
         if (row < 0) continue;
@@ -438,6 +474,19 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
         // 512 bytes apart, which is what the 128x4 tiles would ask for; FC1 fetches these rows as they are)
         *reinterpret_cast<uint32_t*>(base + ex.xq_sf + static_cast<int64_t>(row) * ex.xq_sf_pitch + 4 * g) = quad;
       }
+    };
+    int g = lane;
+    if (token == first_token) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (lane + 32 * u < groups) write(lane + 32 * u, pre[u], pre_quad[u]);
+      g += 64;
+    }
+    for (; g < groups; g += 32) {
+      U32x8 codes;
+      uint32_t quad;
+      quantise(token, g, codes, quad);
+      write(g, codes, quad);
     }
   }
   signal_when_all_ctas_done(ex, 1, ctrl, kCtrlTicketPlace, &s_flag);
@@ -534,34 +583,41 @@ moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, in
   }
 }
 
-// CTA (token, part): quantise a share of the row's 16-element blocks and write it to the rows assigned above
+// counters and control words start at zero (a kernel and not a memset, so that the launches around it may overlap)
+__global__ void moe_clear_kernel(int* words, int n) {
+  grid_dependency_wait();
+  let_dependents_launch();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) words[i] = 0;
+}
+
+// CTA (token, part): a thread quantises one 16-element block of the token and writes it to the rows assigned above
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
 moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_row, uint8_t* xq,
                               uint8_t* xq_sf, int sf_pitch, int hidden, int top_k) {
   __shared__ int s_rows[64];
   const int token = blockIdx.x;
+  const int chunk = blockIdx.y * kThreads + threadIdx.x;
+  const bool mine = chunk < (hidden >> 4);
+  // the tokens are older than the bookkeeping kernel: quantise while that one still runs
+  uint32_t lo = 0, hi = 0, sfb = 0;
+  if (mine) {
+    const U32x8 raw = ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16);
+    uint64_t v2[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(raw.v[i]);
+    quantize_block16<true>(v2, 1.0f, lo, hi, sfb);
+  }
   grid_dependency_wait();
   let_dependents_launch();
   if (threadIdx.x < top_k) s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
   __syncthreads();
-  const int nchunks = hidden >> 4;
-  for (int chunk = blockIdx.y * kThreads + threadIdx.x; chunk < nchunks; chunk += gridDim.y * kThreads) {
-    const U32x8 raw = ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16);
-    float v[16];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      v[2 * i] = Pair16<__nv_bfloat16>::lo(raw.v[i]);
-      v[2 * i + 1] = Pair16<__nv_bfloat16>::hi(raw.v[i]);
-    }
-    uint32_t lo, hi, sfb;
-    quantize_block16<true>(v, 1.0f, lo, hi, sfb);
-    for (int j = 0; j < top_k; ++j) {
-      const int row = s_rows[j];
-      if (row < 0) continue;
-      *reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * (hidden >> 1) + chunk * 8) = make_uint2(lo, hi);
-      xq_sf[static_cast<int64_t>(row) * sf_pitch + chunk] = static_cast<uint8_t>(sfb);
-    }
+  if (!mine) return;
+  for (int j = 0; j < top_k; ++j) {
+    const int row = s_rows[j];
+    if (row < 0) continue;
+    *reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * (hidden >> 1) + chunk * 8) = make_uint2(lo, hi);
+    xq_sf[static_cast<int64_t>(row) * sf_pitch + chunk] = static_cast<uint8_t>(sfb);
   }
 }
 
@@ -842,14 +898,17 @@ cudaError_t launch_in_order(int world, void (*kern)(Params...), dim3 grid, dim3 
 // result), else the caller's ids
 int launch_count(const float* logits, int route_experts, int renormalize, const int* ids_in, int* ids_out,
                  float* weights_out, int tokens, int top_k, int expert_lo, int experts_total, int* my_counts,
-                 int* slot_pos, int* ctrl, const Exchange& ex, cudaStream_t stream) {
+                 int* slot_pos, int* ctrl, const Exchange& ex, cudaStream_t stream, int rows_per_block = 128,
+                 int max_m_blocks = 0, int* num_m_blocks = nullptr, int* m_block_expert = nullptr,
+                 int* m_block_rows = nullptr) {
   const int tpc = tokens >= 4096 ? kCountTokensPerCta : (tokens >= 1024 ? 16 : 8);
   const dim3 grid((tokens + tpc - 1) / tpc);
   const size_t smem = sizeof(int) * 2 * experts_total;
 #define B200_COUNT(PL)                                                                                             \
   launch_in_order(ex.world, moe_count_kernel<PL>, grid, dim3(std::min(count_threads(PL), 32 * tpc)), smem, stream,   \
                   logits, route_experts, renormalize, ids_in, ids_out, weights_out, tokens, top_k, expert_lo,        \
-                  experts_total, my_counts, slot_pos, ctrl, ex, tpc)
+                  experts_total, my_counts, slot_pos, ctrl, ex, tpc, rows_per_block, max_m_blocks, num_m_blocks,     \
+                  m_block_expert, m_block_rows)
   cudaError_t err;
   if (logits == nullptr) err = B200_COUNT(0);
   else if (route_experts <= 64) err = B200_COUNT(2);
@@ -973,13 +1032,13 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
       B200_PREPARE(0);
     }
 #undef B200_PREPARE
-    const int parts = std::max(1, std::min(8, (hidden / 16) / 128));
+    const int parts = (hidden / 16 + 127) / 128;
     B200_CUDA(launch_dependent(moe_scatter_quant_rows_kernel<128>, dim3(static_cast<unsigned>(tokens), parts), dim3(128), 0,
                                stream, static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, sf_row_pitch(hidden), hidden,
                                top_k));
   } else {
-    // two launches for any number of tokens: (route +) count, then scan + quantise + place
-    B200_CUDA(cudaMemsetAsync(ws.ctrl, 0, ws.clear_bytes, stream));
+    // two launches (and the clearing of the counters) for any number of tokens: (route +) count, then scan + quantise + place
+    B200_CUDA(launch_dependent(moe_clear_kernel, dim3(1), dim3(256), 0, stream, ws.ctrl, kCtrlWords + experts));
     Exchange ex{};
     uint8_t* base = static_cast<uint8_t*>(workspace);
     ex.peers.p[0] = base;
@@ -992,11 +1051,11 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     ex.world = 1;
     ex.experts_local = experts;
     int rc = launch_count(logits, route_experts, renormalize, ids, ids, route_w, static_cast<int>(tokens), top_k,
-                          expert_lo, experts, ws.my_counts, ws.slot_pos, ws.ctrl, ex, stream);
+                          expert_lo, experts, ws.my_counts, ws.slot_pos, ws.ctrl, ex, stream, per_block, ws.max_m_blocks,
+                          ws.h.num_m_blocks, ws.h.m_block_expert, ws.h.m_block_rows);
     if (rc) return rc;
     rc = launch_place(x, ids, ws.slot_pos, ex, static_cast<int>(tokens), hidden, top_k, expert_lo, experts,
-                      ws.max_m_blocks, per_block, per_block, ws.h.slot_row, ws.h.num_m_blocks, ws.h.m_block_expert, ws.h.m_block_rows,
-                      ws.ctrl, status, stream);
+                      ws.max_m_blocks, per_block, per_block, ws.h.slot_row, nullptr, nullptr, nullptr, ws.ctrl, status, stream);
     if (rc) return rc;
   }
   int rc;
@@ -1009,7 +1068,7 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
   } else {
     rc = gemm_moe_fc1(ws.xq, ws.xq_sf, w1, w1_sf, ws.act, ws.act_sf, w1_alpha, fc2_input_scale, ws.h.num_m_blocks,
                       ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, 0, status, stream,
-                      nullptr, sf_row_pitch(hidden), slots <= 1024);
+                      nullptr, sf_row_pitch(hidden), 1);
     if (rc) return rc;
     rc = gemm_moe_fc2(ws.act, ws.act_sf, w2, w2_sf, ws.partial, rows_bf16, w2_alpha, ws.h.num_m_blocks, ws.h.m_block_expert,
                       ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, 0, status, stream, 1);
