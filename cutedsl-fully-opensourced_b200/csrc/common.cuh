@@ -62,6 +62,19 @@ __device__ __forceinline__ U32x8 ld_cached_32B(const void* p) {
   return r;
 }
 
+// 16 bytes that nobody reads again: they leave L2 first (the per-slot rows of a prefill step are larger than L2, and what
+// of them is still there need not push out the next step's data: 0.6 % of the step)
+__device__ __forceinline__ uint4 ld_once_16B(const void* p) {
+  uint4 r;
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+               : "l"(p), "l"(policy)
+               : "memory");
+  return r;
+}
+
 // data that the same kernel writes back later (no .nc)
 __device__ __forceinline__ U32x8 ld_32B(const void* p) {
   U32x8 r;

@@ -253,18 +253,19 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
                     "nvfp4_gemm_kernel launch");
 }
 
-template <typename OutT, int kFlavour>
+template <int kFlavour, typename Epilogue>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsa, const CUtensorMap& tsb,
-                const GemmParams& p, const EpilogueStore<OutT>& epi, cudaStream_t stream) {
-  auto kern = nvfp4_gemm_pair_kernel<EpilogueStore<OutT>, kFlavour>;
+                const CUtensorMap& tc, const GemmParams& p, const Epilogue& epi, cudaStream_t stream) {
+  auto kern = nvfp4_gemm_pair_kernel<Epilogue, kFlavour>;
+  constexpr uint32_t kSmem = pair_smem_bytes(Epilogue::kParkWide);
   static std::atomic<bool> configured[kMaxDevices];
-  int rc = configure_smem_once(configured, kern, static_cast<int>(kPairSmemBytes));
+  int rc = configure_smem_once(configured, kern, static_cast<int>(kSmem));
   if (rc) return rc;
   const int pairs = std::min(sm_count_of_current_device() / 2, p.num_m_blocks * p.num_n_blocks);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kPairThreads, 1, 1);
-  cfg.dynamicSmemBytes = kPairSmemBytes;
+  cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -275,7 +276,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, p, epi), "nvfp4_gemm_pair_kernel launch");
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, tc, p, epi), "nvfp4_gemm_pair_kernel launch");
 }
 
 // CTA-pair variant: 256 x 256 tiles on 2-CTA clusters
@@ -307,10 +308,19 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   p.num_n_blocks = (n + 255) / 256;
   rc = device_status_word(&p.status);
   if (rc) return rc;
-  EpilogueStore<OutT> epi{static_cast<OutT*>(c), n, alpha, 0};
-  if (p.sf_block32 == 2) return launch_pair<OutT, 2>(ta, tb, tsa, tsb, p, epi, stream);
-  if (p.sf_block32 == 1) return launch_pair<OutT, 1>(ta, tb, tsa, tsb, p, epi, stream);
-  return launch_pair<OutT, 0>(ta, tb, tsa, tsb, p, epi, stream);
+  auto launch = [&](const CUtensorMap& tc, const auto& epi) {
+    if (p.sf_block32 == 2) return launch_pair<2>(ta, tb, tsa, tsb, tc, p, epi, stream);
+    if (p.sf_block32 == 1) return launch_pair<1>(ta, tb, tsa, tsb, tc, p, epi, stream);
+    return launch_pair<0>(ta, tb, tsa, tsb, tc, p, epi, stream);
+  };
+  CUtensorMap tc{};
+  if constexpr (sizeof(OutT) == 2) {         // 16-bit rows leave through TMA stores
+    rc = make_output_map(&tc, c, m, static_cast<int64_t>(n) * 2, static_cast<int64_t>(n) * 2);
+    if (rc) return rc;
+    return launch(tc, EpilogueStoreWide<OutT>{alpha});
+  } else {
+    return launch(tc, EpilogueStore<OutT>{static_cast<OutT*>(c), n, alpha, 0});
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -760,7 +770,7 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
     if (small_a) return launch_gemm<256, false, 32>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
     if constexpr (sizeof(RowT) == 2) {
       if (park) {
-        EpilogueStoreWide wepi{w2_alpha};
+        EpilogueStoreWide<RowT> wepi{w2_alpha};
         return launch_gemm<256, false>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream);
       }
     }

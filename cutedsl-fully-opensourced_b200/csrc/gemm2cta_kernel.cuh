@@ -24,6 +24,9 @@
 // of movers that each carry two of a stage's four K blocks and report to barriers of their own, the MMAs of
 // blocks 2-3 issued after a second wait (the extra wait, fence and election in the issuing thread cost more than
 // the shorter slab chain saves: 17 % slower).
+// 16-bit rows leave through shared memory and TMA stores (EpilogueStoreWide): with register stores the last wave's drain
+// and the stores' L1 wavefronts showed, 8192^3 252 -> 240 us (1.5 GHz under the power cap), 1024 x 4096 x 4096 12.2 -> 11.3,
+// MXFP8 3001 x 5120 x 4096 69.2 -> 66.5; the 32 KB of parking space fit beside five stages (four: 2 to 3 % slower).
 #pragma once
 
 #include "gemm_kernel.cuh"
@@ -33,7 +36,11 @@ namespace b200fp4 {
 
 constexpr int kPairStages = 5;
 constexpr uint32_t kPairStageBytes = 16384 + 16384 + 2048 + 4096;    // A, B half, SFA, SFB (both halves)
-constexpr uint32_t kPairSmemBytes = kPairStages * kPairStageBytes + 1024 + 256;
+// barriers behind the stages, then (16-bit outputs) 4 KB of parking space per epilogue warp
+constexpr uint32_t kPairParkOffset = (kPairStages * kPairStageBytes + 256 + 1023) & ~1023u;
+constexpr uint32_t pair_smem_bytes(bool park) {
+  return park ? kPairParkOffset + 8 * 4096 + 1024 : kPairStages * kPairStageBytes + 1024 + 256;
+}
 constexpr int kPairThreads = 64 + 8 * 32 + 128;     // TMA, MMA, 8 epilogue warps, 4 scale-slab movers
 
 // kFlavour: GemmParams::sf_block32 (0 NVFP4, 1 MXFP4, 2 MXFP8)
@@ -41,7 +48,7 @@ template <typename Epilogue, int kFlavour>
 __global__ void __launch_bounds__(kPairThreads, 1)
 nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                       const GemmParams p, const Epilogue epi) {
+                       const __grid_constant__ CUtensorMap tmap_c, const GemmParams p, const Epilogue epi) {
   constexpr int kStages = kPairStages;
   constexpr int kBlockN = 256;
   constexpr uint32_t kSfaCol = 256;
@@ -85,6 +92,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     ptx::prefetch_tensormap(&tmap_b);
     ptx::prefetch_tensormap(&tmap_sfa);
     ptx::prefetch_tensormap(&tmap_sfb);
+    if constexpr (Epilogue::kParkWide) ptx::prefetch_tensormap(&tmap_c);
   }
   if (warp == 0) {
     __syncwarp();
@@ -293,9 +301,12 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                                            if (rank == 0) ptx::mbar_arrive(acc_empty_bar);
                                            else ptx::mbar_arrive_cluster_relaxed(acc_empty_bar & ptx::kPeerBitMask);   // tcgen05.wait::ld has returned
                                          }
-                                       });
+                                       },
+                                       Epilogue::kParkWide ? smem_gen + kPairParkOffset + (warp - 2) * 4096 : nullptr, &tmap_c);
       acc_phase ^= 1u;
     }
+    // the TMA stores of this warp's last tiles must have reached global memory
+    if (Epilogue::kParkWide && lane == 0) ptx::bulk_wait_group0();
   }
 
   // ---- teardown: nobody leaves while the peer may still signal this CTA or read its memory

@@ -393,17 +393,20 @@ struct EpilogueStore {
   }
 };
 
-// 256-wide plain tiles with bf16 rows that leave through TMA stores (FC2 of the MoE with short reductions).  The
+// 256-wide plain tiles with 16-bit rows that leave through TMA stores (FC2 of the MoE with short reductions, dense GEMMs
+// on CTA pairs).  The
 // tile has one accumulator, so what counts is how soon it is handed back: each of the eight epilogue warps owns 128
 // columns of its 32 rows as two 32 x 64 boxes and has 4 KB of parking space: it reads and packs the first box into
 // registers, reads the second straight into the parking space, releases the accumulator, stores the second box by
 // TMA and, once that store has read the space, parks and stores the first.  Register stores of the same tile take
 // 64 KB through lanes that each write another row (about 12 bytes per cycle and SM).
+template <typename OutT>
 struct EpilogueStoreWide {
+  static_assert(sizeof(OutT) == 2, "16-bit rows");
   static constexpr int kOutBytes = 2;
   static constexpr bool kUsesOutputMap = true;
   static constexpr bool kParkWide = true;
-  const float* alpha;           // one scale per group, or null
+  const float* alpha;           // one scale per group (dense: one), or null
   template <int kBlockN, typename Loader, typename Release>
   __device__ __forceinline__ void operator()(const GemmParams& p, int m_blk, int n_blk, int group, int row,
                                              int /*rows_valid*/, int part, int parts, Loader&& load, Release&& release,
@@ -416,10 +419,10 @@ struct EpilogueStoreWide {
     const int b0 = part * (4 / parts);                 // first 64-column box of this warp (it owns two: parts == 2)
     auto pack8 = [&](const uint32_t (&r)[32], int q) {
       uint4 v;
-      v.x = Pair16<__nv_bfloat16>::pack(__uint_as_float(r[8 * q]) * scale, __uint_as_float(r[8 * q + 1]) * scale);
-      v.y = Pair16<__nv_bfloat16>::pack(__uint_as_float(r[8 * q + 2]) * scale, __uint_as_float(r[8 * q + 3]) * scale);
-      v.z = Pair16<__nv_bfloat16>::pack(__uint_as_float(r[8 * q + 4]) * scale, __uint_as_float(r[8 * q + 5]) * scale);
-      v.w = Pair16<__nv_bfloat16>::pack(__uint_as_float(r[8 * q + 6]) * scale, __uint_as_float(r[8 * q + 7]) * scale);
+      v.x = Pair16<OutT>::pack(__uint_as_float(r[8 * q]) * scale, __uint_as_float(r[8 * q + 1]) * scale);
+      v.y = Pair16<OutT>::pack(__uint_as_float(r[8 * q + 2]) * scale, __uint_as_float(r[8 * q + 3]) * scale);
+      v.z = Pair16<OutT>::pack(__uint_as_float(r[8 * q + 4]) * scale, __uint_as_float(r[8 * q + 5]) * scale);
+      v.w = Pair16<OutT>::pack(__uint_as_float(r[8 * q + 6]) * scale, __uint_as_float(r[8 * q + 7]) * scale);
       return v;
     };
     auto store_box = [&](int b) {

@@ -770,7 +770,7 @@ __global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ part
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int row = j0 + k < top_k ? s_rows[j0 + k] : -1;
-        u[k] = row >= 0 ? *reinterpret_cast<const uint4*>(partial + static_cast<int64_t>(row) * hidden + c)
+        u[k] = row >= 0 ? ld_once_16B(partial + static_cast<int64_t>(row) * hidden + c)
                         : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
