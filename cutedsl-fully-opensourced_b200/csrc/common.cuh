@@ -42,23 +42,39 @@ struct alignas(32) U32x8 {
   uint32_t v[8];
 };
 
-// read-only, streamed once: bypass L1 allocation
+// No load here is .nc (nor __ldg, nor through a const __restrict__ parameter of a kernel that is launched as a dependent):
+// such a kernel is already running while its predecessor still writes, and a load that is promised read-only data may be
+// moved above the wait for that predecessor.
+// streamed once: bypass L1 allocation
 __device__ __forceinline__ U32x8 ld_stream_32B(const void* p) {
   U32x8 r;
-  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
                  "=r"(r.v[6]), "=r"(r.v[7])
-               : "l"(p));
+               : "l"(p)
+               : "memory");
   return r;
 }
 
-// read-only, read again by other blocks of the SM: through L1
+// one word of a table or a scale
+template <typename T>
+__device__ __forceinline__ T ld_word(const T* p) {
+  static_assert(sizeof(T) == 4, "words");
+  uint32_t v;
+  asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  T r;
+  memcpy(&r, &v, 4);
+  return r;
+}
+
+// read again by other blocks of the SM: through L1
 __device__ __forceinline__ U32x8 ld_cached_32B(const void* p) {
   U32x8 r;
-  asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
                  "=r"(r.v[6]), "=r"(r.v[7])
-               : "l"(p));
+               : "l"(p)
+               : "memory");
   return r;
 }
 
@@ -71,17 +87,6 @@ __device__ __forceinline__ uint4 ld_once_16B(const void* p) {
   asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.b32 {%0, %1, %2, %3}, [%4], %5;"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p), "l"(policy)
-               : "memory");
-  return r;
-}
-
-// data that the same kernel writes back later (no .nc)
-__device__ __forceinline__ U32x8 ld_32B(const void* p) {
-  U32x8 r;
-  asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
-                 "=r"(r.v[6]), "=r"(r.v[7])
-               : "l"(p)
                : "memory");
   return r;
 }

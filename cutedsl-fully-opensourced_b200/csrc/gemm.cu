@@ -330,11 +330,11 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
 // does not depend on timing), applies alpha and rounds once.
 // ---------------------------------------------------------------------------
 template <typename OutT>
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits, int64_t stride,
-                                     const float* __restrict__ alpha, OutT* __restrict__ c, int64_t n4) {
+__global__ void splitk_reduce_kernel(const float* partial, int splits, int64_t stride,
+                                     const float* alpha, OutT* c, int64_t n4) {
   grid_dependency_wait();
   let_dependents_launch();
-  const float scale = alpha == nullptr ? 1.0f : __ldg(alpha);
+  const float scale = alpha == nullptr ? 1.0f : ld_word(alpha);
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     float4 acc = *reinterpret_cast<const float4*>(partial + 4 * i);

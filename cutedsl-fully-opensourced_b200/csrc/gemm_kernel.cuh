@@ -295,7 +295,7 @@ struct EpilogueStore {
   __device__ __forceinline__ void operator()(const GemmParams& p, int m_blk, int n_blk, int group, int row,
                                              int rows_valid, int part, int parts, Loader&& load, Release&& release,
                                              uint8_t* stage = nullptr, const CUtensorMap* cmap = nullptr) const {
-    const float scale = alpha == nullptr ? 1.0f : __ldg(alpha + (alpha_per_group ? group : 0));
+    const float scale = alpha == nullptr ? 1.0f : ld_word(alpha + (alpha_per_group ? group : 0));
     if (stage != nullptr) {
       tma_path<kBlockN>(p, m_blk, n_blk, row, scale, load, stage, cmap, part, parts);
       release();
@@ -412,7 +412,7 @@ struct EpilogueStoreWide {
                                              int /*rows_valid*/, int part, int parts, Loader&& load, Release&& release,
                                              uint8_t* stage = nullptr, const CUtensorMap* cmap = nullptr) const {
     static_assert(kBlockN == 256, "wide parking serves 256-wide tiles");
-    const float scale = alpha == nullptr ? 1.0f : __ldg(alpha + group);
+    const float scale = alpha == nullptr ? 1.0f : ld_word(alpha + group);
     const int lane = row & 31;
     uint8_t* box = stage + lane * 128;
     const int y = m_blk * kBlockM + (row & ~31);
@@ -489,11 +489,11 @@ struct EpiloguePushRows {
   __device__ __forceinline__ void operator()(const GemmParams& p, int m_blk, int n_blk, int group, int row,
                                              int rows_valid, int part, int parts, Loader&& load, Release&& release,
                                              uint8_t* stage = nullptr, const CUtensorMap* /*cmap*/ = nullptr) const {
-    const float scale = alpha == nullptr ? 1.0f : __ldg(alpha + group);
+    const float scale = alpha == nullptr ? 1.0f : ld_word(alpha + group);
     const int lane = row & 31;
     const int64_t grow = static_cast<int64_t>(m_blk) * kBlockM + row;
-    const bool live = __ldg(abort_flag) == 0;
-    const int tag = (row < rows_valid && live) ? __ldg(row_tag + grow) : -1;
+    const bool live = ld_word(abort_flag) == 0;
+    const int tag = (row < rows_valid && live) ? ld_word(row_tag + grow) : -1;
     if constexpr (kBlockN == 128) {
       // park: 2 boxes of 32 rows x 128 bytes, 16-byte chunks XOR-swizzled by the row (no bank conflicts either way);
       // with two warps per TMEM quarter (parts == 2) each warp parks and sends one box: 128 bytes per row
@@ -581,8 +581,8 @@ struct EpilogueSwiglu {
                                              uint8_t* /*stage*/ = nullptr, const CUtensorMap* /*cmap*/ = nullptr) const {
     constexpr int kHalf = kBlockN / 2;
     static_assert(kHalf % 64 == 0, "the SwiGLU epilogue pairs two halves of whole 32-column groups per warp");
-    const float a1 = w1_alpha == nullptr ? 1.0f : __ldg(w1_alpha + group);
-    const float gs = fc2_input_scale == nullptr ? 1.0f : __ldg(fc2_input_scale);
+    const float a1 = w1_alpha == nullptr ? 1.0f : ld_word(w1_alpha + group);
+    const float gs = fc2_input_scale == nullptr ? 1.0f : ld_word(fc2_input_scale);
     const int64_t grow = static_cast<int64_t>(m_blk) * kBlockM + row;
     const int j0 = n_blk * kHalf;
     const int rk2 = (inter + 63) >> 6;
@@ -707,7 +707,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   // grouped launches read the number of row blocks from device memory; never trust it beyond the table size
   const int num_m_blocks =
-      p.num_m_blocks_dev != nullptr ? max(0, min(__ldg(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
+      p.num_m_blocks_dev != nullptr ? max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
   const int num_out_tiles = num_m_blocks * p.num_n_blocks;
   const int splits = p.k_splits > 1 ? p.k_splits : 1;
   const int kt_per_split = (p.num_k_tiles + splits - 1) / splits;
@@ -750,7 +750,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       auto begin_tile = [&](int tile) {
         m_blk = tile_m(tile);
         const int n_blk = tile_n(tile);
-        group = p.m_block_group != nullptr ? max(0, min(__ldg(p.m_block_group + m_blk), p.num_groups - 1)) : 0;
+        group = p.m_block_group != nullptr ? max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1)) : 0;
         sfa_row = p.sfa + static_cast<int64_t>(m_blk) * p.rk * 512;
 #pragma unroll
         for (int i = 0; i < kBPieces; ++i) {
@@ -797,7 +797,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (p.early_trigger) let_dependents_launch();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         begin_tile(tile);
-        if (kARows < kBlockM && p.m_block_rows != nullptr && __ldg(p.m_block_rows + m_blk) > kARows)
+        if (kARows < kBlockM && p.m_block_rows != nullptr && ld_word(p.m_block_rows + m_blk) > kARows)
           atomicOr(p.status, kStatusRowsExceedTile);      // results of this block are wrong: tell the host
         for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end; ++kt) {
           if (!wait_bounded(empty_bar(st.stage), st.phase ^ 1u, abort_flag)) {
@@ -1004,7 +1004,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int m_blk = tile_m(tile);
       const int n_blk = tile_n(tile);
       const int group =
-          p.m_block_group != nullptr ? max(0, min(__ldg(p.m_block_group + m_blk), p.num_groups - 1))
+          p.m_block_group != nullptr ? max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1))
                                      : (splits > 1 ? tile / num_out_tiles : 0);
       if (!wait_bounded<64>(acc_full_bar(acc.stage), acc.phase, abort_flag)) {
         if (lane == 0) atomicOr(p.status, kStatusTimeoutEpilogue);
@@ -1012,7 +1012,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
       ptx::tc_fence_after_sync();
       const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc.stage * kBlockN;
-      const int rows_valid = p.m_block_rows != nullptr ? __ldg(p.m_block_rows + m_blk) : kBlockM;
+      const int rows_valid = p.m_block_rows != nullptr ? ld_word(p.m_block_rows + m_blk) : kBlockM;
       if (quarter * 32 < rows_valid) {                 // a warp whose 32 rows only pad the block has nothing to do
         // parking space of the TMA-store variant: 1024-byte aligned, one slice per epilogue warp
         uint8_t* stage = nullptr;

@@ -47,7 +47,7 @@ __host__ __device__ constexpr StreamLayout stream_layout(int tok) {
 template <int kTok, typename OutT>
 __global__ void __launch_bounds__(kStreamThreads, 2)
 nvfp4_gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                         const GemmParams p, OutT* __restrict__ c, const float* __restrict__ alpha) {
+                         const GemmParams p, OutT* c, const float* alpha) {
   constexpr StreamLayout L = stream_layout(kTok);
   constexpr int kStages = L.stages;
   constexpr uint32_t kSfSetCols = 32;                    // 16 columns of W scales + 16 of X scales per stage
@@ -212,7 +212,7 @@ nvfp4_gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   const int quarter = warp & 3;
   const int channel = quarter * 32 + lane;
   const int n = n_blk * 128 + channel;
-  const float scale = alpha == nullptr ? 1.0f : __ldg(alpha);
+  const float scale = alpha == nullptr ? 1.0f : ld_word(alpha);
   const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
   auto store = [&](int col, float v) {
     const int m = m0 + col;

@@ -51,7 +51,7 @@ constexpr int kRouteMaxPerLane = 32;       // experts <= 1024
 // ---------------------------------------------------------------------------
 // Lane j (< top_k) of the warp returns the j-th choice of the token whose logits start at `row`.
 template <int kPerLane>
-__device__ __forceinline__ void route_one_token(const float* __restrict__ row, int lane, int experts, int top_k,
+__device__ __forceinline__ void route_one_token(const float* row, int lane, int experts, int top_k,
                                                 int renormalize, int& my_id, float& my_w) {
   float v[kPerLane];
   const int per_lane = (experts + 31) >> 5;
@@ -112,7 +112,7 @@ __device__ __forceinline__ void route_one_token(const float* __restrict__ row, i
 }
 
 template <int kPerLane>
-__global__ void route_topk_kernel(const float* __restrict__ logits, int* __restrict__ ids, float* __restrict__ weights,
+__global__ void route_topk_kernel(const float* logits, int* ids, float* weights,
                                   int tokens, int experts, int top_k, int renormalize) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -222,9 +222,9 @@ constexpr int kCountTokensPerCta = 32;
 __host__ __device__ constexpr int count_threads(int per_lane) { return per_lane <= 8 ? 1024 : 256; }
 template <int kPerLane>
 __global__ void __launch_bounds__(count_threads(kPerLane))
-moe_count_kernel(const float* __restrict__ logits, int route_experts, int renormalize, const int* __restrict__ ids_in,
-                 int* __restrict__ ids_out, float* __restrict__ weights_out, int tokens, int top_k, int expert_lo,
-                 int experts_total, int* my_counts, int* __restrict__ slot_pos, int* ctrl, Exchange ex,
+moe_count_kernel(const float* logits, int route_experts, int renormalize, const int* ids_in,
+                 int* ids_out, float* weights_out, int tokens, int top_k, int expert_lo,
+                 int experts_total, int* my_counts, int* slot_pos, int* ctrl, Exchange ex,
                  int tokens_per_cta,
                  int rows_per_block, int max_m_blocks, int* num_m_blocks, int* m_block_expert, int* m_block_rows) {
   const int kCountThreads = blockDim.x;
@@ -333,11 +333,11 @@ moe_count_kernel(const float* __restrict__ logits, int route_experts, int renorm
 // scale bytes (adjacent in the 128x4 tiles) with one store each.  Dynamic shared memory: 3 * experts_total ints.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
-moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ ids,
-                       const int* __restrict__ slot_pos, Exchange ex, int tokens, int hidden, int top_k,
+moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
+                       const int* slot_pos, Exchange ex, int tokens, int hidden, int top_k,
                        int expert_lo, int experts_total, int max_m_blocks, int rows_per_block, int block_stride,
                        int* slot_row, int* num_m_blocks, int* m_block_expert, int* m_block_rows, int* ctrl, int* status,
-                       const float* __restrict__ weights) {
+                       const float* weights) {
   extern __shared__ int s_dyn[];
   int* s_base = s_dyn;                       // blocks before expert e (over all experts, in expert order)
   int* s_myoff = s_dyn + experts_total;      // rows of lower ranks inside expert e's segment
@@ -388,7 +388,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
     if (e < experts_total) {
       int tot = 0, off = 0;
       for (int r = 0; r < ex.world; ++r) {
-        const int c = __ldcg(counts + r * experts_total + e);
+        const int c = *reinterpret_cast<const volatile int*>(counts + r * experts_total + e);      // peers write them
         if (r < ex.rank) off += c;
         tot += c;
       }
@@ -500,7 +500,7 @@ moe_quant_place_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
 // step.  0: the ids are inputs.
 template <int kRoutePerLane>
 __global__ void __launch_bounds__(1024)
-moe_prepare_small_kernel(const float* __restrict__ logits, int route_experts, int renormalize, int top_k, int* ids,
+moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize, int top_k, int* ids,
                          float* weights, int n_slots, int expert_lo, MoeHeader h, int experts, int max_m_blocks,
                          int rows_per_block, int block_stride) {
   __shared__ __align__(16) uint8_t s_cnt[32][1024];      // slots of warp w's 32 that named expert e
@@ -593,7 +593,7 @@ __global__ void moe_clear_kernel(int* words, int n) {
 // CTA (token, part): a thread quantises one 16-element block of the token and writes it to the rows assigned above
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
-moe_scatter_quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ slot_row, uint8_t* xq,
+moe_scatter_quant_rows_kernel(const __nv_bfloat16* x, const int* slot_row, uint8_t* xq,
                               uint8_t* xq_sf, int sf_pitch, int hidden, int top_k) {
   __shared__ int s_rows[64];
   const int token = blockIdx.x;
@@ -635,8 +635,8 @@ __device__ __forceinline__ float4 load_row4(const RowT* p) {
 
 // one CTA per token; every thread owns 4 output columns at a time
 template <typename OutT, typename RowT>
-__global__ void moe_combine_kernel(const RowT* __restrict__ partial, const int* __restrict__ slot_row,
-                                   const float* __restrict__ weights, OutT* __restrict__ out, int hidden,
+__global__ void moe_combine_kernel(const RowT* partial, const int* slot_row,
+                                   const float* weights, OutT* out, int hidden,
                                    int top_k, int accumulate) {
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
@@ -689,8 +689,8 @@ __global__ void moe_combine_kernel(const RowT* __restrict__ partial, const int* 
 // with independent loads (a decode step with one token is nothing but the latency of these reads; with thousands
 // of tokens the plain kernel above is faster).
 template <typename OutT, typename RowT>
-__global__ void moe_combine_few_kernel(const RowT* __restrict__ partial, const int* __restrict__ slot_row,
-                                   const float* __restrict__ weights, OutT* __restrict__ out, int hidden,
+__global__ void moe_combine_few_kernel(const RowT* partial, const int* slot_row,
+                                   const float* weights, OutT* out, int hidden,
                                    int top_k, int accumulate) {
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
@@ -750,8 +750,8 @@ __global__ void moe_combine_few_kernel(const RowT* __restrict__ partial, const i
 // The same sum for bf16 rows and a bf16 output with 16-byte accesses: one CTA per token, a thread owns 8 columns and
 // keeps the loads of four rows in flight.  Same arithmetic as moe_combine_kernel (f32, slot order, one product and
 // one sum per slot, one rounding).
-__global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* __restrict__ partial, const int* __restrict__ slot_row,
-                                          const float* __restrict__ weights, __nv_bfloat16* __restrict__ out,
+__global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* partial, const int* slot_row,
+                                          const float* weights, __nv_bfloat16* out,
                                           int hidden, int top_k, int accumulate) {
   __shared__ int s_rows[64];
   __shared__ float s_w[64];

@@ -118,9 +118,9 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (!p.early_b) grid_dependency_wait();
 
   // block counts read from device memory are never trusted beyond the table size
-  const int num_blocks = max(0, min(__ldg(p.num_m_blocks_dev), p.num_m_blocks));
+  const int num_blocks = max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks));
   const int num_tiles = num_blocks * p.num_n_blocks;
-  auto rows_of = [&](int blk) { return max(0, min(__ldg(p.m_block_rows + blk), kTok)); };
+  auto rows_of = [&](int blk) { return max(0, min(ld_word(p.m_block_rows + blk), kTok)); };
 
   if (warp == 0) {
     // =============================== TMA producer ===============================
@@ -132,7 +132,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       auto begin_tile = [&](int tile) {
         blk = tile / p.num_n_blocks;
         const int n_blk = tile - blk * p.num_n_blocks;
-        group = max(0, min(__ldg(p.m_block_group + blk), p.num_groups - 1));
+        group = max(0, min(ld_word(p.m_block_group + blk), p.num_groups - 1));
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           w_row[i] = Epi::kSwiglu ? n_blk * 128 + i * p.gate_row_offset : n_blk * 256 + i * 128;
@@ -280,7 +280,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     PipeState acc;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const int blk = tile / p.num_n_blocks, n_blk = tile - blk * p.num_n_blocks;
-      const int group = max(0, min(__ldg(p.m_block_group + blk), p.num_groups - 1));
+      const int group = max(0, min(ld_word(p.m_block_group + blk), p.num_groups - 1));
       const int rows = rows_of(blk);
       const int64_t row0 = static_cast<int64_t>(blk) * kTok;
       const bool ready = wait_bounded<64>(acc_full_bar(acc.stage), acc.phase, abort_flag);
@@ -298,8 +298,8 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       };
       auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };   // the four epilogue warps
       if constexpr (Epi::kSwiglu) {
-        const float a1 = epi.w1_alpha == nullptr ? 1.0f : __ldg(epi.w1_alpha + group);
-        const float gs = epi.fc2_input_scale == nullptr ? 1.0f : __ldg(epi.fc2_input_scale);
+        const float a1 = epi.w1_alpha == nullptr ? 1.0f : ld_word(epi.w1_alpha + group);
+        const float gs = epi.fc2_input_scale == nullptr ? 1.0f : ld_word(epi.fc2_input_scale);
         __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(park);
 #pragma unroll 1
         for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -337,7 +337,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         meet();                          // the parking space is free again
       } else {
         using Row = typename Epi::Row;
-        const float a2 = epi.w2_alpha == nullptr ? 1.0f : __ldg(epi.w2_alpha + group);
+        const float a2 = epi.w2_alpha == nullptr ? 1.0f : ld_word(epi.w2_alpha + group);
         Row* out = reinterpret_cast<Row*>(park);
 #pragma unroll 1
         for (int piece = 0; piece < 2; ++piece) {

@@ -95,9 +95,9 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
     if (p.sf_swizzled != nullptr && row < ((p.rows + 127) & ~int64_t{127})) zero_padding_row(p, row, rk, tid, team);
     return;
   }
-  const T* __restrict__ xrow = static_cast<const T*>(p.x) + row * p.x_row_stride;
+  const T* xrow = static_cast<const T*>(p.x) + row * p.x_row_stride;
   T* rrow = static_cast<T*>(p.residual) + (kAdd ? row * p.res_row_stride : 0);
-  const T* __restrict__ wg = static_cast<const T*>(p.weight);
+  const T* wg = static_cast<const T*>(p.weight);
 
   // ---- phase 1: load, (add, round, write residual), sum of squares; all f32 math on register pairs.  Everything the
   // thread reads from DRAM is requested before anything is used.
@@ -109,12 +109,12 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
       const int c = u * kVec + v, chunk = (tid + u * team) * kVec + v;
       if (chunk < nchunks) {
         xin[c] = ld_stream_32B(xrow + chunk * 16);
-        if constexpr (kAdd) rin[c] = ld_32B(rrow + chunk * 16);
+        if constexpr (kAdd) rin[c] = ld_stream_32B(rrow + chunk * 16);
         else win[c] = ld_cached_32B(wg + chunk * 16);
       }
     }
   }
-  const float gs = __ldg(p.global_scale);
+  const float gs = ld_word(p.global_scale);
   // what phase 2 normalises, kept as packed 16-bit pairs so that few registers live across the row reduction
   uint32_t h[kUnits * kVec][8];
   uint64_t ssq2 = 0;                         // {0.0f, 0.0f}
