@@ -398,14 +398,62 @@ __device__ __forceinline__ void quantize_block16(const uint64_t (&v2)[8], float 
   quantize_block16<kImplicitOne, kOneBranch>(value, value, amax, gs, gs, codes_lo, codes_hi, sf_bits);
 }
 
-// the same for sixteen scalars
-template <bool kImplicitOne>
-__device__ __forceinline__ void quantize_block16(const float (&v)[16], float gs, uint32_t& codes_lo,
-                                                 uint32_t& codes_hi, uint32_t& sf_bits) {
+// ---------------------------------------------------------------------------
+// The MoE activation packer (implicit-one reading of the scale byte) on sixteen bf16 values, eight packed pairs.
+//
+// When gs is a power of two -- 1 for the tokens, and for activations unless the caller calibrated a scale -- one
+// conversion is exact.  v * gs is then a bf16 number, 8 significant bits, and a midpoint c (2 or 3 bits) times the divisor
+// s (4 bits) is one too: two of them that differ, differ by more than 2^-8 of either.  So with u = v * gs / s * (1 - 2^-12),
+// the factor approximated to a few ulp, v * gs > c * s puts u above c, v * gs < c * s below it, and a tie, which the golden
+// gives to the smaller magnitude, also below: u is never half way between two codes and the hardware's nearest one is the
+// golden's.  Half of the general routine's multiplications and conversions, and no second path.
+// ---------------------------------------------------------------------------
+struct Block16Codes {
+  uint32_t lo, hi, sf;
+};
+static __device__ __noinline__ Block16Codes quantize_bf16x16_any_scale(uint4 a, uint4 b, float gs) {
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
   uint64_t v2[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v2[i] = f32x2_pack(v[2 * i], v[2 * i + 1]);
-  quantize_block16<kImplicitOne>(v2, gs, codes_lo, codes_hi, sf_bits);
+  for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(w[i]);
+  Block16Codes r;
+  quantize_block16<true>(v2, gs, r.lo, r.hi, r.sf);
+  return r;
+}
+__device__ __forceinline__ bool is_power_of_two(float v) {        // positive and normal
+  const uint32_t u = __float_as_uint(v);
+  return (u & 0x807fffffu) == 0u && u != 0u && u != 0x7f800000u;
+}
+__device__ __forceinline__ Block16Codes quantize_bf16x16_pow2(const uint32_t (&w)[8], float gs) {
+  uint32_t m = Pack16<__nv_bfloat16>::max_abs(w[0], w[1]);
+#pragma unroll
+  for (int i = 2; i < 8; ++i) m = Pack16<__nv_bfloat16>::max_abs(m, w[i]);
+  const float amax = fmaxf(Pair16<__nv_bfloat16>::lo(m), Pair16<__nv_bfloat16>::hi(m));
+  Block16Codes r;
+  r.sf = e4m3_encode_rn(fminf(div_by_6(__fmul_rn(amax, gs)), 448.0f));
+  const float div = e4m3_decode_implicit_one(r.sf);
+  const float k = div > 0.0f ? gs * rcp_approx(div) * 0.999755859375f : 0.0f;      // 1 - 2^-12
+  const uint64_t k2 = f32x2_pack(k, k);
+  uint32_t out[2];
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    float u[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint64_t v = f32x2_mul(pair16_to_f32x2<__nv_bfloat16>(w[4 * g + i]), k2);
+      u[2 * i] = f32x2_lo(v);
+      u[2 * i + 1] = f32x2_hi(v);
+    }
+    out[g] = e2m1x8_drop_negative_zero(e2m1x8_hw(u));
+  }
+  r.lo = out[0];
+  r.hi = out[1];
+  return r;
+}
+// pow2: is_power_of_two(gs)
+__device__ __forceinline__ Block16Codes quantize_bf16x16(const uint32_t (&w)[8], float gs, bool pow2) {
+  if (pow2) return quantize_bf16x16_pow2(w, gs);
+  return quantize_bf16x16_any_scale(make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]), gs);
 }
 
 // exchange buffers of the ranks of an expert-parallel group, as mapped into this process

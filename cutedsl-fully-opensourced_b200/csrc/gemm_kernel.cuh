@@ -592,6 +592,7 @@ struct EpilogueSwiglu {
     // The arithmetic runs on the packed f32x2 instructions where it can (scaling, 1 + e, the product, the bf16
     // round trip): every operation is the same IEEE f32 operation as in scalar form, two per instruction -- the
     // fewer instructions the epilogue issues, the less it holds up the warps that feed the tensor pipe.
+    const bool gs_pow2 = is_power_of_two(gs);
     const uint64_t a1_2 = f32x2_pack(a1, a1);
     const uint64_t one_2 = f32x2_pack(1.0f, 1.0f);
     auto finish = [&](int c0, const uint32_t (&up)[32], const uint32_t (&gate)[32]) {
@@ -600,7 +601,7 @@ struct EpilogueSwiglu {
       uint32_t codes[4];
 #pragma unroll
       for (int b = 0; b < 2; ++b) {
-        uint64_t v2[8];
+        uint32_t w[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const uint64_t u2 = f32x2_mul(f32x2_pack(__uint_as_float(up[16 * b + 2 * i]), __uint_as_float(up[16 * b + 2 * i + 1])), a1_2);
@@ -609,11 +610,11 @@ struct EpilogueSwiglu {
           const uint64_t d2 = f32x2_add(one_2, f32x2_pack(__expf(-g0), __expf(-g1)));
           // silu in f32 (a few ulp; rounded to bf16 next)
           const uint64_t s2 = f32x2_pack(__fdividef(g0, f32x2_lo(d2)), __fdividef(g1, f32x2_hi(d2)));
-          v2[i] = pair16_to_f32x2<__nv_bfloat16>(f32x2_to_pair16<__nv_bfloat16>(f32x2_mul(s2, u2)));
+          w[i] = f32x2_to_pair16<__nv_bfloat16>(f32x2_mul(s2, u2));
         }
-        uint32_t sfb;
-        quantize_block16<true>(v2, gs, codes[2 * b], codes[2 * b + 1], sfb);
-        sfpair |= sfb << (8 * b);
+        const Block16Codes q = quantize_bf16x16(w, gs, gs_pow2);
+        codes[2 * b] = q.lo, codes[2 * b + 1] = q.hi;
+        sfpair |= q.sf << (8 * b);
       }
       *reinterpret_cast<uint4*>(act_codes + grow * (inter >> 1) + ((j0 + c0) >> 1)) =
           make_uint4(codes[0], codes[1], codes[2], codes[3]);

@@ -49,6 +49,12 @@ constexpr int kRouteMaxPerLane = 32;       // experts <= 1024
 // ---------------------------------------------------------------------------
 // route: one warp per token; kPerLane = experts a lane holds (experts <= 32 * kPerLane)
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
 // Lane j (< top_k) of the warp returns the j-th choice of the token whose logits start at `row`.
 template <int kPerLane>
 __device__ __forceinline__ void route_one_token(const float* row, int lane, int experts, int top_k,
@@ -62,8 +68,7 @@ __device__ __forceinline__ void route_one_token(const float* row, int lane, int 
     v[i] = (i < per_lane && e < experts) ? row[e] : -INFINITY;
     mx = fmaxf(mx, v[i]);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  mx = warp_max(mx);
   float sum = 0.0f;
 #pragma unroll
   for (int i = 0; i < kPerLane; ++i) {
@@ -87,15 +92,11 @@ __device__ __forceinline__ void route_one_token(const float* row, int lane, int 
         best_e = lane + 32 * i;
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) {
-        best = ob;
-        best_e = oe;
-      }
-    }
+    // two warp reductions instead of five rounds of shuffles: non-negative floats order as integers (0 = nothing left)
+    const uint32_t key = best >= 0.0f ? __float_as_uint(best) + 1u : 0u;
+    const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+    best_e = static_cast<int>(__reduce_min_sync(0xffffffffu, key == top ? static_cast<uint32_t>(best_e) : 0x7fffffffu));
+    best = top != 0u ? __uint_as_float(top - 1u) : -1.0f;
     if ((best_e & 31) == lane) {
 #pragma unroll
       for (int i = 0; i < kPerLane; ++i)
@@ -357,12 +358,9 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
     quad = 0;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-      uint64_t v2[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(raw[c].v[i]);
-      uint32_t sfb;
-      quantize_block16<true>(v2, 1.0f, codes.v[2 * c], codes.v[2 * c + 1], sfb);
-      quad |= (sfb & 0xffu) << (8 * c);
+      const Block16Codes q = quantize_bf16x16_pow2(raw[c].v, 1.0f);
+      codes.v[2 * c] = q.lo, codes.v[2 * c + 1] = q.hi;
+      quad |= (q.sf & 0xffu) << (8 * c);
     }
   };
   // The tokens are older than the count kernel, so the warp reads and quantises (the start of) its first token while that
@@ -600,14 +598,8 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* x, const int* slot_row, uint8
   const int chunk = blockIdx.y * kThreads + threadIdx.x;
   const bool mine = chunk < (hidden >> 4);
   // the tokens are older than the bookkeeping kernel: quantise while that one still runs
-  uint32_t lo = 0, hi = 0, sfb = 0;
-  if (mine) {
-    const U32x8 raw = ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16);
-    uint64_t v2[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(raw.v[i]);
-    quantize_block16<true>(v2, 1.0f, lo, hi, sfb);
-  }
+  Block16Codes q{};
+  if (mine) q = quantize_bf16x16_pow2(ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16).v, 1.0f);
   grid_dependency_wait();
   let_dependents_launch();
   if (threadIdx.x < top_k) s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];
@@ -616,8 +608,8 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* x, const int* slot_row, uint8
   for (int j = 0; j < top_k; ++j) {
     const int row = s_rows[j];
     if (row < 0) continue;
-    *reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * (hidden >> 1) + chunk * 8) = make_uint2(lo, hi);
-    xq_sf[static_cast<int64_t>(row) * sf_pitch + chunk] = static_cast<uint8_t>(sfb);
+    *reinterpret_cast<uint2*>(xq + static_cast<int64_t>(row) * (hidden >> 1) + chunk * 8) = make_uint2(q.lo, q.hi);
+    xq_sf[static_cast<int64_t>(row) * sf_pitch + chunk] = static_cast<uint8_t>(q.sf);
   }
 }
 

@@ -300,6 +300,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       if constexpr (Epi::kSwiglu) {
         const float a1 = epi.w1_alpha == nullptr ? 1.0f : ld_word(epi.w1_alpha + group);
         const float gs = epi.fc2_input_scale == nullptr ? 1.0f : ld_word(epi.fc2_input_scale);
+        const bool gs_pow2 = is_power_of_two(gs);
         __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(park);
 #pragma unroll 1
         for (int c0 = 0; c0 < rows; c0 += 16) {
@@ -322,15 +323,12 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           const uint4* src = reinterpret_cast<const uint4*>(act + t * 128 + b * 16);
           const uint4 q0 = src[0], q1 = src[1];
           const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          uint64_t v2[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) v2[i] = pair16_to_f32x2<__nv_bfloat16>(w[i]);
-          uint32_t lo, hi, sf;
-          quantize_block16<true>(v2, gs, lo, hi, sf);
+          const Block16Codes q = quantize_bf16x16(w, gs, gs_pow2);
+          uint32_t sf = q.sf;
           sf |= __shfl_down_sync(0xffffffffu, sf, 1) << 8;
           sf |= __shfl_down_sync(0xffffffffu, sf, 2) << 16;
           if (t < rows) {
-            *reinterpret_cast<uint2*>(epi.act_codes + (row0 + t) * (epi.inter >> 1) + n_blk * 64 + b * 8) = make_uint2(lo, hi);
+            *reinterpret_cast<uint2*>(epi.act_codes + (row0 + t) * (epi.inter >> 1) + n_blk * 64 + b * 8) = make_uint2(q.lo, q.hi);
             if ((b & 3) == 0) *reinterpret_cast<uint32_t*>(epi.act_sf + (row0 + t) * epi.sf_pitch + n_blk * 8 + b) = sf;
           }
         }

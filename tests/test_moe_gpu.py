@@ -111,6 +111,23 @@ def test_few_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_r
     test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
 
 
+@pytest.mark.parametrize("tokens,gs2", [(24, 1.0), (24, 0.0625), (24, 3.0), (600, 1.0), (600, 4.0)])
+def test_activation_packer_ties_and_scales(b200, tokens, gs2):
+    """Inputs with few significant bits put many quotients exactly on the midpoints of the code grid (ties go to the smaller
+    magnitude); the activation scale is a power of two, where one conversion is exact, or not.  Weights that copy
+    activations to the output make every code visible."""
+    rng = np.random.default_rng(tokens)
+    experts, hidden, inter, top_k = 4, 256, 128, 1
+    w1c, w1s, w2c, w2s = random_weights(rng, experts, hidden, inter)
+    x = torch.from_numpy(rng.integers(-48, 49, size=(tokens, hidden)).astype(np.float32) / 8.0).to(torch.bfloat16)
+    ids, wts = O.route_topk_ref(torch.randn(tokens, experts), top_k)
+    a1 = torch.full((experts,), 1.0 / 64.0)
+    ref = O.moe_ref(x, w1c, w1s, w2c, w2s, ids, wts, a1.numpy(), None, gs2)
+    out = run_gpu(b200, x, w1c, w1s, w2c, w2s, ids, wts.contiguous(), w1_alpha=a1.cuda(),
+                  fc2_input_scale=torch.tensor([gs2]).cuda(), slot_rows_dtype=torch.float32)
+    assert rel_l2(out, ref) <= 3e-3
+
+
 def test_hot_expert_and_expert_parallel_split(b200):
     """All tokens share one hot expert (several 128-row blocks of one expert), and the same problem computed as two
     expert-parallel halves accumulated into one output."""
