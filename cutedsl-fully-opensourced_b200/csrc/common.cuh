@@ -91,6 +91,11 @@ __device__ __forceinline__ uint4 ld_once_16B(const void* p) {
   return r;
 }
 
+// the 128-byte line at p (aligned) holds nothing that anybody will read: if it is dirty in L2 it need not go to DRAM
+__device__ __forceinline__ void discard_l2_line(const void* p) {
+  asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
+}
+
 __device__ __forceinline__ void st_32B(void* p, const U32x8& r) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(r.v[0]), "r"(r.v[1]),
                "r"(r.v[2]), "r"(r.v[3]), "r"(r.v[4]), "r"(r.v[5]), "r"(r.v[6]), "r"(r.v[7])

@@ -872,7 +872,7 @@ int launch_moe_stream(const void* x, const void* x_sf, int x_sf_pitch, const voi
   p.early_b = early_b;
   p.early_trigger = trigger;
   auto kern = moe_stream_gemm_kernel<kTok, Epi>;
-  constexpr MoeStreamLayout L = moe_stream_layout(kTok, Epi::kParkElem);
+  constexpr MoeStreamLayout L = moe_stream_layout(kTok, Epi::kParkElem, Epi::kSwiglu);
   static std::atomic<bool> configured[kMaxDevices];
   rc = configure_smem_once(configured, kern, static_cast<int>(L.total));
   if (rc) return rc;

@@ -744,7 +744,7 @@ __global__ void moe_combine_few_kernel(const RowT* partial, const int* slot_row,
 // one sum per slot, one rounding).
 __global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* partial, const int* slot_row,
                                           const float* weights, __nv_bfloat16* out,
-                                          int hidden, int top_k, int accumulate) {
+                                          int hidden, int top_k, int accumulate, int discard) {
   __shared__ int s_rows[64];
   __shared__ float s_w[64];
   const int token = blockIdx.x;
@@ -794,6 +794,14 @@ __global__ void moe_combine_bf16x8_kernel(const __nv_bfloat16* partial, const in
     v.z = Pair16<__nv_bfloat16>::pack(acc[4], acc[5]);
     v.w = Pair16<__nv_bfloat16>::pack(acc[6], acc[7]);
     *reinterpret_cast<uint4*>(o) = v;
+  }
+  if (!discard) return;
+  // the rows have been read for the only time and are still dirty in L2 (see the launch)
+  __syncthreads();
+  const int lines = hidden >> 6;             // 128-byte lines of a row
+  for (int i = threadIdx.x; i < lines * top_k; i += blockDim.x) {
+    const int row = s_rows[i / lines];
+    if (row >= 0) discard_l2_line(partial + static_cast<int64_t>(row) * hidden + (i % lines) * 64);
   }
 }
 
@@ -1080,13 +1088,16 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     return combine(
         moe_combine_kernel<float, float>, dim3(static_cast<unsigned>(tokens)), threads, ws.partial, ws.h.slot_row, route_w, static_cast<float*>(out), hidden, top_k, accumulate);
   } else if (rows_bf16) {
+    // Rows that all fit in half of L2 are discarded after they have been read, which saves writing them to DRAM (333 tokens
+    // of hidden 2048: 81.7 -> 80.7 us a step); of the 134 MB of a prefill step most have left L2 by then (0.3 % slower).
     // hidden is a multiple of 64 (checked above): whole 16-byte pieces (32.8 -> 27.9 us at the prefill shape against
     // 8-byte accesses with one row in flight)
     const int t8 = hidden / 8 >= 256 ? 256 : 128;
     return combine(
         moe_combine_bf16x8_kernel, dim3(static_cast<unsigned>(tokens)), t8,
         reinterpret_cast<const __nv_bfloat16*>(ws.partial), ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out),
-        hidden, top_k, accumulate);
+        hidden, top_k, accumulate,
+        static_cast<int>(slots * static_cast<int64_t>(hidden) * 2 <= (64 << 20)));
   } else {
     return combine(
         moe_combine_kernel<__nv_bfloat16, float>, dim3(static_cast<unsigned>(tokens)), threads, ws.partial, ws.h.slot_row, route_w, static_cast<__nv_bfloat16*>(out), hidden, top_k, accumulate);

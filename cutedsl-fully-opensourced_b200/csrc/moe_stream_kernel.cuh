@@ -12,7 +12,7 @@
 //        and quantises them (same arithmetic as EpilogueSwiglu in gemm_kernel.cuh).
 //   FC2: the two pieces are 256 adjacent output columns; rows leave through shared memory as whole lines.
 //
-// Roles as in gemm_kernel.cuh: warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue, warps 6-9 scale-slab movers;
+// Roles as in gemm_kernel.cuh: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 epilogue, warps 10-13 scale-slab movers;
 // persistent over (block, column block), row block outermost; two accumulators; all waits bounded; no multicast.
 //
 // What bounds it: the stream of the weights.  Steps of hidden 7168, 256 experts, intermediate 2048, top-8, 128-row kernels
@@ -24,18 +24,20 @@
 
 namespace b200fp4 {
 
-constexpr int kMoeStreamThreads = 10 * 32;
+constexpr int kMoeStreamThreads = 14 * 32;
 
 struct MoeStreamLayout {
   int stages;
+  int park_rows;               // rows parked at a time: FC1 all of a tile, FC2 of either piece
   uint32_t x_bytes, sfx_bytes, stage_bytes, park_bytes, total;
 };
-__host__ __device__ constexpr MoeStreamLayout moe_stream_layout(int tok, int park_elem) {
+__host__ __device__ constexpr MoeStreamLayout moe_stream_layout(int tok, int park_elem, bool swiglu) {
   MoeStreamLayout s{};
   s.x_bytes = static_cast<uint32_t>(tok) * 128;
   s.sfx_bytes = 1024;                                    // kTok rows of 16 bytes
   s.stage_bytes = 2 * 16384 + s.x_bytes + 2 * 2048 + s.sfx_bytes;
-  s.park_bytes = static_cast<uint32_t>(tok) * 128 * park_elem;
+  s.park_rows = swiglu ? tok : (park_elem == 4 || tok < 32 ? 16 : 32);
+  s.park_bytes = static_cast<uint32_t>(swiglu ? tok : 2 * s.park_rows) * 128 * park_elem;
   s.stages = tok <= 32 ? 5 : 4;
   s.total = s.stages * s.stage_bytes + 1024 + 512 + s.park_bytes;
   return s;
@@ -64,7 +66,7 @@ template <int kTok, typename Epi>
 __global__ void __launch_bounds__(kMoeStreamThreads, 1)
 moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const __grid_constant__ CUtensorMap tmap_sfx, const GemmParams p, const Epi epi) {
-  constexpr MoeStreamLayout L = moe_stream_layout(kTok, Epi::kParkElem);
+  constexpr MoeStreamLayout L = moe_stream_layout(kTok, Epi::kParkElem, Epi::kSwiglu);
   constexpr int kStages = L.stages;
   constexpr uint32_t kAccCols = 2 * kTok;                // two pieces
   constexpr uint32_t kSfaCol = 2 * kAccCols;             // two accumulators first
@@ -98,7 +100,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
     for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(acc_full_bar(s), 1);
-      ptx::mbar_init(acc_empty_bar(s), 4);
+      ptx::mbar_init(acc_empty_bar(s), 8);
     }
     *abort_flag = 0;
     ptx::fence_mbar_init();
@@ -234,7 +236,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       __syncwarp();
       acc.advance(2);
     }
-  } else if (warp >= 6) {
+  } else if (warp >= 10) {
     // =============================== scale-slab movers ===============================
     const int quarter = warp & 3;
     PipeState st;
@@ -273,52 +275,77 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
   } else {
     // =============================== epilogue ===============================
-    const int quarter = warp & 3;
+    // Two groups of four warps, one warp of each per quarter of tensor memory.  FC1: the groups take the rows by sixteens in
+    // turn; FC2: a piece each.
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int channel = quarter * 32 + lane;
-    const int tid = threadIdx.x - 64;                    // 0..127
+    const int tid = threadIdx.x - 64;                    // 0..255
     if (p.early_b) grid_dependency_wait();
+    // what a tile needs from the tables is read one tile ahead: behind the accumulator's barrier the two dependent loads
+    // would be on the path of every tile
+    struct Tile {
+      int blk, n_blk, rows, group;
+      float alpha;
+    };
+    auto look_up = [&](int tile) {
+      Tile t{};
+      if (tile < num_tiles) {
+        t.blk = tile / p.num_n_blocks;
+        t.n_blk = tile - t.blk * p.num_n_blocks;
+        t.rows = rows_of(t.blk);
+        t.group = max(0, min(ld_word(p.m_block_group + t.blk), p.num_groups - 1));
+        const float* alpha;
+        if constexpr (Epi::kSwiglu) alpha = epi.w1_alpha;
+        else alpha = epi.w2_alpha;
+        t.alpha = alpha == nullptr ? 1.0f : ld_word(alpha + t.group);
+      }
+      return t;
+    };
+    float gs = 1.0f;
+    if constexpr (Epi::kSwiglu) {
+      if (epi.fc2_input_scale != nullptr) gs = ld_word(epi.fc2_input_scale);
+    }
+    const bool gs_pow2 = is_power_of_two(gs);
     PipeState acc;
+    Tile next = look_up(blockIdx.x);
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
-      const int blk = tile / p.num_n_blocks, n_blk = tile - blk * p.num_n_blocks;
-      const int group = max(0, min(ld_word(p.m_block_group + blk), p.num_groups - 1));
-      const int rows = rows_of(blk);
-      const int64_t row0 = static_cast<int64_t>(blk) * kTok;
+      const Tile now = next;
+      next = look_up(tile + gridDim.x);
+      const int rows = now.rows, n_blk = now.n_blk;
+      const int64_t row0 = static_cast<int64_t>(now.blk) * kTok;
       const bool ready = wait_bounded<64>(acc_full_bar(acc.stage), acc.phase, abort_flag);
-      // the four warps go on or give up together: they meet at barriers below
-      if (!ptx::bar_all(1, 128, ready)) {
+      // the eight warps go on or give up together: they meet at barriers below
+      if (!ptx::bar_all(1, 256, ready)) {
         if (lane == 0) atomicOr(p.status, kStatusTimeoutEpilogue);
         break;
       }
       ptx::tc_fence_after_sync();
       const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc.stage * kAccCols;
-      auto release = [&] {
+      auto release = [&] {                               // once per warp and tile, after its last read of the accumulator
         ptx::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(acc_empty_bar(acc.stage));
       };
-      auto meet = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };   // the four epilogue warps
       if constexpr (Epi::kSwiglu) {
-        const float a1 = epi.w1_alpha == nullptr ? 1.0f : ld_word(epi.w1_alpha + group);
-        const float gs = epi.fc2_input_scale == nullptr ? 1.0f : ld_word(epi.fc2_input_scale);
-        const bool gs_pow2 = is_power_of_two(gs);
         __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(park);
+        if (16 * half >= rows) release();
 #pragma unroll 1
-        for (int c0 = 0; c0 < rows; c0 += 16) {
+        for (int c0 = 16 * half; c0 < rows; c0 += 32) {
           uint32_t up[16], gate[16];
           ptx::tmem_ld_32x16(t_acc + c0, up);
           ptx::tmem_ld_32x16(t_acc + kTok + c0, gate);
           ptx::tmem_ld_wait();
-          if (c0 + 16 >= rows) release();
+          if (c0 + 32 >= rows) release();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float u = __fmul_rn(__uint_as_float(up[i]), a1), g = __fmul_rn(__uint_as_float(gate[i]), a1);
+            const float u = __fmul_rn(__uint_as_float(up[i]), now.alpha), g = __fmul_rn(__uint_as_float(gate[i]), now.alpha);
             const float s = __fdividef(g, __fadd_rn(1.0f, __expf(-g)));
             act[(c0 + i) * 128 + channel] = __float2bfloat16_rn(__fmul_rn(s, u));
           }
         }
-        meet();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
         // item: 16 adjacent channels of one token; eight lanes hold the 128 channels of a token
-        for (int item = tid; item < ((rows + 15) & ~15) * 8; item += 128) {
+        for (int item = tid; item < ((rows + 15) & ~15) * 8; item += 256) {
           const int t = item >> 3, b = item & 7;
           const uint4* src = reinterpret_cast<const uint4*>(act + t * 128 + b * 16);
           const uint4 q0 = src[0], q1 = src[1];
@@ -332,40 +359,42 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
             if ((b & 3) == 0) *reinterpret_cast<uint32_t*>(epi.act_sf + (row0 + t) * epi.sf_pitch + n_blk * 8 + b) = sf;
           }
         }
-        meet();                          // the parking space is free again
+        asm volatile("bar.sync 1, 256;" ::: "memory");   // the parking space is free again
       } else {
         using Row = typename Epi::Row;
-        const float a2 = epi.w2_alpha == nullptr ? 1.0f : ld_word(epi.w2_alpha + group);
-        Row* out = reinterpret_cast<Row*>(park);
+        constexpr int kParkRows = L.park_rows;
+        Row* out = reinterpret_cast<Row*>(park) + half * kParkRows * 128;
+        auto meet = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory"); };      // the piece's four warps
+        if (rows == 0) release();
 #pragma unroll 1
-        for (int piece = 0; piece < 2; ++piece) {
+        for (int t0 = 0; t0 < rows; t0 += kParkRows) {
+          const int t1 = min(rows, t0 + kParkRows);
 #pragma unroll 1
-          for (int c0 = 0; c0 < rows; c0 += 16) {
+          for (int c0 = t0; c0 < t1; c0 += 16) {
             uint32_t r[16];
-            ptx::tmem_ld_32x16(t_acc + piece * kTok + c0, r);
+            ptx::tmem_ld_32x16(t_acc + half * kTok + c0, r);
             ptx::tmem_ld_wait();
-            if (piece == 1 && c0 + 16 >= rows) release();
+            if (c0 + 16 >= rows) release();
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              const float v = __fmul_rn(__uint_as_float(r[i]), a2);
-              if constexpr (sizeof(Row) == 4) out[(c0 + i) * 128 + channel] = v;
-              else out[(c0 + i) * 128 + channel] = to_out<Row>(v);
+              const float v = __fmul_rn(__uint_as_float(r[i]), now.alpha);
+              if constexpr (sizeof(Row) == 4) out[(c0 - t0 + i) * 128 + channel] = v;
+              else out[(c0 - t0 + i) * 128 + channel] = to_out<Row>(v);
             }
           }
           meet();
           // rows leave as 16-byte pieces, 128 columns of a row side by side
           constexpr int kPer = 16 / sizeof(Row), kChunks = 128 / kPer;
-          const int col0 = n_blk * 256 + piece * 128;
-          for (int i = tid; i < rows * kChunks; i += 128) {
+          const int col0 = n_blk * 256 + half * 128;
+          for (int i = tid & 127; i < (t1 - t0) * kChunks; i += 128) {
             const int t = i / kChunks, c = i % kChunks;
             if (col0 + c * kPer < epi.hidden)
-              *reinterpret_cast<uint4*>(epi.rows + (row0 + t) * epi.hidden + col0 + c * kPer) =
+              *reinterpret_cast<uint4*>(epi.rows + (row0 + t0 + t) * epi.hidden + col0 + c * kPer) =
                   *reinterpret_cast<const uint4*>(out + t * 128 + c * kPer);
           }
           meet();
         }
       }
-      if (rows == 0) release();
       acc.advance(2);
     }
   }

@@ -114,8 +114,7 @@ def test_few_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_r
 @pytest.mark.parametrize("tokens,gs2", [(24, 1.0), (24, 0.0625), (24, 3.0), (600, 1.0), (600, 4.0)])
 def test_activation_packer_ties_and_scales(b200, tokens, gs2):
     """Inputs with few significant bits put many quotients exactly on the midpoints of the code grid (ties go to the smaller
-    magnitude); the activation scale is a power of two, where one conversion is exact, or not.  Weights that copy
-    activations to the output make every code visible."""
+    magnitude); the activation scale is a power of two, where one conversion is exact, or not."""
     rng = np.random.default_rng(tokens)
     experts, hidden, inter, top_k = 4, 256, 128, 1
     w1c, w1s, w2c, w2s = random_weights(rng, experts, hidden, inter)
@@ -125,7 +124,7 @@ def test_activation_packer_ties_and_scales(b200, tokens, gs2):
     ref = O.moe_ref(x, w1c, w1s, w2c, w2s, ids, wts, a1.numpy(), None, gs2)
     out = run_gpu(b200, x, w1c, w1s, w2c, w2s, ids, wts.contiguous(), w1_alpha=a1.cuda(),
                   fc2_input_scale=torch.tensor([gs2]).cuda(), slot_rows_dtype=torch.float32)
-    assert rel_l2(out, ref) <= 3e-3
+    assert rel_l2(out, ref) <= 5e-3      # a wrong side for the ties alone is several per cent
 
 
 def test_hot_expert_and_expert_parallel_split(b200):
