@@ -490,13 +490,14 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
   signal_when_all_ctas_done(ex, 1, ctrl, kCtrlTicketPlace, &s_flag);
 }
 
-// Few slots (<= 1024): count, scan and row assignment in one CTA -- one launch instead of a memset and three
+// Few slots (<= 3072): count, scan and row assignment in one CTA -- one launch instead of a memset and three
 // kernels, which is most of a decode step's bookkeeping time.  Rows of an expert go to its slots in slot order.
 // rows_per_block, block_stride: as in the place kernel.
 // kRoutePerLane > 0: the router runs here first (one warp per token, the CTA's 32 warps take the tokens in turn;
 // experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
 // step.  0: the ids are inputs.
-template <int kRoutePerLane>
+// kPerThread: slots per thread (1, 2 or 3: up to 1024, 2048 or 3072 slots; at most 128 per warp, which its bytes can count).
+template <int kRoutePerLane, int kPerThread>
 __global__ void __launch_bounds__(1024)
 moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize, int top_k, int* ids,
                          float* weights, int n_slots, int expert_lo, MoeHeader h, int experts, int max_m_blocks,
@@ -506,7 +507,7 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
   __shared__ int s_ids[1024];
   __shared__ int s_warp[32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int used = (n_slots + 31) >> 5;                    // warps that hold slots
+  const int used = (n_slots + 32 * kPerThread - 1) / (32 * kPerThread);      // warps that hold slots
   {
     uint4* clear = reinterpret_cast<uint4*>(s_cnt[warp]);
     if (warp < used) clear[lane] = clear[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
@@ -527,19 +528,34 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
     }
     __syncthreads();
   }
-  int e = -1, rank = 0;
-  if (t < n_slots) {
-    e = (kRoutePerLane > 0 ? s_ids[t] : ids[t]) - expert_lo;
-    if (e < 0 || e >= experts) e = -1;
+  // Slot s * 32 + lane of the warp's share, s < kPerThread.  Position of a slot among the slots of its expert, in slot order:
+  // earlier lanes of its group of 32, then earlier groups of the warp, then earlier warps.
+  int e[kPerThread], rank[kPerThread];
+#pragma unroll
+  for (int s = 0; s < kPerThread; ++s) {
+    const int slot = (warp * kPerThread + s) * 32 + lane;
+    e[s] = -1;
+    if (slot < n_slots) {
+      e[s] = (kRoutePerLane > 0 ? s_ids[slot] : ids[slot]) - expert_lo;
+      if (e[s] < 0 || e[s] >= experts) e[s] = -1;
+    }
   }
-  __syncwarp();
-  // position of the slot among the slots of its expert, in slot order: earlier lanes of the warp, then earlier warps
-  const uint32_t same = __match_any_sync(0xffffffffu, e);
-  rank = __popc(same & ((1u << lane) - 1u));
-  if (e >= 0 && rank == 0) s_cnt[warp][e] = static_cast<uint8_t>(__popc(same));
+#pragma unroll
+  for (int s = 0; s < kPerThread; ++s) {
+    __syncwarp();
+    const uint32_t same = __match_any_sync(0xffffffffu, e[s]);
+    rank[s] = __popc(same & ((1u << lane) - 1u));
+    const bool first = rank[s] == 0;
+    if (e[s] >= 0) rank[s] += s_cnt[warp][e[s]];
+    __syncwarp();
+    if (e[s] >= 0 && first) s_cnt[warp][e[s]] = static_cast<uint8_t>(rank[s] + __popc(same));
+  }
   __syncthreads();
-  if (e >= 0)
-    for (int w = 0; w < warp; ++w) rank += s_cnt[w][e];
+#pragma unroll
+  for (int s = 0; s < kPerThread; ++s) {
+    if (e[s] >= 0)
+      for (int w = 0; w < warp; ++w) rank[s] += s_cnt[w][e[s]];
+  }
   int count = 0;
   if (t < experts)
     for (int w = 0; w < used; ++w) count += s_cnt[w][t];
@@ -571,13 +587,16 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
   }
   if (t == experts - 1) *h.num_m_blocks = min(incl, max_m_blocks);
   __syncthreads();
-  if (t < n_slots) {
+#pragma unroll
+  for (int s = 0; s < kPerThread; ++s) {
+    const int slot = (warp * kPerThread + s) * 32 + lane;
+    if (slot >= n_slots) continue;
     int row = -1;
-    if (e >= 0) {
-      row = (s_first[e] + rank / rows_per_block) * block_stride + rank % rows_per_block;
+    if (e[s] >= 0) {
+      row = (s_first[e[s]] + rank[s] / rows_per_block) * block_stride + rank[s] % rows_per_block;
       if (row >= max_m_blocks * block_stride) row = -1;
     }
-    h.slot_row[t] = row;
+    h.slot_row[slot] = row;
   }
 }
 
@@ -813,6 +832,12 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // tools/perf/bench_flashinfer_b12x.py:70-71) gets several blocks instead of wrong results.
 inline bool moe_few_rows(int64_t tokens, int top_k) { return tokens <= 32 && tokens * top_k <= 1024; }
 
+// Up to this many (token, slot) pairs the bookkeeping of a step is one CTA's work (moe_prepare_small_kernel) instead of three
+// launches.  Whole steps of hidden 2048, intermediate 1408, 64 experts, three launches / one CTA, us: 1100 slots 76.7 / 75.2,
+// 2048 74.6 / 74.6 (ids given 75.1 / 73.9), 3000 75.5 / 76.6 (76.9 / 76.7), 4000 84.5 / 86.6.  With logits the router needs a
+// launch of its own beyond 1024 slots, so the line lies lower there.
+inline bool small_front_end(int slots, bool routed) { return slots <= (routed ? 2048 : 3072); }
+
 // Rows per block of the streaming GEMMs (moe_stream_kernel.cuh), 0 = the 128-row kernels.  The narrowest block that an
 // expert with the average number of rows and two standard deviations more still fits (an expert that does not gets a
 // second block, whose weights then come from L2); blocks of 64 up to an average of 60.  Whole steps, us, 128-row kernels /
@@ -1008,28 +1033,35 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     return fail(kInvalidArgument, "workspace holds %zu bytes, %zu needed", workspace_bytes, ws.total);
   const int slots = static_cast<int>(tokens * top_k);
 
-  if (slots <= 1024) {
+  if (small_front_end(slots, logits != nullptr)) {
     // rows that only pad a block keep whatever their scale bytes held: a row of the accumulator depends on its own row of A
     // only, and rows without data are never read back
     // few slots: one CTA counts, scans and assigns rows in slot order; quantisation splits a token's columns
     // over several CTAs (a decode step is mostly the latency of these small kernels)
-#define B200_PREPARE(PL)                                                                                          \
-  B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL>, dim3(1), dim3(1024), 0, stream, logits, route_experts,   \
+#define B200_PREPARE(PL, PT)                                                                                          \
+  B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL, PT>, dim3(1), dim3(1024), 0, stream, logits, route_experts,   \
                              renormalize, top_k, ids, route_w, slots, expert_lo, ws.h, experts, ws.max_m_blocks,    \
                              per_block, per_block))
-    if (logits == nullptr) {
-      B200_PREPARE(0);
+    if (logits == nullptr && slots <= 1024) {
+      B200_PREPARE(0, 1);
+    } else if (logits == nullptr) {
+      B200_PREPARE(0, 3);
+    } else if (slots > 1024) {
+      // more tokens than one CTA should route one after the other
+      int rc = route_topk(logits, ids, route_w, static_cast<int>(tokens), route_experts, top_k, renormalize, stream);
+      if (rc) return rc;
+      B200_PREPARE(0, 2);
     } else if (route_experts <= 64) {
-      B200_PREPARE(2);
+      B200_PREPARE(2, 1);
     } else if (route_experts <= 128) {
-      B200_PREPARE(4);
+      B200_PREPARE(4, 1);
     } else if (route_experts <= 256) {
-      B200_PREPARE(8);
+      B200_PREPARE(8, 1);
     } else {
       // more experts per lane than the 64 registers of a 1024-thread CTA hold: the router keeps its own launch
       int rc = route_topk(logits, ids, route_w, static_cast<int>(tokens), route_experts, top_k, renormalize, stream);
       if (rc) return rc;
-      B200_PREPARE(0);
+      B200_PREPARE(0, 1);
     }
 #undef B200_PREPARE
     const int parts = (hidden / 16 + 127) / 128;

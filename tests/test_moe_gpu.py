@@ -111,6 +111,30 @@ def test_few_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_r
     test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
 
 
+@pytest.mark.parametrize("tokens,top_k,routed", [(512, 2, True), (513, 2, True), (1024, 2, True), (1025, 2, True), (1536, 2, False),
+                                                 (1537, 2, False), (700, 4, False)])
+def test_front_end_switches(b200, tokens, top_k, routed):
+    """The number of slots at which the single-CTA bookkeeping takes one, two or three slots per thread and at which it hands
+    over to the kernels for many slots, with the router inside and with given ids; one hot expert."""
+    rng = np.random.default_rng(tokens)
+    torch.manual_seed(tokens)
+    experts, hidden, inter = 10, 192, 128
+    w1c, w1s, w2c, w2s = random_weights(rng, experts, hidden, inter)
+    x = torch.randn(tokens, hidden).to(torch.bfloat16)
+    logits = torch.randn(tokens, experts)
+    logits[: tokens // 3, 7] += 1e3
+    ids, wts = O.route_topk_ref(logits, top_k)
+    a1 = torch.full((experts,), 0.02)
+    ref = O.moe_ref(x, w1c, w1s, w2c, w2s, ids, wts, a1.numpy())
+    kw = dict(router_logits=logits.cuda()) if routed else {}
+    out = b200.b12x_fused_moe(
+        x.cuda(), torch.from_numpy(O.pack_e2m1(w1c)).cuda(), six_mode(w1s), torch.from_numpy(O.pack_e2m1(w2c)).cuda(), six_mode(w2s),
+        None if routed else ids.cuda(), None if routed else wts.contiguous().cuda(), experts, top_k, w1_alpha=a1.cuda(), **kw)
+    torch.cuda.synchronize()
+    assert b200._lib.device_status() == 0
+    assert rel_l2(out.cpu(), ref) <= 1e-2
+
+
 @pytest.mark.parametrize("tokens,gs2", [(24, 1.0), (24, 0.0625), (24, 3.0), (600, 1.0), (600, 4.0)])
 def test_activation_packer_ties_and_scales(b200, tokens, gs2):
     """Inputs with few significant bits put many quotients exactly on the midpoints of the code grid (ties go to the smaller
