@@ -519,14 +519,15 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
 // Which kernel: the least estimated time.  Times of the variants over 1 <= m <= 8192 and n, k from 1024 to 8192 (launches
 // back to back, operands larger than L2) follow, within 10 to 15 %,
 //
-//   one CTA or pair per tile:  base + waves * k_steps * step      waves = ceil(tiles / SMs or pairs)
-//   streaming kernel:          base + k_steps / splits * step + bytes of B / 6.5 TB/s      (one wave, two CTAs per SM)
+//   128-row tiles of A:        base + waves * k_steps * step + bytes of B / 6.5 TB/s    waves = ceil(tiles / SMs)
+//   CTA pairs:                 base + waves * k_steps * step + 0.8 us per wave beyond the first
+//   streaming kernel:          base + k_steps / splits * step + bytes of B / 6.5 TB/s   (one wave, two CTAs per SM)
 //
 // base: launch, pipeline fill and the last tile's epilogue; step: one 256-wide (128 bytes) K step of a stage, which grows
 // with the bytes a stage brings in.  Where the lines cross:
-//   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 64, n = 2048, k = 7168: 12.5 against 7.4
-//   m = 512, n = k = 4096: 128-wide tiles 10.2 us, 64-wide 15.2; m = 1024: 256-wide pairs 12.9, 128-wide 16.3
-//   m = 2048, n = 2048, k = 7168: pairs 16.8 us, 128-wide 24.5
+//   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 2, n = 7936, k = 2048: 7.3 against 5.7
+//   m = 512, n = k = 4096: 128-wide tiles 10.2 us, 64-wide 15.2; m = 1024: CTA pairs 11.3, 128-wide 16.2
+//   m = 2657, n = 6912, k = 4608: pairs 41.8 us, 256-wide 45.6;  m = 2665, n = 3584, k = 3712: 23.8 against 22.3
 // Returns a tile_n code.
 // ---------------------------------------------------------------------------
 int choose_tile(int m, int n, int k_bytes, int sms) {
@@ -534,26 +535,26 @@ int choose_tile(int m, int n, int k_bytes, int sms) {
   const int kt = (k_bytes + 127) / 128;
   auto blocks = [](int v, int b) { return static_cast<int64_t>((v + b - 1) / b); };
   auto waves = [](int64_t tiles, int slots) { return static_cast<double>((tiles + slots - 1) / slots); };
+  const double b_us = static_cast<double>(n) * k_bytes / 6.5e6;
   int best = 64;
-  double best_us = 3.4 + waves(mb * blocks(n, 64), sms) * kt * 0.345;
+  double best_us = 3.7 + waves(mb * blocks(n, 64), sms) * kt * 0.275 + b_us;
   auto consider = [&](int code, double us) {
     if (us < best_us) best = code, best_us = us;
   };
-  consider(128, 4.3 + waves(mb * blocks(n, 128), sms) * kt * 0.375);
-  consider(256, 5.0 + waves(mb * blocks(n, 256), sms) * kt * 0.50);
-  consider(512, 5.6 + waves(blocks(m, 256) * blocks(n, 256), sms / 2) * kt * 0.43);
-  const int tok = m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128));
-  for (int t = tok; t >= 32 || t == tok; t /= 2) {          // narrower tiles read B again, but spread over more SMs
+  consider(128, 4.0 + waves(mb * blocks(n, 128), sms) * kt * 0.31 + b_us);
+  const double w256 = waves(mb * blocks(n, 256), sms), w512 = waves(blocks(m, 256) * blocks(n, 256), sms / 2);
+  consider(256, 5.0 + w256 * kt * 0.50 + 0.8 * (w256 - 1.0));
+  consider(512, 5.3 + w512 * kt * 0.37 + 0.8 * (w512 - 1.0));
+  // narrower tiles read B again, but spread over more SMs; up to 16 rows tiles of 32 serve where eight CTAs share a tile
+  for (int t = m <= 32 ? 32 : (m <= 64 ? 64 : 128); t >= (m <= 16 ? 16 : 32); t /= 2) {
     const double base = t <= 16 ? 3.9 : (t <= 32 ? 4.3 : (t <= 64 ? 5.2 : 6.6));
     const double step = t <= 32 ? 0.32 : (t <= 64 ? 0.38 : 0.48);
     const int64_t tiles = blocks(m, t) * blocks(n, 128);
     for (int s = 1; s <= 8; s *= 2) {
-      const int steps = (kt + s - 1) / s;
-      // clusters of eight only while every CTA has an SM of its own (two to an SM leave the last ones waiting: m = 281,
-      // n = 1536, k = 5888 took 19.0 instead of 11.5 us)
-      if (4 * s > t || tiles * s > (s == 8 ? sms : 2 * sms) || s > kt) continue;
-      consider(1000 * s + t, base + steps * step + (tiles * s > sms ? 0.8 : 0.0) +
-                                 static_cast<double>(n) * k_bytes * blocks(m, t) / 6.5e6);
+      // clusters of eight only while every CTA has an SM of its own, of whole groups of sixteen (two to an SM leave the last
+      // ones waiting: m = 281, n = 1536, k = 5888 took 19.0 instead of 11.5 us; 144 CTAs did not fit side by side either)
+      if (4 * s > t || tiles * s > (s == 8 ? sms * 7 / 8 : 2 * sms) || s > kt) continue;
+      consider(1000 * s + t, base + (kt + s - 1) / s * step + (tiles * s > sms ? 0.8 : 0.0) + b_us * blocks(m, t));
     }
   }
   return best;
