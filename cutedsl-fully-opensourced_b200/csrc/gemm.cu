@@ -109,16 +109,16 @@ int make_output_map(CUtensorMap* map, void* base, int64_t rows, int64_t row_byte
   return kOk;
 }
 
-// Tiled scale-factor storage viewed as rows of 256 bytes; a box of 8 rows is the 2 KB slab of one
-// 128-row tile and four 64-wide K tiles.  Rows past the end read as zero.
-int make_sf_map(CUtensorMap* map, const void* base, int64_t total_bytes) {
-  const MapKey key{3, reinterpret_cast<uint64_t>(base), static_cast<uint64_t>(total_bytes), 0, 0, 0};
+// Tiled scale-factor storage viewed as rows of 256 bytes; a box is the slab of `tiles` K tiles (512 bytes each) of one
+// 128-row tile: what a stage needs of it.  Rows past the end read as zero.
+int make_sf_map(CUtensorMap* map, const void* base, int64_t total_bytes, int tiles) {
+  const MapKey key{3, reinterpret_cast<uint64_t>(base), static_cast<uint64_t>(total_bytes), static_cast<uint64_t>(tiles), 0, 0};
   if (cached_map(key, map)) return kOk;
   EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr) return fail(kCudaError, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[2] = {256, static_cast<cuuint64_t>(total_bytes / 256)};
   cuuint64_t strides[1] = {256};
-  cuuint32_t box[2] = {256, 8};
+  cuuint32_t box[2] = {256, static_cast<cuuint32_t>(2 * tiles)};
   cuuint32_t elem[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -290,9 +290,10 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   rc = make_operand_map(&tb, b, n, k_nibbles, 1);
   if (rc) return rc;
   const int64_t rk = sf_vec == 32 ? (k + 127) / 128 : (k + 63) / 64;
-  rc = make_sf_map(&tsa, sfa, static_cast<int64_t>((m + 127) / 128) * rk * 512);
+  const int sf_tiles = fmt8 >= 0 ? 1 : (sf_vec == 32 ? 2 : 4);       // scale tiles per stage
+  rc = make_sf_map(&tsa, sfa, static_cast<int64_t>((m + 127) / 128) * rk * 512, sf_tiles);
   if (rc) return rc;
-  rc = make_sf_map(&tsb, sfb, static_cast<int64_t>((n + 127) / 128) * rk * 512);
+  rc = make_sf_map(&tsb, sfb, static_cast<int64_t>((n + 127) / 128) * rk * 512, sf_tiles);
   if (rc) return rc;
   GemmParams p{};
   p.m_rows = m;

@@ -113,7 +113,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     if (lane == 0) {
       PipeState st;
       bool ok = true;
-      const int tps = 4 >> p.sf_block32;                 // 512-byte scale tiles per stage: 4, 2 or 1
+      constexpr int tps = 4 >> kFlavour;                 // 512-byte scale tiles per stage and 128 rows
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const int m2 = tile % p.num_m_blocks;
         const int n_blk = tile / p.num_m_blocks;
@@ -132,8 +132,8 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           // the scale slabs go first: this CTA's own mover warps (local barrier) carry them into tensor memory
           // while the operand tiles are still on their way
           const uint32_t sbar = sf_loaded_bar(st.stage);
-          ptx::mbar_expect_tx(sbar, kSfaBytes + 4096);
-          // a box is four 512-byte scale tiles, whatever the flavour uses of them; rows past the end read as zero
+          ptx::mbar_expect_tx(sbar, 3 * 512 * tps);
+          // boxes of tps scale tiles; rows past the end read as zero
           ptx::tma_load_2d(ssfa, &tmap_sfa, 0, (m_tile * p.rk + tps * kt) * 2, sbar);
 #pragma unroll
           for (int i = 0; i < 2; ++i)
@@ -144,6 +144,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           st.advance(kStages);
         }
       }
+      let_dependents_launch();                             // the last loads are under way: the next kernel's blocks may line up
     }
   } else if (warp == 1) {
     // =============================== MMA issuer (even CTA only) ===============================
@@ -243,16 +244,18 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
         const uint8_t* slab = smem_gen + st.stage * kPairStageBytes + kABytes + kBBytes + lane * 16;
         const uint32_t t_sf = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kSfaCol + st.stage * kSfSetCols;
-        uint32_t ra[16];
+        // the K blocks that the flavour's scale tiles hold: 4 columns of SFA and 8 of SFB each
+        constexpr int tps = 4 >> kFlavour;
+        uint32_t ra[4 * tps];
 #pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
+        for (int kb = 0; kb < tps; ++kb) {
           const uint4 v = *reinterpret_cast<const uint4*>(slab + 512 * kb);
           ra[4 * kb] = v.x, ra[4 * kb + 1] = v.y, ra[4 * kb + 2] = v.z, ra[4 * kb + 3] = v.w;
         }
-        ptx::tmem_st_32x16(t_sf, ra);
-        uint32_t rb[32];
+        ptx::tmem_st_32xn<4 * tps>(t_sf, ra);
+        uint32_t rb[8 * tps];
 #pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
+        for (int kb = 0; kb < tps; ++kb) {
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const uint4 v = *reinterpret_cast<const uint4*>(slab + kSfaBytes + 2048 * i + 512 * kb);
@@ -260,7 +263,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                         rb[8 * kb + 4 * i + 3] = v.w;
           }
         }
-        ptx::tmem_st_32x32(t_sf + 16, rb);
+        ptx::tmem_st_32xn<8 * tps>(t_sf + 16, rb);
         ptx::tmem_st_wait();
         ptx::tc_fence_before_sync();
         __syncwarp();

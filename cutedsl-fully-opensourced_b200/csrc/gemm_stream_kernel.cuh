@@ -121,6 +121,7 @@ nvfp4_gemm_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         ptx::tma_load_2d(sx, &tmap_x, kt * 128, m0, bar);
         st.advance(kStages);
       }
+      let_dependents_launch();       // the last loads are under way (16 x 8192 x 8192: 11.0 -> 10.3 us a call)
     }
     __syncwarp();
   } else if (warp == 1) {
