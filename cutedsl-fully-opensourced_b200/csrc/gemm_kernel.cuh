@@ -815,9 +815,6 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           st.advance(kStages);
         }
       }
-#ifdef TRIG_END
-      let_dependents_launch();
-#endif
     }
   } else if (warp == 1) {
     // =============================== MMA issuer ===============================

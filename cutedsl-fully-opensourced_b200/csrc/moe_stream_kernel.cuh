@@ -188,9 +188,6 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           st.advance(kStages);
         }
       }
-#ifdef TRIG_END
-      let_dependents_launch();
-#endif
     }
   } else if (warp == 1) {
     // =============================== MMA issuer ===============================
