@@ -128,6 +128,41 @@ int make_sf_map(CUtensorMap* map, const void* base, int64_t total_bytes, int til
   return kOk;
 }
 
+// Weights and scale factors of a grouped 256-wide tile, each as one box (GemmParams::joined).  `parts` = 2: a tile is 128
+// rows of the first half of an expert's rows and the same 128 of the second (up and gate); 1: 256 rows in a row.
+int make_joined_maps(CUtensorMap* tb, CUtensorMap* tsf, const void* w, const void* w_sf, int64_t rows, int k, int64_t groups,
+                     int parts) {
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (enc == nullptr) return fail(kCudaError, "cuTensorMapEncodeTiled is not available from this driver");
+  const auto u = [](int64_t v) { return static_cast<cuuint64_t>(v); };
+  const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+  const MapKey kb{5, reinterpret_cast<uint64_t>(w), u(rows), u(k), u(groups), u(parts)};
+  if (!cached_map(kb, tb)) {
+    const int64_t pitch = k / 2, part_rows = rows / parts;
+    const cuuint64_t dims[4] = {u(pitch), u(part_rows), u(parts), u(groups)};
+    const cuuint64_t strides[3] = {u(pitch), u(pitch * part_rows), u(pitch * rows)};
+    const cuuint32_t box[4] = {128, static_cast<cuuint32_t>(256 / parts), static_cast<cuuint32_t>(parts), 1};
+    CUresult r = enc(tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(w), dims, strides, box, elem,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(kCudaError, "cuTensorMapEncodeTiled (weights) failed with CUresult %d", static_cast<int>(r));
+    remember_map(kb, *tb);
+  }
+  const MapKey ks{6, reinterpret_cast<uint64_t>(w_sf), u(rows), u(k), u(groups), u(parts)};
+  if (!cached_map(ks, tsf)) {
+    const int64_t rk = (k + 63) / 64, tiles = rows / parts / 128;
+    const cuuint64_t dims[5] = {256, u(2 * rk), u(tiles), u(parts), u(groups)};
+    const cuuint64_t strides[4] = {256, u(512 * rk), u(512 * rk * tiles), u(512 * rk * tiles * parts)};
+    const cuuint32_t box[5] = {256, 8, static_cast<cuuint32_t>(2 / parts), static_cast<cuuint32_t>(parts), 1};
+    CUresult r = enc(tsf, CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, const_cast<void*>(w_sf), dims, strides, box, elem,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(kCudaError, "cuTensorMapEncodeTiled (weight scales) failed with CUresult %d", static_cast<int>(r));
+    remember_map(ks, *tsf);
+  }
+  return kOk;
+}
+
 // Row-major scale factors of A: [rows][k / 16] bytes, `pitch` bytes between rows; boxes of box_rows rows x 16 bytes (the
 // scale bytes of one 256-wide K step).  Columns beyond k / 16 read as zero.
 int make_sfa_rows_map(CUtensorMap* map, const void* base, int64_t rows, int k, int64_t pitch, int box_rows = 128) {
@@ -234,7 +269,7 @@ int bounded_wait_selftest(long long limit_cycles, int* gave_up_dev, cudaStream_t
 // tc: tensor map of the output for the variants whose tiles leave through TMA stores (others never touch it)
 template <int kBlockN, bool kSwigluB, int kARows = 128, int kEpi = 0, typename Epilogue>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
-                const Epilogue& epi, int max_tiles, cudaStream_t stream) {
+                const Epilogue& epi, int max_tiles, cudaStream_t stream, const CUtensorMap& tsfb = CUtensorMap{}) {
   auto kern = nvfp4_gemm_kernel<kBlockN, kSwigluB, Epilogue, kARows, kEpi>;
   constexpr SmemLayout L = smem_layout<kBlockN, kSwigluB, Epilogue::kOutBytes, kARows, Epilogue::kParkWide>();
   static std::atomic<bool> configured[kMaxDevices];      // per instantiation and device
@@ -245,11 +280,11 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   if (grid < 1) return kOk;
   // the expert-parallel launches keep full stream order: other ranks' kernels follow their own signals
   if (p.peer.world > 1) {
-    kern<<<grid, gemm_threads(kBlockN, kSwigluB, kEpi), L.total, stream>>>(ta, tb, tc, p, epi);
+    kern<<<grid, gemm_threads(kBlockN, kSwigluB, kEpi), L.total, stream>>>(ta, tb, tc, tsfb, p, epi);
     return check_cuda(cudaGetLastError(), "nvfp4_gemm_kernel launch");
   }
   return check_cuda(launch_dependent(kern, dim3(grid), dim3(gemm_threads(kBlockN, kSwigluB, kEpi)), L.total, stream, ta, tb,
-                                     tc, p, epi),
+                                     tc, tsfb, p, epi),
                     "nvfp4_gemm_kernel launch");
 }
 
@@ -651,7 +686,9 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
   const bool small_a = few_rows != 0 && !narrow;
   int rc = make_operand_map(&ta, xq, static_cast<int64_t>(max_m_blocks) * 128, hidden, 0, small_a ? 32 : 128);
   if (rc) return rc;
-  rc = make_operand_map(&tb, w1, 2 * inter, hidden, experts, narrow ? 64 : 128);
+  CUtensorMap tsfb{};
+  rc = narrow ? make_operand_map(&tb, w1, 2 * inter, hidden, experts, 64)
+              : make_joined_maps(&tb, &tsfb, w1, w1_sf, 2 * static_cast<int64_t>(inter), hidden, experts, 2);
   if (rc) return rc;
   GemmParams p{};
   p.sfa = static_cast<const uint8_t*>(xq_sf);
@@ -675,6 +712,7 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
   if (peer != nullptr) p.peer = *peer;
   p.early_b = early_b;
   p.early_trigger = few_rows;
+  p.joined = !narrow;
   CUtensorMap tsfa{};
   if (sfa_row_pitch != 0) {
     rc = make_sfa_rows_map(&tsfa, xq_sf, static_cast<int64_t>(max_m_blocks) * 128, hidden, sfa_row_pitch);
@@ -686,7 +724,7 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
     p.num_n_blocks = inter / 64;
     return launch_gemm<128, true>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
   }
-  if (small_a) return launch_gemm<256, true, 32>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
+  if (small_a) return launch_gemm<256, true, 32>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
   // Sixteen epilogue warps: each reads its 32 up and 32 gate columns in one go and hands the (single) accumulator
   // back before any SwiGLU arithmetic, so the next tile's MMAs wait for a tensor-memory read only; with eight
   // warps half of the arithmetic ran before the release (FC1 of the prefill shape: 104 us with eight, 91 with
@@ -695,8 +733,8 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
     const char* e = getenv("B200FP4_FC1_EPI");
     return e != nullptr && atoi(e) == 8;
   }();
-  if (epi8) return launch_gemm<256, true>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
-  return launch_gemm<256, true, 128, 16>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
+  if (epi8) return launch_gemm<256, true>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+  return launch_gemm<256, true, 128, 16>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
 }
 
 // Epilogue warps of the 128-wide FC2 tiles (short reductions: three K steps per tile at the prefill shape, so the
@@ -741,7 +779,9 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   const bool small_a = few_rows != 0 && wide;
   int rc = make_operand_map(&ta, act_codes, static_cast<int64_t>(max_m_blocks) * 128, inter, 0, small_a ? 32 : 128);
   if (rc) return rc;
-  rc = make_operand_map(&tb, w2, hidden, inter, experts);
+  CUtensorMap tsfb{};
+  rc = wide ? make_joined_maps(&tb, &tsfb, w2, w2_sf, hidden, inter, experts, 1)
+            : make_operand_map(&tb, w2, hidden, inter, experts);
   if (rc) return rc;
   GemmParams p{};
   p.sfa = static_cast<const uint8_t*>(act_sf);
@@ -761,6 +801,7 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   p.status = status;
   p.row_block_major = 1;
   p.early_b = early_b;
+  p.joined = wide;
   EpilogueStore<RowT> epi{partial, hidden, w2_alpha, 1};
   CUtensorMap tc{};
   rc = make_output_map(&tc, partial, static_cast<int64_t>(max_m_blocks) * 128, static_cast<int64_t>(hidden) * sizeof(RowT),
@@ -770,14 +811,14 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   // 128-wide tile has two accumulators, so its epilogue overlaps the next tile's MMAs.
   if (wide) {
     p.num_n_blocks = hidden / 256;
-    if (small_a) return launch_gemm<256, false, 32>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    if (small_a) return launch_gemm<256, false, 32>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
     if constexpr (sizeof(RowT) == 2) {
       if (park) {
         EpilogueStoreWide<RowT> wepi{w2_alpha};
-        return launch_gemm<256, false>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream);
+        return launch_gemm<256, false>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream, tsfb);
       }
     }
-    return launch_gemm<256, false>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    return launch_gemm<256, false>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
   }
   p.num_n_blocks = (hidden + 127) / 128;
   return launch_gemm<128, false>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
