@@ -109,18 +109,19 @@ int make_output_map(CUtensorMap* map, void* base, int64_t rows, int64_t row_byte
   return kOk;
 }
 
-// Tiled scale-factor storage viewed as rows of 256 bytes; a box is the slab of `tiles` K tiles (512 bytes each) of one
-// 128-row tile: what a stage needs of it.  Rows past the end read as zero.
-int make_sf_map(CUtensorMap* map, const void* base, int64_t total_bytes, int tiles) {
-  const MapKey key{3, reinterpret_cast<uint64_t>(base), static_cast<uint64_t>(total_bytes), static_cast<uint64_t>(tiles), 0, 0};
+// Tiled scale-factor storage [128-row tiles][rk K tiles of 512 bytes] viewed as rows of 256 bytes; a box is the slabs of
+// `k_tiles` K tiles of `box_tiles` adjacent row tiles: what a stage needs of them.  Rows and tiles past the end read as zero.
+int make_sf_map(CUtensorMap* map, const void* base, int64_t tiles, int64_t rk, int k_tiles, int box_tiles) {
+  const MapKey key{3, reinterpret_cast<uint64_t>(base), static_cast<uint64_t>(tiles), static_cast<uint64_t>(rk),
+                   static_cast<uint64_t>(k_tiles), static_cast<uint64_t>(box_tiles)};
   if (cached_map(key, map)) return kOk;
   EncodeTiledFn enc = encode_tiled_fn();
   if (enc == nullptr) return fail(kCudaError, "cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t dims[2] = {256, static_cast<cuuint64_t>(total_bytes / 256)};
-  cuuint64_t strides[1] = {256};
-  cuuint32_t box[2] = {256, static_cast<cuuint32_t>(2 * tiles)};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
+  cuuint64_t dims[3] = {256, static_cast<cuuint64_t>(2 * rk), static_cast<cuuint64_t>(tiles)};
+  cuuint64_t strides[2] = {256, static_cast<cuuint64_t>(512 * rk)};
+  cuuint32_t box[3] = {256, static_cast<cuuint32_t>(2 * k_tiles), static_cast<cuuint32_t>(box_tiles)};
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, elem,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(kCudaError, "cuTensorMapEncodeTiled (scale factors) failed with CUresult %d", static_cast<int>(r));
@@ -326,9 +327,9 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   if (rc) return rc;
   const int64_t rk = sf_vec == 32 ? (k + 127) / 128 : (k + 63) / 64;
   const int sf_tiles = fmt8 >= 0 ? 1 : (sf_vec == 32 ? 2 : 4);       // scale tiles per stage
-  rc = make_sf_map(&tsa, sfa, static_cast<int64_t>((m + 127) / 128) * rk * 512, sf_tiles);
+  rc = make_sf_map(&tsa, sfa, (m + 127) / 128, rk, sf_tiles, 1);
   if (rc) return rc;
-  rc = make_sf_map(&tsb, sfb, static_cast<int64_t>((n + 127) / 128) * rk * 512, sf_tiles);
+  rc = make_sf_map(&tsb, sfb, (n + 127) / 128, rk, sf_tiles, 2);
   if (rc) return rc;
   GemmParams p{};
   p.m_rows = m;

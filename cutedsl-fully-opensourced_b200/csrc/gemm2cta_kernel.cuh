@@ -133,11 +133,10 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           // while the operand tiles are still on their way
           const uint32_t sbar = sf_loaded_bar(st.stage);
           ptx::mbar_expect_tx(sbar, 3 * 512 * tps);
-          // boxes of tps scale tiles; rows past the end read as zero
-          ptx::tma_load_2d(ssfa, &tmap_sfa, 0, (m_tile * p.rk + tps * kt) * 2, sbar);
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-            ptx::tma_load_2d(ssfb + i * 2048, &tmap_sfb, 0, ((n_blk * 2 + i) * p.rk + tps * kt) * 2, sbar);
+          // boxes of tps scale tiles (and row tiles); what lies past the end reads as zero
+          // (one load for both row tiles of B: five loads a step were 2 to 5 % slower, 238.5 -> 232.7 us at 8192^3)
+          ptx::tma_load_3d(ssfa, &tmap_sfa, 0, 2 * tps * kt, m_tile, sbar);
+          ptx::tma_load_3d(ssfb, &tmap_sfb, 0, 2 * tps * kt, 2 * n_blk, sbar);      // both 128-row tiles
           if (rank == 0) ptx::mbar_expect_tx(full_bar(st.stage), 2 * (kABytes + kBBytes));
           ptx::tma2_load_2d(sa, &tmap_a, kt * 128, m_tile * 128, bar);
           ptx::tma2_load_3d(sb, &tmap_b, kt * 128, n_blk * 256 + static_cast<int>(rank) * 128, 0, bar);
@@ -258,7 +257,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         for (int kb = 0; kb < tps; ++kb) {
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            const uint4 v = *reinterpret_cast<const uint4*>(slab + kSfaBytes + 2048 * i + 512 * kb);
+            const uint4 v = *reinterpret_cast<const uint4*>(slab + kSfaBytes + 512 * (tps * i + kb));
             rb[8 * kb + 4 * i] = v.x, rb[8 * kb + 4 * i + 1] = v.y, rb[8 * kb + 4 * i + 2] = v.z,
                         rb[8 * kb + 4 * i + 3] = v.w;
           }
