@@ -111,6 +111,15 @@ def test_few_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_r
     test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
 
 
+@pytest.mark.parametrize("tokens,experts,hidden,inter,top_k", [
+    (150, 2, 320, 128, 1), (150, 2, 256, 384, 1), (200, 3, 832, 640, 2), (150, 2, 512, 1408, 1)])
+@pytest.mark.parametrize("slot_rows", [None, torch.float32], ids=["rows_bf16", "rows_f32"])
+def test_many_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_rows):
+    """The 128-row kernels, whose 256-wide tiles fetch both pieces of the weights and of their scales as one box: last K steps
+    that are not full (K = 320, 832, 128, 384, 640, 1408), one and several column blocks, short and long reductions."""
+    test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
+
+
 @pytest.mark.parametrize("tokens,top_k,routed", [(512, 2, True), (513, 2, True), (1024, 2, True), (1025, 2, True), (1536, 2, False),
                                                  (1537, 2, False), (700, 4, False)])
 def test_front_end_switches(b200, tokens, top_k, routed):
