@@ -763,7 +763,9 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
         for (int i = 0; i < kBPieces; ++i) {
           b_row[i] = kSwigluB ? (i == 0 ? 0 : p.gate_row_offset) + n_blk * kBPieceRows : n_blk * kBlockN + kBPieceRows * i;
-          sfb_row[i] = p.sfb + (static_cast<int64_t>(group) * p.b_row_tiles + (b_row[i] >> 7)) * p.rk * 512;
+          // the last 256-wide column block of an odd number of 128-row tiles: its second slab does not exist
+          const int row_tile = min(b_row[i] >> 7, p.b_row_tiles - 1);
+          sfb_row[i] = p.sfb + (static_cast<int64_t>(group) * p.b_row_tiles + row_tile) * p.rk * 512;
         }
       };
       // One K step.  The scale slabs go first and report to their own barrier: the movers carry them into tensor memory
