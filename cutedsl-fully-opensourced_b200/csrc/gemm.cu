@@ -556,8 +556,8 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
 // Which kernel: the least estimated time.  Times of the variants over 1 <= m <= 8192 and n, k from 1024 to 8192 (launches
 // back to back, operands larger than L2) follow, within 10 to 15 %,
 //
-//   128-row tiles of A:        base + waves * k_steps * step + bytes of B / 6.5 TB/s    waves = ceil(tiles / SMs)
-//   CTA pairs:                 base + waves * k_steps * step + 0.8 us per wave beyond the first
+//   64-wide tiles:             base + waves * k_steps * step + bytes of B / 6.5 TB/s    waves = ceil(tiles / SMs)
+//   wider tiles, CTA pairs:    base + waves * k_steps * step + 0.8 to 2.3 us per wave beyond the first (its drain)
 //   streaming kernel:          base + k_steps / splits * step + bytes of B / 6.5 TB/s   (one wave, two CTAs per SM)
 //
 // base: launch, pipeline fill and the last tile's epilogue; step: one 256-wide (128 bytes) K step of a stage, which grows
@@ -565,7 +565,9 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
 //   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 2, n = 7936, k = 2048: 7.3 against 5.7
 //   m = 512, n = k = 4096: 128-wide tiles 10.2 us, 64-wide 15.2; m = 1024: CTA pairs 11.3, 128-wide 16.2
 //   m = 2657, n = 6912, k = 4608: pairs 41.8 us, 256-wide 45.6;  m = 2665, n = 3584, k = 3712: 23.8 against 22.3
-// Over 72 random shapes the choice took 1.02 times the best variant's time on average.
+//   m = 4024, n = 8192, k = 1280: pairs 25.0 us, 128-wide 40.6
+// The constants of the 128- and 256-wide tiles and of the pairs are a least-squares fit to 60 random shapes (mean error 2 to
+// 5 %); with it 80 random shapes of 128 to 8192 rows took 0.96 times what an estimate without drains chose.
 // Returns a tile_n code.
 // ---------------------------------------------------------------------------
 int choose_tile(int m, int n, int k_bytes, int sms) {
@@ -579,10 +581,11 @@ int choose_tile(int m, int n, int k_bytes, int sms) {
   auto consider = [&](int code, double us) {
     if (us < best_us) best = code, best_us = us;
   };
-  consider(128, 4.0 + waves(mb * blocks(n, 128), sms) * kt * 0.26 + b_us);
+  const double w128 = waves(mb * blocks(n, 128), sms);
+  consider(128, 4.6 + w128 * kt * 0.36 + 0.8 * (w128 - 1.0));
   const double w256 = waves(mb * blocks(n, 256), sms), w512 = waves(blocks(m, 256) * blocks(n, 256), sms / 2);
-  consider(256, 5.0 + w256 * kt * 0.50 + 0.8 * (w256 - 1.0));
-  consider(512, 5.3 + w512 * kt * 0.37 + 0.8 * (w512 - 1.0));
+  consider(256, 5.9 + w256 * kt * 0.44 + 2.3 * (w256 - 1.0));
+  consider(512, 5.4 + w512 * kt * 0.335 + 1.5 * (w512 - 1.0));
   // narrower tiles read B again, but spread over more SMs; up to 16 rows tiles of 32 serve where eight CTAs share a tile
   for (int t = m <= 32 ? 32 : (m <= 64 ? 64 : 128); t >= (m <= 16 ? 16 : 32); t /= 2) {
     const double base = t <= 16 ? 3.9 : (t <= 32 ? 4.3 : (t <= 64 ? 5.2 : 6.6));
