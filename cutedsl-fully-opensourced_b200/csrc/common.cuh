@@ -339,16 +339,17 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // a few ulp; exact(i): the same two values exactly as the golden computes them (only evaluated when a bracket is
 // open: one warp in a hundred; a loop over the open values instead of sixteen copies of the exact rounding made the norm
 // kernel 20 to 40 % slower, it keeps the compiler from interleaving a thread's blocks); amax: the exact largest
-// magnitude.  kOneBranch: one branch for the block instead of one per eight values (2 to 3 % faster in the norm kernel,
-// 1 % slower in the epilogue of the MoE's first GEMM).
+// magnitude, NaN ignored; nothing: what `scale` becomes where the scale factor is zero (0, or NaN where it stands for
+// values that are NaN all by themselves, so that their codes are a NaN's).  kOneBranch: one branch for the block instead
+// of one per eight values (2 to 3 % faster in the norm kernel, 1 % slower in the epilogue of the MoE's first GEMM).
 template <bool kImplicitOne, bool kOneBranch, typename Pair, typename Exact>
-__device__ __forceinline__ void quantize_block16(Pair&& pair, Exact&& exact, float amax, float scale, float gs,
-                                                 uint32_t& codes_lo, uint32_t& codes_hi, uint32_t& sf_bits) {
+__device__ __forceinline__ void quantize_block16(Pair&& pair, Exact&& exact, float amax, float scale, float nothing,
+                                                 float gs, uint32_t& codes_lo, uint32_t& codes_hi, uint32_t& sf_bits) {
   const float sf = fminf(div_by_6(__fmul_rn(amax, gs)), 448.0f);
   sf_bits = e4m3_encode_rn(sf);
   const float div = kImplicitOne ? e4m3_decode_implicit_one(sf_bits) : e4m3_decode(sf_bits);
   // k only has to be within a few ulp of scale / div: the brackets are 2^-19 wide
-  const float k = div > 0.0f ? scale * rcp_approx(div) : 0.0f;
+  const float k = div > 0.0f ? scale * rcp_approx(div) : nothing;
   const float k_hi = k * 1.0000019073486328125f;   // 1 + 2^-19
   const float k_lo = k * 0.9999980926513671875f;   // 1 - 2^-19
   const uint64_t k_hi2 = f32x2_pack(k_hi, k_hi);
@@ -400,7 +401,7 @@ __device__ __forceinline__ void quantize_block16(const uint64_t (&v2)[8], float 
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(fmaxf(amax, fabsf(f32x2_lo(v2[i]))), fabsf(f32x2_hi(v2[i])));
   auto value = [&](int i) { return v2[i]; };
-  quantize_block16<kImplicitOne, kOneBranch>(value, value, amax, gs, gs, codes_lo, codes_hi, sf_bits);
+  quantize_block16<kImplicitOne, kOneBranch>(value, value, amax, gs, 0.0f, gs, codes_lo, codes_hi, sf_bits);
 }
 
 // ---------------------------------------------------------------------------

@@ -192,14 +192,16 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
         quantize_block16<false, true>(val, gs, codes[v][0], codes[v][1], sfb[v]);
       } else {
         // h * rstd rounds monotonically in |h|, so the block's largest value comes from its largest |h|, which packed
-        // 16-bit maxima find; the common factor rstd goes into the quantiser's scale
+        // 16-bit maxima find; the common factor rstd goes into the quantiser's scale.  A row with a NaN or an infinity has an
+        // rstd of NaN or 0, a row of zeros with eps = 0 one of infinity: their values are NaN or zero, and a NaN is no
+        // largest value (fmaxf drops it) as it is none in the other variant
         uint32_t m = Pack16<T>::max_abs(h[c][0], h[c][1]);
 #pragma unroll
         for (int i = 2; i < 8; ++i) m = Pack16<T>::max_abs(m, h[c][i]);
-        const float amax = __fmul_rn(fmaxf(Pair16<T>::lo(m), Pair16<T>::hi(m)), rstd);
+        const float amax = fmaxf(__fmul_rn(fmaxf(Pair16<T>::lo(m), Pair16<T>::hi(m)), rstd), 0.0f);
         quantize_block16<false, true>([&](int i) { return pair16_to_f32x2<T>(h[c][i]); },
-                                [&](int i) { return f32x2_mul(pair16_to_f32x2<T>(h[c][i]), rstd2); }, amax, rstd * gs, gs,
-                                codes[v][0], codes[v][1], sfb[v]);
+                                [&](int i) { return f32x2_mul(pair16_to_f32x2<T>(h[c][i]), rstd2); }, amax, rstd * gs, 0.0f * rstd,
+                                gs, codes[v][0], codes[v][1], sfb[v]);
       }
       if (chunk0 + v >= nchunks) sfb[v] = 0;
     }

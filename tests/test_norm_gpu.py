@@ -137,6 +137,27 @@ def test_rows_of_one_warp_and_padding_blocks(b200, rows, hidden):
     test_ragged_shapes_and_layouts(b200, rows, hidden)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hidden", [512, 1024, 4096, 16384])
+def test_rows_with_nan_infinity_and_zeros(b200, hidden, dtype):
+    """A NaN is no largest value: a row whose 1/rms is NaN, 0 or infinite gets zero scale bytes from either operator (with
+    weights of one and a residual of zero they quantise the same values), a block that only NaN weights touch too."""
+    torch.manual_seed(5)
+    x = torch.randn(6, hidden).to(dtype).cuda()
+    x[1] = 0
+    x[2, 5], x[3, 40], x[4, 100] = float("nan"), float("inf"), -float("inf")
+    x[5, 16:32] = float("nan")
+    w = torch.ones(hidden, dtype=dtype, device="cuda")
+    for eps in (1e-6, 0.0):
+        y, s = b200.rmsnorm_fp4quant(x, w, eps=eps)
+        y_add, s_add = b200.add_rmsnorm_fp4quant(x, torch.zeros_like(x), w, eps=eps)
+        assert torch.equal(s, s_add) and torch.equal(y, y_add)
+        assert (s[0] != 0).all() and (s[1:] == 0).all()
+    w[48:64] = float("nan")
+    y, s = b200.rmsnorm_fp4quant(x, w)
+    assert (s[0, 3] == 0) and (s[0, :3] != 0).all() and (s[0, 4:] != 0).all()
+
+
 def test_three_dim_input_and_strided_rows(b200):
     torch.manual_seed(11)
     base = torch.randn(4, 6, 2 * 512).to(torch.bfloat16).cuda()
