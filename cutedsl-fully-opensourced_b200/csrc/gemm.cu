@@ -129,7 +129,7 @@ int make_sf_map(CUtensorMap* map, const void* base, int64_t tiles, int64_t rk, i
   return kOk;
 }
 
-// Weights and scale factors of a grouped 256-wide tile, each as one box (GemmParams::joined).  `parts` = 2: a tile is 128
+// Weights and scale factors of a grouped 256-wide tile, each as one box (kGroupedJoined).  `parts` = 2: a tile is 128
 // rows of the first half of an expert's rows and the same 128 of the second (up and gate); 1: 256 rows in a row.
 int make_joined_maps(CUtensorMap* tb, CUtensorMap* tsf, const void* w, const void* w_sf, int64_t rows, int k, int64_t groups,
                      int parts) {
@@ -268,10 +268,10 @@ int bounded_wait_selftest(long long limit_cycles, int* gave_up_dev, cudaStream_t
 }
 
 // tc: tensor map of the output for the variants whose tiles leave through TMA stores (others never touch it)
-template <int kBlockN, bool kSwigluB, int kARows = 128, int kEpi = 0, typename Epilogue>
+template <int kBlockN, bool kSwigluB, int kARows = 128, int kEpi = 0, int kTiles = kDense, typename Epilogue>
 int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
                 const Epilogue& epi, int max_tiles, cudaStream_t stream, const CUtensorMap& tsfb = CUtensorMap{}) {
-  auto kern = nvfp4_gemm_kernel<kBlockN, kSwigluB, Epilogue, kARows, kEpi>;
+  auto kern = nvfp4_gemm_kernel<kBlockN, kSwigluB, Epilogue, kARows, kEpi, kTiles>;
   constexpr SmemLayout L = smem_layout<kBlockN, kSwigluB, Epilogue::kOutBytes, kARows, Epilogue::kParkWide>();
   static std::atomic<bool> configured[kMaxDevices];      // per instantiation and device
   int rc_cfg = configure_smem_once(configured, kern, static_cast<int>(L.total));
@@ -716,7 +716,6 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
   if (peer != nullptr) p.peer = *peer;
   p.early_b = early_b;
   p.early_trigger = few_rows;
-  p.joined = !narrow;
   CUtensorMap tsfa{};
   if (sfa_row_pitch != 0) {
     rc = make_sfa_rows_map(&tsfa, xq_sf, static_cast<int64_t>(max_m_blocks) * 128, hidden, sfa_row_pitch);
@@ -726,9 +725,9 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
   EpilogueSwiglu epi{static_cast<uint8_t*>(act_codes), static_cast<uint8_t*>(act_sf), w1_alpha, fc2_input_scale, inter};
   if (narrow) {
     p.num_n_blocks = inter / 64;
-    return launch_gemm<128, true>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    return launch_gemm<128, true, 128, 0, kGrouped>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream);
   }
-  if (small_a) return launch_gemm<256, true, 32>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+  if (small_a) return launch_gemm<256, true, 32, 0, kGroupedJoined>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
   // Sixteen epilogue warps: each reads its 32 up and 32 gate columns in one go and hands the (single) accumulator
   // back before any SwiGLU arithmetic, so the next tile's MMAs wait for a tensor-memory read only; with eight
   // warps half of the arithmetic ran before the release (FC1 of the prefill shape: 104 us with eight, 91 with
@@ -737,8 +736,8 @@ int gemm_moe_fc1(const void* xq, const void* xq_sf, const void* w1, const void* 
     const char* e = getenv("B200FP4_FC1_EPI");
     return e != nullptr && atoi(e) == 8;
   }();
-  if (epi8) return launch_gemm<256, true>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
-  return launch_gemm<256, true, 128, 16>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+  if (epi8) return launch_gemm<256, true, 128, 0, kGroupedJoined>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+  return launch_gemm<256, true, 128, 16, kGroupedJoined>(ta, tb, tsfa, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
 }
 
 // Epilogue warps of the 128-wide FC2 tiles (short reductions: three K steps per tile at the prefill shape, so the
@@ -805,7 +804,6 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   p.status = status;
   p.row_block_major = 1;
   p.early_b = early_b;
-  p.joined = wide;
   EpilogueStore<RowT> epi{partial, hidden, w2_alpha, 1};
   CUtensorMap tc{};
   rc = make_output_map(&tc, partial, static_cast<int64_t>(max_m_blocks) * 128, static_cast<int64_t>(hidden) * sizeof(RowT),
@@ -815,17 +813,17 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
   // 128-wide tile has two accumulators, so its epilogue overlaps the next tile's MMAs.
   if (wide) {
     p.num_n_blocks = hidden / 256;
-    if (small_a) return launch_gemm<256, false, 32>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+    if (small_a) return launch_gemm<256, false, 32, 0, kGroupedJoined>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
     if constexpr (sizeof(RowT) == 2) {
       if (park) {
         EpilogueStoreWide<RowT> wepi{w2_alpha};
-        return launch_gemm<256, false>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+        return launch_gemm<256, false, 128, 0, kGroupedJoined>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream, tsfb);
       }
     }
-    return launch_gemm<256, false>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
+    return launch_gemm<256, false, 128, 0, kGroupedJoined>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
   }
   p.num_n_blocks = (hidden + 127) / 128;
-  return launch_gemm<128, false>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
+  return launch_gemm<128, false, 128, 0, kGrouped>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream);
 }
 
 // FC2 of the expert-parallel MoE: as gemm_moe_fc2 with bf16 rows, but every row is stored into the landing zone
@@ -863,13 +861,13 @@ int gemm_moe_fc2_push(const void* act_codes, const void* act_sf, const void* w2,
   EpiloguePushRows epi{row_tag, peers, recv_off, hidden, w2_alpha, abort_flag};
   if (wide) {
     p.num_n_blocks = hidden / 256;
-    if (small_a) return launch_gemm<256, false, 32>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
-    return launch_gemm<256, false>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    if (small_a) return launch_gemm<256, false, 32, 0, kGrouped>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    return launch_gemm<256, false, 128, 0, kGrouped>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
   }
   p.num_n_blocks = (hidden + 127) / 128;
   if (fc2_epilogue_warps() == 8)
-    return launch_gemm<128, false, 128, 8>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
-  return launch_gemm<128, false>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
+    return launch_gemm<128, false, 128, 8, kGrouped>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
+  return launch_gemm<128, false, 128, 0, kGrouped>(ta, tb, CUtensorMap{}, p, epi, max_m_blocks * p.num_n_blocks, stream);
 }
 
 int gemm_moe_fc2(const void* act_codes, const void* act_sf, const void* w2, const void* w2_sf, void* partial,

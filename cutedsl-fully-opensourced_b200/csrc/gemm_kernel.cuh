@@ -84,11 +84,11 @@ struct GemmParams {
   int gate_row_offset;         // SwiGLU epilogue: first row of the gate half inside B
   // tile list: plain GEMM uses ceil(m_rows/128) row blocks of one group; the grouped GEMMs
   // read the number of row blocks and the group of every row block from device memory
-  const int* num_m_blocks_dev; // null -> num_m_blocks
+  const int* num_m_blocks_dev; // grouped tiles only, as the two tables below
   int num_m_blocks;
-  const int* m_block_group;    // null -> group 0
+  const int* m_block_group;    // group of every row block
   int num_groups;              // groups of B (experts); group indices read from device memory are clamped to it
-  const int* m_block_rows;     // null -> all 128 rows of a block hold data; else rows of the block that do
+  const int* m_block_rows;     // rows of the block that hold data
   int* status;                 // device status word (bits of GemmStatusBits)
   // Order of the tile list.  0: column block outermost (CTAs running together share a few column blocks of B
   // and sweep the rows of A).  1: row block outermost: the CTAs running together hold a few row blocks of A
@@ -125,11 +125,6 @@ struct GemmParams {
   // (57.7 against 59.9 us for the step), launches with more than a few tiles per SM lose (a 16 x 8192 x 8192 GEMM 18.3
   // against 16.9 us, a prefill step 3 to 5 us), so only the few-row FC1 sets it.
   int early_trigger;
-  // Grouped 256-wide tiles: the two pieces of B are one box of a map [groups][parts][rows][bytes of K] and their two scale
-  // slabs one box of a map [groups][parts][128-row tiles][256-byte rows] (parts: up and gate, or one).  A K step is then four
-  // loads instead of six; each costs the load path some 80 cycles (a step takes about 1200).  4096 tokens, 128 experts,
-  // hidden 2048, intermediate 768, top-8: 190.6 -> 188.1 us; 32 experts, 4096, 1024, top-4: 208.6 -> 204.3.
-  int joined;
 };
 
 struct SmemLayout {
@@ -645,12 +640,24 @@ struct EpilogueSwiglu {
 // (one 64-row piece for 64-wide tiles).
 // ----------------------------------------------------------------------------
 // kEpi: number of epilogue warps (0 = the default of the tile shape)
-template <int kBlockN, bool kSwigluB, typename Epilogue, int kARows = 128, int kEpi = 0>
+// kTiles: where tiles and B come from (TileSource).  Fixed when compiled: as flags of the launch the producer tested them in
+// every K step, and one thread issues a step's loads (dense 64-wide tiles, 128 x 8192 x 8192: 16.0 us instead of 15.0;
+// 1024 x 1024 x 8192 16.4 instead of 15.4).
+enum TileSource : int {
+  kDense = 0,          // all tiles of one matrix
+  kGrouped = 1,        // row blocks of the tables, each with its group's B
+  // Grouped 256-wide tiles whose two pieces of B are one box of a map [groups][parts][rows][bytes of K] and their two scale
+  // slabs one box of a map [groups][parts][128-row tiles][256-byte rows] (parts: up and gate, or one).  A K step is then four
+  // loads instead of six; each costs the load path some 80 cycles (a step takes about 1200).  4096 tokens, 128 experts,
+  // hidden 2048, intermediate 768, top-8: 190.6 -> 188.1 us; 32 experts, 4096, 1024, top-4: 208.6 -> 204.3.
+  kGroupedJoined = 2,
+};
+template <int kBlockN, bool kSwigluB, typename Epilogue, int kARows = 128, int kEpi = 0, int kTiles = kDense>
 __global__ void __launch_bounds__(gemm_threads(kBlockN, kSwigluB, kEpi), 1)
 nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_aux, const __grid_constant__ CUtensorMap tmap_sfb, const GemmParams p,
                   const Epilogue epi) {
-  static_assert(kARows == 128 || (kBlockN == 256 && kARows == 32), "few-row stages exist for 256-wide tiles");
+  static_assert(kARows == 128 || (kBlockN == 256 && kARows == 32 && kTiles != kDense), "few-row stages exist for grouped 256-wide tiles");
   constexpr SmemLayout L = smem_layout<kBlockN, kSwigluB, Epilogue::kOutBytes, kARows, Epilogue::kParkWide>();
   constexpr int kStages = L.stages;
   constexpr int kAccStages = kBlockN == 256 ? 1 : 2;
@@ -664,6 +671,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   constexpr uint32_t kSfSetCols = 16 + 4 * kSfbColsPerKb;       // columns of one set of scale slabs (SFA + SFB)
   constexpr uint32_t kIdesc = ptx::idesc_mxf4nvf4(kBlockN);
   constexpr int kFirstSfWarp = 2 + kEpiWarps;
+  constexpr bool kIsGrouped = kTiles != kDense, kJoined = kTiles == kGroupedJoined;
+  static_assert(!kJoined || kBlockN == 256, "joined pieces make 256-wide tiles");
+  const bool early_b = kIsGrouped && p.early_b != 0;
+  const bool sfa_rows = kSwigluB && p.sfa_row_major != 0;       // only the MoE's first GEMM has scale bytes as plain rows
   static_assert(kSfaCol + kStages * kSfSetCols <= kTmemCols, "TMEM budget: one set of slab columns per stage");
 
   extern __shared__ uint8_t smem_raw[];
@@ -699,8 +710,8 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&tmap_a);
     ptx::prefetch_tensormap(&tmap_b);
-    if ((L.epi_stage_bytes != 0 && Epilogue::kUsesOutputMap) || p.sfa_row_major) ptx::prefetch_tensormap(&tmap_aux);
-    if (p.joined) ptx::prefetch_tensormap(&tmap_sfb);
+    if ((L.epi_stage_bytes != 0 && Epilogue::kUsesOutputMap) || sfa_rows) ptx::prefetch_tensormap(&tmap_aux);
+    if constexpr (kJoined) ptx::prefetch_tensormap(&tmap_sfb);
   }
   if (warp == 0) {
     __syncwarp();
@@ -711,11 +722,11 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (!p.early_b) grid_dependency_wait();
+  if (!early_b) grid_dependency_wait();
 
   // grouped launches read the number of row blocks from device memory; never trust it beyond the table size
   const int num_m_blocks =
-      p.num_m_blocks_dev != nullptr ? max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
+      kIsGrouped ? max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
   const int num_out_tiles = num_m_blocks * p.num_n_blocks;
   const int splits = p.k_splits > 1 ? p.k_splits : 1;
   const int kt_per_split = (p.num_k_tiles + splits - 1) / splits;
@@ -736,7 +747,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (lane == 0) {
       PipeState st;
       bool ok = true;
-      if (p.peer.wait_flags != nullptr && p.peer.world > 1) {
+      if (kIsGrouped && p.peer.wait_flags != nullptr && p.peer.world > 1) {
         // rows of A come from the other ranks: wait for their "rows placed" signals (bounded)
         const int epoch = *reinterpret_cast<volatile int*>(p.peer.ctrl + kCtrlEpoch) + 1;
         ok = *reinterpret_cast<volatile int*>(p.peer.ctrl + kCtrlAbort) == 0;
@@ -758,7 +769,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       auto begin_tile = [&](int tile) {
         m_blk = tile_m(tile);
         const int n_blk = tile_n(tile);
-        group = p.m_block_group != nullptr ? max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1)) : 0;
+        if constexpr (kIsGrouped) group = max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1));
         sfa_row = p.sfa + static_cast<int64_t>(m_blk) * p.rk * 512;
 #pragma unroll
         for (int i = 0; i < kBPieces; ++i) {
@@ -778,13 +789,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const uint32_t sf_bytes = static_cast<uint32_t>(min(tps, p.rk - tps * kt)) * 512u;
         const uint32_t sbar = sf_loaded_bar(stage), bar = full_bar(stage);
         // B announces the bytes of the whole stage; a box always delivers its full size
-        if constexpr (kB) ptx::mbar_expect_tx(sbar, (p.sfa_row_major ? 2048u : sf_bytes) + (p.joined ? 2048u : sf_bytes) * kBPieces);
+        if constexpr (kB) ptx::mbar_expect_tx(sbar, (sfa_rows ? 2048u : sf_bytes) + (kJoined ? 2048u : sf_bytes) * kBPieces);
         if constexpr (kA) {
-          if (p.sfa_row_major) ptx::tma_load_2d(ssfa, &tmap_aux, kt * 16, m_blk * kBlockM, sbar);
+          if (sfa_rows) ptx::tma_load_2d(ssfa, &tmap_aux, kt * 16, m_blk * kBlockM, sbar);
           else ptx::bulk_load(ssfa, sfa_row + tps * kt * 512, sf_bytes, sbar);
         }
         if constexpr (kB) {
-          if (p.joined) {
+          if constexpr (kJoined) {
             ptx::tma_load_5d(ssfb, &tmap_sfb, 0, 8 * kt, b_row[0] >> 7, 0, group, sbar);
           } else {
 #pragma unroll
@@ -794,7 +805,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         if constexpr (kA) ptx::tma_load_2d(sa, &tmap_a, kt * 128, m_blk * kBlockM, bar);
         if constexpr (kB) {
-          if (p.joined) {
+          if constexpr (kJoined) {
             ptx::tma_load_4d(sb, &tmap_b, kt * 128, b_row[0], 0, group, bar);
           } else {
 #pragma unroll
@@ -804,7 +815,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
       };
       int primed = 0;                    // stages whose B is under way
-      if (p.early_b) {
+      if (early_b) {
         for (int tile = blockIdx.x; tile < num_tiles && primed < kStages; tile += gridDim.x) {
           begin_tile(tile);
           for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end && primed < kStages; ++kt)
@@ -812,10 +823,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         grid_dependency_wait();
       }
-      if (p.early_trigger) let_dependents_launch();
+      if (kIsGrouped && p.early_trigger) let_dependents_launch();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         begin_tile(tile);
-        if (kARows < kBlockM && p.m_block_rows != nullptr && ld_word(p.m_block_rows + m_blk) > kARows)
+        if (kARows < kBlockM && ld_word(p.m_block_rows + m_blk) > kARows)
           atomicOr(p.status, kStatusRowsExceedTile);      // results of this block are wrong: tell the host
         for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end; ++kt) {
           if (!wait_bounded(empty_bar(st.stage), st.phase ^ 1u, abort_flag)) {
@@ -955,7 +966,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const uint8_t* slab = smem_gen + st.stage * L.stage_bytes + L.a_bytes + L.b_bytes + lane * 16;
         const uint32_t t_sf = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kSfaCol + st.stage * kSfSetCols;
         uint32_t ra[16];
-        if (p.sfa_row_major) {
+        if (sfa_rows) {
           // stage holds [128 rows][16 bytes]: the words of row 32 c + lane are K blocks 0..3 of row group c
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
@@ -1016,21 +1027,21 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int quarter = warp & 3;                      // TMEM lanes this warp may touch
     const int part = (warp - 2) >> 2;                  // which share of the columns (two warps per quarter)
     const int row = quarter * 32 + lane;
-    if (p.early_b) grid_dependency_wait();
+    if (early_b) grid_dependency_wait();
     PipeState acc;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
       const int m_blk = tile_m(tile);
       const int n_blk = tile_n(tile);
       const int group =
-          p.m_block_group != nullptr ? max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1))
-                                     : (splits > 1 ? tile / num_out_tiles : 0);
+          kIsGrouped ? max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1))
+                     : (splits > 1 ? tile / num_out_tiles : 0);
       if (!wait_bounded<64>(acc_full_bar(acc.stage), acc.phase, abort_flag)) {
         if (lane == 0) atomicOr(p.status, kStatusTimeoutEpilogue);
         break;
       }
       ptx::tc_fence_after_sync();
       const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc.stage * kBlockN;
-      const int rows_valid = p.m_block_rows != nullptr ? ld_word(p.m_block_rows + m_blk) : kBlockM;
+      const int rows_valid = kIsGrouped ? ld_word(p.m_block_rows + m_blk) : kBlockM;
       if (quarter * 32 < rows_valid) {                 // a warp whose 32 rows only pad the block has nothing to do
         // parking space of the TMA-store variant: 1024-byte aligned, one slice per epilogue warp
         uint8_t* stage = nullptr;
