@@ -107,16 +107,23 @@ at::Tensor bytes(const at::Tensor& t) { return t.element_size() == 1 ? t : t.vie
 void* data(const at::Tensor& t) { return t.data_ptr(); }
 void* data(const at::Tensor* t) { return t == nullptr ? nullptr : t->data_ptr(); }
 
-// `fn(stream)` with the tensor's device current and without the GIL (a launch blocks while the GPU's queue is full)
+// the GIL is given up for as long as this lives, and is held again when an exception passes through
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
+// `fn(stream)` with the tensor's device current and without the GIL (a launch blocks while the GPU's queue is full).
+// `fn` takes the tensors' addresses, which throws for a tensor without storage (a vmap wrapper, a fake tensor).
 template <typename Fn>
 void launch(at::Device dev, Fn&& fn) {
-  int rc;
   c10::cuda::OptionalCUDAGuard guard;
   if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
   void* stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-  PyThreadState* ts = PyEval_SaveThread();
-  rc = fn(stream);
-  PyEval_RestoreThread(ts);
+  const int rc = [&] {
+    WithoutGil released;
+    return fn(stream);
+  }();
   check(rc);
 }
 

@@ -180,6 +180,21 @@ def test_empty_input(b200):
     assert y.shape == (0, 64)
 
 
+def test_tensors_without_storage_are_refused(b200):
+    """A vmap wrapper has no address to launch with: an ordinary exception, with the interpreter's lock held again."""
+    x = torch.randn(3, 4, 128, device="cuda").to(torch.bfloat16)
+    w = torch.ones(128, dtype=torch.bfloat16, device="cuda")
+    logits, sf = torch.randn(3, 4, 8, device="cuda"), torch.zeros(3, 512, dtype=torch.uint8, device="cuda")
+    q = torch.zeros(128, 32, dtype=torch.uint8, device="cuda")
+    for call in (lambda: torch.vmap(lambda t: b200.rmsnorm_fp4quant(t, w))(x),
+                 lambda: torch.vmap(lambda t: b200.topk_route(t, 2))(logits),
+                 lambda: torch.vmap(lambda t: b200.nvfp4_gemm(q, q, t, t))(sf)):
+        with pytest.raises(RuntimeError):
+            call()
+    y, s = b200.rmsnorm_fp4quant(x, w)
+    assert y.shape == (3, 4, 64) and s.shape == (3, 4, 8)
+
+
 def test_argument_errors(b200):
     w = torch.ones(128, dtype=torch.bfloat16, device="cuda")
     x = torch.randn(4, 128, device="cuda").to(torch.bfloat16)
