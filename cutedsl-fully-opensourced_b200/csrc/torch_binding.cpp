@@ -107,6 +107,15 @@ at::Tensor bytes(const at::Tensor& t) { return t.element_size() == 1 ? t : t.vie
 void* data(const at::Tensor& t) { return t.data_ptr(); }
 void* data(const at::Tensor* t) { return t == nullptr ? nullptr : t->data_ptr(); }
 
+// a kernel of `dev` cannot read the address of a CPU tensor or of one on another GPU
+void on_device(const at::Tensor* t, at::Device dev, const char* name) {
+  if (t != nullptr && (!t->is_cuda() || t->device() != dev)) {
+    std::ostringstream s;
+    s << name << " must be a CUDA tensor on " << dev << " (got " << t->device() << ")";
+    value_error("%s", s.str().c_str());
+  }
+}
+
 // the GIL is given up for as long as this lives, and is held again when an exception passes through
 struct WithoutGil {
   PyThreadState* state = PyEval_SaveThread();
@@ -260,15 +269,14 @@ PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // GEMM operands
 // ---------------------------------------------------------------------------------------------------------------------
 struct Matrix {
-  void* ptr;
   int64_t l, rows, cols;
 };
 // [R, C], [L, R, C], or an (R, C, L) view of memory with L slowest; contiguous, never copied
 Matrix matrix(const at::Tensor& t, const char* what) {
-  if (t.dim() == 2 && t.is_contiguous()) return {data(t), 1, t.size(0), t.size(1)};
+  if (t.dim() == 2 && t.is_contiguous()) return {1, t.size(0), t.size(1)};
   if (t.dim() == 3) {
-    if (t.is_contiguous()) return {data(t), t.size(0), t.size(1), t.size(2)};
-    if (t.permute({2, 0, 1}).is_contiguous()) return {data(t), t.size(2), t.size(0), t.size(1)};
+    if (t.is_contiguous()) return {t.size(0), t.size(1), t.size(2)};
+    if (t.permute({2, 0, 1}).is_contiguous()) return {t.size(2), t.size(0), t.size(1)};
   }
   value_error("%s must be contiguous [rows, cols], [L, rows, cols] or an (rows, cols, L) view of it", what);
 }
@@ -284,6 +292,10 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
                   int sf_vec, int fmt8) {
   if (!a.is_cuda() || !b.is_cuda() || !sfa.is_cuda() || !sfb.is_cuda())
     value_error("operands must be CUDA tensors (there is no CPU implementation)");
+  const at::Device dev = a.device();
+  on_device(&b, dev, "b");
+  on_device(&sfa, dev, "sfa");
+  on_device(&sfb, dev, "sfb");
   const Matrix am = matrix(a, "a"), bm = matrix(b, "b");
   if (am.l != bm.l || am.cols != bm.cols)
     value_error("a %s and b %s disagree on batch or K", shape_of(a).c_str(), shape_of(b).c_str());
@@ -294,7 +306,9 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
   if (sfa.element_size() != 1 || sfb.element_size() != 1 || sfa.numel() < need_a || sfb.numel() < need_b)
     value_error("scale factors must be 1-byte tensors in the 128x4 tiled layout (%lld and %lld bytes)",
                 static_cast<long long>(need_a), static_cast<long long>(need_b));
-  const at::Device dev = a.device();
+  // read as the run of bytes at their address: a view with gaps is not one (a permuted view of a run is)
+  if (!sfa.is_non_overlapping_and_dense() || !sfb.is_non_overlapping_and_dense())
+    value_error("scale factors must lie in one run of memory");
   at::Tensor made;
   if (out_arg == Py_None) {
     if (c_code(out_type) < 0)
@@ -303,6 +317,7 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
     made = a.dim() == 2 ? empty({m, n}, out_type, dev) : empty({l, m, n}, out_type, dev);
   }
   const at::Tensor& c = out_arg == Py_None ? made : tensor(out_arg, "out");
+  on_device(&c, dev, "c");
   const Matrix cm = matrix(c, "c");
   if (cm.l != l || cm.rows != m || cm.cols != n || c_code(c.scalar_type()) < 0)
     value_error("c must be [%lld, %lld] (x%lld) in float16, bfloat16 or float32", static_cast<long long>(m),
@@ -310,7 +325,7 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
   const at::Tensor* alpha = maybe(alpha_arg, "alpha");
   if (alpha != nullptr && (alpha->scalar_type() != at::kFloat || !alpha->is_cuda()))
     value_error("alpha must be a float32 CUDA tensor");
-  if (!c.is_cuda()) value_error("c must be a CUDA tensor");
+  on_device(alpha, dev, "alpha");
   void* ws = nullptr;
   size_t ws_bytes = 0;
   if (ws_arg != Py_None && tile_n == 0 && sf_vec == 16 && fmt8 < 0) {
@@ -329,12 +344,13 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
   launch(dev, [&](void* stream) {
     const float* al = static_cast<const float*>(data(alpha));
     const int cc = c_code(c.scalar_type());
+    void *ap = data(a), *bp = data(b), *cp = data(c);
     if (fmt8 >= 0)
-      return b200fp4_mxfp8_gemm(am.ptr, bm.ptr, data(sfa), data(sfb), cm.ptr, al, mi, ni, ki, li, cc, tile_n, fmt8 & 1,
+      return b200fp4_mxfp8_gemm(ap, bp, data(sfa), data(sfb), cp, al, mi, ni, ki, li, cc, tile_n, fmt8 & 1,
                                 fmt8 >> 1, stream);
     if (sf_vec == 32)
-      return b200fp4_mxfp4_gemm(am.ptr, bm.ptr, data(sfa), data(sfb), cm.ptr, al, mi, ni, ki, li, cc, tile_n, stream);
-    return b200fp4_nvfp4_gemm_ws(am.ptr, bm.ptr, data(sfa), data(sfb), cm.ptr, al, mi, ni, ki, li, cc, tile_n, ws, ws_bytes,
+      return b200fp4_mxfp4_gemm(ap, bp, data(sfa), data(sfb), cp, al, mi, ni, ki, li, cc, tile_n, stream);
+    return b200fp4_nvfp4_gemm_ws(ap, bp, data(sfa), data(sfb), cp, al, mi, ni, ki, li, cc, tile_n, ws, ws_bytes,
                                  stream);
   });
   return give(out_arg, made);
@@ -418,14 +434,6 @@ PyObject* topk_route(PyObject*, PyObject* const* v, Py_ssize_t n) {
 // ---------------------------------------------------------------------------------------------------------------------
 // moe(...): see moe.py for the meaning of the arguments
 // ---------------------------------------------------------------------------------------------------------------------
-void on_device(const at::Tensor* t, at::Device dev, const char* name) {
-  if (t != nullptr && (!t->is_cuda() || t->device() != dev)) {
-    std::ostringstream s;
-    s << name << " must be a CUDA tensor on " << dev << " (got " << t->device() << ")";
-    value_error("%s", s.str().c_str());
-  }
-}
-
 // the six-mode view (32, 4, m_tiles, 4, k_tiles, E) of storage [E, m_tiles, k_tiles, 32, 4, 4], or that storage
 at::Tensor scale_storage(const at::Tensor& sf, int64_t experts, int64_t rows, int64_t k, const char* name) {
   const int64_t need = tiled_bytes(rows, k / 16);

@@ -76,6 +76,48 @@ def test_moe_device_check_names_the_offending_argument(b200):
     _on_device(dev, fc2_input_scale=None)            # optional tensors may be absent
 
 
+def _fake(*shape, dtype=torch.uint8, gpu=0):
+    """A tensor that says it lives on a GPU and has no memory: what the checks before a launch look at."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode():
+        return torch.empty(*shape, dtype=dtype, device=f"cuda:{gpu}")
+
+
+def _gemm_args(**changed):
+    args = {"a": _fake(128, 128), "b": _fake(256, 128), "sfa": _fake(2048), "sfb": _fake(4096),
+            "out": _fake(128, 256, dtype=torch.bfloat16), "alpha": _fake(1, dtype=torch.float32)}
+    args.update(changed)
+    return args
+
+
+@pytest.mark.parametrize("name", ["b", "sfa", "sfb", "out", "alpha"])
+def test_gemm_refuses_a_tensor_of_another_gpu(b200, name):
+    good = _gemm_args()
+    other = _fake(*good[name].shape, dtype=good[name].dtype, gpu=1)
+    with pytest.raises(ValueError, match="must be a CUDA tensor on cuda:0"):
+        b200.nvfp4_gemm(**_gemm_args(**{name: other}))
+    with pytest.raises(ValueError, match="must be a CUDA tensor on cuda:0"):
+        b200.nvfp4_gemm(**_gemm_args(**{name: other}), sf_vec_size=32)
+    fp8 = {n: t.view(torch.float8_e4m3fn) for n, t in (("a", good["a"]), ("b", good["b"]))}
+    if name == "b":
+        other = other.view(torch.float8_e4m3fn)
+    with pytest.raises(ValueError, match="must be a CUDA tensor on cuda:0"):
+        b200.mxfp8_gemm(**_gemm_args(**{**fp8, name: other}))
+    with pytest.raises(RuntimeError):                  # the same call with every tensor on its GPU gets past the checks
+        b200.nvfp4_gemm(**good)
+
+
+def test_gemm_refuses_scale_factors_with_gaps(b200):
+    for name, n in (("sfa", 2048), ("sfb", 4096)):
+        with pytest.raises(ValueError, match="one run of memory"):
+            b200.nvfp4_gemm(**_gemm_args(**{name: _fake(2 * n)[::2]}))
+        with pytest.raises(ValueError, match="one run of memory"):
+            b200.nvfp4_gemm(**_gemm_args(**{name: _fake(n // 16, 32)[:, :16]}))
+        for view in (_fake(n // 512, 32, 4, 4).permute(1, 2, 3, 0), _fake(16, n // 16).t(), _fake(1, 2 * n)[:, :n]):
+            with pytest.raises(RuntimeError):          # one run, whatever the order of its dimensions
+                b200.nvfp4_gemm(**_gemm_args(**{name: view}))
+
+
 def test_pack_moe_weights_matches_the_oracle_quantiser_and_layout(b200):
     torch.manual_seed(0)
     e, inter, hidden = 3, 128, 256
