@@ -554,20 +554,23 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
 
 // ---------------------------------------------------------------------------
 // Which kernel: the least estimated time.  Times of the variants over 1 <= m <= 8192 and n, k from 1024 to 8192 (launches
-// back to back, operands larger than L2) follow, within 10 to 15 %,
+// back to back in a graph, operands larger than L2) follow, within 10 to 15 %,
 //
-//   64-wide tiles:             base + waves * k_steps * step + bytes of B / 6.5 TB/s    waves = ceil(tiles / SMs)
-//   wider tiles, CTA pairs:    base + waves * k_steps * step + 0.8 to 2.3 us per wave beyond the first (its drain)
-//   streaming kernel:          base + k_steps / splits * step + bytes of B / 6.5 TB/s   (one wave, two CTAs per SM)
+//   64-wide tiles:                base + waves * k_steps * step + share * bytes of B / 6.5 TB/s    waves = ceil(tiles / SMs)
+//   128-wide tiles:               the same + 0.9 us per wave beyond the first (its drain)
+//   256-wide tiles, CTA pairs:    base + waves * k_steps * step + 1.5 to 2.3 us per wave beyond the first
+//   streaming kernel:             base + k_steps / splits * step + bytes of B / 6.5 TB/s   (one wave, two CTAs per SM)
 //
 // base: launch, pipeline fill and the last tile's epilogue; step: one 256-wide (128 bytes) K step of a stage, which grows
-// with the bytes a stage brings in.  Where the lines cross:
+// with the bytes a stage brings in; share: how much of the stream of B does not hide behind the steps.  Where the lines cross:
 //   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 2, n = 7936, k = 2048: 7.3 against 5.7
-//   m = 512, n = k = 4096: 128-wide tiles 10.2 us, 64-wide 15.2; m = 1024: CTA pairs 11.3, 128-wide 16.2
+//   m = 128, n = k = 8192: 64-wide tiles 14.2 us, 128-wide 14.9, streaming 4 x 128 15.5;  f32 results 14.2 against 17.2
+//   m = 1280, n = k = 1024: 128-wide tiles 5.6 us, 64-wide 7.0;  m = 512, n = k = 4096: 10.0 against 14.0
 //   m = 2657, n = 6912, k = 4608: pairs 41.8 us, 256-wide 45.6;  m = 2665, n = 3584, k = 3712: 23.8 against 22.3
 //   m = 4024, n = 8192, k = 1280: pairs 25.0 us, 128-wide 40.6
-// The constants of the 128- and 256-wide tiles and of the pairs are a least-squares fit to 60 random shapes (mean error 2 to
-// 5 %); with it 80 random shapes of 128 to 8192 rows took 0.96 times what an estimate without drains chose.
+// The constants of the 64- and 128-wide tiles are a fit to 528 shapes under every variant (three flavours, 16-bit and f32
+// results): the chosen kernel takes 2 % more than the fastest one on average.  Those of the 256-wide tiles and of the pairs
+// are a least-squares fit to 60 random shapes (mean error 2 to 5 %).
 // Returns a tile_n code.
 // ---------------------------------------------------------------------------
 int choose_tile(int m, int n, int k_bytes, int sms) {
@@ -577,12 +580,12 @@ int choose_tile(int m, int n, int k_bytes, int sms) {
   auto waves = [](int64_t tiles, int slots) { return static_cast<double>((tiles + slots - 1) / slots); };
   const double b_us = static_cast<double>(n) * k_bytes / 6.5e6;
   int best = 64;
-  double best_us = 3.7 + waves(mb * blocks(n, 64), sms) * kt * 0.275 + b_us;
+  double best_us = 4.6 + waves(mb * blocks(n, 64), sms) * kt * 0.253 + 0.57 * b_us;
   auto consider = [&](int code, double us) {
     if (us < best_us) best = code, best_us = us;
   };
   const double w128 = waves(mb * blocks(n, 128), sms);
-  consider(128, 4.6 + w128 * kt * 0.36 + 0.8 * (w128 - 1.0));
+  consider(128, 5.2 + w128 * kt * 0.246 + 0.9 * (w128 - 1.0) + 0.56 * b_us);
   const double w256 = waves(mb * blocks(n, 256), sms), w512 = waves(blocks(m, 256) * blocks(n, 256), sms / 2);
   consider(256, 5.9 + w256 * kt * 0.44 + 2.3 * (w256 - 1.0));
   consider(512, 5.4 + w512 * kt * 0.335 + 1.5 * (w512 - 1.0));
