@@ -38,6 +38,7 @@ struct NormParams {
   int64_t x_row_stride;     // elements
   int64_t res_row_stride;   // elements
   bool y_vec16;             // rows of y are 16-byte aligned
+  bool sf_rows_vec4;        // rows of sf_rowmajor are 4-byte aligned
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
       if (p.sf_swizzled != nullptr) *reinterpret_cast<uint32_t*>(p.sf_swizzled + sf_swizzled_offset(row, chunk0, rk)) = quad;
       if (p.sf_rowmajor != nullptr) {
         uint8_t* dst = p.sf_rowmajor + row * nchunks + chunk0;
-        if ((nchunks & 3) == 0) {            // row-major rows are 4-byte aligned
+        if (p.sf_rows_vec4) {
           *reinterpret_cast<uint32_t*>(dst) = quad;
         } else {
           for (int j = 0; j < 4 && chunk0 + j < nchunks; ++j) dst[j] = static_cast<uint8_t>(quad >> (8 * j));
@@ -322,6 +323,7 @@ int norm_fp4quant_launch(const void* x, void* residual, const void* weight, void
   p.res_row_stride = res_row_stride;
 
   p.y_vec16 = hidden % 32 == 0 && (reinterpret_cast<uintptr_t>(y_fp4) & 15) == 0;
+  p.sf_rows_vec4 = hidden % 64 == 0 && (reinterpret_cast<uintptr_t>(p.sf_rowmajor) & 3) == 0;
   if (rows > (1LL << 30)) return fail(kUnsupported, "too many rows");
   const bool add = residual != nullptr;
   if (dtype == 1) return add ? dispatch<__nv_bfloat16, true>(p, stream) : dispatch<__nv_bfloat16, false>(p, stream);

@@ -228,8 +228,9 @@ PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       if (sfup == nullptr) {
         sfu = flat ? empty({rows, kb}, at::kByte, dev) : empty({x.size(0), x.size(1), kb}, at::kByte, dev);
         sfup = &sfu;
-      } else if (sfup->numel() < rows * kb || sfup->element_size() != 1) {
-        value_error("block_scale_unswizzled is too small");
+      } else if (sfup->element_size() != 1 || sfup->numel() < rows * kb || !sfup->is_contiguous()) {
+        value_error("block_scale_unswizzled must be a contiguous 1-byte tensor with at least %lld elements",
+                    static_cast<long long>(rows * kb));
       }
     }
     for (const at::Tensor* t : {yp, sfp, sfup})

@@ -118,6 +118,23 @@ def test_gemm_refuses_scale_factors_with_gaps(b200):
                 b200.nvfp4_gemm(**_gemm_args(**{name: view}))
 
 
+def _norm_args(**changed):
+    bf16 = torch.bfloat16
+    args = {"input": _fake(8, 256, dtype=bf16), "residual": _fake(8, 256, dtype=bf16), "weight": _fake(256, dtype=bf16),
+            "y_fp4": _fake(8, 128), "block_scale": _fake(128, 16), "block_scale_unswizzled": _fake(8, 16),
+            "global_scale": _fake(1, dtype=torch.float32), "output_both_sf_layouts": True}
+    args.update(changed)
+    return args
+
+
+@pytest.mark.parametrize("view", [lambda: _fake(8, 32)[:, :16], lambda: _fake(16, 8).t(), lambda: _fake(256)[::2]])
+def test_norm_refuses_row_major_scales_that_are_no_run_of_rows(b200, view):
+    with pytest.raises(ValueError, match="block_scale_unswizzled must be a contiguous"):
+        b200.add_rmsnorm_fp4quant(**_norm_args(block_scale_unswizzled=view()))
+    with pytest.raises(RuntimeError):                  # a contiguous one, also at an odd offset, gets past the checks
+        b200.add_rmsnorm_fp4quant(**_norm_args(block_scale_unswizzled=_fake(200)[1:129].view(8, 16)))
+
+
 def test_pack_moe_weights_matches_the_oracle_quantiser_and_layout(b200):
     torch.manual_seed(0)
     e, inter, hidden = 3, 128, 256

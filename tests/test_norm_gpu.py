@@ -158,6 +158,22 @@ def test_rows_with_nan_infinity_and_zeros(b200, hidden, dtype):
     assert (s[0, 3] == 0) and (s[0, :3] != 0).all() and (s[0, 4:] != 0).all()
 
 
+@pytest.mark.parametrize("hidden", [512, 1008, 4096])
+def test_row_major_scales_at_any_offset(b200, hidden):
+    """The third output of the two-layout call may start at any byte: rows that are not 4-byte aligned take byte stores."""
+    torch.manual_seed(3)
+    x, r = (torch.randn(5, hidden).to(torch.bfloat16).cuda() for _ in range(2))
+    w = torch.ones(hidden, dtype=torch.bfloat16, device="cuda")
+    n = 5 * hidden // 16
+    y, s, u = b200.add_rmsnorm_fp4quant(x, r.clone(), w, output_both_sf_layouts=True)
+    for offset in range(5):
+        buf = torch.full((n + 16,), 0xA5, dtype=torch.uint8, device="cuda")
+        out = b200.add_rmsnorm_fp4quant(x, r.clone(), w, output_both_sf_layouts=True,
+                                        block_scale_unswizzled=buf[offset:offset + n].view(5, -1))
+        assert torch.equal(out[0], y) and torch.equal(out[1], s) and torch.equal(out[2], u)
+        assert (buf[:offset] == 0xA5).all() and (buf[offset + n:] == 0xA5).all()
+
+
 def test_three_dim_input_and_strided_rows(b200):
     torch.manual_seed(11)
     base = torch.randn(4, 6, 2 * 512).to(torch.bfloat16).cuda()
