@@ -252,8 +252,9 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
 
 template <typename T, bool kAdd, int kVec, int kUnits, bool kWarpRow, int kCap, int kMinCtas>
 int launch_one(const NormParams& p, int threads, cudaStream_t stream) {
-  const int64_t rows = p.sf_swizzled != nullptr ? (p.rows + 127) / 128 * 128 : p.rows;
   const int64_t per_cta = kWarpRow ? kCap / 32 : 1;
+  if (p.rows > (0x7fffffffLL - 128) * per_cta) return fail(kUnsupported, "too many rows");      // blocks of a grid
+  const int64_t rows = p.sf_swizzled != nullptr ? (p.rows + 127) / 128 * 128 : p.rows;
   return check_cuda(launch_dependent(norm_quant_kernel<T, kAdd, kVec, kUnits, kWarpRow, kCap, kMinCtas>,
                                      dim3(static_cast<unsigned>((rows + per_cta - 1) / per_cta)),
                                      dim3(kWarpRow ? kCap : threads), 0, stream, p),
@@ -324,7 +325,6 @@ int norm_fp4quant_launch(const void* x, void* residual, const void* weight, void
 
   p.y_vec16 = hidden % 32 == 0 && (reinterpret_cast<uintptr_t>(y_fp4) & 15) == 0;
   p.sf_rows_vec4 = hidden % 64 == 0 && (reinterpret_cast<uintptr_t>(p.sf_rowmajor) & 3) == 0;
-  if (rows > (1LL << 30)) return fail(kUnsupported, "too many rows");
   const bool add = residual != nullptr;
   if (dtype == 1) return add ? dispatch<__nv_bfloat16, true>(p, stream) : dispatch<__nv_bfloat16, false>(p, stream);
   return add ? dispatch<__half, true>(p, stream) : dispatch<__half, false>(p, stream);

@@ -187,6 +187,17 @@ def test_three_dim_input_and_strided_rows(b200):
                        exact=False)
 
 
+def test_more_rows_than_two_to_the_thirty(b200):
+    """What bounds the rows is the grid (four short rows per block) and memory; one row stands for all of the input."""
+    rows = (1 << 30) + 5
+    row = torch.randn(1, 64, device="cuda").to(torch.bfloat16)
+    y, s = b200.rmsnorm_fp4quant(row.expand(rows, 64), torch.ones(64, dtype=torch.bfloat16, device="cuda"))
+    y, s = y.view(torch.int64), s.view(torch.int32)
+    for part in (slice(0, 1 << 20), slice((1 << 30) - (1 << 20), rows)):
+        assert (y[part] == y[0]).all() and (s[part] == s[0]).all()
+    assert s[0, 0] != 0
+
+
 def test_empty_input(b200):
     x = torch.empty(0, 128, dtype=torch.bfloat16, device="cuda")
     w = torch.ones(128, dtype=torch.bfloat16, device="cuda")
