@@ -74,12 +74,38 @@ const at::Tensor& tensor(PyObject* o, const char* name) {
 // null: None was passed
 const at::Tensor* maybe(PyObject* o, const char* name) { return o == Py_None ? nullptr : &tensor(o, name); }
 
+// Undefined: not a dtype
 at::ScalarType dtype(PyObject* o) {
-  if (!THPDtype_Check(o)) throw Raise{PyExc_TypeError, "dtype must be a torch.dtype"};
-  return reinterpret_cast<THPDtype*>(o)->scalar_type;
+  return THPDtype_Check(o) ? reinterpret_cast<THPDtype*>(o)->scalar_type : at::ScalarType::Undefined;
+}
+// the type of a result that the call makes: None is torch's default type; nothing is asked of it where the caller gives
+// the result's tensor
+at::ScalarType result_dtype(PyObject* o, PyObject* out) {
+  if (o == Py_None) return c10::get_default_dtype_as_scalartype();
+  if (out == Py_None && !THPDtype_Check(o)) throw Raise{PyExc_TypeError, "out_dtype must be a torch.dtype"};
+  return dtype(o);
 }
 int64_t integer(PyObject* o) {
   const int64_t v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw std::exception();
+  return v;
+}
+// o == v in Python's sense (16.0 is 16)
+bool equals(PyObject* o, long v) {
+  if (PyLong_CheckExact(o)) return integer(o) == v;
+  PyObject* want = PyLong_FromLong(v);
+  const int eq = want == nullptr ? -1 : PyObject_RichCompareBool(o, want, Py_EQ);
+  Py_XDECREF(want);
+  if (eq < 0) throw std::exception();
+  return eq != 0;
+}
+// int(o)
+int64_t to_integer(PyObject* o) {
+  if (PyLong_CheckExact(o)) return integer(o);
+  PyObject* i = PyNumber_Long(o);
+  if (i == nullptr) throw std::exception();
+  const int64_t v = PyLong_AsLongLong(i);
+  Py_DECREF(i);
   if (v == -1 && PyErr_Occurred()) throw std::exception();
   return v;
 }
@@ -178,7 +204,7 @@ PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
       value_error("%s", s.str().c_str());
     }
     if (w.scalar_type() != type || w.device() != x.device()) value_error("weight must have the dtype and device of input");
-    if (integer(a[8]) != 16) not_implemented("only NVFP4 (block_size=16, e4m3 scale factors) is implemented");
+    if (!equals(a[8], 16)) not_implemented("only NVFP4 (block_size=16, e4m3 scale factors) is implemented");
     if (a[9] != Py_None && !(PyUnicode_Check(a[9]) && PyUnicode_CompareWithASCIIString(a[9], "e4m3") == 0))
       not_implemented("scale_format: only e4m3 is implemented");
     if (x.dim() != 2 && x.dim() != 3) value_error("input must be [B, H] or [B, S, H]");
@@ -361,7 +387,8 @@ PyObject* product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& sf
 PyObject* nvfp4_gemm(PyObject*, PyObject* const* v, Py_ssize_t n) {
   return guarded(n, 10, [&]() -> PyObject* {
     return product(bytes(tensor(v[0], "a")), bytes(tensor(v[1], "b")), tensor(v[2], "sfa"), tensor(v[3], "sfb"), v[4], v[5],
-                   dtype(v[6]), static_cast<int>(integer(v[7])), v[8], static_cast<int>(integer(v[9])), -1);
+                   result_dtype(v[6], v[5]), static_cast<int>(integer(v[7])), v[8],
+                   equals(v[9], 16) ? 16 : (equals(v[9], 32) ? 32 : 0), -1);
   });
 }
 
@@ -374,8 +401,8 @@ PyObject* mxfp8_gemm(PyObject*, PyObject* const* v, Py_ssize_t n) {
       if (t->scalar_type() == at::kFloat8_e5m2) fmt8 |= t == &a ? 1 : 2;
       else if (t->scalar_type() != at::kFloat8_e4m3fn) value_error("a and b must be float8_e4m3fn or float8_e5m2 tensors");
     }
-    return product(a, b, tensor(v[2], "sfa"), tensor(v[3], "sfb"), v[4], v[5], dtype(v[6]), static_cast<int>(integer(v[7])),
-                   Py_None, 32, fmt8);
+    return product(a, b, tensor(v[2], "sfa"), tensor(v[3], "sfb"), v[4], v[5], result_dtype(v[6], v[5]),
+                   static_cast<int>(integer(v[7])), Py_None, 32, fmt8);
   });
 }
 
@@ -385,11 +412,7 @@ PyObject* mm_fp4(PyObject*, PyObject* const* v, Py_ssize_t n) {
   return guarded(n, 7, [&]() -> PyObject* {
     at::Tensor b = bytes(tensor(v[1], "b")), sfa = tensor(v[2], "a_descale"), sfb = tensor(v[3], "b_descale");
     const at::ScalarType out_type = dtype(v[6]);
-    if (c_code(out_type) < 0) {
-      std::ostringstream s;
-      s << "out_dtype " << out_type;
-      not_implemented("%s", s.str().c_str());
-    }
+    if (c_code(out_type) < 0) not_implemented("out_dtype must be torch.float16, torch.bfloat16 or torch.float32");
     auto storage = [](at::Tensor& t) {
       if (t.dim() != 2 || t.is_contiguous()) return;
       at::Tensor tt = t.t();
@@ -481,7 +504,7 @@ PyObject* moe(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (!x.is_cuda()) value_error("x must be a CUDA tensor (there is no CPU implementation)");
     if (x.dim() != 2 || !x.is_contiguous()) value_error("x must be contiguous [tokens, hidden]");
     const int64_t tokens = x.size(0), hidden = x.size(1);
-    const int64_t num_experts = integer(v[kExperts]), top_k = integer(v[kTopK]), offset = integer(v[kOffset]);
+    const int64_t num_experts = integer(v[kExperts]), top_k = integer(v[kTopK]), offset = to_integer(v[kOffset]);
     const int64_t local = v[kLocal] == Py_None ? num_experts : integer(v[kLocal]);
     const bool accumulate = truth(v[kAccumulate]);
     const at::Device dev = x.device();

@@ -135,6 +135,44 @@ def test_norm_refuses_row_major_scales_that_are_no_run_of_rows(b200, view):
         b200.add_rmsnorm_fp4quant(**_norm_args(block_scale_unswizzled=_fake(200)[1:129].view(8, 16)))
 
 
+def _moe_args(**changed):
+    """hidden 256, intermediate 128, 2 experts, 4 tokens, top-1"""
+    f32 = torch.float32
+    args = {"x": _fake(4, 256, dtype=torch.bfloat16), "w1_weight": _fake(2, 256, 128), "w1_weight_sf": _fake(2, 2 * 4 * 512),
+            "w2_weight": _fake(2, 256, 64), "w2_weight_sf": _fake(2, 2 * 2 * 512),
+            "token_selected_experts": _fake(4, 1, dtype=torch.int32), "token_final_scales": _fake(4, 1, dtype=f32),
+            "num_experts": 2, "top_k": 1, "w1_alpha": _fake(2, dtype=f32), "w2_alpha": _fake(2, dtype=f32),
+            "fc2_input_scale": _fake(1, dtype=f32), "router_logits": _fake(4, 2, dtype=f32),
+            "output": _fake(4, 256, dtype=torch.bfloat16), "workspace": _fake(1 << 22)}
+    args.update(changed)
+    return args
+
+
+def test_argument_forms_that_python_takes_for_the_same(b200):
+    """16.0 is 16, a result type is not looked at beside the result's tensor, and None is torch's default type."""
+    past_the_checks = pytest.raises(RuntimeError)
+    for call in (lambda: b200.add_rmsnorm_fp4quant(**_norm_args(block_size=16.0)),
+                 lambda: b200.nvfp4_gemm(**_gemm_args(), sf_vec_size=16.0),
+                 lambda: b200.nvfp4_gemm(**_gemm_args(), sf_vec_size=32.0),
+                 lambda: b200.nvfp4_gemm(**_gemm_args(), out_dtype=None),
+                 lambda: b200.nvfp4_gemm(**_gemm_args(out=None), out_dtype=None),
+                 lambda: b200.b12x_fused_moe(**_moe_args(local_expert_offset=0.0))):
+        with past_the_checks:
+            call()
+    with pytest.raises(NotImplementedError):
+        b200.add_rmsnorm_fp4quant(**_norm_args(block_size=16.5))
+    with pytest.raises(NotImplementedError):
+        b200.nvfp4_gemm(**_gemm_args(), sf_vec_size=16.5)
+    with pytest.raises(TypeError):
+        b200.nvfp4_gemm(**_gemm_args(out=None), out_dtype="bf16")
+    z = _fake(128, 128)
+    with pytest.raises(NotImplementedError):
+        b200.mm_fp4(z, z.t(), _fake(2048), _fake(2048), out_dtype=None)
+    x, w1, s1, w2, s2, ids, w = _cpu_moe_args()
+    with pytest.raises(NotImplementedError):
+        b200.b12x_fused_moe(x, w1, s1, w2, s2, ids, w, 2, 1, output_dtype=None)
+
+
 def test_pack_moe_weights_matches_the_oracle_quantiser_and_layout(b200):
     torch.manual_seed(0)
     e, inter, hidden = 3, 128, 256
