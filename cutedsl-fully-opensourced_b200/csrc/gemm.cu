@@ -588,7 +588,8 @@ int choose_tile(int m, int n, int k_bytes, int sms) {
   consider(128, 5.2 + w128 * kt * 0.246 + 0.9 * (w128 - 1.0) + 0.56 * b_us);
   const double w256 = waves(mb * blocks(n, 256), sms), w512 = waves(blocks(m, 256) * blocks(n, 256), sms / 2);
   consider(256, 5.9 + w256 * kt * 0.44 + 2.3 * (w256 - 1.0));
-  consider(512, 5.4 + w512 * kt * 0.335 + 1.5 * (w512 - 1.0));
+  static const bool no_pairs = getenv("B200FP4_NO_PAIRS") != nullptr;
+  if (!no_pairs) consider(512, 5.4 + w512 * kt * 0.335 + 1.5 * (w512 - 1.0));
   // narrower tiles read B again, but spread over more SMs; up to 16 rows tiles of 32 serve where eight CTAs share a tile
   for (int t = m <= 32 ? 32 : (m <= 64 ? 64 : 128); t >= (m <= 16 ? 16 : 32); t /= 2) {
     const double base = t <= 16 ? 3.9 : (t <= 32 ? 4.3 : (t <= 64 ? 5.2 : 6.6));

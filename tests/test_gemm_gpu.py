@@ -8,10 +8,15 @@
   CPU's, tolerance rel-L2 <= 1e-5 (the stated bar for N(0,1) operands against
   the de-quantised f32 reference is rel-L2 <= 1e-2).
 """
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
 
+from conftest import ROOT
 from oracle import nvfp4_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -378,3 +383,26 @@ def _mx_flavours(b200, m, n, k, tile_n):
                      (got8, O.gemm_mxfp8_ref(ab, sfa, bb, sfb, alpha=1.0, a_e5m2=False, b_e5m2=True))):
         err = torch.linalg.vector_norm(got.cpu() - ref) / torch.linalg.vector_norm(ref)
         assert err <= 1e-5, float(err)
+
+
+@pytest.mark.parametrize("switch", [None, "1"])
+def test_switch_that_keeps_large_gemms_on_single_cta_tiles(switch):
+    """B200FP4_NO_PAIRS is read once per process: a child that runs one GEMM under a profiler names its kernels."""
+    code = """
+import torch
+import cutedsl_fully_opensourced_b200 as b200
+q, sf = torch.zeros(2048, 1024, dtype=torch.uint8, device="cuda"), torch.zeros(16 * 32 * 512, dtype=torch.uint8, device="cuda")
+b200.nvfp4_gemm(q, q, sf, sf)
+torch.cuda.synchronize()
+with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+    b200.nvfp4_gemm(q, q, sf, sf)
+    torch.cuda.synchronize()
+print([e.key for e in prof.key_averages()])
+"""
+    env = {k: v for k, v in os.environ.items() if k != "B200FP4_NO_PAIRS"}
+    env["PYTHONPATH"] = ROOT
+    if switch is not None:
+        env["B200FP4_NO_PAIRS"] = switch
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert "nvfp4_gemm" in r.stdout and ("nvfp4_gemm_pair_kernel" in r.stdout) == (switch is None), r.stdout
