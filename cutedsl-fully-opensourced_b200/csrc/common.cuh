@@ -67,6 +67,27 @@ __device__ __forceinline__ T ld_word(const T* p) {
   return r;
 }
 
+// What a kernel reads BEFORE its own grid_dependency_wait() (see there): from L2, whatever a line of an earlier launch in
+// this SM's L1 may hold.
+template <typename T>
+__device__ __forceinline__ T ld_early_word(const T* p) {
+  static_assert(sizeof(T) == 4, "words");
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  T r;
+  memcpy(&r, &v, 4);
+  return r;
+}
+__device__ __forceinline__ U32x8 ld_early_32B(const void* p) {
+  U32x8 r;
+  asm volatile("ld.relaxed.gpu.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+                 "=r"(r.v[6]), "=r"(r.v[7])
+               : "l"(p)
+               : "memory");
+  return r;
+}
+
 // read again by other blocks of the SM: through L1
 __device__ __forceinline__ U32x8 ld_cached_32B(const void* p) {
   U32x8 r;
@@ -226,6 +247,11 @@ struct Pack16<__half> {
 // stream drains.  grid_dependency_wait() returns when that kernel is complete and its writes are visible: nothing that
 // an earlier kernel may write or read is touched before it.  let_dependents_launch() lets the next kernel's blocks be
 // scheduled as soon as every block of this one has called it (or has exited).
+// A few reads come before a kernel's own wait: block tables, weights and tokens, all written before its predecessor
+// started.  They rely on every kernel here calling grid_dependency_wait() before let_dependents_launch() unless its
+// dependents read nothing early (the norm): when a dependent may start, the kernels before its predecessor are complete and
+// their writes in L2.  The wait makes those writes visible to the kernel that executes it, not to its dependents, so such
+// words are read past L1 (ld_early_*; TMA reads L2 anyway).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -726,7 +726,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   // grouped launches read the number of row blocks from device memory; never trust it beyond the table size
   const int num_m_blocks =
-      kIsGrouped ? max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
+      kIsGrouped ? max(0, min(ld_early_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
   const int num_out_tiles = num_m_blocks * p.num_n_blocks;
   const int splits = p.k_splits > 1 ? p.k_splits : 1;
   const int kt_per_split = (p.num_k_tiles + splits - 1) / splits;
@@ -766,10 +766,13 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       // what the loads of a tile have in common
       int m_blk = 0, group = 0, b_row[kBPieces];
       const uint8_t *sfa_row = nullptr, *sfb_row[kBPieces];
-      auto begin_tile = [&](int tile) {
+      auto begin_tile = [&](int tile, auto before_wait) {
         m_blk = tile_m(tile);
         const int n_blk = tile_n(tile);
-        if constexpr (kIsGrouped) group = max(0, min(ld_word(p.m_block_group + m_blk), p.num_groups - 1));
+        if constexpr (kIsGrouped) {
+          const int* g = p.m_block_group + m_blk;
+          group = max(0, min(decltype(before_wait)::value ? ld_early_word(g) : ld_word(g), p.num_groups - 1));
+        }
         sfa_row = p.sfa + static_cast<int64_t>(m_blk) * p.rk * 512;
 #pragma unroll
         for (int i = 0; i < kBPieces; ++i) {
@@ -817,7 +820,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int primed = 0;                    // stages whose B is under way
       if (early_b) {
         for (int tile = blockIdx.x; tile < num_tiles && primed < kStages; tile += gridDim.x) {
-          begin_tile(tile);
+          begin_tile(tile, std::true_type{});
           for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end && primed < kStages; ++kt)
             issue(kt, primed++, std::false_type{}, std::true_type{});
         }
@@ -825,7 +828,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
       if (kIsGrouped && p.early_trigger) let_dependents_launch();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        begin_tile(tile);
+        begin_tile(tile, std::false_type{});
         if (kARows < kBlockM && ld_word(p.m_block_rows + m_blk) > kARows)
           atomicOr(p.status, kStatusRowsExceedTile);      // results of this block are wrong: tell the host
         for (int kt = tile_kt0(tile), kt_end = tile_kt1(tile); kt < kt_end; ++kt) {

@@ -354,7 +354,7 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
     const __nv_bfloat16* xrow = x + static_cast<int64_t>(token) * hidden;
     U32x8 raw[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) raw[c] = ld_stream_32B(xrow + g * 64 + c * 16);
+    for (int c = 0; c < 4; ++c) raw[c] = ld_early_32B(xrow + g * 64 + c * 16);
     quad = 0;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -618,7 +618,7 @@ moe_scatter_quant_rows_kernel(const __nv_bfloat16* x, const int* slot_row, uint8
   const bool mine = chunk < (hidden >> 4);
   // the tokens are older than the bookkeeping kernel: quantise while that one still runs
   Block16Codes q{};
-  if (mine) q = quantize_bf16x16_pow2(ld_stream_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16).v, 1.0f);
+  if (mine) q = quantize_bf16x16_pow2(ld_early_32B(x + static_cast<int64_t>(token) * hidden + chunk * 16).v, 1.0f);
   grid_dependency_wait();
   let_dependents_launch();
   if (threadIdx.x < top_k) s_rows[threadIdx.x] = slot_row[static_cast<int64_t>(token) * top_k + threadIdx.x];

@@ -120,7 +120,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (!p.early_b) grid_dependency_wait();
 
   // block counts read from device memory are never trusted beyond the table size
-  const int num_blocks = max(0, min(ld_word(p.num_m_blocks_dev), p.num_m_blocks));
+  const int num_blocks = max(0, min(ld_early_word(p.num_m_blocks_dev), p.num_m_blocks));
   const int num_tiles = num_blocks * p.num_n_blocks;
   auto rows_of = [&](int blk) { return max(0, min(ld_word(p.m_block_rows + blk), kTok)); };
 
@@ -131,10 +131,11 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       bool ok = true;
       int blk = 0, group = 0, w_row[2];
       const uint8_t* sfw[2];
-      auto begin_tile = [&](int tile) {
+      auto begin_tile = [&](int tile, auto before_wait) {
         blk = tile / p.num_n_blocks;
         const int n_blk = tile - blk * p.num_n_blocks;
-        group = max(0, min(ld_word(p.m_block_group + blk), p.num_groups - 1));
+        const int* g = p.m_block_group + blk;
+        group = max(0, min(decltype(before_wait)::value ? ld_early_word(g) : ld_word(g), p.num_groups - 1));
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           w_row[i] = Epi::kSwiglu ? n_blk * 128 + i * p.gate_row_offset : n_blk * 256 + i * 128;
@@ -165,14 +166,14 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       int primed = 0;                    // stages whose weights are under way
       if (p.early_b) {
         for (int tile = blockIdx.x; tile < num_tiles && primed < kStages; tile += gridDim.x) {
-          begin_tile(tile);
+          begin_tile(tile, std::true_type{});
           for (int kt = 0; kt < p.num_k_tiles && primed < kStages; ++kt) issue(kt, primed++, std::false_type{}, std::true_type{});
         }
         grid_dependency_wait();
       }
       if (p.early_trigger) let_dependents_launch();
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        begin_tile(tile);
+        begin_tile(tile, std::false_type{});
         for (int kt = 0; kt < p.num_k_tiles; ++kt) {
           if (!wait_bounded(empty_bar(st.stage), st.phase ^ 1u, abort_flag)) {
             atomicOr(p.status, kStatusTimeoutProducer);
@@ -196,6 +197,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     const uint64_t w_desc0 = ptx::smem_desc_sw128(smem_base);
     const uint64_t x_desc0 = ptx::smem_desc_sw128(smem_base + 32768);
     const int last_kblocks = ((p.k_bytes - (p.num_k_tiles - 1) * 128) + 31) >> 5;
+    if (p.early_b) grid_dependency_wait();               // nothing can be multiplied before the rows are there anyway
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       // N of the instructions: the rows of the block, rounded up to 16
       const int n = kTok == 16 ? 16 : max(16, (rows_of(tile / p.num_n_blocks) + 15) & ~15);

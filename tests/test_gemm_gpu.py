@@ -406,3 +406,42 @@ print([e.key for e in prof.key_averages()])
     r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert "nvfp4_gemm" in r.stdout and ("nvfp4_gemm_pair_kernel" in r.stdout) == (switch is None), r.stdout
+
+
+def test_queued_norm_and_gemm_chains_in_one_place(b200):
+    """norm -> GEMM -> norm -> GEMM without a synchronisation, every buffer reused: each step gives what it gives alone."""
+    torch.manual_seed(29)
+    hidden, rows = 1024, [1, 16, 200, 640]
+    w = torch.ones(hidden, dtype=torch.bfloat16, device="cuda")
+    weights = [b200.gemm.quantize_operand(torch.randn(hidden, hidden, device="cuda")) for _ in range(2)]
+    gs = torch.full((1,), 448.0, device="cuda")
+    alphas = [torch.full((1,), 1.0 / (448.0 * g), device="cuda") for _, _, g in weights]
+    most = max(rows)
+    x, res, c = (torch.empty(most, hidden, dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    y = torch.empty(most, hidden // 2, dtype=torch.uint8, device="cuda")
+    sf = torch.empty(-(-most // 128) * 128 * hidden // 16, dtype=torch.uint8, device="cuda")
+    inputs = [(torch.randn(m, hidden, device="cuda").to(torch.bfloat16), torch.randn(m, hidden, device="cuda").to(torch.bfloat16))
+              for m in rows * 4]
+
+    def step(tokens, residual):
+        m = tokens.shape[0]
+        x[:m].copy_(tokens)
+        res[:m].copy_(residual)
+        for (b, sfb, _), alpha in zip(weights, alphas):
+            b200.add_rmsnorm_fp4quant(x[:m], res[:m], w, y[:m], sf, global_scale=gs, is_sf_swizzled_layout=True)
+            b200.nvfp4_gemm(y[:m], b, sf, sfb, alpha=alpha, out=c[:m])
+            x[:m].copy_(c[:m])
+        b200.add_rmsnorm_fp4quant(c[:m], res[:m], w, y[:m], sf, global_scale=gs, is_sf_swizzled_layout=True)
+        b, sfb, _ = weights[0]
+        return b200.nvfp4_gemm(y[:m], b, sf, sfb, alpha=alphas[0]), res[:m].clone()
+
+    alone = []
+    for s in inputs:
+        torch.cuda.synchronize()
+        alone.append(step(*s))
+        torch.cuda.synchronize()
+    for _ in range(3):
+        queued = [step(*s) for s in inputs]
+        torch.cuda.synchronize()
+        for a, q in zip(alone, queued):
+            assert torch.equal(a[0], q[0]) and torch.equal(a[1], q[1])

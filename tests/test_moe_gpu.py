@@ -389,3 +389,56 @@ def test_packed_checkpoint_weights_run_through_the_operator(b200):
             act = torch.nn.functional.silu(fc1[:, inter:]) * fc1[:, :inter]
             ref[m] += wts[m, j:j + 1] * (act @ w2[e].t())
     assert rel_l2(out, ref) <= 0.35      # 4-bit weights and activations in both GEMMs: ~20 % is the format's own noise
+
+
+def test_queued_calls_with_changing_operands_in_one_place(b200):
+    """Calls that follow one another without a synchronisation on one workspace, with tokens, logits and weights rewritten in
+    place between them, small and large front ends, streaming and 128-row GEMMs: each gives what it gives alone."""
+    torch.manual_seed(23)
+    experts, top_k, hidden, inter, most = 32, 4, 512, 256, 1200
+    packed = [b200.pack_moe_weights(0.05 * torch.randn(experts, 2 * inter, hidden, device="cuda"),
+                                    0.05 * torch.randn(experts, hidden, inter, device="cuda")) for _ in range(2)]
+    w = {k: v.clone() for k, v in packed[0].items()}
+    moe = b200.B12xMoEWrapper(experts, top_k, hidden, inter, max_num_tokens=most)
+    x, logits = torch.empty(most, hidden, dtype=torch.bfloat16, device="cuda"), torch.empty(most, experts, device="cuda")
+    sizes = [1, 7, 64, 300, 600, most]
+    steps = []
+    for i in range(36):
+        n = sizes[(5 * i + i // 6) % 6]
+        bias = torch.zeros(experts, device="cuda").index_fill_(0, torch.randperm(experts, device="cuda")[:4], 3.0)
+        steps.append((i % 2, torch.randn(n, hidden, device="cuda").to(torch.bfloat16),
+                      torch.randn(n, experts, device="cuda") + bias))
+
+    def step(which, tokens, scores):
+        n = tokens.shape[0]
+        for k in ("w1_weight", "w2_weight", "w1_alpha", "w2_alpha"):
+            w[k].copy_(packed[which][k])
+        for k in ("w1_weight_sf", "w2_weight_sf"):
+            w[k].view(torch.uint8).copy_(packed[which][k].view(torch.uint8))
+        x[:n].copy_(tokens)
+        logits[:n].copy_(scores)
+        return moe.run(x[:n], w["w1_weight"], w["w1_weight_sf"], w["w2_weight"], w["w2_weight_sf"],
+                       router_logits=logits[:n], w1_alpha=w["w1_alpha"], w2_alpha=w["w2_alpha"])
+
+    alone = []
+    for s in steps:
+        torch.cuda.synchronize()
+        alone.append(step(*s))
+        torch.cuda.synchronize()
+    for _ in range(3):
+        queued = [step(*s) for s in steps]
+        torch.cuda.synchronize()
+        for a, q in zip(alone, queued):
+            assert torch.equal(a, q)
+    # without the copies in between: the operators' own kernels follow one another directly
+    w1, w2 = packed[0], packed[1]
+    args = [(s[1], p["w1_weight"], p["w1_weight_sf"], p["w2_weight"], p["w2_weight_sf"]) for s in steps for p in (w1, w2)]
+    kw = [dict(router_logits=s[2], w1_alpha=p["w1_alpha"], w2_alpha=p["w2_alpha"]) for s in steps for p in (w1, w2)]
+    alone = []
+    for a, k in zip(args, kw):
+        alone.append(moe.run(*a, **k))
+        torch.cuda.synchronize()
+    queued = [moe.run(*a, **k) for a, k in zip(args, kw)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, q) for a, q in zip(alone, queued))
+    assert b200._lib.device_status() == 0
