@@ -691,10 +691,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint8_t* tail_gen = smem_gen + kStages * L.stage_bytes + 8 * (4 * kStages + 4);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail_gen);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail_gen + 4);
+  volatile int* early_blocks = reinterpret_cast<volatile int*>(tail_gen + 8);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  if (early_b && threadIdx.x == 32) *early_blocks = ld_early_word(p.num_m_blocks_dev);      // one read per CTA: past L1 they add up
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(full_bar(s), 1);
@@ -726,7 +728,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   // grouped launches read the number of row blocks from device memory; never trust it beyond the table size
   const int num_m_blocks =
-      kIsGrouped ? max(0, min(ld_early_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
+      kIsGrouped ? max(0, min(early_b ? *early_blocks : ld_word(p.num_m_blocks_dev), p.num_m_blocks)) : p.num_m_blocks;
   const int num_out_tiles = num_m_blocks * p.num_n_blocks;
   const int splits = p.k_splits > 1 ? p.k_splits : 1;
   const int kt_per_split = (p.num_k_tiles + splits - 1) / splits;

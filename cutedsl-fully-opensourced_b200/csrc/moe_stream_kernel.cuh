@@ -86,11 +86,13 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   uint8_t* tail_gen = smem_gen + kStages * L.stage_bytes + 8 * (4 * kStages + 4);
   volatile uint32_t* tmem_ptr_smem = reinterpret_cast<volatile uint32_t*>(tail_gen);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail_gen + 4);
+  volatile int* early_blocks = reinterpret_cast<volatile int*>(tail_gen + 8);
   uint8_t* park = smem_gen + kStages * L.stage_bytes + 512;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  if (p.early_b && threadIdx.x == 32) *early_blocks = ld_early_word(p.num_m_blocks_dev);    // one read per CTA: past L1 they add up
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(full_bar(s), 1);
@@ -120,7 +122,7 @@ moe_stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (!p.early_b) grid_dependency_wait();
 
   // block counts read from device memory are never trusted beyond the table size
-  const int num_blocks = max(0, min(ld_early_word(p.num_m_blocks_dev), p.num_m_blocks));
+  const int num_blocks = max(0, min(p.early_b ? *early_blocks : ld_word(p.num_m_blocks_dev), p.num_m_blocks));
   const int num_tiles = num_blocks * p.num_n_blocks;
   auto rows_of = [&](int blk) { return max(0, min(ld_word(p.m_block_rows + blk), kTok)); };
 
