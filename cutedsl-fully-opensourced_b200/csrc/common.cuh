@@ -248,10 +248,9 @@ struct Pack16<__half> {
 // an earlier kernel may write or read is touched before it.  let_dependents_launch() lets the next kernel's blocks be
 // scheduled as soon as every block of this one has called it (or has exited).
 // A few reads come before a kernel's own wait: block tables, weights and tokens, all written before its predecessor
-// started.  They rely on every kernel here calling grid_dependency_wait() before let_dependents_launch() unless its
-// dependents read nothing early (the norm): when a dependent may start, the kernels before its predecessor are complete and
-// their writes in L2.  The wait makes those writes visible to the kernel that executes it, not to its dependents, so such
-// words are read past L1 (ld_early_*; TMA reads L2 anyway).
+// started.  They rely on every kernel here calling grid_dependency_wait() before let_dependents_launch(): when a dependent
+// may start, the kernels before its predecessor are complete and their writes in L2.  The wait makes those writes visible
+// to the kernel that executes it, not to its dependents, so such words are read past L1 (ld_early_*; TMA reads L2 anyway).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -90,8 +90,10 @@ __global__ void __launch_bounds__(kCap, kMinCtas) norm_quant_kernel(const NormPa
   if constexpr (!kWarpRow) {
     if (tid < kSlots && tid >= (team >> 5)) red[tid] = 0.0f;       // slots without a warp
   }
-  let_dependents_launch();
+  // (the other way round the blocks of several calls to come line up and hold the slots: add, [128, 16384] bf16, one call after
+  // the other in a graph, 6.2 us instead of 4.8)
   grid_dependency_wait();
+  let_dependents_launch();
   if (row >= p.rows) {                       // only tiled outputs have blocks past the data
     if (p.sf_swizzled != nullptr && row < ((p.rows + 127) & ~int64_t{127})) zero_padding_row(p, row, rk, tid, team);
     return;
