@@ -279,7 +279,8 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   int grid = sm_count_of_current_device();
   if (grid > max_tiles) grid = max_tiles;
   if (grid < 1) return kOk;
-  // the expert-parallel launches keep full stream order: other ranks' kernels follow their own signals
+  // expert-parallel launches that wait for or signal other ranks keep full stream order.  FC2 of the per-rank return does
+  // neither (its rows stay on this GPU) and overlaps FC1's tail like any other: it waits before it reads a row
   if (p.peer.world > 1) {
     kern<<<grid, gemm_threads(kBlockN, kSwigluB, kEpi), L.total, stream>>>(ta, tb, tc, tsfb, p, epi);
     return check_cuda(cudaGetLastError(), "nvfp4_gemm_kernel launch");
@@ -606,8 +607,9 @@ int choose_tile(int m, int n, int k_bytes, int sms) {
 }
 
 // workspace: optional f32 scratch of gemm_workspace_bytes(m, n, k) bytes; with it, problems with few output tiles
-// and a long reduction run split-K (tile_n 0 only).  Without it they run unsplit.
-// sf_vec: 16 = NVFP4 (e4m3 scale per 16 elements), 32 = MXFP4 (ue8m0 scale per 32 elements; single-CTA tiles only)
+// and a long reduction run split-K through global memory (NVFP4, tile_n 0 only).  Without it choose_tile picks a kernel, the
+// streaming one among them, which splits the reduction over a cluster.
+// sf_vec: 16 = NVFP4 (e4m3 scale per 16 elements), 32 = MXFP4 and MXFP8 (ue8m0 scale per 32 elements)
 int gemm_dense(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha, int m, int n,
                int k, int l, int c_dtype, int tile_n, void* workspace, size_t workspace_bytes, int sf_vec, int fmt8,
                cudaStream_t stream) {

@@ -121,9 +121,10 @@ struct GemmParams {
   // Launched as a dependent of the kernel before it (programmatic dependent launch): the block tables and B are older
   // than that kernel, so the producer asks for the first stages of B before it waits for the rows of A.
   int early_b;
-  // Let the next kernel's blocks take over the SMs of blocks that have finished.  Measured: FC1 of a one-token step gains
-  // (57.7 against 59.9 us for the step), launches with more than a few tiles per SM lose (a 16 x 8192 x 8192 GEMM 18.3
-  // against 16.9 us, a prefill step 3 to 5 us), so only the few-row FC1 sets it.
+  // Grouped launches: let the next kernel's blocks take over the SMs of blocks that have finished.  Measured: FC1 of a
+  // one-token step gains (57.7 against 59.9 us for the step, with 128-row tiles), launches with more than a few tiles per SM
+  // lose (a prefill step 3 to 5 us).  Set by the streaming FC1 of up to 1024 slots (moe_stream_kernel.cuh) and by the FC1 of
+  // expert-parallel steps of at most 32 tokens, where it only matters while FC2 is launched as a dependent (per-rank return).
   int early_trigger;
 };
 

@@ -869,7 +869,6 @@ struct MoeWorkspace {
   uint8_t* act;
   uint8_t* act_sf;
   float* partial;
-  size_t clear_bytes;      // ctrl + my_counts
   size_t total;
   int max_m_blocks;
 };
@@ -895,7 +894,6 @@ MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int expert
   w.h.slot_row = reinterpret_cast<int*>(take(sizeof(int) * slots));
   w.ctrl = reinterpret_cast<int*>(take(sizeof(int) * (kCtrlWords + experts)));
   w.my_counts = w.ctrl == nullptr ? nullptr : w.ctrl + kCtrlWords;
-  w.clear_bytes = sizeof(int) * (kCtrlWords + experts);
   w.counts_all = reinterpret_cast<int*>(take(sizeof(int) * experts));
   w.slot_pos = reinterpret_cast<int*>(take(sizeof(int) * slots));
   w.row_tag = reinterpret_cast<int*>(take(sizeof(int) * rows));
@@ -909,8 +907,8 @@ MoeWorkspace carve(void* base, int64_t tokens, int hidden, int inter, int expert
   return w;
 }
 
-// a launch that may overlap the tail of its predecessor on a single GPU; the expert-parallel steps, whose kernels wait for
-// and signal other ranks, keep full stream order
+// a launch that may overlap the tail of its predecessor on a single GPU; in expert-parallel steps the kernels that wait for
+// or signal other ranks keep full stream order
 template <typename... Params, typename... Args>
 cudaError_t launch_in_order(int world, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                             Args&&... args) {
