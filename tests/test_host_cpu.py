@@ -148,6 +148,17 @@ def _moe_args(**changed):
     return args
 
 
+@pytest.mark.parametrize("name", [n for n, v in _moe_args().items() if isinstance(v, torch.Tensor) and n != "x"])
+def test_moe_operator_refuses_a_tensor_of_another_gpu_or_the_cpu(b200, name):
+    """The single-GPU operator checks for itself (the test above covers what the expert-parallel classes call)."""
+    good = _moe_args()
+    for other in (_fake(*good[name].shape, dtype=good[name].dtype, gpu=1), torch.zeros(good[name].shape, dtype=good[name].dtype)):
+        with pytest.raises(ValueError, match=f"{name} must be a CUDA tensor on cuda:0"):
+            b200.b12x_fused_moe(**_moe_args(**{name: other}))
+    with pytest.raises(RuntimeError):                  # with every tensor on its GPU the call gets past the checks
+        b200.b12x_fused_moe(**good)
+
+
 def test_argument_forms_that_python_takes_for_the_same(b200):
     """16.0 is 16, a result type is not looked at beside the result's tensor, and None is torch's default type."""
     past_the_checks = pytest.raises(RuntimeError)
