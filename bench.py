@@ -307,8 +307,8 @@ class GemmPart(Part):
         self.alg_bytes = self.m * k // 2 + n * k // 2 + (self.m + n) * k // 16 + 2 * self.m * n
         # M = 128 streams the weights once: HBM-bound; the larger problems are bound by the tensor pipe
         self.bound = "hbm" if m <= 256 else "tensor"
-        self.kernel = ("nvfp4_gemm_pair_kernel (256x256 tiles on CTA pairs) for a full wave of such tiles, else "
-                       "nvfp4_gemm_kernel<256|128|64>")
+        self.kernel = ("the least estimated time of nvfp4_gemm_pair_kernel (256x256 tiles on CTA pairs), "
+                       "nvfp4_gemm_kernel<256|128|64> and nvfp4_gemm_stream_kernel")
         self.sets = max(3, math.ceil(2 * L2_BYTES / max(1, self.alg_bytes)) + 1)
         # the small problems take less device time than an eager launch through Python costs on the host: they
         # are replayed from CUDA graphs (one per operand set); the large ones are launched eagerly

@@ -74,27 +74,27 @@ int b200fp4_nvfp4_gemm(const void* a, const void* b, const void* sfa, const void
                        int m, int n, int k, int l, int c_dtype, int tile_n, void* stream);
 
 /* The same GEMM with scratch memory for split-K.  Problems with few 128 x 256 output tiles and a long reduction
- * (M = 128 against an 8192 x 8192 weight matrix: a 40 MB weight stream for 32 tiles) leave most SMs idle; with a
+ * (M = 128 against an 8192 x 8192 weight matrix: a 40 MB weight stream for 32 tiles) can be split; with a
  * workspace of b200fp4_nvfp4_gemm_workspace_bytes(m, n, k) bytes (0 = this shape does not split; f32, 16-byte aligned,
  * caller-owned) and tile_n = 0 the K tiles of every output tile are dealt to several CTAs and a second small kernel
  * sums their partial matrices in slice order, applies alpha and rounds once.  workspace = NULL behaves exactly as
- * b200fp4_nvfp4_gemm.  (Measured at M = 128, N = K = 8192: the split kernel takes the same 15 us as the unsplit
- * 64-wide tiles and the reduction adds 4, so nothing selects this by default.)  Same reference interface as above. */
+ * b200fp4_nvfp4_gemm, whose choice of kernels covers such problems: M = 17 / 64 / 128 / 256, N = K = 8192 take 10.7 /
+ * 12.7 / 13.9 / 15.3 us without a workspace and 12.2 / 13.3 / 16.2 / 19.4 with one.  Same reference interface as above. */
 size_t b200fp4_nvfp4_gemm_workspace_bytes(int m, int n, int k);
 int b200fp4_nvfp4_gemm_ws(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha,
                           int m, int n, int k, int l, int c_dtype, int tile_n, void* workspace, size_t workspace_bytes,
                           void* stream);
 
 /* MXFP4 flavour of the same GEMM (sf_vec_size 32 of the demo): e2m1 codes as above, one ue8m0 scale byte (2^(b-127))
- * per 32 K-elements, in the same 128x4 tiles ([l][ceil(rows/128)][ceil(k/128)][32][4][4]).  Single-CTA tiles only
- * (tile_n 0, 64, 128 or 256).  Stands in for the (Float4E2M1FN, Float4E2M1FN, Float8E8M0FNU, 32) configuration of
+ * per 32 K-elements, in the same 128x4 tiles ([l][ceil(rows/128)][ceil(k/128)][32][4][4]).  tile_n as for
+ * b200fp4_nvfp4_gemm.  Stands in for the (Float4E2M1FN, Float4E2M1FN, Float8E8M0FNU, 32) configuration of
  *   .../blockscaled_gemm/blockscaled_gemm_dispatch.py:34-43 and dense_blockscaled_gemm_persistent_cooperative.py:60-68. */
 int b200fp4_mxfp4_gemm(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha,
                        int m, int n, int k, int l, int c_dtype, int tile_n, void* stream);
 
 /* MXFP8 flavour: A [l][m][k] and B [l][n][k] are 8-bit floats (e4m3, or e5m2 where a_e5m2 / b_e5m2 != 0), one ue8m0
  * scale byte per 32 K-elements in 128x4 tiles ([l][ceil(rows/128)][ceil(k/128)][32][4][4]); k a multiple of 16.
- * Single-CTA tiles only.  Stands in for the (Float8E4M3FN | Float8E5M2, ..., Float8E8M0FNU, 32) configurations of
+ * tile_n as for b200fp4_nvfp4_gemm.  Stands in for the (Float8E4M3FN | Float8E5M2, ..., Float8E8M0FNU, 32) configurations of
  *   .../blockscaled_gemm/blockscaled_gemm_dispatch.py:34-43. */
 int b200fp4_mxfp8_gemm(const void* a, const void* b, const void* sfa, const void* sfb, void* c, const float* alpha,
                        int m, int n, int k, int l, int c_dtype, int tile_n, int a_e5m2, int b_e5m2, void* stream);
