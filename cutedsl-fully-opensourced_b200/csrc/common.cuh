@@ -454,7 +454,8 @@ __device__ __forceinline__ Block16Codes quantize_bf16x16_pow2(const uint32_t (&w
   uint32_t m = Pack16<__nv_bfloat16>::max_abs(w[0], w[1]);
 #pragma unroll
   for (int i = 2; i < 8; ++i) m = Pack16<__nv_bfloat16>::max_abs(m, w[i]);
-  const float amax = fmaxf(Pair16<__nv_bfloat16>::lo(m), Pair16<__nv_bfloat16>::hi(m));
+  // (not below zero: the largest of sixteen NaN is a NaN, which is no largest value, here as in the general routine)
+  const float amax = fmaxf(fmaxf(Pair16<__nv_bfloat16>::lo(m), Pair16<__nv_bfloat16>::hi(m)), 0.0f);
   Block16Codes r;
   r.sf = e4m3_encode_rn(fminf(div_by_6(__fmul_rn(amax, gs)), 448.0f));
   const float div = e4m3_decode_implicit_one(r.sf);

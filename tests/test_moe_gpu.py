@@ -391,6 +391,31 @@ def test_packed_checkpoint_weights_run_through_the_operator(b200):
     assert rel_l2(out, ref) <= 0.35      # 4-bit weights and activations in both GEMMs: ~20 % is the format's own noise
 
 
+@pytest.mark.parametrize("tokens", [1, 40, 300, 1500])
+@pytest.mark.parametrize("fc2_input_scale", [None, 3.0])
+def test_blocks_of_nan_get_a_zero_scale(b200, tokens, fc2_input_scale):
+    """Sixteen NaN have no largest value: their scale byte is zero and they add nothing, in the tokens as in the activations
+    (an expert whose alpha is NaN), whatever front end and GEMM the number of tokens takes, whatever the packer's scale."""
+    torch.manual_seed(31)
+    experts, top_k, hidden, inter = 8, 2, 512, 256
+    p = b200.pack_moe_weights(0.05 * torch.randn(experts, 2 * inter, hidden, device="cuda"),
+                              0.05 * torch.randn(experts, hidden, inter, device="cuda"))
+    x = torch.randn(tokens, hidden, device="cuda").to(torch.bfloat16)
+    ids, scales = b200.topk_route(torch.randn(tokens, experts, device="cuda"), top_k)
+    gs = None if fc2_input_scale is None else torch.tensor([fc2_input_scale], device="cuda")
+
+    def run(value, alpha):
+        t, a = x.clone(), p["w1_alpha"].clone()
+        t[0, 32:48] = value
+        t[tokens // 2, :16] = value
+        a[int(ids[0, 0])] = alpha
+        return b200.b12x_fused_moe(t, p["w1_weight"], p["w1_weight_sf"], p["w2_weight"], p["w2_weight_sf"], ids, scales,
+                                   experts, top_k, w1_alpha=a, w2_alpha=p["w2_alpha"], fc2_input_scale=gs)
+
+    nan, zero = run(float("nan"), float("nan")), run(0.0, 0.0)
+    assert torch.isfinite(zero).all() and torch.equal(nan, zero)
+
+
 def test_queued_calls_with_changing_operands_in_one_place(b200):
     """Calls that follow one another without a synchronisation on one workspace, with tokens, logits and weights rewritten in
     place between them, small and large front ends, streaming and 128-row GEMMs: each gives what it gives alone."""
