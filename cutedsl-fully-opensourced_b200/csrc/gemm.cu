@@ -291,16 +291,15 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 }
 
 template <int kFlavour, typename Epilogue>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tsa, const CUtensorMap& tsb,
-                const CUtensorMap& tc, const GemmParams& p, const Epilogue& epi, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_part, const CUtensorMap& tsa, const CUtensorMap& tsb,
+                const CUtensorMap& tc, const GemmParams& p, const PairUnits& units, const Epilogue& epi, cudaStream_t stream) {
   auto kern = nvfp4_gemm_pair_kernel<Epilogue, kFlavour>;
   constexpr uint32_t kSmem = pair_smem_bytes(Epilogue::kParkWide);
   static std::atomic<bool> configured[kMaxDevices];
   int rc = configure_smem_once(configured, kern, static_cast<int>(kSmem));
   if (rc) return rc;
-  const int pairs = std::min(sm_count_of_current_device() / 2, p.num_m_blocks * p.num_n_blocks);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.gridDim = dim3(2 * std::min(sm_count_of_current_device() / 2, units.num), 1, 1);
   cfg.blockDim = dim3(kPairThreads, 1, 1);
   cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;
@@ -313,7 +312,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tsa, tsb, tc, p, epi), "nvfp4_gemm_pair_kernel launch");
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, ta, tb, tb_part, tsa, tsb, tc, p, units, epi), "nvfp4_gemm_pair_kernel launch");
 }
 
 // CTA-pair variant: 256 x 256 tiles on 2-CTA clusters
@@ -346,10 +345,16 @@ int gemm_dense_pair(const void* a, const void* b, const void* sfa, const void* s
   p.num_n_blocks = (n + 255) / 256;
   rc = device_status_word(&p.status);
   if (rc) return rc;
+  CUtensorMap tb_part{};                 // half a unit's rows of B
+  const PairUnits units(p.num_m_blocks * p.num_n_blocks, sm_count_of_current_device() / 2, sizeof(OutT) == 2);
+  if (units.parts != 1) {
+    rc = make_operand_map(&tb_part, b, n, k_nibbles, 1, 128 / units.parts);
+    if (rc) return rc;
+  }
   auto launch = [&](const CUtensorMap& tc, const auto& epi) {
-    if (p.sf_block32 == 2) return launch_pair<2>(ta, tb, tsa, tsb, tc, p, epi, stream);
-    if (p.sf_block32 == 1) return launch_pair<1>(ta, tb, tsa, tsb, tc, p, epi, stream);
-    return launch_pair<0>(ta, tb, tsa, tsb, tc, p, epi, stream);
+    if (p.sf_block32 == 2) return launch_pair<2>(ta, tb, tb_part, tsa, tsb, tc, p, units, epi, stream);
+    if (p.sf_block32 == 1) return launch_pair<1>(ta, tb, tb_part, tsa, tsb, tc, p, units, epi, stream);
+    return launch_pair<0>(ta, tb, tb_part, tsa, tsb, tc, p, units, epi, stream);
   };
   CUtensorMap tc{};
   if constexpr (sizeof(OutT) == 2) {         // 16-bit rows leave through TMA stores

@@ -34,6 +34,33 @@
 namespace b200fp4 {
 
 
+// How the tiles of a launch are dealt to the pairs.  Whole waves of 256 x 256 tiles, then the tiles that are left over: where
+// they are at most half (a quarter) as many as there are pairs, each becomes two (four) units of 128 (64) columns for as many
+// pairs.  A unit loads all rows of A and fewer of B (26 or 30 KB per CTA and K step instead of 38), has narrower MMAs and a
+// quarter or half of the tile to drain; every output is the same sum in the same order.  Only behind whole waves: alone, units
+// take as long as tiles (475 x 2280 x 2048, 18 tiles: 7.4 us either way, 36 tiles 7.6 against 7.9).  Measured with bf16
+// results, us before and now, tiles as waves of 74 + rest: 2267 x 2280 x 2048 (1 + 7) 11.6 -> 10.4, 2523 x 2536 x 2048
+// (1 + 26) 11.9 -> 11.5, 2779 x 2536 x 2048 (1 + 36) 12.1 -> 12.0, 3035 x 3304 x 6144 (2 + 8) 31.2 -> 29.5,
+// 3035 x 4840 x 6144 (3 + 6) 40.4 -> 38.4, 4059 x 5096 x 2048 (4 + 24) 24.4 -> 23.9; MXFP8 3001 x 5120 x 4096 (3 + 18) in a
+// long loop 61.9 -> 61.1.  Four units where two would do as well (9 to 18 tiles left) makes no difference.
+// f32 results leave through registers and keep whole tiles.
+struct PairUnits {
+  int whole, parts, num;       // tiles of whole waves; units of each further tile; units in all
+  PairUnits(int tiles, int pairs, bool split) {
+    const int left = tiles % pairs;
+    whole = tiles - left;
+    parts = !split || left == 0 || whole == 0 ? 1 : (4 * left <= pairs ? 4 : (2 * left <= pairs ? 2 : 1));
+    num = whole + left * parts;
+  }
+  __device__ __forceinline__ void locate(int unit, int& tile, int& cols, int& col0) const {
+    tile = unit, cols = 256, col0 = 0;
+    if (unit >= whole && parts != 1) {
+      const int u = unit - whole;
+      tile = whole + u / parts, cols = 256 / parts, col0 = u % parts * cols;
+    }
+  }
+};
+
 constexpr int kPairStages = 5;
 constexpr uint32_t kPairStageBytes = 16384 + 16384 + 2048 + 4096;    // A, B half, SFA, SFB (both halves)
 // barriers behind the stages, then (16-bit outputs) 4 KB of parking space per epilogue warp
@@ -47,14 +74,13 @@ constexpr int kPairThreads = 64 + 8 * 32 + 128;     // TMA, MMA, 8 epilogue warp
 template <typename Epilogue, int kFlavour>
 __global__ void __launch_bounds__(kPairThreads, 1)
 nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                       const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                       const __grid_constant__ CUtensorMap tmap_c, const GemmParams p, const Epilogue epi) {
+                       const __grid_constant__ CUtensorMap tmap_b_part, const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
+                       const __grid_constant__ CUtensorMap tmap_c, const GemmParams p, const PairUnits units, const Epilogue epi) {
   constexpr int kStages = kPairStages;
   constexpr int kBlockN = 256;
   constexpr uint32_t kSfaCol = 256;
   constexpr uint32_t kSfSetCols = 48;                    // 16 columns of SFA + 32 of SFB per stage
   static_assert(kSfaCol + kPairStages * kSfSetCols <= kTmemCols, "TMEM budget");
-  constexpr uint32_t kIdesc = ptx::idesc_mxf4nvf4_m256(kBlockN);
   constexpr uint32_t kABytes = 16384, kBBytes = 16384, kSfaBytes = 2048;
 
   extern __shared__ uint8_t smem_raw[];
@@ -106,7 +132,6 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   const uint32_t tmem_base = *tmem_ptr_smem;
   grid_dependency_wait();
 
-  const int num_tiles = p.num_m_blocks * p.num_n_blocks; // num_m_blocks counts 256-row blocks here
 
   if (warp == 0) {
     // =============================== TMA producer (both CTAs) ===============================
@@ -114,9 +139,14 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       PipeState st;
       bool ok = true;
       constexpr int tps = 4 >> kFlavour;                 // 512-byte scale tiles per stage and 128 rows
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      for (int unit = pair; unit < units.num && ok; unit += num_pairs) {
+        int tile, cols, col0;
+        units.locate(unit, tile, cols, col0);
         const int m2 = tile % p.num_m_blocks;
         const int n_blk = tile / p.num_m_blocks;
+        const CUtensorMap* map_b = cols == 256 ? &tmap_b : &tmap_b_part;
+        const int b_row = n_blk * 256 + col0 + static_cast<int>(rank) * (cols >> 1);
+        const uint32_t operand_bytes = 2 * (kABytes + static_cast<uint32_t>(cols) * 64);
         const int m_tile = 2 * m2 + static_cast<int>(rank);          // 128-row tile of A owned by this CTA
         for (int kt = 0; kt < p.num_k_tiles; ++kt) {
           if (!wait_bounded(empty_bar(st.stage), st.phase ^ 1u, abort_flag)) {
@@ -137,9 +167,9 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           // (one load for both row tiles of B: five loads a step were 2 to 5 % slower, 238.5 -> 232.7 us at 8192^3)
           ptx::tma_load_3d(ssfa, &tmap_sfa, 0, 2 * tps * kt, m_tile, sbar);
           ptx::tma_load_3d(ssfb, &tmap_sfb, 0, 2 * tps * kt, 2 * n_blk, sbar);      // both 128-row tiles
-          if (rank == 0) ptx::mbar_expect_tx(full_bar(st.stage), 2 * (kABytes + kBBytes));
+          if (rank == 0) ptx::mbar_expect_tx(full_bar(st.stage), operand_bytes);
           ptx::tma2_load_2d(sa, &tmap_a, kt * 128, m_tile * 128, bar);
-          ptx::tma2_load_3d(sb, &tmap_b, kt * 128, n_blk * 256 + static_cast<int>(rank) * 128, 0, bar);
+          ptx::tma2_load_3d(sb, map_b, kt * 128, b_row, 0, bar);
           st.advance(kStages);
         }
       }
@@ -156,7 +186,11 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       const uint64_t b_desc0 = ptx::smem_desc_sw128(smem_base + kABytes);
       const int last_kblocks = ((p.k_bytes - (p.num_k_tiles - 1) * 128) + 31) >> 5;
       B200_ACCT(MmaAcct acct; acct.start();)
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      for (int unit = pair; unit < units.num && ok; unit += num_pairs) {
+        int tile, cols, col0;
+        units.locate(unit, tile, cols, col0);
+        const uint32_t n_field = static_cast<uint32_t>(cols >> 3) << 17;       // of the instruction descriptor
+        const uint32_t sf_col = 16 + (static_cast<uint32_t>(col0) >> 5);
         B200_ACCT(acct.skip();)
         if (!wait_bounded(acc_empty_bar, acc_phase ^ 1u, abort_flag)) {
           if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
@@ -183,7 +217,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           const uint64_t stage_off = static_cast<uint64_t>(st.stage * (kPairStageBytes >> 4));
           const uint64_t da = a_desc0 + stage_off, db = b_desc0 + stage_off;
           const uint32_t sfa_t = tmem_base + kSfaCol + st.stage * kSfSetCols;
-          const uint32_t sfb_t = sfa_t + 16;
+          const uint32_t sfb_t = sfa_t + sf_col;
           const int kblocks = kt + 1 == p.num_k_tiles ? last_kblocks : 4;
           if (ptx::elect_one()) {
             if constexpr (kFlavour == 2) {               // one scale tile per stage, instruction kb reads byte kb
@@ -191,7 +225,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
               for (int kb = 0; kb < 4; ++kb) {
                 if (kb < kblocks)
                   ptx::mma2_mxf8_block32(tmem_base, da + 2 * kb, db + 2 * kb,
-                                         ptx::idesc_m256(ptx::idesc_mxf8_block32(kBlockN, p.a_fmt8, p.b_fmt8, kb)), sfa_t, sfb_t,
+                                         ptx::idesc_m256(ptx::idesc_mxf8_block32(0, p.a_fmt8, p.b_fmt8, kb)) | n_field, sfa_t, sfb_t,
                                          (kt != 0 || kb != 0) ? 1u : 0u);
               }
             } else if constexpr (kFlavour == 1) {        // a scale tile serves two instructions
@@ -199,15 +233,16 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
               for (int kb = 0; kb < 4; ++kb) {
                 if (kb < kblocks)
                   ptx::mma2_mxf4_block32(tmem_base, da + 2 * kb, db + 2 * kb,
-                                         ptx::idesc_m256(ptx::idesc_mxf4_block32(kBlockN, (kb & 1) * 2)), sfa_t + 4 * (kb >> 1),
+                                         ptx::idesc_m256(ptx::idesc_mxf4_block32(0, (kb & 1) * 2)) | n_field, sfa_t + 4 * (kb >> 1),
                                          sfb_t + 8 * (kb >> 1), (kt != 0 || kb != 0) ? 1u : 0u);
               }
             } else {
-              ptx::mma2_mxf4nvf4(tmem_base, da, db, kIdesc, sfa_t, sfb_t, kt != 0 ? 1u : 0u);
+              const uint32_t idesc = ptx::idesc_mxf4nvf4_m256(0) | n_field;
+              ptx::mma2_mxf4nvf4(tmem_base, da, db, idesc, sfa_t, sfb_t, kt != 0 ? 1u : 0u);
 #pragma unroll
               for (int kb = 1; kb < 4; ++kb) {
                 if (kb < kblocks)
-                  ptx::mma2_mxf4nvf4(tmem_base, da + 2 * kb, db + 2 * kb, kIdesc, sfa_t + 4 * kb, sfb_t + 8 * kb, 1u);
+                  ptx::mma2_mxf4nvf4(tmem_base, da + 2 * kb, db + 2 * kb, idesc, sfa_t + 4 * kb, sfb_t + 8 * kb, 1u);
               }
             }
             ptx::tc2_commit_mcast(empty_bar(st.stage), 3);      // frees the stage in both CTAs
@@ -234,7 +269,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const int quarter = warp & 3;
     PipeState st;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+    for (int unit = pair; unit < units.num && ok; unit += num_pairs) {
       for (int kt = 0; kt < p.num_k_tiles; ++kt) {
         if (!wait_bounded(sf_loaded_bar(st.stage), st.phase, abort_flag)) {
           if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
@@ -282,7 +317,9 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const int part = (warp - 2) >> 2;
     const int row = quarter * 32 + lane;
     uint32_t acc_phase = 0;
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    for (int unit = pair; unit < units.num; unit += num_pairs) {
+      int tile, cols, col0;
+      units.locate(unit, tile, cols, col0);
       const int m2 = tile % p.num_m_blocks;
       const int n_blk = tile / p.num_m_blocks;
       if (!wait_bounded<64>(acc_full_bar, acc_phase, abort_flag)) {
@@ -291,20 +328,29 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
       ptx::tc_fence_after_sync();
       const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      epi.template operator()<kBlockN>(p, 2 * m2 + static_cast<int>(rank), n_blk, 0, row, kBlockM, part, 2,
-                                       [&](int c0, uint32_t (&r)[32]) {
-                                         ptx::tmem_ld_32x32(t_acc + c0, r);
-                                         ptx::tmem_ld_wait();
-                                       },
-                                       [&]() {      // called once the warp has read its share of the accumulator
-                                         ptx::tc_fence_before_sync();
-                                         __syncwarp();
-                                         if (lane == 0) {
-                                           if (rank == 0) ptx::mbar_arrive(acc_empty_bar);
-                                           else ptx::mbar_arrive_cluster_relaxed(acc_empty_bar & ptx::kPeerBitMask);   // tcgen05.wait::ld has returned
-                                         }
-                                       },
-                                       Epilogue::kParkWide ? smem_gen + kPairParkOffset + (warp - 2) * 4096 : nullptr, &tmap_c);
+      auto load = [&](int c0, uint32_t (&r)[32]) {
+        ptx::tmem_ld_32x32(t_acc + c0, r);
+        ptx::tmem_ld_wait();
+      };
+      auto release = [&]() {      // called once the warp has read its share of the accumulator
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (rank == 0) ptx::mbar_arrive(acc_empty_bar);
+          else ptx::mbar_arrive_cluster_relaxed(acc_empty_bar & ptx::kPeerBitMask);   // tcgen05.wait::ld has returned
+        }
+      };
+      uint8_t* stage = Epilogue::kParkWide ? smem_gen + kPairParkOffset + (warp - 2) * 4096 : nullptr;
+      const int m_tile = 2 * m2 + static_cast<int>(rank);
+      if constexpr (Epilogue::kParkWide) {
+        if (cols != 256) {        // a box of 64 columns per warp, or none
+          if (64 * part < cols) epi.one_box(p, m_tile, row, 64 * part, n_blk * 256 + col0 + 64 * part, load, release, stage, &tmap_c);
+          else release();
+          acc_phase ^= 1u;
+          continue;
+        }
+      }
+      epi.template operator()<kBlockN>(p, m_tile, n_blk, 0, row, kBlockM, part, 2, load, release, stage, &tmap_c);
       acc_phase ^= 1u;
     }
     // the TMA stores of this warp's last tiles must have reached global memory

@@ -408,6 +408,32 @@ struct EpilogueStoreWide {
   static constexpr bool kUsesOutputMap = true;
   static constexpr bool kParkWide = true;
   const float* alpha;           // one scale per group (dense: one), or null
+  // 64 columns only: accumulator columns from `acc_col` on, columns from `col` on of the output
+  template <typename Loader, typename Release>
+  __device__ __forceinline__ void one_box(const GemmParams& p, int m_blk, int row, int acc_col, int col, Loader&& load,
+                                          Release&& release, uint8_t* stage, const CUtensorMap* cmap) const {
+    const float scale = alpha == nullptr ? 1.0f : ld_word(alpha);
+    const int lane = row & 31, y = m_blk * kBlockM + (row & ~31);
+    uint8_t* box = stage + lane * 128;
+    if (lane == 0) ptx::bulk_wait_group_read0();       // the previous tile's last store has read the box
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t r[32];
+      load(acc_col + 32 * h, r);
+      auto pk = [&](int i) { return Pair16<OutT>::pack(__uint_as_float(r[i]) * scale, __uint_as_float(r[i + 1]) * scale); };
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<uint4*>(box + (((4 * h + q) ^ (lane & 7)) << 4)) = make_uint4(pk(8 * q), pk(8 * q + 2), pk(8 * q + 4), pk(8 * q + 6));
+    }
+    release();
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      if (col < p.n_cols && y < p.m_rows) ptx::tma_store_2d(cmap, col * 2, y, ptx::smem_u32(stage));
+      ptx::bulk_commit_group();
+    }
+  }
   template <int kBlockN, typename Loader, typename Release>
   __device__ __forceinline__ void operator()(const GemmParams& p, int m_blk, int n_blk, int group, int row,
                                              int /*rows_valid*/, int part, int parts, Loader&& load, Release&& release,

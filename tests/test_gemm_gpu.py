@@ -369,6 +369,28 @@ def test_mx_flavours_on_cta_pairs(b200, m, n, k):
     _check_status(b200)
 
 
+@pytest.mark.parametrize("m,n,k", [(1277, 4088, 320), (1277, 4088, 64), (2050, 2568, 1056), (1024, 4872, 256)])
+def test_pair_tiles_of_a_last_wave_in_parts(b200, m, n, k):
+    """One wave of 256 x 256 tiles on 74 CTA pairs and 6, 25 or 6 more, whose columns are dealt to four, two or four pairs
+    each: ragged rows, columns and K steps, all flavours.  Integer-valued operands exact; elsewhere a unit adds the same
+    products in the same order as a whole tile, which is what f32 results still come from: equal after rounding."""
+    ac, sfa, bc, sfb = O.integer_gemm_operands(m, n, k, seed=m + n + k)
+    ref = O.gemm_nvfp4_ref(ac, sfa, bc, sfb, alpha=0.5)
+    a, b, sa, sb = _dev_operands(ac, sfa, bc, sfb)
+    alpha = torch.tensor([0.5], device="cuda")
+    for out_dtype in (torch.bfloat16, torch.float16):
+        c = b200.nvfp4_gemm(a, b, sa, sb, alpha=alpha, out_dtype=out_dtype, tile_n=512)
+        assert torch.equal(c.cpu().float(), ref.to(out_dtype).float())
+    torch.manual_seed(k)
+    sa, sb = (torch.randint(122, 131, (-(-r // 128) * 128 * (-(-k // 128)) * 4,), dtype=torch.uint8, device="cuda") for r in (m, n))
+    f32 = b200.nvfp4_gemm(a, b, sa, sb, alpha=alpha, out_dtype=torch.float32, tile_n=512, sf_vec_size=32)
+    assert torch.equal(b200.nvfp4_gemm(a, b, sa, sb, alpha=alpha, tile_n=512, sf_vec_size=32), f32.bfloat16())
+    a, b = (torch.randn(r, k, device="cuda").to(torch.float8_e4m3fn) for r in (m, n))
+    f32 = b200.mxfp8_gemm(a, b, sa, sb, alpha=alpha, out_dtype=torch.float32, tile_n=512)
+    assert torch.equal(b200.mxfp8_gemm(a, b, sa, sb, alpha=alpha, tile_n=512), f32.bfloat16())
+    _check_status(b200)
+
+
 def _mx_flavours(b200, m, n, k, tile_n):
     rng = np.random.default_rng(m + n + k)
     kb = -(-k // 32)
