@@ -827,7 +827,7 @@ int gemm_moe_fc2_typed(const void* act_codes, const void* act_sf, const void* w2
     if (small_a) return launch_gemm<256, false, 32, 0, kGroupedJoined>(ta, tb, tc, p, epi, max_m_blocks * p.num_n_blocks, stream, tsfb);
     if constexpr (sizeof(RowT) == 2) {
       if (park) {
-        EpilogueStoreWide<RowT> wepi{w2_alpha};
+        const EpilogueStoreWide<RowT, true> wepi{w2_alpha};
         return launch_gemm<256, false, 128, 0, kGroupedJoined>(ta, tb, tc, p, wepi, max_m_blocks * p.num_n_blocks, stream, tsfb);
       }
     }

@@ -78,6 +78,7 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
                        const __grid_constant__ CUtensorMap tmap_c, const GemmParams p, const PairUnits units, const Epilogue epi) {
   constexpr int kStages = kPairStages;
   constexpr int kBlockN = 256;
+  static_assert(!Epilogue::kHalves, "one accumulator barrier");
   constexpr uint32_t kSfaCol = 256;
   constexpr uint32_t kSfSetCols = 48;                    // 16 columns of SFA + 32 of SFB per stage
   static_assert(kSfaCol + kPairStages * kSfSetCols <= kTmemCols, "TMEM budget");

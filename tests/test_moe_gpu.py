@@ -120,6 +120,13 @@ def test_many_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_
     test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
 
 
+@pytest.mark.parametrize("inter", [128, 256, 640, 1024])
+def test_down_projection_drained_by_halves(b200, inter):
+    """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose first and last K step are
+    issued half by half; one and several column blocks, blocks whose upper row quarters are empty."""
+    test_topk_random_against_oracle(b200, 150, 2, 512, inter, 1, None)
+
+
 @pytest.mark.parametrize("tokens,top_k,routed", [(512, 2, True), (513, 2, True), (1024, 2, True), (1025, 2, True), (1536, 2, False),
                                                  (1537, 2, False), (700, 4, False)])
 def test_front_end_switches(b200, tokens, top_k, routed):
