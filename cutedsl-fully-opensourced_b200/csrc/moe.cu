@@ -865,7 +865,7 @@ inline bool moe_few_rows(int64_t tokens, int top_k) { return tokens <= 32 && tok
 // Up to this many (token, slot) pairs the bookkeeping of a step is one CTA's work (moe_prepare_small_kernel) instead of three
 // launches.  Whole steps of hidden 2048, intermediate 1408, 64 experts, three launches / one CTA, us: 1100 slots 76.7 / 75.2,
 // 2048 74.6 / 74.6 (ids given 75.1 / 73.9), 3000 75.5 / 76.6 (76.9 / 76.7), 4000 84.5 / 86.6.  With logits the router needs a
-// launch of its own beyond 1024 slots, so the line lies lower there.
+// launch of its own beyond 32 tokens, so the line lies lower there.
 inline bool small_front_end(int slots, bool routed) { return slots <= (routed ? 2048 : 3072); }
 
 // Few tokens: the bookkeeping kernel quantises and writes them itself (moe_prepare_small_kernel<..., true>) on up to eight
@@ -1097,11 +1097,19 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
       B200_PREPARE(0, 1);
     } else if (logits == nullptr) {
       B200_PREPARE(0, 3);
-    } else if (slots > 1024) {
-      // more tokens than one CTA should route one after the other
+    } else if (tokens > 32) {
+      // One CTA routes a token per warp; with more tokens than warps a launch of its own, with all SMs, is the shorter way.
+      // Whole steps in a graph, us, in the CTA / in its own launch: 128 experts, hidden 2048, intermediate 768, top-8:
+      // 24 tokens 58.0 / 57.9, 32 62.3 / 62.2, 33 64.1 / 62.4, 40 67.1 / 64.2, 64 72.0 / 68.0, 128 81.1 / 71.2;
+      // 256 experts, 7168, 2048, top-8: 32 601.7 / 597.4, 40 670 / 662, 64 831.6 / 826.8; 8 experts, 4096, 3584, top-2:
+      // 16 44.9 / 45.8, 32 45.7 / 45.9, 64 48.2 / 46.7, 512 87.6 / 68.2.
       int rc = route_topk(logits, ids, route_w, static_cast<int>(tokens), route_experts, top_k, renormalize, stream);
       if (rc) return rc;
-      B200_PREPARE(0, 2);
+      if (slots > 1024) {
+        B200_PREPARE(0, 2);
+      } else {
+        B200_PREPARE(0, 1);
+      }
     } else if (route_experts <= 64) {
       B200_PREPARE(2, 1);
     } else if (route_experts <= 128) {

@@ -120,6 +120,12 @@ def test_many_rows_per_expert(b200, tokens, experts, hidden, inter, top_k, slot_
     test_topk_random_against_oracle(b200, tokens, experts, hidden, inter, top_k, slot_rows)
 
 
+@pytest.mark.parametrize("tokens,top_k", [(32, 8), (33, 8), (128, 8), (129, 8)])
+def test_router_inside_or_in_a_launch_of_its_own(b200, tokens, top_k):
+    """As many tokens as the bookkeeping CTA has warps and one more, and either side of 1024 slots with the router apart."""
+    test_front_end_switches(b200, tokens, top_k, True)
+
+
 @pytest.mark.parametrize("tokens,experts,hidden,top_k", [(1, 4, 64, 1), (1, 70, 4096, 24), (3, 4, 1088, 2), (4, 8, 4096, 6),
                                                           (4, 8, 4096, 7), (2, 130, 4160, 3), (4, 300, 192, 2)])
 def test_few_tokens_placed_by_the_bookkeeping(b200, tokens, experts, hidden, top_k):
