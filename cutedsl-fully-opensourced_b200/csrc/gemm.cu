@@ -943,10 +943,10 @@ int moe_stream_gemms_tok(const void* xq, const void* xq_sf, int xq_sf_pitch, con
                          void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
                          const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
                          const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
-                         int trigger, int early, int* status, cudaStream_t stream) {
+                         int trigger, int* status, cudaStream_t stream) {
   const MoeStreamFc1 e1{static_cast<uint8_t*>(act), static_cast<uint8_t*>(act_sf), w1_alpha, fc2_input_scale, inter, act_sf_pitch};
   int rc = launch_moe_stream<kTok>(xq, xq_sf, xq_sf_pitch, w1, w1_sf, 2 * inter, hidden, inter, inter / 128, num_blocks_dev,
-                                   block_expert, block_rows, max_blocks, experts, early, trigger, status, e1, stream);
+                                   block_expert, block_rows, max_blocks, experts, 1, trigger, status, e1, stream);
   if (rc) return rc;
   const int n_blocks = (hidden + 255) / 256;
   if (rows_bf16) {
@@ -963,12 +963,11 @@ int moe_stream_gemms(int tok, const void* xq, const void* xq_sf, int xq_sf_pitch
                      void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
                      const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
                      const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
-                     int trigger, int early, int* status, cudaStream_t stream) {
-  // early: the block tables are older than the kernel before FC1
+                     int trigger, int* status, cudaStream_t stream) {
   auto run = [&](auto fn) {
     return fn(xq, xq_sf, xq_sf_pitch, w1, w1_sf, act, act_sf, act_sf_pitch, w2, w2_sf, partial, rows_bf16, w1_alpha, w2_alpha,
-              fc2_input_scale, num_blocks_dev, block_expert, block_rows, max_blocks, hidden, inter, experts, trigger, early,
-              status, stream);
+              fc2_input_scale, num_blocks_dev, block_expert, block_rows, max_blocks, hidden, inter, experts, trigger, status,
+              stream);
   };
   if (tok == 16) return run(moe_stream_gemms_tok<16>);
   if (tok == 32) return run(moe_stream_gemms_tok<32>);

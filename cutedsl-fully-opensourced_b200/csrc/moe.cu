@@ -38,7 +38,7 @@ int moe_stream_gemms(int tok, const void* xq, const void* xq_sf, int xq_sf_pitch
                      void* act_sf, int act_sf_pitch, const void* w2, const void* w2_sf, void* partial, int rows_bf16,
                      const float* w1_alpha, const float* w2_alpha, const float* fc2_input_scale, const int* num_blocks_dev,
                      const int* block_expert, const int* block_rows, int max_blocks, int hidden, int inter, int experts,
-                     int trigger, int early, int* status, cudaStream_t stream);
+                     int trigger, int* status, cudaStream_t stream);
 
 int sm_count_of_current_device();
 
@@ -497,18 +497,11 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
 // experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
 // step.  0: the ids are inputs.
 // kPerThread: slots per thread (1, 2 or 3: up to 1024, 2048 or 3072 slots; at most 128 per warp, which its bytes can count).
-// kTokens: the tokens as well, quantised and written to their rows (few_tokens).  Several CTAs: each assigns all rows, the first
-// one writes the tables, and the blocks of sixteen elements are dealt to the threads of all.
-struct FewTokens {
-  const __nv_bfloat16* x;
-  uint8_t *xq, *xq_sf;
-  int sf_pitch, hidden;
-};
-template <int kRoutePerLane, int kPerThread, bool kTokens = false>
+template <int kRoutePerLane, int kPerThread>
 __global__ void __launch_bounds__(1024)
 moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize, int top_k, int* ids,
                          float* weights, int n_slots, int expert_lo, MoeHeader h, int experts, int max_m_blocks,
-                         int rows_per_block, int block_stride, FewTokens few) {
+                         int rows_per_block, int block_stride) {
   __shared__ __align__(16) uint8_t s_cnt[32][1024];      // slots of warp w's 32 that named expert e
   __shared__ int s_first[1024];                            // expert -> its first block
   __shared__ int s_ids[1024];
@@ -528,21 +521,13 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
       route_one_token<kRoutePerLane>(logits + static_cast<int64_t>(token) * route_experts, lane, route_experts, top_k,
                                      renormalize, my_id, my_w);
       if (lane < top_k) {
-        if (!kTokens || blockIdx.x == 0) {
-          ids[token * top_k + lane] = my_id;
-          weights[token * top_k + lane] = my_w;
-        }
+        ids[token * top_k + lane] = my_id;
+        weights[token * top_k + lane] = my_w;
         s_ids[token * top_k + lane] = my_id;               // handed to the slot's thread below
       }
     }
+    __syncthreads();
   }
-  // kTokens: block `chunk` of sixteen elements of all tokens; the first one while the routing warps still choose
-  const int chunks = kTokens ? few.hidden >> 4 : 0, all_chunks = kTokens ? n_slots / top_k * chunks : 0;
-  Block16Codes q{};
-  const int first_chunk = kTokens ? static_cast<int>(blockIdx.x) + t * static_cast<int>(gridDim.x) : 0;
-  if (kTokens && first_chunk < all_chunks)
-    q = quantize_bf16x16_pow2(ld_stream_32B(few.x + static_cast<int64_t>(first_chunk) * 16).v, 1.0f);
-  if constexpr (kRoutePerLane > 0) __syncthreads();
   // Slot s * 32 + lane of the warp's share, s < kPerThread.  Position of a slot among the slots of its expert, in slot order:
   // earlier lanes of its group of 32, then earlier groups of the warp, then earlier warps.
   int e[kPerThread], rank[kPerThread];
@@ -592,8 +577,7 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
   incl += warp == 0 ? 0 : __shfl_sync(0xffffffffu, before, warp - 1);
   const int excl = incl - blocks;
   s_first[t] = excl;
-  const bool tables = !kTokens || blockIdx.x == 0;         // every CTA comes to the same rows, one writes them down
-  if (tables && t < experts) {
+  if (t < experts) {
     for (int b = 0; b < blocks; ++b) {
       if (excl + b < max_m_blocks) {
         h.m_block_expert[excl + b] = t;
@@ -601,7 +585,7 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
       }
     }
   }
-  if (tables && t == experts - 1) *h.num_m_blocks = min(incl, max_m_blocks);
+  if (t == experts - 1) *h.num_m_blocks = min(incl, max_m_blocks);
   __syncthreads();
 #pragma unroll
   for (int s = 0; s < kPerThread; ++s) {
@@ -612,21 +596,7 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
       row = (s_first[e[s]] + rank[s] / rows_per_block) * block_stride + rank[s] % rows_per_block;
       if (row >= max_m_blocks * block_stride) row = -1;
     }
-    if (tables) h.slot_row[slot] = row;
-    if constexpr (kTokens) s_ids[slot] = row;              // (the ids are in registers)
-  }
-  if constexpr (kTokens) {
-    __syncthreads();
-    for (int i = first_chunk; i < all_chunks; i += 1024 * static_cast<int>(gridDim.x)) {
-      if (i != first_chunk) q = quantize_bf16x16_pow2(ld_stream_32B(few.x + static_cast<int64_t>(i) * 16).v, 1.0f);
-      const int token = i / chunks, chunk = i - token * chunks;
-      for (int j = 0; j < top_k; ++j) {
-        const int row = s_ids[token * top_k + j];
-        if (row < 0) continue;
-        *reinterpret_cast<uint2*>(few.xq + static_cast<int64_t>(row) * (few.hidden >> 1) + chunk * 8) = make_uint2(q.lo, q.hi);
-        few.xq_sf[static_cast<int64_t>(row) * few.sf_pitch + chunk] = static_cast<uint8_t>(q.sf);
-      }
-    }
+    h.slot_row[slot] = row;
   }
 }
 
@@ -868,17 +838,6 @@ inline bool moe_few_rows(int64_t tokens, int top_k) { return tokens <= 32 && tok
 // launch of its own beyond 32 tokens, so the line lies lower there.
 inline bool small_front_end(int slots, bool routed) { return slots <= (routed ? 2048 : 3072); }
 
-// Few tokens: the bookkeeping kernel quantises and writes them itself (moe_prepare_small_kernel<..., true>) on up to eight
-// CTAs, which all do the bookkeeping and share the tokens.  The first GEMM gets its blocks ready meanwhile; the block tables are
-// as young as the rows then, so it asks for its first weights later, and where those are many or one launch has much to write
-// that costs more than the launch saved.  Whole steps in a graph, us, two launches / one: 128 experts, hidden 2048,
-// intermediate 768, top-8: one token 19.3 / 18.4, two 20.4 / 19.8, four 24.3 / 24.4; 8 experts, 4096, 3584, top-2: one
-// 22.8 / 21.8, two 23.4 / 22.1, four 33.6 / 33.0, eight 46.0 / 45.5; 256 experts, 7168, 2048, top-8: one 46.6 / 46.4, two
-// 76.2 / 76.4, four 130.7 / 132.1.  route_experts: 0 = the ids are given.
-inline bool few_tokens(int64_t tokens, int hidden, int slots, int tok, int route_experts) {
-  return tok != 0 && tokens <= 4 && slots <= 24 && hidden <= 4096 && route_experts <= 256;
-}
-
 // Rows per block of the streaming GEMMs (moe_stream_kernel.cuh), 0 = the 128-row kernels.  The narrowest block that an
 // expert with the average number of rows and two standard deviations more still fits (an expert that does not gets a
 // second block, whose weights then come from L2); blocks of 64 up to an average of 60.  Whole steps, us, 128-row kernels /
@@ -1071,29 +1030,17 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
   if (workspace_bytes < ws.total)
     return fail(kInvalidArgument, "workspace holds %zu bytes, %zu needed", workspace_bytes, ws.total);
   const int slots = static_cast<int>(tokens * top_k);
-  const bool merged = few_tokens(tokens, hidden, slots, tok, logits != nullptr ? route_experts : 0);
 
   if (small_front_end(slots, logits != nullptr)) {
     // rows that only pad a block keep whatever their scale bytes held: a row of the accumulator depends on its own row of A
     // only, and rows without data are never read back
     // few slots: one CTA counts, scans and assigns rows in slot order; quantisation splits a token's columns
     // over several CTAs (a decode step is mostly the latency of these small kernels)
-#define B200_PREPARE_TOKENS(PL, PT, TOKENS)                                                                           \
-  B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL, PT, TOKENS>, dim3(TOKENS ? few_ctas : 1), dim3(1024), 0, stream, logits, \
-                             route_experts, renormalize, top_k, ids, route_w, slots, expert_lo, ws.h, experts,          \
-                             ws.max_m_blocks, per_block, per_block, few))
-#define B200_PREPARE(PL, PT) B200_PREPARE_TOKENS(PL, PT, false)
-    const int few_ctas = static_cast<int>(std::min<int64_t>(8, (tokens * hidden / 16 + 63) / 64));
-    const FewTokens few{static_cast<const __nv_bfloat16*>(x), ws.xq, ws.xq_sf, sf_row_pitch(hidden), hidden};
-    if (merged && logits == nullptr) {
-      B200_PREPARE_TOKENS(0, 1, true);
-    } else if (merged && route_experts <= 64) {
-      B200_PREPARE_TOKENS(2, 1, true);
-    } else if (merged && route_experts <= 128) {
-      B200_PREPARE_TOKENS(4, 1, true);
-    } else if (merged) {
-      B200_PREPARE_TOKENS(8, 1, true);
-    } else if (logits == nullptr && slots <= 1024) {
+#define B200_PREPARE(PL, PT)                                                                                          \
+  B200_CUDA(launch_dependent(moe_prepare_small_kernel<PL, PT>, dim3(1), dim3(1024), 0, stream, logits, route_experts,   \
+                             renormalize, top_k, ids, route_w, slots, expert_lo, ws.h, experts, ws.max_m_blocks,    \
+                             per_block, per_block))
+    if (logits == nullptr && slots <= 1024) {
       B200_PREPARE(0, 1);
     } else if (logits == nullptr) {
       B200_PREPARE(0, 3);
@@ -1123,9 +1070,8 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
       B200_PREPARE(0, 1);
     }
 #undef B200_PREPARE
-#undef B200_PREPARE_TOKENS
     const int parts = (hidden / 16 + 127) / 128;
-    if (!merged) B200_CUDA(launch_dependent(moe_scatter_quant_rows_kernel<128>, dim3(static_cast<unsigned>(tokens), parts), dim3(128), 0,
+    B200_CUDA(launch_dependent(moe_scatter_quant_rows_kernel<128>, dim3(static_cast<unsigned>(tokens), parts), dim3(128), 0,
                                stream, static_cast<const __nv_bfloat16*>(x), ws.h.slot_row, ws.xq, ws.xq_sf, sf_row_pitch(hidden), hidden,
                                top_k));
   } else {
@@ -1155,7 +1101,7 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
     rc = moe_stream_gemms(tok, ws.xq, ws.xq_sf, sf_row_pitch(hidden), w1, w1_sf, ws.act, ws.act_sf, sf_row_pitch(inter), w2,
                           w2_sf, ws.partial, rows_bf16, w1_alpha, w2_alpha, fc2_input_scale, ws.h.num_m_blocks,
                           ws.h.m_block_expert, ws.h.m_block_rows, ws.max_m_blocks, hidden, inter, experts, slots <= 1024,
-                          merged ? 0 : 1, status, stream);
+                          status, stream);
     if (rc) return rc;
   } else {
     rc = gemm_moe_fc1(ws.xq, ws.xq_sf, w1, w1_sf, ws.act, ws.act_sf, w1_alpha, fc2_input_scale, ws.h.num_m_blocks,

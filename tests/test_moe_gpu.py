@@ -126,32 +126,6 @@ def test_router_inside_or_in_a_launch_of_its_own(b200, tokens, top_k):
     test_front_end_switches(b200, tokens, top_k, True)
 
 
-@pytest.mark.parametrize("tokens,experts,hidden,top_k", [(1, 4, 64, 1), (1, 70, 4096, 24), (3, 4, 1088, 2), (4, 8, 4096, 6),
-                                                          (4, 8, 4096, 7), (2, 130, 4160, 3), (4, 300, 192, 2)])
-def test_few_tokens_placed_by_the_bookkeeping(b200, tokens, experts, hidden, top_k):
-    """One to eight CTAs that share the tokens' blocks, a thread with several blocks, the most slots and the widest token and one
-    more of either (two launches again), with given ids and with the router inside (up to 64, 128, 256 experts and beyond); the
-    same ids once more per token."""
-    rng = np.random.default_rng(tokens + hidden)
-    torch.manual_seed(hidden + top_k)
-    inter = 128
-    shared = [np.repeat(w[:1], experts, axis=0) for w in random_weights(rng, 1, hidden, inter)]
-    x = torch.randn(tokens, hidden).to(torch.bfloat16)
-    logits = torch.randn(tokens, experts)
-    ids, wts = O.route_topk_ref(logits, top_k)
-    a1 = torch.tensor(rng.uniform(0.01, 0.03, experts), dtype=torch.float32)
-    a2 = torch.tensor(rng.uniform(0.5, 2.0, experts), dtype=torch.float32)
-    alphas = dict(w1_alpha=a1.cuda(), w2_alpha=a2.cuda())
-    repeated = ids.clone()
-    repeated[:, -1] = repeated[:, 0]
-    for given in (ids, repeated):
-        ref = O.moe_ref(x, *shared, given, wts, a1.numpy(), a2.numpy())
-        assert rel_l2(run_gpu(b200, x, *shared, given, wts.contiguous(), **alphas), ref) <= 1e-2
-    ref = O.moe_ref(x, *shared, ids, wts, a1.numpy(), a2.numpy())
-    out = run_gpu(b200, x, *shared, torch.full_like(ids, -1), torch.zeros_like(wts), router_logits=logits.cuda(), **alphas)
-    assert rel_l2(out, ref) <= 1e-2
-
-
 @pytest.mark.parametrize("inter", [128, 256, 640, 1024])
 def test_down_projection_drained_by_halves(b200, inter):
     """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose first and last K step are
