@@ -493,7 +493,7 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
 // Few slots (<= 3072): count, scan and row assignment in one CTA -- one launch instead of a memset and three
 // kernels, which is most of a decode step's bookkeeping time.  Rows of an expert go to its slots in slot order.
 // rows_per_block, block_stride: as in the place kernel.
-// kRoutePerLane > 0: the router runs here first (one warp per token, the CTA's 32 warps take the tokens in turn;
+// kRoutePerLane > 0: the router runs here first (one warp per token, so for up to 32 tokens;
 // experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
 // step.  0: the ids are inputs.
 // kPerThread: slots per thread (1, 2 or 3: up to 1024, 2048 or 3072 slots; at most 128 per warp, which its bytes can count).
