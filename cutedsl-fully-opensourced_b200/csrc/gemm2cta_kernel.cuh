@@ -14,7 +14,8 @@
 // is fetched by the CTA that needs it.  All waits are bounded as in the single-CTA kernel.
 //
 // Measured at M = N = K = 8192 (cycle accounting of the MMA-issuing thread, -DB200FP4_ACCT): 720 cycles per K step
-// against 875 for the single-CTA kernel with 128 x 256 tiles (512 would keep the tensor pipe busy).  40 % of the
+// against 875 for the single-CTA kernel with 128 x 256 tiles (512 would keep the tensor pipe busy); 632 since both row tiles
+// of B's scales are one load, 93 of them per MMA for issuing, 71 operands, 60 slabs, 40 accumulator.  Of the 720, 40 % of the
 // issuing thread's cycles go into issuing MMAs, 15 % into waiting for operand tiles and 26 % into waiting for
 // scale slabs that reach tensor memory after the operands have landed.  Tried against that slab wait, without
 // gain: a second group of mover warps (unchanged: one group keeps up); a slab ring of its own, twice as deep as
