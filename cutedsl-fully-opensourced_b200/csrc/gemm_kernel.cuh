@@ -402,8 +402,8 @@ struct EpilogueStore {
 // registers, reads the second straight into the parking space, releases the accumulator, stores the second box by
 // TMA and, once that store has read the space, parks and stores the first.  Register stores of the same tile take
 // 64 KB through lanes that each write another row (about 12 bytes per cycle and SM).
-// kHalves_ (FC2): the two warps of a tensor-memory quarter have an accumulator barrier each, and the MMAs of a tile's first and
-// last K step come half by half (see the MMA issuer).
+// kHalves_ (FC2): the two warps of a tensor-memory quarter have an accumulator barrier each, and MMAs come half by half (see the
+// MMA issuer).
 template <typename OutT, bool kHalves_ = false>
 struct EpilogueStoreWide {
   static_assert(sizeof(OutT) == 2, "16-bit rows");
@@ -702,11 +702,12 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   constexpr uint32_t kSfbColsPerKb = kBlockN >= 128 ? kBlockN / 32 : 4;
   constexpr uint32_t kSfaCol = kAccStages * kBlockN;            // TMEM columns: accumulators first
   constexpr uint32_t kSfSetCols = 16 + 4 * kSfbColsPerKb;       // columns of one set of scale slabs (SFA + SFB)
-  constexpr uint32_t kIdesc = ptx::idesc_mxf4nvf4(kBlockN);
   constexpr int kFirstSfWarp = 2 + kEpiWarps;
   constexpr bool kIsGrouped = kTiles != kDense, kJoined = kTiles == kGroupedJoined;
   // a pair of barriers for each half of the one accumulator's columns
   constexpr bool kHalves = Epilogue::kHalves;
+  constexpr int kMmaN = kHalves ? kBlockN / 2 : kBlockN;        // columns of every MMA of the kernel
+  constexpr uint32_t kIdesc = ptx::idesc_mxf4nvf4(kMmaN);
   static_assert(!kHalves || (kBlockN == 256 && !kSwigluB && kIsGrouped && kEpiWarps == 8), "halves of a 256-wide tile");
   static_assert(!kJoined || kBlockN == 256, "joined pieces make 256-wide tiles");
   const bool early_b = kIsGrouped && p.early_b != 0;
@@ -943,38 +944,39 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sfa_t = tmem_base + kSfaCol + st.stage * kSfSetCols;
           const int kblocks = kt + 1 == p.num_k_tiles ? last_kblocks : 4;
           if constexpr (kHalves) {
-            // The epilogue warps of a half hand it back as soon as they have read it.  In a tile's first and last K step the
-            // MMAs come half by half (two of 128 columns take as long as one of 256), so that one half is drained while the
-            // tensor core works on the other: with three or four K steps a tile the one accumulator is what a tile waits for.
-            // FC2 of 4096 tokens: 53.1 -> 52.4 us (128 experts, 2048, 768, top-8), 57.7 -> 55.8 (32 experts, 4096, 1024, top-4).
-            const bool first = kt == kt_first, last = kt + 1 == p.num_k_tiles;
-            if (first || last) {
+            // The epilogue warps of a half hand it back as soon as they have read it.  The MMAs of a K step come half by half
+            // (two of 128 columns take as long as one of 256), so that one half is drained while the tensor core works on the
+            // other: with three or four K steps a tile the one accumulator is what a tile waits for.  All MMAs into a half have
+            // the same shape: only MMAs of one shape into one accumulator are sure to be executed in the order of their issue.
+            // FC2 of 4096 tokens alone, one accumulator barrier and whole MMAs / halves: four K steps (32 experts, 4096, 1024,
+            // top-4) 58.4-58.9 / 56.6-56.8 us, three (128 experts, 2048, 768, top-8) 52.9-53.2 / 53.3.  (Whole MMAs in the K
+            // steps between a tile's first and last would save another 0.6 us with three and nothing with four, but mix shapes.)
+            const bool first = kt == kt_first, last = kt + 1 == kt_end;
 #pragma unroll
-              for (int i = 0; i < 2; ++i) {
-                if (first) {
-                  ok = wait_bounded(acc_empty_bar(i), acc.phase ^ 1u, abort_flag);
-                  if (!ok) break;
-                  ptx::tc_fence_after_sync();
-                }
-                if (ptx::elect_one()) {
+            for (int i = 0; i < 2; ++i) {
+              if (first) {
+                ok = wait_bounded(acc_empty_bar(i), acc.phase ^ 1u, abort_flag);
+                if (!ok) break;
+                ptx::tc_fence_after_sync();
+              }
+              if (ptx::elect_one()) {
 #pragma unroll
-                  for (int kb = 0; kb < 4; ++kb) {
-                    if (kb < kblocks)
-                      ptx::mma_mxf4nvf4(d_tmem + 128 * i, da + 2 * kb, db + 1024 * i + 2 * kb, ptx::idesc_mxf4nvf4(128),
-                                        sfa_t + 4 * kb, sfb_t + kSfbColsPerKb * kb + 4 * i, (!first || kb != 0) ? 1u : 0u);
-                  }
-                  if (i == 1) ptx::tc_commit(empty_bar(st.stage));
-                  if (last) ptx::tc_commit(acc_full_bar(i));
+                for (int kb = 0; kb < 4; ++kb) {
+                  if (kb < kblocks)
+                    ptx::mma_mxf4nvf4(d_tmem + kMmaN * i, da + 2 * kb, db + 8 * kMmaN * i + 2 * kb, kIdesc, sfa_t + 4 * kb,
+                                      sfb_t + kSfbColsPerKb * kb + kMmaN / 32 * i, (!first || kb != 0) ? 1u : 0u);
                 }
-                __syncwarp();
+                if (i == 1) ptx::tc_commit(empty_bar(st.stage));
+                if (last) ptx::tc_commit(acc_full_bar(i));
               }
-              if (!ok) {
-                if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
-                break;
-              }
-              st.advance(kStages);
-              continue;
+              __syncwarp();
             }
+            if (!ok) {
+              if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
+              break;
+            }
+            st.advance(kStages);
+            continue;
           }
           if (ptx::elect_one()) {
             if (p.sf_block32 == 2) {
@@ -983,7 +985,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               for (int kb = 0; kb < 4; ++kb) {
                 if (kb < kblocks)
                   ptx::mma_mxf8_block32(d_tmem, da + 2 * kb, db + 2 * kb,
-                                        ptx::idesc_mxf8_block32(kBlockN, p.a_fmt8, p.b_fmt8, kb), sfa_t, sfb_t,
+                                        ptx::idesc_mxf8_block32(kMmaN, p.a_fmt8, p.b_fmt8, kb), sfa_t, sfb_t,
                                         (kt != kt_first || kb != 0) ? 1u : 0u);
               }
             } else if (p.sf_block32 == 1) {
@@ -991,7 +993,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
               for (int kb = 0; kb < 4; ++kb) {
                 if (kb < kblocks)
-                  ptx::mma_mxf4_block32(d_tmem, da + 2 * kb, db + 2 * kb, ptx::idesc_mxf4_block32(kBlockN, (kb & 1) * 2),
+                  ptx::mma_mxf4_block32(d_tmem, da + 2 * kb, db + 2 * kb, ptx::idesc_mxf4_block32(kMmaN, (kb & 1) * 2),
                                         sfa_t + 4 * (kb >> 1), sfb_t + kSfbColsPerKb * (kb >> 1),
                                         (kt != kt_first || kb != 0) ? 1u : 0u);
               }
