@@ -126,11 +126,39 @@ def test_router_inside_or_in_a_launch_of_its_own(b200, tokens, top_k):
     test_front_end_switches(b200, tokens, top_k, True)
 
 
-@pytest.mark.parametrize("inter", [128, 256, 640, 1024])
+@pytest.mark.parametrize("inter", [128, 256, 512, 640, 1024])
 def test_down_projection_drained_by_halves(b200, inter):
-    """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose first and last K step are
-    issued half by half; one and several column blocks, blocks whose upper row quarters are empty."""
+    """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose MMAs are issued half by
+    half: four tiles, none with a successor on its CTA, blocks whose upper row quarters are empty."""
     test_topk_random_against_oracle(b200, 150, 2, 512, inter, 1, None)
+
+
+@pytest.mark.parametrize("inter", [128, 512, 640, 1024])
+def test_accumulator_halves_change_hands(b200, inter):
+    """The same with more tiles than two to an SM, so that either half is filled, drained and filled again: full blocks, short
+    ones and one with a single row in turn.  One expert per token under weight 1: the result is the row of FC2 rounded to bf16,
+    bit by bit the same as with f32 rows, which 128-wide tiles with accumulators of their own compute."""
+    g = torch.Generator(device="cuda").manual_seed(inter)
+    experts, hidden = 6, 8192
+
+    def operand(rows, k):
+        sf = torch.randint(0x18, 0x30, (experts, rows // 128, (k // 16 + 3) // 4, 32, 4, 4), generator=g, device="cuda", dtype=torch.uint8)
+        codes = torch.randint(0, 256, (experts, rows, k // 2), generator=g, device="cuda", dtype=torch.uint8)
+        return codes, sf.view(torch.float8_e4m3fn).permute(3, 4, 1, 5, 2, 0)
+
+    (w1, w1s), (w2, w2s) = operand(2 * inter, hidden), operand(hidden, inter)
+    rows = [1, 401, 128, 150, 257, 33]                     # of each expert: 1 + 4 + 1 + 2 + 3 + 1 blocks, 32 column blocks each
+    tiles = sum(-(-r // 128) for r in rows) * hidden // 256
+    assert tiles > 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    ids = torch.repeat_interleave(torch.arange(experts), torch.tensor(rows))
+    ids = ids[torch.randperm(ids.numel(), generator=torch.Generator().manual_seed(inter))].int()[:, None].contiguous().cuda()
+    x = torch.randn(ids.shape[0], hidden, generator=g, device="cuda").to(torch.bfloat16)
+    alpha = torch.full((experts,), 0.01, device="cuda")
+    out, ref = (b200.b12x_fused_moe(x, w1, w1s, w2, w2s, ids, torch.ones(ids.shape, device="cuda"), experts, 1, w1_alpha=alpha,
+                                    slot_rows_dtype=dt) for dt in (None, torch.float32))
+    torch.cuda.synchronize()
+    assert b200._lib.device_status() == 0
+    assert bool((ref.float().abs().amax(-1) > 0).all()) and torch.equal(out, ref)
 
 
 @pytest.mark.parametrize("tokens,top_k,routed", [(512, 2, True), (513, 2, True), (1024, 2, True), (1025, 2, True), (1536, 2, False),
