@@ -906,7 +906,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
           break;
         }
-        B200_ACCT(acct.mark(acct.acc); ++acct.tiles;)
+        B200_ACCT(if (!kHalves) acct.mark(acct.acc); ++acct.tiles;)
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc.stage * kBlockN;
         // a 64-wide tile uses half of a 128-row slab of B scale factors: its row groups start at column 0 or 2
@@ -955,8 +955,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
               if (first) {
+                B200_ACCT(acct.skip();)
                 ok = wait_bounded(acc_empty_bar(i), acc.phase ^ 1u, abort_flag);
                 if (!ok) break;
+                B200_ACCT(acct.mark(acct.acc);)
                 ptx::tc_fence_after_sync();
               }
               if (ptx::elect_one()) {
@@ -970,6 +972,7 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 if (last) ptx::tc_commit(acc_full_bar(i));
               }
               __syncwarp();
+              B200_ACCT(acct.mark(acct.issue);)
             }
             if (!ok) {
               if (lane == 0) atomicOr(p.status, kStatusTimeoutMma);
