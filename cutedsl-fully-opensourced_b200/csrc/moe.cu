@@ -493,8 +493,8 @@ moe_quant_place_kernel(const __nv_bfloat16* x, const int* ids,
 // Few slots (<= 3072): count, scan and row assignment in one CTA -- one launch instead of a memset and three
 // kernels, which is most of a decode step's bookkeeping time.  Rows of an expert go to its slots in slot order.
 // rows_per_block, block_stride: as in the place kernel.
-// kRoutePerLane > 0: the router runs here first (one warp per token, so for up to 32 tokens;
-// experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
+// kRoutePerLane > 0: the router runs here first (one warp per token: at most 32 tokens, and at most 1024 slots, which
+// s_ids holds; experts per lane as in route_one_token) and writes its choice to ids / weights -- one launch fewer in a decode
 // step.  0: the ids are inputs.
 // kPerThread: slots per thread (1, 2 or 3: up to 1024, 2048 or 3072 slots; at most 128 per warp, which its bytes can count).
 template <int kRoutePerLane, int kPerThread>
@@ -515,7 +515,7 @@ moe_prepare_small_kernel(const float* logits, int route_experts, int renormalize
   grid_dependency_wait();
   let_dependents_launch();
   if constexpr (kRoutePerLane > 0) {
-    for (int token = warp; token * top_k < n_slots; token += 32) {
+    if (const int token = warp; token * top_k < n_slots) {
       int my_id;
       float my_w;
       route_one_token<kRoutePerLane>(logits + static_cast<int64_t>(token) * route_experts, lane, route_experts, top_k,
@@ -1044,7 +1044,7 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
       B200_PREPARE(0, 1);
     } else if (logits == nullptr) {
       B200_PREPARE(0, 3);
-    } else if (tokens > 32) {
+    } else if (tokens > 32 || slots > 1024) {
       // One CTA routes a token per warp; with more tokens than warps a launch of its own, with all SMs, is the shorter way.
       // Whole steps in a graph, us, in the CTA / in its own launch: 128 experts, hidden 2048, intermediate 768, top-8:
       // 24 tokens 58.0 / 57.9, 32 62.3 / 62.2, 33 64.1 / 62.4, 40 67.1 / 64.2, 64 72.0 / 68.0, 128 81.1 / 71.2;

@@ -126,6 +126,25 @@ def test_router_inside_or_in_a_launch_of_its_own(b200, tokens, top_k):
     test_front_end_switches(b200, tokens, top_k, True)
 
 
+def test_router_inside_with_as_many_slots_as_it_holds(b200):
+    """32 tokens of 32 experts each: every warp of the bookkeeping CTA routes a token, and its table of 1024 slots is full."""
+    rng = np.random.default_rng(32)
+    torch.manual_seed(32)
+    tokens, top_k, experts, hidden, inter = 32, 32, 48, 192, 128
+    weights = random_weights(rng, experts, hidden, inter)
+    x, logits = torch.randn(tokens, hidden).to(torch.bfloat16), torch.randn(tokens, experts)
+    ids, wts = O.route_topk_ref(logits, top_k)
+    ref = O.moe_ref(x, *weights, ids, wts, np.full(experts, 0.02, np.float32))
+    out = run_gpu(b200, x, *weights, ids, wts.contiguous(), w1_alpha=torch.full((experts,), 0.02).cuda())
+    w1c, w1s, w2c, w2s = weights
+    routed = b200.b12x_fused_moe(
+        x.cuda(), torch.from_numpy(O.pack_e2m1(w1c)).cuda(), six_mode(w1s), torch.from_numpy(O.pack_e2m1(w2c)).cuda(), six_mode(w2s),
+        None, None, experts, top_k, w1_alpha=torch.full((experts,), 0.02).cuda(), router_logits=logits.cuda())
+    torch.cuda.synchronize()
+    assert b200._lib.device_status() == 0
+    assert rel_l2(out, ref) <= 1e-2 and rel_l2(routed.cpu(), ref) <= 1e-2
+
+
 @pytest.mark.parametrize("inter", [128, 256, 512, 640, 1024])
 def test_down_projection_drained_by_halves(b200, inter):
     """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose MMAs are issued half by
