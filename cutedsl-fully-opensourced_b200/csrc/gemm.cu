@@ -291,8 +291,9 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 }
 
 template <int kFlavour, typename Epilogue>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_part, const CUtensorMap& tsa, const CUtensorMap& tsb,
-                const CUtensorMap& tc, const GemmParams& p, const PairUnits& units, const Epilogue& epi, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_part, const CUtensorMap& tsa,
+                const CUtensorMap& tsb, const CUtensorMap& tc, const GemmParams& p, const PairUnits& units, const Epilogue& epi,
+                cudaStream_t stream) {
   auto kern = nvfp4_gemm_pair_kernel<Epilogue, kFlavour>;
   constexpr uint32_t kSmem = pair_smem_bytes(Epilogue::kParkWide);
   static std::atomic<bool> configured[kMaxDevices];
@@ -572,7 +573,8 @@ int gemm_dense_typed(const void* a, const void* b, const void* sfa, const void* 
 //   m = 16, n = k = 4096: 128 x 64 tiles 8.8 us, streaming 5.5;  m = 2, n = 7936, k = 2048: 7.3 against 5.7
 //   m = 128, n = k = 8192: 64-wide tiles 14.2 us, 128-wide 14.9, streaming 4 x 128 15.5;  f32 results 14.2 against 17.2
 //   m = 1280, n = k = 1024: 128-wide tiles 5.6 us, 64-wide 7.0;  m = 512, n = k = 4096: 10.0 against 14.0
-//   m = 2657, n = 6912, k = 4608: pairs 41.8 us, 256-wide 45.6;  m = 2665, n = 3584, k = 3712: 23.8 against 22.3
+//   m = 2657, n = 6912, k = 4608: pairs 38.7 us, 256-wide 42.7;  m = 2665, n = 3584, k = 3712: 21.5 against 21.3 (154 tiles
+//   on 74 pairs; the estimate charges pairs a whole wave for the six tiles left, which they deal out in parts)
 //   m = 4024, n = 8192, k = 1280: pairs 25.0 us, 128-wide 40.6
 // The constants of the 64- and 128-wide tiles are a fit to 528 shapes under every variant (three flavours, 16-bit and f32
 // results): the chosen kernel takes 2 % more than the fastest one on average.  Those of the 256-wide tiles and of the pairs

@@ -13,11 +13,11 @@
 // tensor memory with tcgen05.st, each CTA for itself; they report to the even CTA).  No TMA multicast is used anywhere: every tile
 // is fetched by the CTA that needs it.  All waits are bounded as in the single-CTA kernel.
 //
-// Measured at M = N = K = 8192 (cycle accounting of the MMA-issuing thread, -DB200FP4_ACCT): 720 cycles per K step
-// against 875 for the single-CTA kernel with 128 x 256 tiles (512 would keep the tensor pipe busy); 632 since both row tiles
-// of B's scales are one load, 93 of them per MMA for issuing, 71 operands, 60 slabs, 40 accumulator.  Of the 720, 40 % of the
-// issuing thread's cycles go into issuing MMAs, 15 % into waiting for operand tiles and 26 % into waiting for
-// scale slabs that reach tensor memory after the operands have landed.  Tried against that slab wait, without
+// Measured at M = N = K = 8192 (cycle accounting of the MMA-issuing thread, -DB200FP4_ACCT): 617 cycles per K step
+// against 850 for the single-CTA kernel with 128 x 256 tiles (512 would keep the tensor pipe busy).  Of the 617, 296 (48 %) go
+// into issuing the four MMAs, 110 (18 %) into waiting for operand tiles, 74 (12 %) for scale slabs that reach tensor memory
+// after the operands have landed, 49 (8 %) for the accumulator, 88 (14 %) into the rest of the loop.  Before both row tiles of
+// B's scales were one load it was 720, 26 % of it for slabs.  Tried at that time against the slab wait, without
 // gain: a second group of mover warps (unchanged: one group keeps up); a slab ring of its own, twice as deep as
 // the operand ring, with the slabs requested five K steps early and held in the movers' registers until the
 // columns are free (slab wait down to 7 %, operand wait up to 45 %, 15 to 25 % slower overall); loading only A
@@ -39,11 +39,10 @@ namespace b200fp4 {
 // they are at most half (a quarter) as many as there are pairs, each becomes two (four) units of 128 (64) columns for as many
 // pairs.  A unit loads all rows of A and fewer of B (26 or 30 KB per CTA and K step instead of 38), has narrower MMAs and a
 // quarter or half of the tile to drain; every output is the same sum in the same order.  Only behind whole waves: alone, units
-// take as long as tiles (475 x 2280 x 2048, 18 tiles: 7.4 us either way, 36 tiles 7.6 against 7.9).  Measured with bf16
-// results, us before and now, tiles as waves of 74 + rest: 2267 x 2280 x 2048 (1 + 7) 11.6 -> 10.4, 2523 x 2536 x 2048
-// (1 + 26) 11.9 -> 11.5, 2779 x 2536 x 2048 (1 + 36) 12.1 -> 12.0, 3035 x 3304 x 6144 (2 + 8) 31.2 -> 29.5,
-// 3035 x 4840 x 6144 (3 + 6) 40.4 -> 38.4, 4059 x 5096 x 2048 (4 + 24) 24.4 -> 23.9; MXFP8 3001 x 5120 x 4096 (3 + 18) in a
-// long loop 61.9 -> 61.1.  Four units where two would do as well (9 to 18 tiles left) makes no difference.
+// take as long as tiles (475 x 2280 x 2048, 18 tiles: 7.4 us either way, 36 tiles 7.6 against 7.9).  Whole tiles / units, us,
+// operands from HBM, tiles as waves of 74 + rest: 11.9 / 10.6 (2267 x 2280 x 2048, 1 + 7), 22.9 / 21.5 (2665 x 3584 x 3712,
+// 2 + 6), 41.7 / 40.8 (3035 x 4840 x 6144, 3 + 6), 12.8 / 12.4 (2779 x 2536 x 2048, 1 + 36).  Four units
+// where two would do as well (9 to 18 tiles left) makes no difference.
 // f32 results leave through registers and keep whole tiles.
 struct PairUnits {
   int whole, parts, num;       // tiles of whole waves; units of each further tile; units in all
@@ -75,8 +74,9 @@ constexpr int kPairThreads = 64 + 8 * 32 + 128;     // TMA, MMA, 8 epilogue warp
 template <typename Epilogue, int kFlavour>
 __global__ void __launch_bounds__(kPairThreads, 1)
 nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                       const __grid_constant__ CUtensorMap tmap_b_part, const __grid_constant__ CUtensorMap tmap_sfa, const __grid_constant__ CUtensorMap tmap_sfb,
-                       const __grid_constant__ CUtensorMap tmap_c, const GemmParams p, const PairUnits units, const Epilogue epi) {
+                       const __grid_constant__ CUtensorMap tmap_b_part, const __grid_constant__ CUtensorMap tmap_sfa,
+                       const __grid_constant__ CUtensorMap tmap_sfb, const __grid_constant__ CUtensorMap tmap_c, const GemmParams p,
+                       const PairUnits units, const Epilogue epi) {
   constexpr int kStages = kPairStages;
   constexpr int kBlockN = 256;
   static_assert(!Epilogue::kHalves, "one accumulator barrier");
@@ -133,7 +133,6 @@ nvfp4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
   grid_dependency_wait();
-
 
   if (warp == 0) {
     // =============================== TMA producer (both CTAs) ===============================

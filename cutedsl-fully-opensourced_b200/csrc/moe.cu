@@ -1048,8 +1048,8 @@ int moe_fused(const void* x, const void* w1, const void* w1_sf, const void* w2, 
       // One CTA routes a token per warp; with more tokens than warps a launch of its own, with all SMs, is the shorter way.
       // Whole steps in a graph, us, in the CTA / in its own launch: 128 experts, hidden 2048, intermediate 768, top-8:
       // 24 tokens 58.0 / 57.9, 32 62.3 / 62.2, 33 64.1 / 62.4, 40 67.1 / 64.2, 64 72.0 / 68.0, 128 81.1 / 71.2;
-      // 256 experts, 7168, 2048, top-8: 32 601.7 / 597.4, 40 670 / 662, 64 831.6 / 826.8; 8 experts, 4096, 3584, top-2:
-      // 16 44.9 / 45.8, 32 45.7 / 45.9, 64 48.2 / 46.7, 512 87.6 / 68.2.
+      // 256 experts, 7168, 2048, top-8: 32 601.7 / 597.4, 40 670 / 662, 64 831.6 / 826.8 (within the spread of two runs);
+      // 8 experts, 4096, 3584, top-2: 16 44.9 / 45.8, 32 45.7 / 45.9, 64 48.2 / 46.7, 512 87.6 / 68.2.
       int rc = route_topk(logits, ids, route_w, static_cast<int>(tokens), route_experts, top_k, renormalize, stream);
       if (rc) return rc;
       if (slots > 1024) {

@@ -14,8 +14,8 @@
 // quantisation, and the last rows spread over all SMs.  (A persistent grid that looped over rows with the weights parked
 // in shared memory as f32 was 10 % slower on the largest shapes and 40 % on middle ones: a last wave that was nearly
 // empty, and a launch that had to load the weights first.)  What bounds it: DRAM for the add variant -- [8192, 7168]
-// bf16, 385 MB: 61 us = 6.3 TB/s as a burst (66 before), 66 in a long loop (72) -- and the issue slots for the plain one
-// ([4096, 5120] fp16: 22.6 -> 13.7 us; [8192, 7168] bf16: 45 -> 34 us).
+// bf16, 385 MB: 61 us = 6.3 TB/s as a burst (66 before), 66 in a long loop (72).  The plain one ([4096, 5120] fp16: 22.6 -> 13.7
+// us; [8192, 7168] bf16: 45 -> 34 us) fills neither DRAM (3.9 TB/s, 61 % of a copy) nor the issue slots (64 % busy).
 #include "common.cuh"
 
 namespace b200fp4 {
