@@ -402,8 +402,8 @@ struct EpilogueStore {
 // registers, reads the second straight into the parking space, releases the accumulator, stores the second box by
 // TMA and, once that store has read the space, parks and stores the first.  Register stores of the same tile take
 // 64 KB through lanes that each write another row (about 12 bytes per cycle and SM).
-// kHalves_ (FC2): the two warps of a tensor-memory quarter have an accumulator barrier each, and MMAs come half by half (see the
-// MMA issuer).
+// kHalves_ (FC2 but for three K steps): the two warps of a tensor-memory quarter have an accumulator barrier each, and MMAs come
+// half by half (see the MMA issuer).
 template <typename OutT, bool kHalves_ = false>
 struct EpilogueStoreWide {
   static_assert(sizeof(OutT) == 2, "16-bit rows");
@@ -946,11 +946,10 @@ nvfp4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if constexpr (kHalves) {
             // The epilogue warps of a half hand it back as soon as they have read it.  The MMAs of a K step come half by half
             // (two of 128 columns take as long as one of 256), so that one half is drained while the tensor core works on the
-            // other: with three or four K steps a tile the one accumulator is what a tile waits for.  All MMAs into a half have
-            // the same shape: only MMAs of one shape into one accumulator are sure to be executed in the order of their issue.
-            // FC2 of 4096 tokens alone, one accumulator barrier and whole MMAs / halves: four K steps (32 experts, 4096, 1024,
-            // top-4) 58.4-58.9 / 56.6-56.8 us, three (128 experts, 2048, 768, top-8) 52.9-53.2 / 53.3.  (Whole MMAs in the K
-            // steps between a tile's first and last would save another 0.6 us with three and nothing with four, but mix shapes.)
+            // other: with few K steps a tile the one accumulator is what a tile waits for (figures at the launch of FC2).  All
+            // MMAs into a half have the same shape: only MMAs of one shape into one accumulator are sure to be executed in the
+            // order of their issue, so whole MMAs in the K steps between a tile's first and last (0.6 us of 53 with three) are
+            // no choice.
             const bool first = kt == kt_first, last = kt + 1 == kt_end;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {

@@ -148,7 +148,7 @@ def test_router_inside_with_as_many_slots_as_it_holds(b200):
 @pytest.mark.parametrize("inter", [128, 256, 512, 640, 1024])
 def test_down_projection_drained_by_halves(b200, inter):
     """FC2 with one to four K steps (a last one that is not full among them) on 256-wide tiles, whose MMAs are issued half by
-    half: four tiles, none with a successor on its CTA, blocks whose upper row quarters are empty."""
+    half but for three steps: four tiles, none with a successor on its CTA, blocks whose upper row quarters are empty."""
     test_topk_random_against_oracle(b200, 150, 2, 512, inter, 1, None)
 
 
